@@ -322,6 +322,50 @@ __device__ __forceinline__ bool warp_emit(const PairSink& s, WarpChunk& c, uint3
     return ok;
 }
 
+// Append, for every lane, `cnt` pairs which the lane produces one after the
+// other: body(put) calls put(key, value) exactly cnt times.  For sparse hits,
+// where most lanes have none or one or two.  One reservation at most, of whole
+// chunks.  Whole warp must call.  Returns false on overflow (pairs dropped; the
+// batch will be re-run).
+template <typename Body>
+__device__ __forceinline__ bool warp_emit_serial(const PairSink& s, WarpChunk& c, uint32_t cnt, Body&& body) {
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane_id() >= (uint32_t)o) incl += t;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if (total == 0) return true;
+    const uint32_t room = c.cap != 0 ? c.cap - c.used : 0u;
+    const unsigned long long p0 = c.base + c.used;   // the first `room` pairs
+    unsigned long long p1 = 0;                       // the rest
+    if (total > room) {
+        const uint32_t need = (total - room + kSinkChunk - 1) / kSinkChunk * kSinkChunk;
+        if (lane_id() == 0) p1 = atomicAdd(s.cursor, (unsigned long long)need);
+        p1 = __shfl_sync(0xffffffffu, p1, 0);
+        if (p1 + need > s.capacity) {
+            if (lane_id() == 0) atomicExch(s.overflow, 1u);
+            c.cap = 0;
+            c.used = 0;
+            return false;
+        }
+        c.base = p1;
+        c.used = total - room;
+        c.cap = need;
+    } else {
+        c.used += total;
+    }
+    uint32_t r = incl - cnt;
+    body([&](uint32_t key, uint32_t val) {
+        const unsigned long long pos = r < room ? p0 + r : p1 + (r - room);
+        s.keys[pos] = key;
+        s.vals[pos] = val;
+        ++r;
+    });
+    return true;
+}
+
 // Append the pairs named by every lane's 32-bit hit mask, written out in
 // coalesced runs: output slot i of the warp's hits is produced by lane i % 32,
 // which finds the hit's owner lane (binary search over the inclusive prefix of

@@ -190,19 +190,21 @@ hj_status geometry_t(const T* db, uint32_t n, uint32_t d, uint32_t k, T eps, dou
 // ---- index build -----------------------------------------------------------------------
 template <typename T>
 __global__ void k_cell_ids(const T* __restrict__ db, uint32_t n, uint32_t d, GeoT<T> geo, HjGrid grid,
-                           unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* alias) {
+                           unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* alias, uint32_t* silent) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     unsigned long long lid = 0;
-    bool al = false;
+    bool al = false, zero = false;
     for (uint32_t j = 0; j < grid.k; ++j) {
         uint32_t c = cell_coord(db[(uint64_t)i * d + j], geo.min_arr[j], geo.eps);
         al |= c >= grid.n_cells[j];
+        zero |= c == 0u;
         lid += (unsigned long long)c * grid.mult[j];
     }
     keys[i] = lid;
     vals[i] = i;
     if (al) atomicExch(alias, 1u);
+    if (zero) atomicExch(silent, 1u);
 }
 
 __global__ void k_run_flags(const unsigned long long* __restrict__ keys, uint32_t n, uint32_t* __restrict__ flags) {
@@ -295,23 +297,24 @@ __global__ void k_max_u32(const uint32_t* __restrict__ a, uint32_t n, uint32_t* 
 }
 
 __global__ void k_block_counts(const uint32_t* __restrict__ order, const uint32_t* __restrict__ cell_start, uint32_t nC,
-                               uint32_t qb, uint32_t* __restrict__ cnt) {
+                               uint32_t qb, uint32_t align, uint32_t* __restrict__ cnt) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nC) return;
     uint32_t c = order[i];
-    uint32_t pop = cell_start[c + 1] - cell_start[c];
-    cnt[i] = (pop + qb - 1) / qb;
+    uint32_t s = cell_start[c] & ~(align - 1u);
+    cnt[i] = (cell_start[c + 1] - s + qb - 1) / qb;
 }
 
 __global__ void k_make_blocks(const uint32_t* __restrict__ order, const uint32_t* __restrict__ cell_start,
                               const uint32_t* __restrict__ cell_nb, const uint32_t* __restrict__ off, uint32_t nC,
-                              uint32_t qb, HjBlock* __restrict__ blocks) {
+                              uint32_t qb, uint32_t align, HjBlock* __restrict__ blocks) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nC) return;
     uint32_t c = order[i];
     uint32_t s = cell_start[c], e = cell_start[c + 1];
     uint32_t o = off[i];
-    for (uint32_t q = s; q < e; q += qb, ++o) blocks[o] = HjBlock{c, q, min(e, q + qb), cell_nb[c]};
+    for (uint32_t q = s & ~(align - 1u); q < e; q += qb, ++o)
+        blocks[o] = HjBlock{c, max(q, s), min(e, q + qb), cell_nb[c]};
 }
 
 __global__ void k_origin_index(const uint32_t* __restrict__ order, const uint32_t* __restrict__ cell_start,
@@ -378,7 +381,8 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
     HJ_TRY(tmp.alloc(&scalars, 4));
     HJ_CUDA(cudaMemsetAsync(scalars, 0, 4 * sizeof(uint32_t), st));
     unsigned grid1 = (n + 255) / 256;
-    k_cell_ids<T><<<grid1, 256, 0, st>>>(d_db, n, d, geo, ix->grid, keys, ix->perm, scalars);
+    k_cell_ids<T><<<grid1, 256, 0, st>>>(d_db, n, d, geo, ix->grid, keys, ix->perm, scalars,
+                                          scalars + 2);
     HJ_LAUNCHED();
     uint32_t nbits = bits_for(ix->total_cells > 0 ? ix->total_cells - 1 : 0);
     HJ_TRY(radix_sort_u64_u32(reinterpret_cast<uint64_t*>(keys), ix->perm, reinterpret_cast<uint64_t*>(keys_tmp),
@@ -401,11 +405,12 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
     unsigned grid2 = (unsigned)std::min<uint64_t>(((uint64_t)n * d + 255) / 256, (uint64_t)num_sms() * 16);
     k_gather_rows<T><<<grid2, 256, 0, st>>>(d_db, ix->perm, n, d, pts);
     HJ_LAUNCHED();
-    uint32_t hs[2];
+    uint32_t hs[3];
     HJ_CUDA(cudaMemcpyAsync(hs, scalars, sizeof(hs), cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaStreamSynchronize(st));
     ix->aliasing = hs[0];
     ix->nC = hs[1];
+    ix->any_silent = hs[2];
     if (ix->aliasing) {
         set_error("grid aliasing: a point's cell coordinate reaches nCells in some indexed dimension "
                   "(epsilon below the coordinates' rounding granularity); unsupported");
@@ -512,19 +517,19 @@ void free_index(hj_index* ix, cudaStream_t st) {
     dfree(ix->cell_order, st);
     dfree(ix->tc_a, st);
     dfree(ix->tc_b, st);
-    dfree(ix->tc_err, st);
-    dfree(ix->tc_pband, st);
+    dfree(ix->perm_flag, st);
 }
 
 }  // namespace
 
-hj_status build_blocks(const hj_index* ix, uint32_t qb, HjBlock** d_blocks, uint32_t* n_blocks, cudaStream_t st) {
+hj_status build_blocks(const hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
+                       cudaStream_t st) {
     uint32_t nC = ix->nC;
     Scratch tmp(st);
     uint32_t* cnt = nullptr;
     HJ_TRY(tmp.alloc(&cnt, (size_t)nC + 1));
     unsigned g = (nC + 255) / 256;
-    k_block_counts<<<g, 256, 0, st>>>(ix->cell_order, ix->cell_start, nC, qb, cnt);
+    k_block_counts<<<g, 256, 0, st>>>(ix->cell_order, ix->cell_start, nC, qb, align, cnt);
     HJ_LAUNCHED();
     HJ_CUDA(cudaMemsetAsync(cnt + nC, 0, 4, st));
     HJ_TRY(scan_u32_inplace(cnt, (uint64_t)nC + 1, st));
@@ -533,7 +538,8 @@ hj_status build_blocks(const hj_index* ix, uint32_t qb, HjBlock** d_blocks, uint
     HJ_CUDA(cudaStreamSynchronize(st));
     HjBlock* blocks = nullptr;
     HJ_TRY(tmp.alloc_pool(&blocks, (size_t)std::max<uint32_t>(nb, 1)));   // handed to the caller
-    k_make_blocks<<<g, 256, 0, st>>>(ix->cell_order, ix->cell_start, ix->cell_nb, cnt, nC, qb, blocks);
+    k_make_blocks<<<g, 256, 0, st>>>(ix->cell_order, ix->cell_start, ix->cell_nb, cnt, nC, qb, align,
+                                      blocks);
     HJ_LAUNCHED();
     *d_blocks = tmp.keep(blocks);
     *n_blocks = nb;

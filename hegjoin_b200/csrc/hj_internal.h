@@ -58,6 +58,7 @@ struct hj_index {
     HjGrid grid = {};
     uint64_t total_cells = 0;
     uint32_t aliasing = 0;
+    uint32_t any_silent = 0;   // some cell has a coordinate of 0 and visits no cell (kernel.cu:780 wraps)
     int device = 0;
     cudaStream_t stream = nullptr;   // stream the index was built on; its memory is freed in that order
 
@@ -81,14 +82,13 @@ struct hj_index {
     uint32_t max_nb = 0;
 
     // tensor-core operands (built on first use)
-    void* tc_a = nullptr;            // n x kpad, query form
-    void* tc_b = nullptr;            // n x kpad, candidate form
-    float* tc_err = nullptr;         // per sorted point: quantisation error norm (rounded up)
-    float* tc_pband = nullptr;       // per sorted point: its part of the guard band (rounded up)
+    void* tc_a = nullptr;            // query form: K-block planes (hj_refine_tc.cu)
+    void* tc_b = nullptr;            // candidate form
+    uint32_t* perm_flag = nullptr;   // perm with bit 31 set for points of silent cells (built on first use)
     uint32_t tc_kpad = 0;
     int plain_shape = 0;             // exact refine tile shape (0 or 1; autotuned per d and dtype)
     int tc_kind = -1;                // HJ_REFINE_TC_F16 / _BF16 the operands hold
-    void* tc_state = nullptr;        // tensor maps and error maxima (hj_refine_tc.cu)
+    void* tc_state = nullptr;        // scale, threshold and error maxima (hj_refine_tc.cu)
 };
 
 namespace hj {
@@ -103,7 +103,10 @@ void init_memory_pool();
 void tc_release(hj_index* ix);
 
 // hj_index.cu
-hj_status build_blocks(const hj_index* ix, uint32_t qb, HjBlock** d_blocks, uint32_t* n_blocks,
+// Work items of up to qb queries per cell, in the workload order; `align` (a
+// power of two): a cell's items after its first start at multiples of it and
+// fill whole groups, the first begins at the cell's first point.
+hj_status build_blocks(const hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
                        cudaStream_t st);
 
 constexpr unsigned long long kEmptyLid = ~0ull;

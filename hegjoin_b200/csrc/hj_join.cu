@@ -40,22 +40,20 @@ hj_status launch_refine_plain(const hj_index* ix, const HjBlock* blocks, uint32_
                               const PairSink& sink, uint32_t count_only, unsigned long long* block_counts,
                               uint32_t* qcount, cudaStream_t st);
 hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st);
-uint32_t tc_query_block();
-hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
-                           const PairSink& sink, const PairSink& band, uint32_t count_only,
+uint32_t tc_query_block(const hj_index* ix);
+hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
+                           const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
                            unsigned long long* block_counts, unsigned long long* stats, uint32_t* err,
                            cudaStream_t st);
-hj_status launch_band_recheck(const hj_index* ix, const uint32_t* bq, const uint32_t* bc,
+hj_status launch_band_recheck(hj_index* ix, const uint32_t* bq, const uint32_t* bc,
                               const unsigned long long* band_used, unsigned long long band_cap,
-                              const PairSink& sink, uint32_t nblocks, cudaStream_t st);
+                              const PairSink& sink, uint32_t nblocks, bool sym, cudaStream_t st);
 uint64_t plain_emit_warps(uint32_t nblocks);
 uint64_t tc_emit_warps(uint32_t nblocks);
 double tc_delta(const hj_index* ix);
 double tc_band_ratio(const hj_index* ix);
 bool tc_supported(const hj_index* ix, int kind);
-int tc_get_epi(const hj_index* ix);
-void tc_set_epi(hj_index* ix, int epi);
-void tc_set_defer(hj_index* ix, bool defer);
+void tc_set_dense(hj_index* ix, bool dense);
 }  // namespace hj
 
 struct hj_result {
@@ -405,12 +403,12 @@ bool tuning_enabled() {
     return !(e && e[0] == '0');
 }
 
-// Tensor-core epilogue: with fewer than ~3% of its 32 x 32 chunks holding a hit, one vote
-// per accumulator and a re-read of the hit chunks beats a vote per chunk (measured at
-// d = 18 with 1.6% and at d = 90 with 6.4%).  HJ_TC_DEFER=0/1 forces either form (tests).
-bool defer_for(double pairs, double cand) {
-    if (const char* e = std::getenv("HJ_TC_DEFER")) return e[0] == '1';
-    return cand > 0 && pairs * 1024.0 < 0.03 * cand;
+// Tensor-core epilogue: with fewer than ~3% of its 32 x 32 chunks holding a hit, ORing the
+// signs and reading the hit chunks again beats building every chunk's mask.
+// HJ_TC_DEFER=0/1 forces masks or ORs (tests).
+bool dense_for(double pairs, double cand) {
+    if (const char* e = std::getenv("HJ_TC_DEFER")) return e[0] != '1';
+    return !(cand > 0 && pairs * 1024.0 < 0.03 * cand);
 }
 
 float ms_since(std::chrono::steady_clock::time_point t0) {
@@ -617,11 +615,11 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     }
     S.refine_used = (uint32_t)refine;
     // the tile shape of each refine kernel fixes its work-item size
-    const uint32_t qb = tc ? tc_query_block() : plain_query_block(ix->dtype);
+    const uint32_t qb = tc ? tc_query_block(ix) : plain_query_block(ix->dtype);
 
     HjBlock* blocks = nullptr;
     uint32_t nblocks = 0;
-    HJ_TRY(build_blocks(ix, qb, &blocks, &nblocks, st));
+    HJ_TRY(build_blocks(ix, qb, tc ? 8u : 1u, &blocks, &nblocks, st));
     tmp.adopt(blocks);
     if (!tc && nblocks >= kLightMinItems) {
         // the light items' tail in cell order (kLightCandidates)
@@ -699,7 +697,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     // head_reset: zero the work-item queue head first (batches reset it with the rest)
     auto run_refine = [&](const HjBlock* blk, uint32_t nb, const PairSink& sink, const PairSink& band,
                           uint32_t count_only, unsigned long long* bc, bool head_reset = true,
-                          uint32_t* qcount = nullptr) -> hj_status {
+                          uint32_t* qcount = nullptr, bool sym = false) -> hj_status {
         if (head_reset) HJ_CUDA(cudaMemsetAsync(head, 0, sizeof(unsigned int), st));
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (!count_only) {
@@ -710,7 +708,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             e1 = kev.ev.back().second;
             HJ_CUDA(cudaEventRecord(e0, st));
         }
-        HJ_TRY(tc ? launch_refine_tc(ix, blk, nb, head, sink, band, count_only, bc,
+        HJ_TRY(tc ? launch_refine_tc(ix, blk, nb, head, sink, band, count_only, sym, bc,
                                      count_only ? nullptr : &ctl->tc_acc, &ctl->timeout, st)
                   : launch_refine_plain(ix, blk, nb, head, sink, count_only, bc, qcount, st));
         if (!count_only) HJ_CUDA(cudaEventRecord(e1, st));
@@ -757,48 +755,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         PairSink none{nullptr, nullptr, nullptr, 0, overflow};
         int tuned = 0;
         const std::string key = tune_key(refine, ix->d, ix->dtype);
-        if (tc && !tune_lookup(key, &tuned) && tuning_enabled()) {
-            // the vote form follows the hit density: measure it on the sample first, so the
-            // shapes are timed in the form the refine will use
-            HJ_TRY(run_refine(sblocks, nsamp, none, no_band, 1, scnt));
-            HJ_TRY(check_timeout());
-            {
-                std::vector<unsigned long long> h0(nsamp);
-                std::vector<HjBlock> hs0(nsamp);
-                HJ_CUDA(cudaMemcpyAsync(h0.data(), scnt, nsamp * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                        st));
-                HJ_CUDA(cudaMemcpyAsync(hs0.data(), sblocks, nsamp * sizeof(HjBlock), cudaMemcpyDeviceToHost, st));
-                HJ_CUDA(cudaStreamSynchronize(st));
-                double sp = 0, sc = 0;
-                for (uint32_t q = 0; q < nsamp; ++q) {
-                    sp += (double)h0[q];
-                    sc += (double)hs0[q].nb * (hs0[q].q1 - hs0[q].q0);
-                }
-                tc_set_defer(ix, defer_for(sp, sc));
-            }
-            // time each epilogue shape on the sample; the last run's counts are the estimate.
-            // Shapes: warp groups | 8 * (one warp set per accumulator)
-            const int cands[4] = {2, 4, 10, 12};
-            float best = 1e30f;
-            int best_epi = tc_get_epi(ix);
-            EventPairs tev;
-            tev.ev.emplace_back(nullptr, nullptr);
-            HJ_TRY(event_acquire(&tev.ev[0].first));
-            HJ_TRY(event_acquire(&tev.ev[0].second));
-            for (int c : cands) {
-                tc_set_epi(ix, c);
-                HJ_CUDA(cudaMemsetAsync(scnt, 0, nsamp * sizeof(unsigned long long), st));
-                HJ_CUDA(cudaEventRecord(tev.ev[0].first, st));
-                HJ_TRY(run_refine(sblocks, nsamp, none, no_band, 1, scnt));
-                HJ_CUDA(cudaEventRecord(tev.ev[0].second, st));
-                HJ_TRY(check_timeout());
-                float ms = 0;
-                HJ_CUDA(cudaEventElapsedTime(&ms, tev.ev[0].first, tev.ev[0].second));
-                if (ms < best) { best = ms; best_epi = c; }
-            }
-            tc_set_epi(ix, best_epi);
-            tune_store(key, best_epi);
-        } else if (!tc && nsamp >= 16 && !tune_lookup(key, &tuned) && tuning_enabled()) {
+        if (!tc && nsamp >= 16 && !tune_lookup(key, &tuned) && tuning_enabled()) {
             // the exact refine's two tile shapes, timed on the sample (each run twice, the
             // faster run kept: the first run of a shape also pays its one-time setup); the
             // last run's counts are the estimate, and they are the same for either shape
@@ -824,7 +781,6 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             ix->plain_shape = best_shape;   // the exact counts of the last run do not depend on the shape
             tune_store(key, best_shape);
         } else {
-            if (tc && tuned) tc_set_epi(ix, tuned);
             if (!tc) ix->plain_shape = tuned;
             HJ_TRY(run_refine(sblocks, nsamp, none, no_band, 1, scnt));
             HJ_TRY(check_timeout());
@@ -847,7 +803,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     }
     S.estimated_pairs = (uint64_t)total_est;
     S.ms_estimate = ms_since(t_est);
-    if (tc) tc_set_defer(ix, defer_for(total_est, cand_total));
+    if (tc) tc_set_dense(ix, dense_for(total_est, cand_total));
 
     // ---- result buffer capacity
     // slack for partly filled warp chunks: every warp that can emit during a batch holds
@@ -972,8 +928,12 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         PairSink sink{keys, vals, &ctl->cursor, cap, overflow};
         PairSink band = tc ? PairSink{band_q, band_c, &ctl->band_cursor, cap, overflow} : no_band;
         if (fused_counts) HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
-        HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, fused_counts ? qoff : nullptr));
-        if (tc) HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, st));
+        // all items of the join in this one batch: every unordered pair once (a query's pairs
+        // must lie in one batch, and a shard owns its queries' pairs only)
+        const bool sym = tc && opts.shard_count <= 1 && b.b0 == 0 && b.b1 == nblocks;
+        HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, fused_counts ? qoff : nullptr,
+                          sym));
+        if (tc) HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, st));
         JoinCtl hc;
         HJ_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));

@@ -5,46 +5,52 @@
 // loop is a dense distance evaluation; here each (candidate tile x query block)
 // is a GEMM on the 5th-generation tensor cores:
 //
-//   A (M = 128 candidates, streamed by TMA) = [-2 c~, 1, 1, |c~|^2_hi, |c~|^2_lo, 0...]
-//   B (N = 2 x 256 queries, resident)       = [  q~, |q~|^2_hi, |q~|^2_lo, 1, 1, 0...]
-//   D = A B^T = |q~|^2 + |c~|^2 - 2 q~.c~ = |q~ - c~|^2        (FP32 accumulate in TMEM)
+//   A (M = 128 candidates, streamed by TMA) = [-2 c~, 1, 1, N_c hi, N_c lo, 0...]
+//   B (N = 256 queries, resident)           = [  q~, N_q hi, N_q lo, 1, 1, 0...]
+//   D' = A B^T = N_q + N_c - 2 q~.c~        (FP32 accumulate in TMEM)
 //
-// where x~ is the FP16 (or BF16) rounding of (x - origin) * 2^s.  The origin
-// is the per-dimension minimum and s is a power-of-two scale chosen per
-// dataset so that the largest |x - origin|^2 * 4^s lies in [2^12, 2^14]: every
-// stored half (coordinates up to 128, -2x up to 256, norm halves up to 2^14)
-// is finite with a 4x margin below FP16's 65504 whatever the data's units, and
-// small-valued data stays clear of the FP16 subnormals.  Scaling by 2^s is
-// exact, so the threshold becomes T * 4^s exactly.  The norms ride in the K
-// padding (d + 4 rounded up to 32), so the MMA yields the (scaled) squared
-// distance directly and the epilogue is one compare per pair.  A pair is
-//   accepted  if D <= T - delta,
-//   rejected  if D >  T + delta,
-//   rechecked otherwise, in FP32 in the reference's order (fma chain),
-// with T the exact squared threshold and delta a per-candidate-row bound on
-// |D - d2_ref| (quantisation error, norm-split residual, tensor-core
-// accumulation error and the reference's own FP32 rounding; derivation in
-// tc_band_p / tc_band_q below).  A D that is NaN counts as "in the band", never as a
-// reject.  The result set is therefore identical to the exact path.
+// where x~ is the FP16 (or BF16) rounding of (x - origin) * 2^s and the norm
+// terms carry the threshold: N_c = |c~|^2 - P(c), N_q = |q~|^2 - T - Q(q), with T
+// the exact squared threshold and P + Q the pair's guard band (quantisation,
+// tensor-core accumulation and the reference's own FP32 rounding; derivation at
+// tc_band_p below).  So D' = |q~ - c~|^2 - (T + P + Q), and the sign of the MMA
+// output is the filter's decision.  The origin is the per-dimension minimum and s
+// is a power-of-two scale chosen per dataset so that the largest
+// |x - origin|^2 * 4^s lies in [2^12, 2^14]: every stored half (coordinates up
+// to 128, -2x up to 256, norm terms in [-60000, 2^14]) is finite whatever the
+// data's units, and small-valued data stays clear of the FP16 subnormals.
+// Scaling by 2^s is exact, so the threshold becomes T * 4^s exactly.  A pair is
+//   rejected  if D' > 0 (the sign bit is clear),
+//   accepted  if D' <= lo, below the band's lower edge for every pair,
+//   rechecked otherwise, in FP32 in the reference's order (fma chain).
+// The result set is therefore identical to the exact path.
 //
-// Kernel shape (one CTA per SM, persistent, 96 + 128 * EPI threads):
-//   warp 0      TMA producer: the work item's 256 queries once, candidate tiles
-//               through a ring of shared-memory stages;
-//   warps 1, 2  MMA issuers: candidate tile t is computed as M = 128 x N = 256
-//               MMAs into TMEM accumulator t % 2 (2 x 256 columns, all of TMEM)
-//               by issuer 1 + t % 2.  The accumulators form a ring over the
-//               tiles, so the MMAs of tile t + 1 run while the epilogue drains
-//               tile t.  N = 256 matters: a microbenchmark of this pattern
-//               issued 128 x 128 x 16 MMAs at 42% of the tensor pipe's rate and
-//               128 x 256 x 16 ones at 98%;
-//   warps 3..   epilogue, EPI groups of 4 warps (one per TMEM lane quarter),
-//               either all draining every tile or split into one set per
-//               accumulator (every other tile; autotuned): tcgen05.ld,
-//               min-reduce, compare, warp-aggregated emission; an accumulator
-//               is released as soon as its warps have read it.
-// Every wait is bounded; a timeout raises an error flag, drains and returns.
+// Kernel shape (one CTA per SM, persistent, 19 warps):
+//   warp 0      loads: the work item's up to 512 query columns once, candidate
+//               tiles through a ring of shared-memory stages, by bulk copies;
+//   warps 1, 2  MMA issuers, one per TMEM accumulator (2 x 256 columns, all of
+//               TMEM): M = 128 x N = 256 MMAs.  N = 256 matters: a microbenchmark
+//               of this pattern issued 128 x 128 x 16 MMAs at 42% of the tensor
+//               pipe's rate and 128 x 256 x 16 ones at 98%;
+//   warps 3..18 epilogue, a set of 8 per accumulator: tcgen05.ld, signs ORed or
+//               gathered into masks, accumulator released, hits emitted.
+//
+// What bounds it, at d = 18 (two K steps per tile; 400,000 points, 12,500
+// accumulator uses per SM): the hand-over chain of an accumulator, ~1,700 cycles
+// for a use (issue ~200, MMAs 273, wake ~100, four TMEM reads with their ORs ~600,
+// release ~100, and the hits' emission, which holds back its own set), two
+// accumulators overlapping.  The floor of each part is 273 cycles per use on the
+// tensor pipe and 256 on the ALU (one OR per value at 128 per cycle).  Measured
+// there: 15.9 ms before the sign test, symmetric form and whole-warp waits, 6.4 ms
+// now; at 90-D and 150,000 points 6.7 -> 2.5 ms; at 18-D and 100,000 points, where
+// half of the 32 x 32 chunks hold a hit, 4.7 -> 1.2 ms.  Tried and not kept: one
+// set of 16 warps on every use (a warp that emits holds back both accumulators:
+// 8.6 ms), 64-column reads (spills: 9.8 ms), named barriers instead of mbarriers
+// for the release (6.5 ms), three accumulators of 160 columns.
+// Every wait is bounded; a timeout raises an error flag that ends every later wait
+// at once, and the roles walk their loops to the end (on garbage that the host
+// discards, within the item's ranges), leave time for copies in flight and return.
 
-#include <cudaTypedefs.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 
@@ -58,48 +64,56 @@
 namespace hj {
 namespace {
 
-constexpr int kQT = 2;                       // 128-row query loads per work item
-constexpr int kTileRows = 128;               // rows per tile (M for A) and per query load
-constexpr int kQB = kQT * kTileRows;         // queries per work item (N of every MMA)
-constexpr int kAcc = 2;                      // TMEM accumulators: a ring over the candidate tiles
-constexpr int kAccCols = 256;                // N of one MMA: the work item's queries
-constexpr int kProbeThreads = 192;   // tile probe: TMA warp, MMA warp, 4 epilogue warps
-constexpr int kProbeQT = 4;                  // the tile probe evaluates 512 query rows ...
-constexpr int kProbeQB = kProbeQT * kTileRows;
+constexpr int kTileRows = 128;               // candidate rows per tile (M of every MMA)
+constexpr int kAcc = 2;                      // TMEM accumulators
+constexpr int kAccCols = 256;                // N of one MMA: columns of one accumulator
+constexpr int kQBMax = 2 * kAccCols;         // query columns per work item at most
+constexpr int kProbeThreads = 192;   // tile probe: load warp, MMA warp, 4 epilogue warps
+constexpr int kProbeQB = 512;                // the tile probe evaluates 512 query rows
 constexpr int kMaxStages = 8;
-constexpr uint32_t kKBlockBytes = kTileRows * 64;   // one 32-element K block of a 128-row tile
-constexpr uint32_t kBKBlockBytes = kQB * 64;        // one 32-element K block of the whole query block
-constexpr uint32_t kProbeBKBlockBytes = kProbeQB * 64;
+constexpr uint32_t kRowBytes = 64;           // one row of one K block: 32 halves
+constexpr uint32_t kKBlockBytes = kTileRows * kRowBytes;   // one K block of a candidate tile
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kMaxRanges = 256;
+constexpr int kEpiWarps = 16;                // 8 per accumulator: 4 TMEM lane quarters x 2 column halves
+constexpr int kThreads = 32 * (1 + kAcc + kEpiWarps);
 constexpr long long kWaitCycles = 4000000000ll;     // ~2 s at 1.9 GHz
+
+// Operand forms in memory: K-block planes [kb][row][64 bytes], a row's four
+// 16-byte chunks permuted the way the 64-byte swizzle of shared memory wants
+// them (chunk ^ (row / 2) % 4, a pattern of 8 rows).  128 rows of a plane from a
+// multiple of 8 are then the shared-memory image of one K block, fetched by one
+// contiguous bulk copy of 8 KB.  (A tensor-map load with a box of 64-byte rows
+// delivered ~8 bytes per cycle and SM whatever d, and the refine ran at its pace.)
+// Planes are padded by kRowPad zero rows: a tile may start at the last points.
+constexpr uint32_t kRowPad = 512 + 8;
+__host__ __device__ __forceinline__ uint64_t plane_rows(uint32_t n) { return ((uint64_t)n + 7u) / 8u * 8u + kRowPad; }
 
 struct TcArgs {
     const HjBlock* blocks;
     uint32_t nblocks;
+    uint32_t parts;             // work items per block: each takes 1/parts of the block's candidate tiles
     unsigned int* head;
-    const uint32_t* perm;
+    const uint32_t* perm;       // sorted position -> original id, bit 31 set for points of silent cells
     const unsigned long long* cell_lid;
     const uint32_t* cell_start;
-    uint32_t nC;
     HjCellHash hash;
     HjGrid grid;
-    const float4* pinfo;        // per sorted point: quantisation error norm, |x~|^2, norm-split residual
-    const float* pband;         // per sorted point: its part of the guard band (tc_band_p)
-    uint32_t n;
+    const uint8_t* qform;       // operand planes
+    const uint8_t* cform;
+    unsigned long long plane;   // bytes of one plane
     uint32_t nkb;               // K blocks of 32 elements
+    uint32_t qcols;             // query columns per work item: 512, or 256 where shared memory is short
     uint32_t stages;
-    float thr;
-    float gamma_acc;
-    float s_t;                  // sqrt(T (1 + 1e-4))
-    float ref_rel;              // (d + 2) 2^-24 (1.01)
+    float lo;                   // accepted outright: D' <= lo (negative)
+    uint32_t sym;               // every unordered pair once: see the symmetric form below
     PairSink sink;              // accepted pairs: (query id, candidate id)
     PairSink band;              // band pairs: (query sorted position, candidate sorted position)
     uint32_t count_only;
     unsigned long long* block_counts;
     unsigned long long* stats;  // [0] accepted, [1] band
     uint32_t* err;
-    uint32_t idesc;
+    uint32_t fmt;               // operand format of the instruction descriptor (0 FP16, 1 BF16)
     long long wait_cycles;      // bound of every mbarrier wait (SM cycles)
 };
 
@@ -112,14 +126,18 @@ struct TcShared {
     uint32_t tmem_base;
     uint32_t item;
     uint32_t abort;
-    uint32_t nq, ntiles, nr, q0;
-    uint32_t max_e, max_n, max_r;          // float bits (non-negative)
-    uint32_t qid[kQB];
+    uint32_t ntiles, nr;
+    uint32_t qid[kQBMax];                  // original ids of the query columns
     uint32_t rs[kMaxRanges];               // range start (sorted position)
     uint32_t rl[kMaxRanges];               // range length
     uint32_t tp[kMaxRanges + 1];           // tile prefix
 };
 
+// Tiles start at multiples of 8 rows (the swizzle pattern), so a range's first
+// tile may begin with up to 7 rows of other points, which the epilogue masks.
+__device__ __forceinline__ uint32_t range_tiles(uint32_t start, uint32_t len) {
+    return len ? ((start & 7u) + len + kTileRows - 1) / kTileRows : 0u;
+}
 
 // Tiles are visited in order, so the range of tile t is found by walking r
 // forward from the previous tile's range (the last r with tp[r] <= t; ranges
@@ -127,8 +145,8 @@ struct TcShared {
 // current range's first tile, end tile, start row and length stay in registers,
 // so a tile inside the same range costs no shared-memory reads.
 struct TileWalk {
-    uint32_t r = 0, start = 0, valid = 0;
-    uint32_t t0 = 0, t1 = 0, rs = 0, rl = 0;   // range r: tiles [t0, t1), rows [rs, rs + rl)
+    uint32_t start = 0, first = 0, end = 0;    // the tile's rows start + [0, 128); [first, end) are the range's
+    uint32_t r = 0, t0 = 0, t1 = 0, rs = 0, rl = 0;   // range r: tiles [t0, t1), rows [rs, rs + rl)
     __device__ __forceinline__ void locate(const TcShared& S, uint32_t t) {
         if (t >= t1) {
             while (r + 1 < S.nr && S.tp[r + 1] <= t) ++r;
@@ -137,103 +155,108 @@ struct TileWalk {
             rs = S.rs[r];
             rl = S.rl[r];
         }
-        const uint32_t off = (t - t0) * kTileRows;
-        start = rs + off;
-        valid = min((uint32_t)kTileRows, rl - off);
+        const uint32_t off = (t - t0) * kTileRows, skip = rs & 7u;
+        start = (rs & ~7u) + off;
+        first = off ? 0u : skip;
+        end = min((uint32_t)kTileRows, skip + rl - off);
     }
 };
 
-// The guard band of a candidate row c against the whole query block:
-//   |D - d2_ref| <= acc + res + e (2 sT + 3 e) + ref_rel (sT + e)^2
-//   e   = e_c + max e_q       (|x~ - x| norms; |(|q~-c~|) - |q-c|| <= e)
-//   acc = gamma (2.01 (|c~|^2 + max |q~|^2))   (tensor-core accumulation; 2|a.b| <= |a|^2 + |b|^2)
-//   res = r_c + max r_q       (norm split residuals)
+// The guard band of a pair (q, c): the tensor-core value D of |q~ - c~|^2 differs
+// from the reference's FP32 d2 (near the threshold T) by at most
+//   acc + e (2 sT + 3 e) + ref_rel (sT + e)^2
+//   e   = e_c + e_q           (|x~ - x| norms; |(|q~-c~|) - |q-c|| <= e)
+//   acc = gamma (2.01 (|c~|^2 + |q~|^2) + 1.01 T)  (tensor-core accumulation; 2|a.b| <= |a|^2 + |b|^2;
+//                              T for the shift in the norm terms, below)
 //   the last term bounds the reference's own FP32 rounding of d2 (d + 2 roundings).
-// With (e_c + m)^2 <= 2 e_c^2 + 2 m^2 it splits into a candidate part and a
-// query-block part, delta <= P(c) + Q(block):
-//   P(c) = gamma 2.01 |c~|^2 + r_c + e_c (2 sT + 6 e_c) + ref_rel (2 sT e_c + 2 e_c^2)
-//   Q    = gamma 2.01 max|q~|^2 + max r_q + m (2 sT + 6 m) + ref_rel (sT^2 + 2 sT m + 2 m^2),  m = max e_q
-// each with a 1% margin for its own FP32 evaluation.  P is computed once per
-// point (k_tc_pband, rounded up), Q once per work item, and a row's band edges
-// are two additions rounded outwards: hi = (thr + Q) + P, lo = (thr - Q) - P.
-__host__ __device__ __forceinline__ double tc_band_p(double gamma, double s_t, double ref_rel, double e, double n2,
-                                                     double r) {
-    return (gamma * 2.01 * n2 + r + e * (2.0 * s_t + 6.0 * e) + ref_rel * (2.0 * s_t * e + 2.0 * e * e)) * 1.01;
+// With (e_c + m)^2 <= 2 e_c^2 + 2 m^2 (m = e_q) it splits into a candidate part and a
+// query part, delta <= P(c) + Q(q):
+//   P(c) = gamma 2.01 |c~|^2 + e_c (2 sT + 6 e_c) + ref_rel (2 sT e_c + 2 e_c^2)
+//   Q(q) = gamma (2.01 |q~|^2 + 1.01 T) + m (2 sT + 6 m) + ref_rel (sT^2 + 2 sT m + 2 m^2)
+// each with a 2% margin (gamma (P + Q) of the shift itself, and rounding).
+//
+// The band's upper edge T + P(c) + Q(q) rides in the norm terms of the operands,
+//   N_c = |c~|^2 - P(c),   N_q = |q~|^2 - T - Q(q),
+// each stored as two halves that are never above it, so the MMA gives
+//   D' = |q~ - c~|^2 - (T + P + Q) - (split residuals >= 0):
+// a pair is rejected iff D' > 0 -- its sign bit is clear -- and accepted outright
+// if D' <= -(2 P + 2 Q + residuals).  The sign test is what the epilogue is made
+// of: no threshold per row or column, and three-input ORs cover two values per
+// instruction where a minimum covers one.
+__host__ __device__ __forceinline__ double tc_band_p(double gamma, double s_t, double ref_rel, double e, double n2) {
+    return (gamma * 2.01 * n2 + e * (2.0 * s_t + 6.0 * e) + ref_rel * (2.0 * s_t * e + 2.0 * e * e)) * 1.02;
 }
-__host__ __device__ __forceinline__ double tc_band_q(double gamma, double s_t, double ref_rel, double me, double mn,
-                                                     double mr) {
-    return (gamma * 2.01 * mn + mr + me * (2.0 * s_t + 6.0 * me) +
-            ref_rel * (s_t * s_t + 2.0 * s_t * me + 2.0 * me * me)) * 1.01 + 1e-30;
+__host__ __device__ __forceinline__ double tc_band_q(double gamma, double s_t, double ref_rel, double e, double n2) {
+    return (gamma * (2.01 * n2 + 1.01 * s_t * s_t) + e * (2.0 * s_t + 6.0 * e) +
+            ref_rel * (s_t * s_t + 2.0 * s_t * e + 2.0 * e * e)) * 1.02 + 1e-30;
 }
 
-// Tree minimum of N values with three-input minima.  The .NaN forms return NaN
-// when any input is NaN, so a NaN accumulator reaches the band test below
-// (where "not above the upper edge" counts it as a hit) instead of being
-// dropped by the minimum.
-__device__ __forceinline__ float fmin3(float a, float b, float c) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ float fmin2(float a, float b) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-// A value is a candidate hit unless it is known to lie above the band: NaN is
-// kept (and, failing `v <= lo`, goes to the exact recheck).
-__device__ __forceinline__ bool not_above(float v, float hi) { return !(v > hi); }
-template <uint32_t N>
-__device__ __forceinline__ float minN(const float (&v)[N]) {
-    if constexpr (N == 1) {
-        return v[0];
-    } else if constexpr (N == 2) {
-        return fmin2(v[0], v[1]);
-    } else {
-        constexpr uint32_t M = (N + 2) / 3;
-        float m[M];
+// OR of 32 words in eight independent chains (two-input ORs run at twice the rate
+// of three-input ones, so the value rate is the same).
+__device__ __forceinline__ uint32_t or_all(const uint32_t (&v)[32]) {
+    uint32_t m[8];
 #pragma unroll
-        for (uint32_t i = 0; i < N / 3; ++i) m[i] = fmin3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
-        if constexpr (N % 3 == 1) m[M - 1] = v[N - 1];
-        if constexpr (N % 3 == 2) m[M - 1] = fmin2(v[N - 2], v[N - 1]);
-        return minN<M>(m);
-    }
+    for (int i = 0; i < 8; ++i) m[i] = (v[i] | v[i + 8]) | (v[i + 16] | v[i + 24]);
+    return ((m[0] | m[1]) | (m[2] | m[3])) | ((m[4] | m[5]) | (m[6] | m[7]));
 }
+// Bit i = sign of v[i].
+__device__ __forceinline__ uint32_t sign_mask(const uint32_t (&v)[32]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 31; i >= 0; --i) m = __funnelshift_l(v[i], m, 1);
+    return m;
+}
+// Bit i = (v[i] < lo), lo negative.
+__device__ __forceinline__ uint32_t below_mask(const uint32_t (&v)[32], float lo) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 31; i >= 0; --i) m = __funnelshift_l(__float_as_uint(__uint_as_float(v[i]) - lo), m, 1);
+    return m;
+}
+__device__ __forceinline__ uint32_t low_bits(uint32_t n) { return n >= 32u ? 0xFFFFFFFFu : (1u << n) - 1u; }
 
-// EPI = epilogue warp groups (4 warps each, one per TMEM lane quarter).  SPLIT:
-// the epilogue warps form one set per accumulator, so a warp drains every other
-// tile (with two tiles' MMA time for it) instead of every tile.  Which is faster
-// depends on d: the autotuner times all four shapes.  DEFER: one vote per
-// accumulator instead of one per chunk, chunks with a hit read again before the
-// release; it pays where hits are rare (picked from the estimated pair density).
-template <int EPI, bool SPLIT, bool DEFER>
-__global__ void __launch_bounds__(32 * (1 + kAcc) + 128 * EPI, 1)
-    k_refine_tc(const __grid_constant__ CUtensorMap tm_cand, const __grid_constant__ CUtensorMap tm_query, TcArgs a) {
-    static_assert(EPI == 2 || EPI == 4, "an epilogue set needs whole groups of 4 warps");
+// DENSE: every chunk's signs go into a mask at once (one instruction per value);
+// otherwise they are only ORed (half an instruction per value) and the chunks
+// with a hit are read again before the accumulator is released.
+//
+// Symmetric form (a.sym): d2 is the same number for (q, c) and (c, q), so a join
+// that runs all its work items in one batch evaluates each unordered pair once
+// and emits both orders.  An item then takes only the cells after its own in
+// linear-id order (the stencil is symmetric) and, of its own cell, the points from
+// its first query on; candidates before the query are masked.  Cells with a
+// coordinate of 0 visit no cell in the reference's stencil (kernel.cu:780 wraps)
+// although their neighbours visit them: an item of such a "silent" cell emits
+// only (candidate, query) orders, and a silent candidate (bit 31 of perm) only
+// (query, candidate).
+//
+// Work of one item.  With more than 256 query columns every tile is multiplied
+// with both halves of the columns, half h by issuer h into accumulator h; an item
+// of up to 256 columns alternates its tiles between the accumulators.
+template <bool DENSE>
+__global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
     extern __shared__ uint8_t smem_raw[];
     // operand tiles need 1024-byte alignment for the swizzle pattern
     uint32_t base = tc::smem_u32(smem_raw);
     uint8_t* smem = smem_raw + ((1024u - (base & 1023u)) & 1023u);
     const uint32_t tile_bytes = a.nkb * kKBlockBytes;
-    uint8_t* b_tiles = smem;                                   // query block: [K block][256 rows]
-    uint8_t* a_tiles = smem + kQT * tile_bytes;                // a.stages tiles: [K block][128 rows]
+    const uint32_t bkb_bytes = a.qcols * kRowBytes;            // one K block of the query columns
+    uint8_t* b_tiles = smem;                                   // queries: [K block][qcols rows]
+    uint8_t* a_tiles = smem + a.nkb * bkb_bytes;               // a.stages tiles: [K block][128 rows]
     TcShared& S = *reinterpret_cast<TcShared*>(a_tiles + a.stages * tile_bytes);
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (tid == 0) {
         for (uint32_t s = 0; s < a.stages; ++s) {
             tc::mbar_init(&S.full_a[s], 1);
-            tc::mbar_init(&S.empty_a[s], 1);   // released by the one issuer of the tile it holds
+            tc::mbar_init(&S.empty_a[s], 2);   // two commits: one by each issuer, or both by the tile's
         }
         for (int j = 0; j < kAcc; ++j) {
             tc::mbar_init(&S.full_acc[j], 1);
-            tc::mbar_init(&S.empty_acc[j], SPLIT ? 2 * EPI : 4 * EPI);   // the warps draining it
+            tc::mbar_init(&S.empty_acc[j], kEpiWarps / kAcc);   // the warps draining it
         }
         tc::mbar_init(&S.bfull, 1);
         S.abort = 0;
         tc::fence_mbar_init();
-        tc::tma_prefetch_desc(&tm_cand);
-        tc::tma_prefetch_desc(&tm_query);
     }
     if (warp == 1) {
         tc::tmem_alloc(&S.tmem_base, kTmemCols);
@@ -246,8 +269,8 @@ __global__ void __launch_bounds__(32 * (1 + kAcc) + 128 * EPI, 1)
     volatile uint32_t* abort = &S.abort;
 
     // role state carried across work items (barrier phases)
-    uint32_t it = 0;            // candidate tiles issued / consumed
-    uint32_t acc_use[kAcc] = {0, 0};   // uses of each accumulator seen by this thread
+    uint32_t stage = 0, use_a = 0;   // the next tile's stage and how often it has been filled before
+    uint32_t uses = 0;          // uses of its accumulator issued / drained
     uint32_t items_loaded = 0;
     WarpChunk wc_acc, wc_band;
     warp_chunk_init(wc_acc);
@@ -255,336 +278,287 @@ __global__ void __launch_bounds__(32 * (1 + kAcc) + 128 * EPI, 1)
 
     for (;;) {
         __syncthreads();
-        if (tid == 0) {
-            S.item = *abort ? 0xFFFFFFFFu : atomicAdd(a.head, 1u);
-            S.max_e = S.max_n = S.max_r = 0u;
-        }
+        if (tid == 0) S.item = *abort ? 0xFFFFFFFFu : atomicAdd(a.head, 1u);
         __syncthreads();
         const uint32_t item = S.item;
-        if (item >= a.nblocks) break;
-        const HjBlock blk = a.blocks[item];
-        const uint32_t nq = blk.q1 - blk.q0;
-        // query ids and block maxima of the error terms
+        const uint32_t bi = item / a.parts;
+        if (item == 0xFFFFFFFFu || bi >= a.nblocks) break;
+        const HjBlock blk = a.blocks[bi];
+        // query columns: positions qbase + [0, ncols), of which the first q0 - qbase are not the item's
+        const uint32_t q0 = blk.q0, qbase = q0 & ~7u, ncols = blk.q1 - qbase;
+        const bool both = ncols > (uint32_t)kAccCols;
+        bool q_silent = false;
         {
-            float me = 0.f, mn = 0.f, mr = 0.f;
-            for (uint32_t i = tid; i < (uint32_t)kQB; i += blockDim.x) {
-                S.qid[i] = i < nq ? a.perm[blk.q0 + i] : 0u;
-                if (i < nq) {
-                    float4 p = a.pinfo[blk.q0 + i];
-                    me = fmaxf(me, p.x); mn = fmaxf(mn, p.y); mr = fmaxf(mr, p.z);
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                me = fmaxf(me, __shfl_xor_sync(0xffffffffu, me, o));
-                mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-                mr = fmaxf(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-            }
-            if (lane == 0) {
-                atomicMax(&S.max_e, __float_as_uint(me));
-                atomicMax(&S.max_n, __float_as_uint(mn));
-                atomicMax(&S.max_r, __float_as_uint(mr));
-            }
-        }
-        if (warp == 0) {
-            // stencil rows of the block's cell -> candidate ranges -> 128-row tiles
+            // stencil rows of the block's cell -> candidate ranges, a row per thread
             const unsigned long long L = a.cell_lid[blk.cell];
             const uint32_t k = a.grid.k;
             uint32_t lo[kMaxK], w[kMaxK];
             uint32_t rows = 1;
-            bool empty = false;
             const uint32_t cl = lane_cell_coord(a.grid, L);
             for (uint32_t j = 0; j < k; ++j) {
                 const uint32_t c = __shfl_sync(0xffffffffu, cl, j);
-                uint32_t l = c - 1u;                                // kernel.cu:780, wraps at 0
-                uint32_t h = min(a.grid.n_cells[j] - 1u, c + 1u);   // kernel.cu:781
-                empty |= l > h;
-                lo[j] = l;
-                w[j] = h - l + 1u;
+                const uint32_t h = min(a.grid.n_cells[j] - 1u, c + 1u);   // kernel.cu:781
+                q_silent |= c == 0u;                                      // kernel.cu:780 wraps at 0
+                lo[j] = c == 0u ? 0u : c - 1u;
+                w[j] = h - lo[j] + 1u;
                 if (j > 0) rows *= w[j];
             }
-            if (empty) rows = 0;
+            if (q_silent && !a.sym) rows = 0;
             const StencilRows sr = stencil_rows(a.grid, lo, rows);
-            uint32_t tiles_mine[kMaxRanges / 32];
-            uint32_t my_tiles = 0;
-#pragma unroll
-            for (uint32_t s = 0; s < kMaxRanges / 32; ++s) {
-                uint32_t r = lane * (kMaxRanges / 32) + s;
-                uint32_t len = 0, st = 0;
-                if (r < rows) {
-                    const uint2 sp = cell_span(a.hash, a.cell_start, stencil_row_id(a.grid, sr, lo, w, r), w[0]);
-                    st = sp.x;
-                    len = sp.y - sp.x;
-                    S.rs[r] = st;
-                    S.rl[r] = len;
+            for (uint32_t r = tid; r < rows; r += blockDim.x) {
+                unsigned long long id = stencil_row_id(a.grid, sr, lo, w, r);
+                uint32_t wid = w[0];
+                bool own = false;
+                if (a.sym) {
+                    // rows before the cell's own are skipped; its own row starts at the cell itself
+                    own = id <= L && L < id + wid;
+                    if (own) {
+                        wid -= (uint32_t)(L - id);
+                        id = L;
+                    } else if (id < L) {
+                        wid = 0;
+                    }
                 }
-                tiles_mine[s] = (len + kTileRows - 1) / kTileRows;
-                my_tiles += tiles_mine[s];
+                uint2 sp = make_uint2(0u, 0u);
+                if (wid) sp = cell_span(a.hash, a.cell_start, id, wid);
+                if (own) sp.x = q0;
+                S.rs[r] = sp.x;
+                S.rl[r] = sp.y - sp.x;
             }
-            uint32_t incl = my_tiles;
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= (uint32_t)o) incl += t;
-            }
-            uint32_t run = incl - my_tiles;
-            const uint32_t nr = min(rows, kMaxRanges);
+            for (uint32_t i = tid; i < ncols; i += blockDim.x) S.qid[i] = a.perm[qbase + i] & 0x7FFFFFFFu;
+            __syncthreads();
+            if (warp == 0) {
+                // tiles of 128 rows: their prefix over the ranges
+                const uint32_t nr = rows;
+                uint32_t tiles_mine[kMaxRanges / 32];
+                uint32_t my_tiles = 0;
 #pragma unroll
-            for (uint32_t s = 0; s < kMaxRanges / 32; ++s) {
-                uint32_t r = lane * (kMaxRanges / 32) + s;
-                if (r < nr) S.tp[r] = run;
-                run += tiles_mine[s];
-            }
-            if (lane == 31) {
-                S.tp[nr] = incl;
-                S.ntiles = incl;
-                S.nr = nr;
-                S.nq = nq;
-                S.q0 = blk.q0;
+                for (uint32_t s = 0; s < kMaxRanges / 32; ++s) {
+                    const uint32_t r = lane * (kMaxRanges / 32) + s;
+                    tiles_mine[s] = r < nr ? range_tiles(S.rs[r], S.rl[r]) : 0u;
+                    my_tiles += tiles_mine[s];
+                }
+                uint32_t incl = my_tiles;
+                for (int o = 1; o < 32; o <<= 1) {
+                    uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= (uint32_t)o) incl += t;
+                }
+                uint32_t run = incl - my_tiles;
+#pragma unroll
+                for (uint32_t s = 0; s < kMaxRanges / 32; ++s) {
+                    const uint32_t r = lane * (kMaxRanges / 32) + s;
+                    if (r < nr) S.tp[r] = run;
+                    run += tiles_mine[s];
+                }
+                if (lane == 31) {
+                    S.tp[nr] = incl;
+                    S.ntiles = incl;
+                    S.nr = nr;
+                }
             }
         }
         __syncthreads();
-        const uint32_t ntiles = S.ntiles;
-        if (ntiles == 0) continue;
+        // this item's tiles [t_lo, t_hi) of the block's
+        const uint32_t part = item - bi * a.parts;
+        const uint32_t t_lo = (uint32_t)((unsigned long long)S.ntiles * part / a.parts);
+        const uint32_t t_hi = (uint32_t)((unsigned long long)S.ntiles * (part + 1) / a.parts);
+        if (t_lo == t_hi) continue;
 
+        // Every role's warp walks its loop as a whole and one elected lane issues: a wait
+        // inside a one-lane branch took 600 to 1,250 cycles per hand-over against 250 converged.
         if (warp == 0) {
-            if (lane == 0) {
-                // ---------------- TMA producer
-                // both query tiles: rows past the item's queries are masked in the epilogue,
-                // rows past n are zero-filled
-                tc::mbar_arrive_expect_tx(&S.bfull, kQT * tile_bytes);
-                for (uint32_t j = 0; j < (uint32_t)kQT; ++j)
-                    for (uint32_t kb = 0; kb < a.nkb; ++kb)
-                        tc::tma_load_2d(b_tiles + kb * kBKBlockBytes + j * kKBlockBytes, &tm_query, &S.bfull,
-                                        (int)(kb * 32), (int)(blk.q0 + j * kTileRows));
-                TileWalk tw;
-                for (uint32_t t = 0; t < ntiles; ++t) {
-                    const uint32_t s = it % a.stages, use = it / a.stages;
-                    if (use > 0 && !tc::mbar_wait(&S.empty_a[s], (use - 1) & 1u, abort, a.err, a.wait_cycles)) break;
-                    tw.locate(S, t);
-                    tc::mbar_arrive_expect_tx(&S.full_a[s], tile_bytes);
-                    for (uint32_t kb = 0; kb < a.nkb; ++kb)
-                        tc::tma_load_2d(a_tiles + s * tile_bytes + kb * kKBlockBytes, &tm_cand, &S.full_a[s],
-                                        (int)(kb * 32), (int)tw.start);
-                    ++it;
-                }
+            // ---------------- loads: the query columns once, then the candidate tiles
+            const uint32_t qbytes = ((ncols + 31u) & ~31u) * kRowBytes;
+            if (tc::elect_one()) {
+                tc::mbar_arrive_expect_tx(&S.bfull, a.nkb * qbytes);
+                for (uint32_t kb = 0; kb < a.nkb; ++kb)
+                    tc::bulk_load(b_tiles + kb * bkb_bytes, a.qform + kb * a.plane + (size_t)qbase * kRowBytes, qbytes,
+                                  &S.bfull);
             }
             __syncwarp();
-            it = __shfl_sync(0xffffffffu, it, 0);
+            TileWalk tw;
+            for (uint32_t t = t_lo; t < t_hi; ++t) {
+                if (use_a > 0) tc::mbar_wait(&S.empty_a[stage], (use_a - 1) & 1u, abort, a.err, a.wait_cycles);
+                tw.locate(S, t);
+                if (tc::elect_one()) {
+                    tc::mbar_arrive_expect_tx(&S.full_a[stage], tile_bytes);
+                    for (uint32_t kb = 0; kb < a.nkb; ++kb)
+                        tc::bulk_load(a_tiles + stage * tile_bytes + kb * kKBlockBytes,
+                                      a.cform + kb * a.plane + (size_t)tw.start * kRowBytes, kKBlockBytes,
+                                      &S.full_a[stage]);
+                }
+                __syncwarp();
+                if (++stage == a.stages) { stage = 0; ++use_a; }
+            }
         } else if (warp <= kAcc) {
-            if (lane == 0) {
-                // ---------------- MMA issuer h (warp 1: h = 0, warp 2: h = 1) of the tiles t with
-                // t % 2 == h, into accumulator h.  Two issuers: every barrier wait stalls the
-                // issuing thread's MMA stream for ~160 cycles (measured), and the other issuer
-                // keeps the tensor pipe busy meanwhile.
-                const uint32_t h = warp - 1;
-                bool ok = tc::mbar_wait(&S.bfull, items_loaded & 1u, abort, a.err, a.wait_cycles);
-                tc::fence_after();
-                const uint32_t ksteps = a.nkb * 2;
-                const uint32_t a_base = tc::smem_u32(a_tiles), b_base = tc::smem_u32(b_tiles);
-                for (uint32_t t = 0; ok && t < ntiles; ++t) {
-                    const uint32_t s = it % a.stages, use = it / a.stages;
-                    ++it;
-                    if ((t & 1u) != h) continue;
-                    if (!tc::mbar_wait(&S.full_a[s], use & 1u, abort, a.err, a.wait_cycles)) break;
-                    if (acc_use[h] > 0 &&
-                        !tc::mbar_wait(&S.empty_acc[h], (acc_use[h] - 1) & 1u, abort, a.err, a.wait_cycles))
-                        break;
-                    tc::fence_after();
-                    // M = 128 candidates x N = 256 queries per MMA: the shape that keeps the
-                    // tensor pipe busy (N = 128 MMAs issue at well under half its rate)
-                    for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                        const uint32_t kin = (ks & 1u) * 32u;
-                        uint64_t ad = tc::desc_kmajor_sw64(a_base + s * tile_bytes + (ks >> 1) * kKBlockBytes + kin);
-                        uint64_t bd = tc::desc_kmajor_sw64(b_base + (ks >> 1) * kBKBlockBytes + kin);
-                        tc::mma_f16(tmem + h * kAccCols, ad, bd, a.idesc, ks > 0 ? 1u : 0u);
+            // ---------------- MMA issuer h (warp 1: h = 0, warp 2: h = 1), into accumulator h.
+            const uint32_t h = warp - 1;
+            tc::mbar_wait(&S.bfull, items_loaded & 1u, abort, a.err, a.wait_cycles);
+            const uint64_t a_desc = tc::desc_kmajor_sw64(tc::smem_u32(a_tiles));
+            const uint64_t b_desc =
+                tc::desc_kmajor_sw64(tc::smem_u32(b_tiles) + (both ? h * (uint32_t)kAccCols * kRowBytes : 0u));
+            // N = this half's query columns in whole groups of 32
+            const uint32_t cols = both ? (h ? ncols - kAccCols : (uint32_t)kAccCols) : ncols;
+            const uint32_t idesc = tc::idesc_f16(a.fmt, kTileRows, (cols + 31u) & ~31u);
+            // both: this issuer takes every tile; otherwise every second one
+            for (uint32_t t = t_lo; t < t_hi; ++t) {
+                if (both || ((t - t_lo) & 1u) == h) {
+                    tc::mbar_wait(&S.full_a[stage], use_a & 1u, abort, a.err, a.wait_cycles);
+                    if (uses > 0) tc::mbar_wait(&S.empty_acc[h], (uses - 1) & 1u, abort, a.err, a.wait_cycles);
+                    ++uses;
+                    if (tc::elect_one()) {
+                        tc::fence_after();
+                        // M = 128 candidates x N = 256 queries per MMA: the shape that keeps the
+                        // tensor pipe busy (N = 128 MMAs issue at well under half its rate)
+                        uint64_t ad = a_desc + ((stage * tile_bytes) >> 4), bd = b_desc;
+                        tc::mma_f16(tmem + h * kAccCols, ad, bd, idesc, 0u);
+                        tc::mma_f16(tmem + h * kAccCols, ad + 2u, bd + 2u, idesc, 1u);
+                        for (uint32_t kb = 1; kb < a.nkb; ++kb) {
+                            ad += kKBlockBytes >> 4;
+                            bd += bkb_bytes >> 4;
+                            tc::mma_f16(tmem + h * kAccCols, ad, bd, idesc, 1u);
+                            tc::mma_f16(tmem + h * kAccCols, ad + 2u, bd + 2u, idesc, 1u);
+                        }
+                        tc::mma_commit(&S.full_acc[h]);
+                        tc::mma_commit(&S.empty_a[stage]);
+                        if (!both) tc::mma_commit(&S.empty_a[stage]);
                     }
-                    tc::mma_commit(&S.full_acc[h]);
-                    ++acc_use[h];
-                    tc::mma_commit(&S.empty_a[s]);
+                    __syncwarp();
                 }
+                if (++stage == a.stages) { stage = 0; ++use_a; }
             }
-            __syncwarp();
-            it = __shfl_sync(0xffffffffu, it, 0);
-#pragma unroll
-            for (int j = 0; j < kAcc; ++j) acc_use[j] = __shfl_sync(0xffffffffu, acc_use[j], 0);
             ++items_loaded;
         } else {
-            // ---------------- epilogue: warps 3 .. 3 + 4*EPI.  SPLIT: two sets of 2*EPI warps,
-            // one per accumulator (tiles of one parity), so a warp has two tiles' MMA time to
-            // drain its share and a slow warp holds back only its own accumulator; otherwise
-            // one set of 4*EPI warps drains every tile.  TMEM lane quarter = warp % 4; column
-            // group within the set = (index in set) / 4.
-            constexpr uint32_t SETW = SPLIT ? 2 * EPI : 4 * EPI;
+            // ---------------- epilogue: warps 3 .. 18, a set of 8 per accumulator, so that a slow
+            // warp holds back only its own accumulator.  TMEM lane quarter = warp % 4; each warp
+            // reads half of the accumulator's columns.
             const uint32_t ew = warp - 1 - kAcc;
-            const uint32_t hset = ew / SETW;   // SPLIT: the accumulator (tile parity) this warp drains
+            const uint32_t j = ew / (kEpiWarps / kAcc);   // the accumulator this warp drains
             const uint32_t quarter = warp & 3u;
-            const uint32_t grp = (ew % SETW) >> 2;
             const uint32_t row = quarter * 32u + lane;
-            const uint32_t lane_base = (quarter * 32u) << 16;
             // per-thread pair counts of one launch stay far below 2^32 (bounded by the sink)
             uint32_t n_acc = 0, n_band = 0;
-            bool ok = true;
-            // this warp's columns of an accumulator: COLS = 256 / (SETW / 4), read in chunks
-            // of LDW by tcgen05.ld, W chunks per wait ("wave").
-            constexpr uint32_t COLS = kAccCols / (SETW / 4);
-            constexpr uint32_t LDW = EPI == 4 ? 32u : 64u;
-            constexpr uint32_t NCH = COLS / LDW;
-            constexpr uint32_t W = (EPI == 2 || !SPLIT) ? 2u : 1u;
-            static_assert(NCH % W == 0, "whole waves per accumulator");
-            const uint32_t t_first = SPLIT ? hset : 0u, t_step = SPLIT ? 2u : 1u;
-            const uint32_t ncols = min((uint32_t)kAccCols, S.nq);
-            const uint32_t q0 = S.q0;
-            // the query block's part of the guard band, added to the threshold once per item
-            const float qb = __double2float_ru(tc_band_q(a.gamma_acc, a.s_t, a.ref_rel, __uint_as_float(S.max_e),
-                                                         __uint_as_float(S.max_n), __uint_as_float(S.max_r)));
-            const float thr_hi = __fadd_ru(a.thr, qb), thr_lo = __fsub_rd(a.thr, qb);
+            // this warp's columns of the accumulator, read in chunks of 32
+            constexpr uint32_t COLS = kAccCols / 2, NCH = COLS / 32;
+            const uint32_t acc_col = ((ew >> 2) & 1u) * COLS;
+            const uint32_t acc = tmem + ((quarter * 32u) << 16) + j * kAccCols + acc_col;
+            const uint32_t col_base = acc_col + (both ? j * kAccCols : 0u);   // in query columns
+            // chunks that hold queries of this item (the rest of the accumulator is stale)
+            const uint32_t nch = ncols > col_base ? min(NCH, (ncols - col_base + 31u) / 32u) : 0u;
             TileWalk tw;
-            // the row's band term and original id, loaded one tile ahead: a global load on
-            // the hit path stalls the warp, and a stalled warp holds back the release of the
-            // next accumulator
-            float pb_next = 0.f;
-            uint32_t cid_next = 0u;
-            if (t_first < ntiles) {
-                tw.locate(S, t_first);
-                if (row < tw.valid) {
-                    pb_next = a.pband[tw.start + row];
-                    if (!a.count_only) cid_next = a.perm[tw.start + row];
-                }
-            }
-            for (uint32_t t = t_first; ok && t < ntiles; t += t_step) {
-                const uint32_t j = t & 1u;
-                const uint32_t cpos = tw.start + row;
-                const bool vrow = row < tw.valid;
-                const float hi = vrow ? __fadd_ru(thr_hi, pb_next) : -INFINITY;
-                const float lo = vrow ? __fsub_rd(thr_lo, pb_next) : -INFINITY;
-                const uint32_t cid = cid_next;   // the owner lane's id reaches the writing lane by a shuffle
-                if (t + t_step < ntiles) {
-                    // the next tile's rows, loaded while this tile is processed
-                    tw.locate(S, t + t_step);
-                    if (row < tw.valid) {
-                        pb_next = a.pband[tw.start + row];
-                        if (!a.count_only) cid_next = a.perm[tw.start + row];
-                    }
-                }
-                if (!tc::mbar_wait(&S.full_acc[j], acc_use[j] & 1u, abort, a.err, a.wait_cycles)) {
-                    ok = false;
-                    break;
-                }
+            for (uint32_t t = t_lo + (both ? 0u : j); t < t_hi; t += both ? 1u : 2u) {
+                tc::mbar_wait(&S.full_acc[j], uses & 1u, abort, a.err, a.wait_cycles);
                 tc::fence_after();
-                if constexpr (DEFER) {
-                    // fast pass: min-reduce every chunk and note, per row, the chunks with a value
-                    // not above the upper band edge; no vote or branch per chunk
-                    uint32_t hitw = 0;
-                    auto load_chunk = [&](float (&v)[LDW], uint32_t c) {
-                        const uint32_t col = grp * COLS + c * LDW;
-                        if constexpr (LDW == 64) tc::tmem_ld_32x64(tmem + lane_base + j * kAccCols + col, v);
-                        else tc::tmem_ld_32x32(tmem + lane_base + j * kAccCols + col, v);
-                    };
+                // per chunk: signs (candidate hits) and outright accepts of this lane's row
+                uint32_t hm[NCH], am[NCH];
 #pragma unroll
-                    for (uint32_t c0 = 0; c0 < NCH; c0 += W) {
-                        float v[W][LDW];
+                for (uint32_t c = 0; c < NCH; ++c) hm[c] = am[c] = 0u;
+                if constexpr (DENSE) {
 #pragma unroll
-                        for (uint32_t w = 0; w < W; ++w) load_chunk(v[w], c0 + w);
-                        tc::tmem_ld_wait();
-#pragma unroll
-                        for (uint32_t w = 0; w < W; ++w) hitw |= (uint32_t)not_above(minN<LDW>(v[w]), hi) << (c0 + w);
+                    for (uint32_t c = 0; c < NCH; ++c) {
+                        if (c >= nch) break;
+                        uint32_t v[32];
+                        tc::tmem_ld_32(acc + c * 32u, v);
+                        tc::tmem_wait_32(v);
+                        hm[c] = sign_mask(v);
+                        if (!a.count_only && __any_sync(0xffffffffu, hm[c])) am[c] = hm[c] & below_mask(v, a.lo);
                     }
-                    // chunks where some row hit are read again (rare: the accumulator is still
-                    // held) and classified pair by pair
-                    uint32_t wave_hits = __reduce_or_sync(0xffffffffu, hitw);
-                    while (wave_hits) {
-                        const uint32_t c = __ffs(wave_hits) - 1;
-                        wave_hits &= wave_hits - 1;
-                        float v[LDW];
-                        load_chunk(v, c);
-                        tc::tmem_ld_wait();
-                        const bool any_hit = (hitw >> c) & 1u;
-                        const uint32_t col0 = grp * COLS + c * LDW;
-#pragma unroll
-                        for (uint32_t h = 0; h < LDW / 32; ++h) {
-                            const uint32_t qcol = col0 + h * 32u;
-                            uint32_t hmask = 0, amask = 0;
-                            if (any_hit) {
-#pragma unroll
-                                for (int i = 0; i < 32; ++i) {
-                                    bool inq = qcol + i < ncols;
-                                    hmask |= (uint32_t)(inq && not_above(v[h * 32 + i], hi)) << i;
-                                    amask |= (uint32_t)(inq && v[h * 32 + i] <= lo) << i;
-                                }
-                            }
-                            const uint32_t bmask = hmask & ~amask;
-                            n_acc += __popc(amask);
-                            n_band += __popc(bmask);
-                            if (a.count_only) continue;
-                            // coalesced output: each lane writes every 32nd pair of the warp's
-                            // hits; the owner lane's row gives the candidate
-                            warp_emit_masks_v(a.sink, wc_acc, amask, cid, [&](uint32_t, uint32_t b, uint32_t ocid) {
-                                return make_uint2(S.qid[qcol + b], ocid);
-                            });
-                            warp_emit_masks_v(a.band, wc_band, bmask, cpos, [&](uint32_t, uint32_t b, uint32_t opos) {
-                                return make_uint2(q0 + qcol + b, opos);
-                            });
-                        }
-                    }
-                    // every column of this warp has been read: release the accumulator
-                    tc::fence_before();
-                    __syncwarp();
-                    if (lane == 0) tc::mbar_arrive(&S.empty_acc[j]);
                 } else {
-                    // per chunk: min-reduce, vote, and classify at once; the accumulator is
-                    // released as soon as the last wave is in registers
-#pragma unroll 1
-                    for (uint32_t c0 = 0; c0 < NCH; c0 += W) {
-                        float v[W][LDW];
+                    uint32_t seen = 0, v[32];
 #pragma unroll
-                        for (uint32_t w = 0; w < W; ++w) {
-                            const uint32_t col = grp * COLS + (c0 + w) * LDW;
-                            if constexpr (LDW == 64) {
-                                tc::tmem_ld_32x64(tmem + lane_base + j * kAccCols + col, v[w]);
-                            } else {
-                                tc::tmem_ld_32x32(tmem + lane_base + j * kAccCols + col, v[w]);
-                            }
-                        }
-                        tc::tmem_ld_wait();
-                        if (c0 + W >= NCH) {
-                            // all of this warp's columns are in registers: release the accumulator
-                            tc::fence_before();
-                            __syncwarp();
-                            if (lane == 0) tc::mbar_arrive(&S.empty_acc[j]);
-                        }
+                    for (uint32_t c = 0; c < NCH; ++c) {
+                        if (c >= nch) break;
+                        tc::tmem_ld_32(acc + c * 32u, v);
+                        tc::tmem_wait_32(v);
+                        seen |= (or_all(v) >> 31) << c;
+                    }
+                    seen = __reduce_or_sync(0xffffffffu, seen);
+                    if (seen) {
+                        // rare: the accumulator is still held
 #pragma unroll
-                        for (uint32_t w = 0; w < W; ++w) {
-                            const uint32_t col0 = grp * COLS + (c0 + w) * LDW;
-                            const bool any_hit = not_above(minN<LDW>(v[w]), hi);
-                            if (!__any_sync(0xffffffffu, any_hit)) continue;
-#pragma unroll
-                            for (uint32_t h = 0; h < LDW / 32; ++h) {
-                                const uint32_t qcol = col0 + h * 32u;
-                                uint32_t hmask = 0, amask = 0;
-                                if (any_hit) {
-#pragma unroll
-                                    for (int i = 0; i < 32; ++i) {
-                                        bool inq = qcol + i < ncols;
-                                        hmask |= (uint32_t)(inq && not_above(v[w][h * 32 + i], hi)) << i;
-                                        amask |= (uint32_t)(inq && v[w][h * 32 + i] <= lo) << i;
-                                    }
-                                }
-                                const uint32_t bmask = hmask & ~amask;
-                                n_acc += __popc(amask);
-                                n_band += __popc(bmask);
-                                if (a.count_only) continue;
-                                // coalesced output: each lane writes every 32nd pair of the warp's
-                                // hits; the owner lane's row gives the candidate
-                                warp_emit_masks_v(a.sink, wc_acc, amask, cid, [&](uint32_t, uint32_t b, uint32_t ocid) {
-                                    return make_uint2(S.qid[qcol + b], ocid);
-                                });
-                                warp_emit_masks_v(a.band, wc_band, bmask, cpos, [&](uint32_t, uint32_t b, uint32_t opos) {
-                                    return make_uint2(q0 + qcol + b, opos);
-                                });
-                            }
+                        for (uint32_t c = 0; c < NCH; ++c) {
+                            if (!((seen >> c) & 1u)) continue;
+                            tc::tmem_ld_32(acc + c * 32u, v);
+                            tc::tmem_wait_32(v);
+                            hm[c] = sign_mask(v);
+                            am[c] = hm[c] & below_mask(v, a.lo);
                         }
                     }
                 }
-                ++acc_use[j];
+                // every column of this warp has been read: release the accumulator
+                tc::fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&S.empty_acc[j]);
+                ++uses;
+                uint32_t any = 0;
+#pragma unroll
+                for (uint32_t c = 0; c < NCH; ++c) any |= hm[c];
+                if (!__any_sync(0xffffffffu, any)) continue;
+
+                // rows past the range's end and columns past the queries are other points'; in the
+                // symmetric form a candidate pairs with the queries up to its own position
+                tw.locate(S, t);
+                const uint32_t cpos = tw.start + row;
+                const bool in = row >= tw.first && row < tw.end;
+                const uint32_t lim = in ? (a.sym ? min(ncols, cpos - qbase + 1u) : ncols) : 0u;
+                const uint32_t skip = q0 - qbase;   // columns below 8 that precede the item's queries
+                uint32_t na = 0, nb = 0;
+                uint32_t self = 0xFFFFFFFFu;   // column of the candidate itself
+                if (a.sym && in && cpos < blk.q1) self = cpos - qbase - col_base;
+#pragma unroll
+                for (uint32_t c = 0; c < NCH; ++c) {
+                    const uint32_t c0 = col_base + c * 32u;
+                    hm[c] &= lim > c0 ? low_bits(lim - c0) : 0u;
+                    if (c0 == 0u) hm[c] &= ~low_bits(skip);
+                    am[c] &= hm[c];
+                    hm[c] &= ~am[c];          // band
+                    na += __popc(am[c]);
+                    nb += __popc(hm[c]);
+                }
+                if (a.count_only) {
+                    n_band += na + nb;
+                    continue;
+                }
+                // accepted pairs go out in both orders (symmetric form), the pair of a point with itself once
+                if (__any_sync(0xffffffffu, na)) {
+                    const uint32_t cw = na ? a.perm[cpos] : 0u;
+                    const uint32_t cid = cw & 0x7FFFFFFFu;
+                    const bool fwd = !q_silent;
+                    const bool rev = a.sym && !(cw >> 31);
+                    uint32_t self_hit = 0;
+#pragma unroll
+                    for (uint32_t c = 0; c < NCH; ++c)
+                        if (self - c * 32u < 32u) self_hit |= (am[c] >> (self - c * 32u)) & 1u;
+                    const uint32_t cnt = (fwd ? na : 0u) + (rev ? na - self_hit : 0u);
+                    n_acc += cnt;
+                    warp_emit_serial(a.sink, wc_acc, cnt, [&](auto&& put) {
+#pragma unroll
+                        for (uint32_t c = 0; c < NCH; ++c) {
+                            uint32_t m = am[c];
+                            while (m) {
+                                const uint32_t col = c * 32u + __ffs(m) - 1u;
+                                m &= m - 1u;
+                                const uint32_t qid = S.qid[col_base + col];
+                                if (fwd) put(qid, cid);
+                                if (rev && col != self) put(cid, qid);
+                            }
+                        }
+                    });
+                }
+                if (__any_sync(0xffffffffu, nb)) {
+                    n_band += a.sym ? 2u * nb : nb;
+                    warp_emit_serial(a.band, wc_band, nb, [&](auto&& put) {
+#pragma unroll
+                        for (uint32_t c = 0; c < NCH; ++c) {
+                            uint32_t m = hm[c];
+                            while (m) {
+                                const uint32_t col = c * 32u + __ffs(m) - 1u;
+                                m &= m - 1u;
+                                put(qbase + col_base + col, cpos);
+                            }
+                        }
+                    });
+                }
             }
             unsigned long long w_acc = n_acc, w_band = n_band;
             for (int o = 16; o > 0; o >>= 1) {
@@ -593,18 +567,22 @@ __global__ void __launch_bounds__(32 * (1 + kAcc) + 128 * EPI, 1)
             }
             if (lane == 0) {
                 if (a.count_only) {
-                    if (w_acc + w_band) atomicAdd(&a.block_counts[item], w_acc + w_band);
+                    if (w_acc + w_band) atomicAdd(&a.block_counts[bi], w_acc + w_band);
                 } else if (a.stats) {
                     if (w_acc) atomicAdd(&a.stats[0], w_acc);
                     if (w_band) atomicAdd(&a.stats[1], w_band);
                 }
             }
-            it += ntiles;
         }
     }
     if (warp > kAcc && !a.count_only) {
         warp_chunk_close(a.sink, wc_acc);
         warp_chunk_close(a.band, wc_band);
+    }
+    if (*abort) {
+        // after a timeout copies may still be in flight (a microsecond or two): let them land
+        const long long t0 = clock64();
+        while (clock64() - t0 < 200000ll) {}
     }
     tc::fence_before();
     __syncthreads();
@@ -615,22 +593,23 @@ __global__ void __launch_bounds__(32 * (1 + kAcc) + 128 * EPI, 1)
 }
 
 // Band pairs: exact FP32 refine in the reference's order (kernel.cu:350-355).
+// sym: a pair stands for both orders (see the symmetric form above).
 __global__ void k_band_recheck(const float* __restrict__ pts, const uint32_t* __restrict__ perm, uint32_t d,
                                float thr, const uint32_t* __restrict__ bq, const uint32_t* __restrict__ bc,
                                const unsigned long long* __restrict__ band_used, unsigned long long band_cap,
-                               PairSink sink) {
+                               uint32_t sym, PairSink sink) {
     const unsigned long long n = min(*band_used, band_cap);
     WarpChunk wc;
     warp_chunk_init(wc);
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < n; base += stride) {
         unsigned long long i = base + threadIdx.x;
-        bool hit = false;
-        uint32_t qp = 0, cp = 0;
+        uint32_t qid = 0, cid = 0;
+        bool fwd = false, rev = false;
         if (i < n) {
-            qp = bq[i];
+            const uint32_t qp = bq[i];
             if (qp != kSentinelKey) {
-                cp = bc[i];
+                const uint32_t cp = bc[i];
                 const float* q = pts + (size_t)qp * d;
                 const float* c = pts + (size_t)cp * d;
                 float acc = 0.f;
@@ -638,10 +617,18 @@ __global__ void k_band_recheck(const float* __restrict__ pts, const uint32_t* __
                     float diff = __fsub_rn(c[l], q[l]);
                     acc = __fmaf_rn(diff, diff, acc);
                 }
-                hit = acc <= thr;
+                if (acc <= thr) {
+                    const uint32_t qw = perm[qp], cw = perm[cp];
+                    qid = qw & 0x7FFFFFFFu;
+                    cid = cw & 0x7FFFFFFFu;
+                    fwd = !(qw >> 31);
+                    rev = sym && !(cw >> 31) && qp != cp;
+                }
             }
         }
-        warp_emit(sink, wc, hit ? 1u : 0u, [&](uint32_t) { return make_uint2(perm[qp], perm[cp]); });
+        warp_emit(sink, wc, (fwd ? 1u : 0u) + (rev ? 1u : 0u), [&](uint32_t j) {
+            return fwd && j == 0 ? make_uint2(qid, cid) : make_uint2(cid, qid);
+        });
     }
     warp_chunk_close(sink, wc);
 }
@@ -689,56 +676,151 @@ __global__ void k_tc_range(const float* __restrict__ pts, uint32_t n, uint32_t d
     block_max_into(bad ? 0.0 : n2, max_n2);
 }
 
-// Operand forms of one sorted point (one thread each), in units scaled by
-// `scale` (a power of two): x~ = half((x - origin) * scale).  Also folds the
-// maxima of the per-point bound terms into maxima[0..2] (float bits).
+// The two halves of a norm term N: their sum is never above it (the filter may
+// only err towards the recheck).  N is at least -60000, finite in FP16: a term
+// cut off there belongs to a pair whose D' is negative anyway (the other terms
+// are at most 2^14).
 template <typename H>
-__global__ void k_tc_prep(const float* __restrict__ pts, uint32_t n, uint32_t d, uint32_t kpad,
-                          const float* __restrict__ origin, double scale, H* __restrict__ qform,
-                          H* __restrict__ cform, float4* __restrict__ pinfo, unsigned int* __restrict__ maxima) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < n) {
+__device__ __forceinline__ H to_h_down(double x);
+template <>
+__device__ __forceinline__ __half to_h_down<__half>(double x) { return __float2half_rd(__double2float_rd(x)); }
+template <>
+__device__ __forceinline__ __nv_bfloat16 to_h_down<__nv_bfloat16>(double x) {
+    return __float2bfloat16_rd(__double2float_rd(x));
+}
+template <typename H>
+__device__ __forceinline__ double split_norm(double n, H& hi, H& lo) {
+    n = fmax(n, -60000.0);
+    hi = to_h<H>(n);
+    lo = to_h_down<H>(n - from_h(hi));
+    return n - from_h(hi) - from_h(lo);   // the residual, >= 0
+}
+
+// Constants of the guard band (scaled units).
+struct TcBand {
+    double thr, gamma, s_t, ref_rel;
+};
+
+// Operand forms of sorted points [row0, row0 + rows), one thread each, written to
+// plane rows 0..; rows past n and up to plane_n are zero.  Units are scaled by
+// `scale` (a power of two): x~ = half((x - origin) * scale).  shift: the norm
+// terms carry the threshold and the guard band (the filter); otherwise they are
+// |x~|^2 (the tile probe).  Folds the maxima of the bound terms into
+// maxima[0..4] (float bits): e, |x~|^2, residual, 2 P + residual, 2 Q + residual.
+// A block stages its 64 points in shared memory with coalesced loads (rows padded
+// to an odd stride); a thread writes its rows in 16-byte chunks, neighbouring
+// threads neighbouring rows.  Either form may be null.
+constexpr int kTcMaxima = 5;
+constexpr int kPrepRows = 64;
+template <typename H>
+__global__ void __launch_bounds__(kPrepRows)
+    k_tc_prep(const float* __restrict__ pts, uint32_t n, uint32_t d, uint32_t nkb, const float* __restrict__ origin,
+              double scale, TcBand band, uint32_t shift, uint32_t row0, unsigned long long plane_n,
+              H* __restrict__ qform, H* __restrict__ cform, unsigned int* __restrict__ maxima) {
+    extern __shared__ float prep_s[];
+    const uint32_t stride = d | 1u;
+    const unsigned long long first = (unsigned long long)blockIdx.x * kPrepRows;   // plane row
+    const uint32_t src0 = row0 + (uint32_t)first;
+    const uint32_t have = src0 < n ? min((uint32_t)kPrepRows, n - src0) : 0u;
+    for (uint32_t f = threadIdx.x; f < have * d; f += kPrepRows) {
+        const uint32_t i = f / d, l = f - i * d;
+        prep_s[i * stride + l] = pts[(size_t)src0 * d + f];
+    }
+    __syncthreads();
+    const unsigned long long row = first + threadIdx.x;
+    float m[kTcMaxima] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    if (row < plane_n) {
+        const bool real = threadIdx.x < have;
+        const float* x_s = prep_s + threadIdx.x * stride;
+        const H zero = to_h<H>(0.0), one = to_h<H>(1.0);
         double n2 = 0, e2 = 0;
-        H* qr = qform + (size_t)i * kpad;
-        H* cr = cform + (size_t)i * kpad;
-        for (uint32_t l = 0; l < d; ++l) {
-            double x = ((double)pts[(size_t)i * d + l] - (double)origin[l]) * scale;   // exact: scale is 2^s
-            H h = to_h<H>(x);
-            double xt = from_h(h);
+        auto put = [&](uint32_t chunk, const H (&q)[8], const H (&c)[8]) {
+            const unsigned long long at = ((unsigned long long)(chunk >> 2) * plane_n + row) * 4u +
+                                          ((chunk & 3u) ^ ((uint32_t)(row >> 1) & 3u));
+            if (qform) reinterpret_cast<uint4*>(qform)[at] = *reinterpret_cast<const uint4*>(q);
+            if (cform) reinterpret_cast<uint4*>(cform)[at] = *reinterpret_cast<const uint4*>(c);
+        };
+        const uint32_t whole = d / 8u;   // chunks of coordinates only
+        for (uint32_t ch = 0; ch < whole; ++ch) {
+            __align__(16) H q[8], c[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                const uint32_t l = ch * 8u + i;
+                const double x = real ? ((double)x_s[l] - (double)origin[l]) * scale : 0.0;   // exact: scale is 2^s
+                const double xt = from_h(q[i] = to_h<H>(x));
+                c[i] = to_h<H>(-2.0 * xt);
+                e2 += (xt - x) * (xt - x);
+                n2 += xt * xt;
+            }
+            if (!real)
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) q[i] = c[i] = zero;
+            put(ch, q, c);
+        }
+        // the last coordinates, then the norm terms and zeros
+        for (uint32_t l = whole * 8u; l < d; ++l) {
+            const double x = real ? ((double)x_s[l] - (double)origin[l]) * scale : 0.0;
+            const double xt = from_h(to_h<H>(x));
             e2 += (xt - x) * (xt - x);
             n2 += xt * xt;
-            qr[l] = h;
-            cr[l] = to_h<H>(-2.0 * xt);
         }
-        H nh = to_h<H>(n2);
-        H nl = to_h<H>(n2 - from_h(nh));
-        double res = fabs(n2 - from_h(nh) - from_h(nl));
-        H one = to_h<H>(1.0), zero = to_h<H>(0.0);
-        qr[d] = nh; qr[d + 1] = nl; qr[d + 2] = one; qr[d + 3] = one;
-        cr[d] = one; cr[d + 1] = one; cr[d + 2] = nh; cr[d + 3] = nl;
-        for (uint32_t l = d + 4; l < kpad; ++l) { qr[l] = zero; cr[l] = zero; }
-        // round the bounds up: float conversion is to nearest, so scale by 1 + 2^-20
-        const float up = 1.0f + 9.6e-7f;
-        p = make_float4((float)sqrt(e2) * up, (float)n2 * up, (float)res * up + 1e-30f, 0.f);
-        pinfo[i] = p;
-    }
-    float m[3] = {p.x, p.y, p.z};
+        const double e = sqrt(e2);
+        const double P = tc_band_p(band.gamma, band.s_t, band.ref_rel, e, n2);
+        const double Q = tc_band_q(band.gamma, band.s_t, band.ref_rel, e, n2);
+        H qh, ql, cnh, cnl;
+        const double rq = split_norm<H>(shift ? n2 - band.thr - Q : n2, qh, ql);
+        const double rc = split_norm<H>(shift ? n2 - P : n2, cnh, cnl);
+        for (uint32_t ch = whole; ch < nkb * 4u; ++ch) {
+            __align__(16) H q[8], c[8];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+            for (uint32_t i = 0; i < 8; ++i) {
+                const uint32_t l = ch * 8u + i;
+                q[i] = c[i] = zero;
+                if (!real) continue;
+                if (l < d) {
+                    const double x = ((double)x_s[l] - (double)origin[l]) * scale;
+                    q[i] = to_h<H>(x);
+                    c[i] = to_h<H>(-2.0 * from_h(q[i]));
+                } else if (l < d + 4u) {
+                    const uint32_t w = l - d;
+                    q[i] = w == 0 ? qh : w == 1 ? ql : one;
+                    c[i] = w == 2 ? cnh : w == 3 ? cnl : one;
+                }
+            }
+            put(ch, q, c);
+        }
+        if (real) {
+            // round the bounds up: float conversion is to nearest, so scale by 1 + 2^-20
+            const float up = 1.0f + 9.6e-7f;
+            m[0] = (float)e * up;
+            m[1] = (float)n2 * up;
+            m[2] = (float)fmax(rq, rc) * up + 1e-30f;
+            m[3] = (float)(2.0 * P + rc) * up + 1e-30f;
+            m[4] = (float)(2.0 * Q + rq) * up + 1e-30f;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kTcMaxima; ++j) {
         float v = m[j];
         for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
         if (lane_id() == 0 && v > 0.f) atomicMax(&maxima[j], __float_as_uint(v));
     }
 }
 
-// Each point's part of the guard band (tc_band_p), rounded up.
-__global__ void k_tc_pband(const float4* __restrict__ pinfo, uint32_t n, double gamma, double s_t, double ref_rel,
-                           float* __restrict__ out) {
+// Marks the points of silent cells (a coordinate of 0) in bit 31 of a copy of perm.
+__global__ void k_flag_silent(const unsigned long long* __restrict__ cell_lid, const uint32_t* __restrict__ cell_start,
+                              uint32_t nC, HjGrid g, uint32_t* __restrict__ perm) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pinfo[i];
-    out[i] = __double2float_ru(tc_band_p(gamma, s_t, ref_rel, p.x, p.y, p.z));
+    if (i >= nC) return;
+    unsigned long long L = cell_lid[i];
+    bool silent = false;
+    for (uint32_t j = 0; j < g.k; ++j) {
+        const unsigned long long q = L / g.n_cells[j];
+        silent |= L == q * g.n_cells[j];
+        L = q;
+    }
+    if (!silent) return;
+    for (uint32_t p = cell_start[i]; p < cell_start[i + 1]; ++p) perm[p] |= 0x80000000u;
 }
 
 // Per-dimension minimum of the points: lanes walk a row's dimensions (coalesced
@@ -765,19 +847,20 @@ __global__ void k_fill_f32(float* p, uint32_t n, float v) {
     if (i < n) p[i] = v;
 }
 
-// Debug/test kernel: one candidate tile (rows a0..a0+127) against four query
-// tiles (rows b0..b0+511) through the same TMA maps, descriptors and MMA
-// sequence as k_refine_tc; writes every accumulator value to out[128][512].
+// Debug/test kernel: one candidate tile (plane rows 0..127 of cform) against 512
+// query rows (plane rows 0..511 of qform) through the same copies, descriptors and
+// MMA sequence as k_refine_tc; writes every accumulator value to out[128][512].
 __global__ void __launch_bounds__(kProbeThreads, 1)
-    k_tc_tile_probe(const __grid_constant__ CUtensorMap tm_cand, const __grid_constant__ CUtensorMap tm_query,
-                    uint32_t nkb, uint32_t idesc, uint32_t a0, uint32_t b0, float* __restrict__ out, uint32_t* err,
-                    uint32_t skip_mma, long long wait_cycles) {
+    k_tc_tile_probe(const uint8_t* __restrict__ cform, const uint8_t* __restrict__ qform, unsigned long long plane,
+                    uint32_t nkb, uint32_t idesc, float* __restrict__ out, uint32_t* err, uint32_t skip_mma,
+                    long long wait_cycles) {
     extern __shared__ uint8_t smem_raw[];
     uint32_t base = tc::smem_u32(smem_raw);
     uint8_t* smem = smem_raw + ((1024u - (base & 1023u)) & 1023u);
     const uint32_t tile_bytes = nkb * kKBlockBytes;
+    constexpr uint32_t bkb_bytes = kProbeQB * kRowBytes;
     uint8_t* b_tiles = smem;
-    uint8_t* a_tile = smem + kProbeQT * tile_bytes;
+    uint8_t* a_tile = smem + nkb * bkb_bytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(a_tile + tile_bytes);   // [0] loads, [1] mma
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
     uint32_t* abortp = tslot + 1;
@@ -797,12 +880,10 @@ __global__ void __launch_bounds__(kProbeThreads, 1)
     tc::fence_after();
     const uint32_t tmem = *tslot;
     if (tid == 0) {
-        tc::mbar_arrive_expect_tx(&bars[0], (kProbeQT + 1) * tile_bytes);
+        tc::mbar_arrive_expect_tx(&bars[0], nkb * (bkb_bytes + kKBlockBytes));
         for (uint32_t kb = 0; kb < nkb; ++kb) {
-            tc::tma_load_2d(a_tile + kb * kKBlockBytes, &tm_cand, &bars[0], (int)(kb * 32), (int)a0);
-            for (uint32_t j = 0; j < kProbeQT; ++j)
-                tc::tma_load_2d(b_tiles + kb * kProbeBKBlockBytes + j * kKBlockBytes, &tm_query, &bars[0], (int)(kb * 32),
-                                (int)(b0 + j * kTileRows));
+            tc::bulk_load(a_tile + kb * kKBlockBytes, cform + kb * plane, kKBlockBytes, &bars[0]);
+            tc::bulk_load(b_tiles + kb * bkb_bytes, qform + kb * plane, bkb_bytes, &bars[0]);
         }
     }
     if (tid == 32) {
@@ -816,7 +897,7 @@ __global__ void __launch_bounds__(kProbeThreads, 1)
                     const uint32_t kin = (ks & 1u) * 32u;
                     tc::mma_f16(tmem + j * kAccCols,
                                 tc::desc_kmajor_sw64(tc::smem_u32(a_tile) + (ks >> 1) * kKBlockBytes + kin),
-                                tc::desc_kmajor_sw64(tc::smem_u32(b_tiles) + (ks >> 1) * kProbeBKBlockBytes +
+                                tc::desc_kmajor_sw64(tc::smem_u32(b_tiles) + (ks >> 1) * bkb_bytes +
                                                      j * (kAccCols * 64u) + kin),
                                 idesc, ks > 0 ? 1u : 0u);
                 }
@@ -830,11 +911,12 @@ __global__ void __launch_bounds__(kProbeThreads, 1)
         tc::fence_after();
         if (ok) {
             for (uint32_t col = 0; col < (uint32_t)kProbeQB; col += 32) {
-                float v[32];
-                tc::tmem_ld_32x32(tmem + ((quarter * 32u) << 16) + col, v);
-                tc::tmem_ld_wait();
+                uint32_t v[32];
+                tc::tmem_ld_32(tmem + ((quarter * 32u) << 16) + col, v);
+                tc::tmem_wait_32(v);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) out[(size_t)(quarter * 32 + lane) * kProbeQB + col + i] = v[i];
+                for (int i = 0; i < 32; ++i)
+                    out[(size_t)(quarter * 32 + lane) * kProbeQB + col + i] = __uint_as_float(v[i]);
             }
         }
     }
@@ -847,35 +929,6 @@ __global__ void __launch_bounds__(kProbeThreads, 1)
 }
 
 // ---- host side -------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }
-    return fn;
-}
-
-hj_status make_map(CUtensorMap* m, const void* base, uint32_t rows, uint32_t kpad, int kind) {
-    auto fn = encode_fn();
-    if (!fn) { set_error("cuTensorMapEncodeTiled is not available"); return HJ_ERR_CUDA; }
-    cuuint64_t dims[2] = {kpad, rows};
-    cuuint64_t strides[1] = {(cuuint64_t)kpad * 2};
-    cuuint32_t box[2] = {32, (cuuint32_t)kTileRows};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = fn(m, kind == HJ_REFINE_TC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                    2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
-        return HJ_ERR_CUDA;
-    }
-    return HJ_OK;
-}
-
 uint32_t kpad_for(uint32_t d) { return ((d + 4 + 31) / 32) * 32; }
 
 // The float constants of the guard band, shared by the per-point terms and the kernel.
@@ -886,31 +939,30 @@ float band_ref_rel(uint32_t d) { return (float)((d + 2) * std::ldexp(1.0, -24) *
 // (alignment and truncation); bound = (steps + 1) * 32 * 2^-23 * sum|terms|.
 float band_gamma(uint32_t kpad) { return (float)((kpad / 16 + 1) * 32 * std::ldexp(1.0, -23)); }
 
-size_t tc_smem_bytes(uint32_t nkb, uint32_t stages) {
-    return 1024 + (size_t)(kQT + stages) * nkb * kKBlockBytes + sizeof(TcShared);
+size_t tc_smem_bytes(uint32_t nkb, uint32_t qcols, uint32_t stages) {
+    return 1024 + (size_t)nkb * ((size_t)qcols * kRowBytes + (size_t)stages * kKBlockBytes) + sizeof(TcShared);
 }
+constexpr size_t kSmemBudget = 225 * 1024;
+
+// Query columns per work item: 512 (each candidate tile fetched once for both
+// accumulators: half the L2 traffic per pair) where three stages fit beside them.
+uint32_t tc_qcols(uint32_t nkb) { return tc_smem_bytes(nkb, kQBMax, 3) <= kSmemBudget ? kQBMax : kAccCols; }
 
 uint32_t tc_stages(uint32_t nkb) {
-    size_t budget = 225 * 1024;
     uint32_t s = kMaxStages;
-    while (s > 2 && tc_smem_bytes(nkb, s) > budget) --s;
+    while (s > 2 && tc_smem_bytes(nkb, tc_qcols(nkb), s) > kSmemBudget) --s;
     return s;
 }
-
-struct TcMaps {
-    CUtensorMap cand, query;
-};
 
 }  // namespace
 
 struct TcState {
-    TcMaps maps;
-    int epi = 4;              // epilogue shape code, EPI | 8 * SPLIT (autotuned: 2, 4, 10, 12)
-    bool defer = false;       // one vote per accumulator (set from the estimated pair density)
+    bool dense = false;       // masks at once (set from the estimated pair density)
     float gamma_acc = 0;
     int scale_exp = 0;        // operand forms hold (x - origin) * 2^scale_exp
     double thr_s = 0;         // the squared threshold in those units: thr * 4^scale_exp, exact
     float max_e = 0, max_n = 0, max_r = 0;   // maxima of the per-point bound terms (scaled units)
+    float lo = 0;             // accepted outright: D' <= lo
 };
 
 static TcState* tc_state(const hj_index* ix) { return reinterpret_cast<TcState*>(ix->tc_state); }
@@ -919,13 +971,20 @@ bool tc_supported(const hj_index* ix, int kind) {
     if (ix->dtype != HJ_F32 || ix->d < 8) return false;
     if (kind != HJ_REFINE_TC_F16 && kind != HJ_REFINE_TC_BF16) return false;
     uint32_t nkb = kpad_for(ix->d) / 32;
-    if (tc_smem_bytes(nkb, 2) > 225 * 1024) return false;
+    if (tc_smem_bytes(nkb, kAccCols, 2) > kSmemBudget) return false;
     uint32_t rows = 1;
     for (uint32_t j = 1; j < ix->k; ++j) rows *= 3;
     return rows <= kMaxRanges && ix->n < 0x7FFFFF00u;
 }
 
-uint32_t tc_query_block() { return kQB; }
+uint32_t tc_query_block(const hj_index* ix) { return tc_qcols(kpad_for(ix->d) / 32); }
+
+// Work items per block of queries: a list too short to fill the SMs evenly (16
+// items each) has its blocks' candidate tiles cut into up to 32 parts.
+static uint32_t tc_parts(uint32_t nblocks) {
+    const uint32_t want = 16u * (uint32_t)num_sms(), nb = std::max<uint32_t>(nblocks, 1);
+    return std::min<uint32_t>(32u, (want + nb - 1) / nb);
+}
 
 // Band recheck grid for a refine over nblocks work items: as many blocks as there
 // are SMs x 8, but no more than 8 per refine CTA (small joins have small bands).
@@ -937,14 +996,14 @@ static unsigned recheck_grid(uint32_t nblocks) {
 // refine's epilogue warps (at most 16 per CTA, one CTA per SM) and the band
 // recheck's warps (8 per block), each holding at most one partly filled chunk.
 uint64_t tc_emit_warps(uint32_t nblocks) {
-    return (uint64_t)std::min<uint32_t>((uint32_t)num_sms(), std::max<uint32_t>(nblocks, 1)) * 16ull +
+    return std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)std::max<uint32_t>(nblocks, 1) * tc_parts(nblocks)) * 16ull +
            (uint64_t)recheck_grid(nblocks) * 8ull;
 }
 
 // Half-width of the guard band for the worst pair of the dataset, in scaled units.
 static double tc_delta_scaled(const hj_index* ix, const TcState* s) {
     const double sT = band_s_t(s->thr_s), ref = band_ref_rel(ix->d), g = s->gamma_acc;
-    return tc_band_p(g, sT, ref, s->max_e, s->max_n, s->max_r) + tc_band_q(g, sT, ref, s->max_e, s->max_n, s->max_r);
+    return tc_band_p(g, sT, ref, s->max_e, s->max_n) + tc_band_q(g, sT, ref, s->max_e, s->max_n) + 2.0 * s->max_r;
 }
 
 // The same in the dataset's units (the figure the join reports).
@@ -994,6 +1053,38 @@ static bool choose_scale(double max_n2, double thr, int* out) {
     return true;
 }
 
+// Per-dimension minima of the points (the operand forms' origin).
+static hj_status launch_col_min(const hj_index* ix, float* origin, cudaStream_t st) {
+    const uint32_t n = ix->n, d = ix->d;
+    k_fill_f32<<<(d + 255) / 256, 256, 0, st>>>(origin, d, INFINITY);
+    HJ_LAUNCHED();
+    const unsigned blocks = (unsigned)std::min<uint32_t>(num_sms() * 2, std::max<uint32_t>(1, n / 64));
+    k_col_min<<<blocks, 256, (size_t)8 * d * sizeof(float), st>>>((const float*)ix->pts, n, d, origin);
+    HJ_LAUNCHED();
+    return HJ_OK;
+}
+
+// Operand forms of `rows` plane rows from sorted point row0 (all planes, padding rows zero).
+static hj_status launch_prep(const hj_index* ix, int kind, const float* origin, int sexp, const TcBand& band,
+                             uint32_t shift, uint32_t row0, uint64_t rows, void* qf, void* cf, unsigned int* mx,
+                             cudaStream_t st) {
+    const uint32_t n = ix->n, d = ix->d, nkb = kpad_for(d) / 32;
+    const unsigned blocks = (unsigned)((rows + kPrepRows - 1) / kPrepRows);
+    const size_t smem = (size_t)kPrepRows * (d | 1u) * sizeof(float);
+    const double scale = std::ldexp(1.0, sexp);
+    if (kind == HJ_REFINE_TC_BF16) {
+        HJ_TRY(ensure_smem(k_tc_prep<__nv_bfloat16>, smem));
+        k_tc_prep<__nv_bfloat16><<<blocks, kPrepRows, smem, st>>>((const float*)ix->pts, n, d, nkb, origin, scale, band,
+                                                                  shift, row0, rows, (__nv_bfloat16*)qf,
+                                                                  (__nv_bfloat16*)cf, mx);
+    } else {
+        HJ_TRY(ensure_smem(k_tc_prep<__half>, smem));
+        k_tc_prep<__half><<<blocks, kPrepRows, smem, st>>>((const float*)ix->pts, n, d, nkb, origin, scale, band, shift,
+                                                           row0, rows, (__half*)qf, (__half*)cf, mx);
+    }
+    return launch_status(__FILE__, __LINE__);
+}
+
 hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st) {
     if (ix->tc_kind == kind && ix->tc_state) return HJ_OK;
     // Drop the previous operand forms before anything else: if a step below
@@ -1002,38 +1093,26 @@ hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st) {
     ix->tc_kind = -1;
     dfree(ix->tc_a, st);
     dfree(ix->tc_b, st);
-    dfree(ix->tc_err, st);
-    dfree(ix->tc_pband, st);
     const uint32_t kpad = kpad_for(ix->d), n = ix->n, d = ix->d;
     uint16_t *qf = nullptr, *cf = nullptr;
     float* origin = nullptr;
-    float4* pinfo = nullptr;
-    float* pband = nullptr;
     unsigned long long* rng = nullptr;   // [0] max |x - origin|^2 (FP64 bits), [1] non-finite flag
     unsigned int* mx = nullptr;          // maxima of the bound terms (float bits)
     auto fail = [&](hj_status e) {
         cudaGetLastError();
-        dfree(qf, st); dfree(cf, st); dfree(pinfo, st); dfree(origin, st); dfree(rng, st); dfree(mx, st);
-        dfree(pband, st);
+        dfree(qf, st); dfree(cf, st); dfree(origin, st); dfree(rng, st); dfree(mx, st);
         return e;
     };
 #define TC_TRY(x) do { hj_status e_ = (x); if (e_ != HJ_OK) return fail(e_); } while (0)
-    TC_TRY(dalloc(&qf, (size_t)n * kpad, st));
-    TC_TRY(dalloc(&cf, (size_t)n * kpad, st));
-    TC_TRY(dalloc(&pinfo, n, st));
-    TC_TRY(dalloc(&pband, n, st));
+    const uint64_t rows = plane_rows(n);
+    TC_TRY(dalloc(&qf, (size_t)rows * kpad, st));
+    TC_TRY(dalloc(&cf, (size_t)rows * kpad, st));
     TC_TRY(dalloc(&origin, d, st));
     TC_TRY(dalloc(&rng, 2, st));
-    TC_TRY(dalloc(&mx, 4, st));
+    TC_TRY(dalloc(&mx, kTcMaxima, st));
     TC_TRY(cuda_status(cudaMemsetAsync(rng, 0, 2 * sizeof(unsigned long long), st), "clear range scratch"));
-    TC_TRY(cuda_status(cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned int), st), "clear maxima"));
-    k_fill_f32<<<(d + 255) / 256, 256, 0, st>>>(origin, d, INFINITY);
-    TC_TRY(launch_status(__FILE__, __LINE__));
-    {
-        const unsigned blocks = (unsigned)std::min<uint32_t>(num_sms() * 2, std::max<uint32_t>(1, n / 64));
-        k_col_min<<<blocks, 256, (size_t)8 * d * sizeof(float), st>>>((const float*)ix->pts, n, d, origin);
-        TC_TRY(launch_status(__FILE__, __LINE__));
-    }
+    TC_TRY(cuda_status(cudaMemsetAsync(mx, 0, kTcMaxima * sizeof(unsigned int), st), "clear maxima"));
+    TC_TRY(launch_col_min(ix, origin, st));
     const unsigned pblocks = std::max<uint32_t>(1, (n + 255) / 256);
     k_tc_range<<<pblocks, 256, 0, st>>>((const float*)ix->pts, n, d, origin, rng,
                                         reinterpret_cast<uint32_t*>(rng + 1));
@@ -1053,110 +1132,97 @@ hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st) {
                   ix->thr / max_n2);
         return fail(HJ_ERR_UNSUPPORTED);
     }
-    const double scale = std::ldexp(1.0, sexp);
-    if (kind == HJ_REFINE_TC_BF16)
-        k_tc_prep<__nv_bfloat16><<<pblocks, 256, 0, st>>>((const float*)ix->pts, n, d, kpad, origin, scale,
-                                                           (__nv_bfloat16*)qf, (__nv_bfloat16*)cf, pinfo, mx);
-    else
-        k_tc_prep<__half><<<pblocks, 256, 0, st>>>((const float*)ix->pts, n, d, kpad, origin, scale, (__half*)qf,
-                                                    (__half*)cf, pinfo, mx);
-    TC_TRY(launch_status(__FILE__, __LINE__));
-    unsigned int hm[4] = {0, 0, 0, 0};
+    const double thr_s = std::ldexp(ix->thr, 2 * sexp);
+    const TcBand band{thr_s, band_gamma(kpad), band_s_t(thr_s), band_ref_rel(d)};
+    TC_TRY(launch_prep(ix, kind, origin, sexp, band, 1u, 0, rows, qf, cf, mx, st));
+    float hm[kTcMaxima];
     TC_TRY(cuda_status(cudaMemcpyAsync(hm, mx, sizeof(hm), cudaMemcpyDeviceToHost, st), "maxima to host"));
     TC_TRY(cuda_status(cudaStreamSynchronize(st), "maxima sync"));
-    TcMaps maps;
-    TC_TRY(make_map(&maps.query, qf, n, kpad, kind));
-    TC_TRY(make_map(&maps.cand, cf, n, kpad, kind));
-    // each point's part of the guard band
-    const float gamma_acc = band_gamma(kpad);
-    const double thr_s = std::ldexp(ix->thr, 2 * sexp);
-    k_tc_pband<<<pblocks, 256, 0, st>>>(pinfo, n, gamma_acc, band_s_t(thr_s), band_ref_rel(d), pband);
-    TC_TRY(launch_status(__FILE__, __LINE__));
 #undef TC_TRY
     dfree(origin, st);
     dfree(rng, st);
     dfree(mx, st);
     TcState* s = new TcState();
-    s->maps = maps;
-    s->gamma_acc = gamma_acc;
+    s->gamma_acc = (float)band.gamma;
     s->scale_exp = sexp;
     s->thr_s = thr_s;
-    std::memcpy(&s->max_e, &hm[0], 4);
-    std::memcpy(&s->max_n, &hm[1], 4);
-    std::memcpy(&s->max_r, &hm[2], 4);
+    s->max_e = hm[0];
+    s->max_n = hm[1];
+    s->max_r = hm[2];
+    s->lo = -std::nextafter(hm[3] + hm[4], INFINITY);
     ix->tc_a = qf;
     ix->tc_b = cf;
-    ix->tc_err = reinterpret_cast<float*>(pinfo);
-    ix->tc_pband = pband;
     ix->tc_kpad = kpad;
     ix->tc_state = s;
     ix->tc_kind = kind;
     return HJ_OK;
 }
 
-int tc_get_epi(const hj_index* ix) {
+void tc_set_dense(hj_index* ix, bool dense) {
     TcState* s = tc_state(ix);
-    return s ? s->epi : 0;
-}
-void tc_set_epi(hj_index* ix, int epi) {
-    TcState* s = tc_state(ix);
-    if (s && (epi == 2 || epi == 4 || epi == 10 || epi == 12)) s->epi = epi;
+    if (s) s->dense = dense;
 }
 
-void tc_set_defer(hj_index* ix, bool defer) {
-    TcState* s = tc_state(ix);
-    if (s) s->defer = defer;
+// perm with the points of silent cells marked (bit 31), for the symmetric form;
+// the index's own perm where no cell is silent.
+static hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st) {
+    *out = ix->perm;
+    if (!ix->any_silent) return HJ_OK;
+    if (!ix->perm_flag) {
+        uint32_t* p = nullptr;
+        HJ_TRY(dalloc(&p, ix->n, st));
+        ix->perm_flag = p;
+        HJ_CUDA(cudaMemcpyAsync(p, ix->perm, (size_t)ix->n * 4, cudaMemcpyDeviceToDevice, st));
+        k_flag_silent<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->nC, ix->grid, p);
+        HJ_LAUNCHED();
+    }
+    *out = ix->perm_flag;
+    return HJ_OK;
 }
 
-hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
-                           const PairSink& sink, const PairSink& band, uint32_t count_only,
+// sym: blocks[0..nblocks) is the join's whole list, each unordered pair once.
+hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
+                           const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
                            unsigned long long* block_counts, unsigned long long* stats, uint32_t* err,
                            cudaStream_t st) {
     if (nblocks == 0) return HJ_OK;
     TcState* s = tc_state(ix);
     if (!s) { set_error("tensor-core operands not prepared"); return HJ_ERR_INVALID; }
-    const uint32_t nkb = ix->tc_kpad / 32, stages = tc_stages(nkb);
-    size_t smem = tc_smem_bytes(nkb, stages);
+    const uint32_t nkb = ix->tc_kpad / 32, qcols = tc_qcols(nkb), stages = tc_stages(nkb);
+    size_t smem = tc_smem_bytes(nkb, qcols, stages);
     // one CTA per SM: ask for more than half of the SM's shared memory
     smem = std::max<size_t>(smem, 116 * 1024);
-    const int code = s->epi;
-    auto kern = s->defer ? (code == 2    ? k_refine_tc<2, false, true>
-                            : code == 10 ? k_refine_tc<2, true, true>
-                            : code == 12 ? k_refine_tc<4, true, true>
-                                         : k_refine_tc<4, false, true>)
-                         : (code == 2    ? k_refine_tc<2, false, false>
-                            : code == 10 ? k_refine_tc<2, true, false>
-                            : code == 12 ? k_refine_tc<4, true, false>
-                                         : k_refine_tc<4, false, false>);
-    const int epi = (code & 7) == 2 ? 2 : 4;
+    auto kern = s->dense ? k_refine_tc<true> : k_refine_tc<false>;
     HJ_TRY(ensure_smem(kern, smem));
     TcArgs a{};
-    a.blocks = blocks; a.nblocks = nblocks; a.head = head;
-    a.perm = ix->perm; a.cell_lid = ix->cell_lid; a.cell_start = ix->cell_start; a.nC = ix->nC; a.grid = ix->grid;
+    a.blocks = blocks; a.nblocks = nblocks; a.parts = tc_parts(nblocks); a.head = head;
+    a.perm = ix->perm;
+    if (sym) HJ_TRY(flagged_perm(ix, &a.perm, st));
+    a.cell_lid = ix->cell_lid; a.cell_start = ix->cell_start; a.grid = ix->grid;
     a.hash = cell_hash(ix);
-    a.pinfo = reinterpret_cast<const float4*>(ix->tc_err);
-    a.pband = ix->tc_pband;
-    a.n = ix->n; a.nkb = nkb; a.stages = stages;
-    a.thr = (float)s->thr_s;   // exact: thr * 4^s
-    a.gamma_acc = s->gamma_acc;
-    a.s_t = band_s_t(s->thr_s);
-    a.ref_rel = band_ref_rel(ix->d);
+    a.qform = (const uint8_t*)ix->tc_a; a.cform = (const uint8_t*)ix->tc_b;
+    a.plane = plane_rows(ix->n) * kRowBytes;
+    a.nkb = nkb; a.qcols = qcols; a.stages = stages;
+    a.lo = s->lo;
+    a.sym = sym ? 1u : 0u;
     a.sink = sink; a.band = band;
     a.count_only = count_only; a.block_counts = block_counts; a.stats = stats; a.err = err;
-    a.idesc = tc::idesc_f16(ix->tc_kind == HJ_REFINE_TC_BF16 ? 1u : 0u, kTileRows, kAccCols);
+    a.fmt = ix->tc_kind == HJ_REFINE_TC_BF16 ? 1u : 0u;
     a.wait_cycles = kWaitCycles;
-    unsigned grid = (unsigned)std::min<uint32_t>((uint32_t)num_sms(), nblocks);
-    kern<<<grid, 32 * (1 + kAcc) + 128 * epi, smem, st>>>(s->maps.cand, s->maps.query, a);
+    unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)nblocks * a.parts);
+    kern<<<grid, kThreads, smem, st>>>(a);
     HJ_LAUNCHED();
     return HJ_OK;
 }
 
-hj_status launch_band_recheck(const hj_index* ix, const uint32_t* bq, const uint32_t* bc,
+hj_status launch_band_recheck(hj_index* ix, const uint32_t* bq, const uint32_t* bc,
                               const unsigned long long* band_used, unsigned long long band_cap, const PairSink& sink,
-                              uint32_t nblocks, cudaStream_t st) {
+                              uint32_t nblocks, bool sym, cudaStream_t st) {
     const unsigned grid = recheck_grid(nblocks);
-    k_band_recheck<<<grid, 256, 0, st>>>((const float*)ix->pts, ix->perm, ix->d, (float)ix->thr, bq, bc, band_used,
-                                         band_cap, sink);
+    const uint32_t* perm = ix->perm;
+    if (sym) HJ_TRY(flagged_perm(ix, &perm, st));
+    k_band_recheck<<<grid, 256, 0, st>>>((const float*)ix->pts, perm, ix->d, (float)ix->thr, bq, bc, band_used,
+                                         band_cap, sym ? 1u : 0u, sink);
     HJ_LAUNCHED();
     return HJ_OK;
 }
@@ -1172,26 +1238,47 @@ static hj_status run_tile_probe(hj_index* ix, int kind, uint32_t a0, uint32_t b0
     HJ_TRY(tc_prepare(ix, kind, st));
     TcState* s = tc_state(ix);
     const uint32_t nkb = ix->tc_kpad / 32;
-    size_t smem = 1024 + (size_t)(kProbeQT + 1) * nkb * kKBlockBytes + 64;
+    size_t smem = 1024 + (size_t)nkb * (kProbeQB + kTileRows) * kRowBytes + 64;
     smem = std::max<size_t>(smem, 116 * 1024);
     HJ_TRY(ensure_smem(k_tc_tile_probe, smem));
     Scratch tmp(st);
     uint32_t* err = nullptr;
     HJ_TRY(tmp.alloc(&err, 1));
     HJ_CUDA(cudaMemsetAsync(err, 0, 4, st));
-    k_tc_tile_probe<<<1, kProbeThreads, smem, st>>>(s->maps.cand, s->maps.query, nkb,
+    // the probe's operand forms: its rows only, with plain norms, so its accumulators are
+    // squared distances
+    uint16_t *qf = nullptr, *cf = nullptr;
+    float* origin = nullptr;
+    unsigned int* mx = nullptr;
+    const size_t words = (size_t)kProbeQB * ix->tc_kpad;   // halves per form (512 plane rows)
+    HJ_TRY(tmp.alloc(&qf, words));
+    HJ_TRY(tmp.alloc(&cf, words));
+    HJ_TRY(tmp.alloc(&origin, ix->d));
+    HJ_TRY(tmp.alloc(&mx, kTcMaxima));
+    HJ_TRY(launch_col_min(ix, origin, st));
+    HJ_TRY(launch_prep(ix, kind, origin, s->scale_exp, TcBand{}, 0u, b0, kProbeQB, qf, nullptr, mx, st));
+    HJ_TRY(launch_prep(ix, kind, origin, s->scale_exp, TcBand{}, 0u, a0, kProbeQB, nullptr, cf, mx, st));
+    k_tc_tile_probe<<<1, kProbeThreads, smem, st>>>((const uint8_t*)cf, (const uint8_t*)qf,
+                                               (unsigned long long)kProbeQB * kRowBytes, nkb,
                                                tc::idesc_f16(kind == HJ_REFINE_TC_BF16 ? 1u : 0u, kTileRows, kAccCols),
-                                               a0, b0, d_out, err, skip_mma, wait_cycles);
+                                               d_out, err, skip_mma, wait_cycles);
     HJ_LAUNCHED();
     uint32_t herr = 0;
     HJ_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
-    if (h_query_rows)
-        HJ_CUDA(cudaMemcpyAsync(h_query_rows, (const uint16_t*)ix->tc_a + (size_t)b0 * ix->tc_kpad,
-                                (size_t)std::min<uint32_t>(kProbeQB, ix->n - b0) * ix->tc_kpad * 2, cudaMemcpyDeviceToHost, st));
-    if (h_cand_rows)
-        HJ_CUDA(cudaMemcpyAsync(h_cand_rows, (const uint16_t*)ix->tc_b + (size_t)a0 * ix->tc_kpad,
-                                (size_t)std::min<uint32_t>(kTileRows, ix->n - a0) * ix->tc_kpad * 2,
-                                cudaMemcpyDeviceToHost, st));
+    // rows back in row order: out[row][kb * 32 + e] from the swizzled planes
+    auto fetch = [&](const uint16_t* form, uint32_t rows, void* out) -> hj_status {
+        std::vector<uint16_t> h(words);
+        HJ_CUDA(cudaMemcpyAsync(h.data(), form, words * 2, cudaMemcpyDeviceToHost, st));
+        HJ_CUDA(cudaStreamSynchronize(st));
+        uint16_t* o = static_cast<uint16_t*>(out);
+        for (uint32_t r = 0; r < rows; ++r)
+            for (uint32_t ch = 0; ch < nkb * 4; ++ch)
+                std::memcpy(o + (size_t)r * ix->tc_kpad + ch * 8,
+                            h.data() + (((size_t)(ch >> 2) * kProbeQB + r) * 4 + ((ch & 3u) ^ ((r >> 1) & 3u))) * 8, 16);
+        return HJ_OK;
+    };
+    if (h_query_rows) HJ_TRY(fetch(qf, std::min<uint32_t>(kProbeQB, ix->n - b0), h_query_rows));
+    if (h_cand_rows) HJ_TRY(fetch(cf, std::min<uint32_t>(kTileRows, ix->n - a0), h_cand_rows));
     HJ_CUDA(cudaStreamSynchronize(st));
     if (herr) { set_error("tensor-core tile probe: a bounded wait expired"); return HJ_ERR_TIMEOUT; }
     return HJ_OK;

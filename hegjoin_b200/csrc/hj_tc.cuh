@@ -1,11 +1,10 @@
-// hj_tc.cuh -- inline-PTX wrappers for mbarriers, TMA and tcgen05 (sm_100a).
+// hj_tc.cuh -- inline-PTX wrappers for mbarriers, bulk copies and tcgen05 (sm_100a).
 //
-// Written from the PTX ISA descriptions of these instructions.  TMA loads are
-// plain tiled loads into this CTA's own shared memory, and tcgen05.commit
-// signals this CTA's own barriers.
+// Written from the PTX ISA descriptions of these instructions.  Bulk copies go
+// into this CTA's own shared memory, and tcgen05.commit signals this CTA's own
+// barriers.
 #pragma once
 
-#include <cuda.h>
 #include <cstdint>
 
 namespace hj {
@@ -13,6 +12,15 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// One lane of the (converged) warp.  Instructions that take warp-uniform operands
+// (bulk copies, MMAs, commits) go under it: under `lane == 0` the compiler cannot
+// tell that one thread is left and serialises over the warp's active threads.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
 }
 
 // ---- mbarrier -----------------------------------------------------------------------
@@ -61,38 +69,32 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Bounded wait: gives up after ~`limit_cycles` SM cycles or when *abort is
+// Bounded wait: gives up after ~`limit_cycles` SM cycles or as soon as *abort is
 // raised by another role, records the timeout in *err and returns false.
 template <bool kSleep = true>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort,
                                           uint32_t* err, long long limit_cycles) {
     if (mbar_try_wait<kSleep>(bar, parity)) return true;
-    long long t0 = clock64();
-    uint32_t spins = 0;
+    const long long t0 = clock64();
     while (true) {
+        if (*abort) return false;
         if (mbar_try_wait<kSleep>(bar, parity)) return true;
-        if ((++spins & 255u) == 0) {
-            if (*abort) return false;
-            if (clock64() - t0 > limit_cycles) {
-                *abort = 1u;
-                atomicExch(err, 1u);
-                return false;
-            }
+        if (clock64() - t0 > limit_cycles) {
+            *abort = 1u;
+            atomicExch(err, 1u);
+            return false;
         }
     }
 }
 
-// ---- TMA ------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
-}
-// 2-D tiled load; x is the inner (element) coordinate, y the row.
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-        : "memory");
+// ---- bulk copies (TMA) ----------------------------------------------------------------
+// Contiguous bulk copy global -> this CTA's shared memory (16-byte aligned
+// addresses, a multiple of 16 bytes), completing on `bar`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
 }
 
 // ---- tcgen05 --------------------------------------------------------------------------
@@ -127,44 +129,35 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 }
 
 // 32 lanes x 32 columns of 32-bit accumulators: thread t of the warp gets lane
-// (base lane + t), columns [col, col + 32).  The outputs are float registers
-// (a .b32 destination takes any 32-bit register), so no copies follow the load.
-__device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, float (&v)[32]) {
+// (base lane + t), columns [col, col + 32).  The registers hold the values only
+// after tmem_wait_32, which takes and returns them so that no use can move
+// before it; other work may go in between.
+__device__ __forceinline__ void tmem_ld_32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
         "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
-          "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
-          "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
-          "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr)
         : "memory");
 }
-// 32 lanes x 64 columns: thread t gets lane (base lane + t), columns [col, col + 64).
-__device__ __forceinline__ void tmem_ld_32x64(uint32_t taddr, float (&v)[64]) {
+// Waits for every tcgen05.ld of this thread so far.
+__device__ __forceinline__ void tmem_wait_32(uint32_t (&v)[32]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
-        "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
-        "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
-          "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
-          "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
-          "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31]),
-          "=f"(v[32]), "=f"(v[33]), "=f"(v[34]), "=f"(v[35]), "=f"(v[36]), "=f"(v[37]), "=f"(v[38]), "=f"(v[39]),
-          "=f"(v[40]), "=f"(v[41]), "=f"(v[42]), "=f"(v[43]), "=f"(v[44]), "=f"(v[45]), "=f"(v[46]), "=f"(v[47]),
-          "=f"(v[48]), "=f"(v[49]), "=f"(v[50]), "=f"(v[51]), "=f"(v[52]), "=f"(v[53]), "=f"(v[54]), "=f"(v[55]),
-          "=f"(v[56]), "=f"(v[57]), "=f"(v[58]), "=f"(v[59]), "=f"(v[60]), "=f"(v[61]), "=f"(v[62]), "=f"(v[63])
-        : "r"(taddr)
+        "tcgen05.wait::ld.sync.aligned;"
+        : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+          "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+          "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+          "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+        :
         : "memory");
 }
-
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor for a K-major operand stored as rows of 64
-// bytes (32 half-precision elements) with the 64-byte swizzle TMA writes:
+// bytes (32 half-precision elements) with the 64-byte swizzle:
 // 8-row groups are 512 bytes apart (stride byte offset); the leading byte
 // offset is not used by swizzled K-major layouts.
 __device__ __forceinline__ uint64_t desc_kmajor_sw64(uint32_t saddr) {
