@@ -520,7 +520,38 @@ void free_index(hj_index* ix, cudaStream_t st) {
     dfree(ix->perm_flag, st);
 }
 
+// Marks the points of silent cells (a coordinate of 0) in bit 31 of a copy of perm.
+__global__ void k_flag_silent(const unsigned long long* __restrict__ cell_lid, const uint32_t* __restrict__ cell_start,
+                              uint32_t nC, HjGrid g, uint32_t* __restrict__ perm) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nC) return;
+    unsigned long long L = cell_lid[i];
+    bool silent = false;
+    for (uint32_t j = 0; j < g.k; ++j) {
+        const unsigned long long q = L / g.n_cells[j];
+        silent |= L == q * g.n_cells[j];
+        L = q;
+    }
+    if (!silent) return;
+    for (uint32_t p = cell_start[i]; p < cell_start[i + 1]; ++p) perm[p] |= 0x80000000u;
+}
+
 }  // namespace
+
+hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st) {
+    *out = ix->perm;
+    if (!ix->any_silent) return HJ_OK;
+    if (!ix->perm_flag) {
+        uint32_t* p = nullptr;
+        HJ_TRY(dalloc(&p, ix->n, st));
+        ix->perm_flag = p;
+        HJ_CUDA(cudaMemcpyAsync(p, ix->perm, (size_t)ix->n * 4, cudaMemcpyDeviceToDevice, st));
+        k_flag_silent<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->nC, ix->grid, p);
+        HJ_LAUNCHED();
+    }
+    *out = ix->perm_flag;
+    return HJ_OK;
+}
 
 hj_status build_blocks(const hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
                        cudaStream_t st) {

@@ -102,6 +102,14 @@ void init_memory_pool();
 // hj_refine_tc.cu
 void tc_release(hj_index* ix);
 
+// Largest d of the warp-per-item exact refine (hj_refine_warp.cu).
+constexpr int kWarpMaxD32 = 12;
+constexpr int kWarpMaxD64 = 8;
+
+// perm with the points of silent cells marked (bit 31), for the refines' symmetric
+// form; the index's own perm where no cell is silent.
+hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st);
+
 // hj_index.cu
 // Work items of up to qb queries per cell, in the workload order; `align` (a
 // power of two): a cell's items after its first start at multiples of it and

@@ -35,10 +35,18 @@
 
 namespace hj {
 uint32_t plain_query_block(int dtype);
-bool plain_counts_queries(const hj_index* ix);
 hj_status launch_refine_plain(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                               const PairSink& sink, uint32_t count_only, unsigned long long* block_counts,
-                              uint32_t* qcount, cudaStream_t st);
+                              cudaStream_t st);
+bool warp_refine_supported(const hj_index* ix);
+uint32_t warp_query_block(uint32_t n);
+uint64_t warp_chunk_slack(uint32_t nblocks, double avg);
+hj_status launch_refine_warp(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
+                             const PairSink& sink, uint32_t count_only, bool sym, unsigned long long* block_counts,
+                             uint32_t* qcount, cudaStream_t st);
+hj_status launch_refine_digest(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
+                               uint32_t* d_count, unsigned long long* d_sum, unsigned long long* d_xor,
+                               unsigned long long* total, cudaStream_t st);
 hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st);
 uint32_t tc_query_block(const hj_index* ix);
 hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
@@ -70,12 +78,20 @@ struct hj_result {
 namespace hj {
 namespace {
 
+// The estimator's sample: every stride-th work item, of each at most max_q queries
+// (the estimate is a rate per query).
 __global__ void k_pick_samples(const HjBlock* __restrict__ blocks, uint32_t nblocks, uint32_t stride,
-                               uint32_t nsamp, HjBlock* __restrict__ out) {
+                               uint32_t nsamp, uint32_t max_q, HjBlock* __restrict__ out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nsamp) return;
-    out[i] = blocks[min(nblocks - 1, i * stride)];
+    HjBlock b = blocks[min(nblocks - 1, i * stride)];
+    b.q1 = min(b.q1, b.q0 + max_q);
+    out[i] = b;
 }
+
+// Queries per sampled item of the warp refine, whose cost is queries x candidates
+// (the tensor-core filter's is candidate tiles: it takes whole items).
+constexpr uint32_t kSampleQueries = 8;
 
 // Estimated pairs per work item, on the device: the sampled rate (pairs per
 // query) of the item's sample group, or the larger of its group's and the next
@@ -691,6 +707,13 @@ struct EventPairs {
     }
 };
 
+// Per-query digest arrays of a join (hj_result_digest's values, added up).
+struct DigestOut {
+    uint32_t* count = nullptr;
+    unsigned long long* sum = nullptr;
+    unsigned long long* xr = nullptr;
+};
+
 // What a join does with each grouped batch.
 struct BatchHandler {
     virtual ~BatchHandler() = default;
@@ -706,6 +729,8 @@ struct BatchHandler {
     // (if any) after which the last batch's set may be reused.
     virtual bool can_overlap() const { return false; }
     virtual cudaEvent_t take_release() { return nullptr; }
+    // Whether all that is wanted are digests (into *out), not the batches.
+    virtual bool digest_only(DigestOut*) const { return false; }
 };
 
 // The batched join (distanceTableNDGridBatches, GPU.cu:787-1702): refine kind,
@@ -754,8 +779,9 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         if (tc) S.filter_delta = tc_delta(ix);
     }
     S.refine_used = (uint32_t)refine;
+    const bool warp = !tc && warp_refine_supported(ix);   // exact: an item per warp, or block-tiled
     // the tile shape of each refine kernel fixes its work-item size
-    const uint32_t qb = tc ? tc_query_block(ix) : plain_query_block(ix->dtype);
+    const uint32_t qb = tc ? tc_query_block(ix) : warp ? warp_query_block(ix->n) : plain_query_block(ix->dtype);
 
     HjBlock* blocks = nullptr;
     uint32_t nblocks = 0;
@@ -794,6 +820,9 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             tmp.release(cell);
         }
     }
+    const double avg_work = (double)ix->total_candidates / std::max<uint32_t>(1, nblocks);   // pairs evaluated per item
+    // items hold 8 queries on average: enough for the digest kernel, whose lanes are queries
+    const bool crowded = (uint64_t)ix->n >= 8ull * nblocks;
     if (opts.shard_count > 1) {
         // the item list on the host, for the costs of the share
         std::vector<HjBlock> hblocks(nblocks);
@@ -850,7 +879,8 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         }
         HJ_TRY(tc ? launch_refine_tc(ix, blk, nb, head, sink, band, count_only, sym, bc,
                                      count_only ? nullptr : &ctl->tc_acc, &ctl->timeout, st)
-                  : launch_refine_plain(ix, blk, nb, head, sink, count_only, bc, qcount, st));
+               : warp ? launch_refine_warp(ix, blk, nb, avg_work, head, sink, count_only, sym, bc, qcount, st)
+                      : launch_refine_plain(ix, blk, nb, head, sink, count_only, bc, st));
         if (!count_only) HJ_CUDA(cudaEventRecord(e1, st));
         return HJ_OK;
     };
@@ -864,6 +894,32 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         }
         return HJ_OK;
     };
+
+    // ---- digests that nobody wants the pairs of: one launch, no estimate, no batches.  Only
+    // without limits on buffers and batches, which such a join would never meet.
+    DigestOut dig;
+    if (warp && crowded && !opts.result_capacity && !opts.device_bytes_cap && !opts.max_batches &&
+        handler.digest_only(&dig)) {
+        S.ms_setup = ms_since(t_start);
+        kev.ev.emplace_back(nullptr, nullptr);
+        HJ_TRY(event_acquire(&kev.ev[0].first));
+        HJ_TRY(event_acquire(&kev.ev[0].second));
+        HJ_CUDA(cudaEventRecord(kev.ev[0].first, st));
+        HJ_TRY(launch_refine_digest(ix, blocks, nblocks, avg_work, head, dig.count, dig.sum, dig.xr, &ctl->valid, st));
+        HJ_CUDA(cudaEventRecord(kev.ev[0].second, st));
+        JoinCtl hc;
+        HJ_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
+        HJ_CUDA(cudaStreamSynchronize(st));
+        HJ_CUDA(cudaEventElapsedTime(&S.ms_refine_kernel, kev.ev[0].first, kev.ev[0].second));
+        S.total_pairs = S.estimated_pairs = hc.valid;
+        S.n_batches = nblocks ? 1 : 0;
+        S.refine_launches = nblocks ? 1 : 0;
+        S.ms_total = ms_since(t_start);
+        S.ms_refine = S.ms_total - S.ms_setup;
+        S.kernel_launches = (uint32_t)(thread_launch_count() - launches0);
+        if (stats) *stats = S;
+        return HJ_OK;
+    }
 
     // ---- estimator (GPUBatchEst_v2, GPU.cu:403-779)
     auto t_est = std::chrono::steady_clock::now();
@@ -890,12 +946,13 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         HJ_TRY(tmp.alloc(&sblocks, nsamp));
         HJ_TRY(tmp.alloc(&scnt, nsamp));
         HJ_CUDA(cudaMemsetAsync(scnt, 0, nsamp * sizeof(unsigned long long), st));
-        k_pick_samples<<<(nsamp + 255) / 256, 256, 0, st>>>(blocks, nblocks, stride, nsamp, sblocks);
+        k_pick_samples<<<(nsamp + 255) / 256, 256, 0, st>>>(blocks, nblocks, stride, nsamp,
+                                                           warp ? kSampleQueries : 0x7FFFFFFFu, sblocks);
         HJ_LAUNCHED();
         PairSink none{nullptr, nullptr, nullptr, 0, overflow};
         int tuned = 0;
         const std::string key = tune_key(refine, ix->d, ix->dtype);
-        if (!tc && nsamp >= 16 && !tune_lookup(key, &tuned) && tuning_enabled()) {
+        if (!tc && !warp && nsamp >= 16 && !tune_lookup(key, &tuned) && tuning_enabled()) {
             // the exact refine's two tile shapes, timed on the sample (each run twice, the
             // faster run kept: the first run of a shape also pays its one-time setup); the
             // last run's counts are the estimate, and they are the same for either shape
@@ -948,7 +1005,9 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     // ---- result buffer capacity
     // slack for partly filled warp chunks: every warp that can emit during a batch holds
     // at most one (sized from the launch grids, so small joins get small buffers)
-    const uint64_t chunk_slack = (tc ? tc_emit_warps(nblocks) : plain_emit_warps(nblocks)) * kSinkChunk;
+    const uint64_t chunk_slack = tc     ? tc_emit_warps(nblocks) * kSinkChunk
+                                 : warp ? warp_chunk_slack(nblocks, avg_work)
+                                        : plain_emit_warps(nblocks) * kSinkChunk;
     // keys, vals, their grouped copies (+ band pair ids; + a second set of grouped copies)
     const bool overlap = opts.stream_overlap && handler.can_overlap();
     const uint32_t base_words = tc ? 6u : 4u;
@@ -1047,10 +1106,6 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     cudaEvent_t release[2] = {nullptr, nullptr};   // a sink's events: the set is still being read
     uint32_t* qoff = nullptr;   // per-query counters, then first slots, of the grouping
     HJ_TRY(tmp.alloc(&qoff, (size_t)ix->n + 1));
-    // the exact refine counts each query's pairs itself when every item takes its block path
-    // (no warp path below k = 4): the grouping then skips its counting pass
-    const bool fused_counts = !tc && plain_counts_queries(ix);
-
     auto t_ref = std::chrono::steady_clock::now();
     float ms_group = 0;
     uint64_t total = 0;
@@ -1067,10 +1122,13 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         HJ_LAUNCHED();
         PairSink sink{keys, vals, &ctl->cursor, cap, overflow};
         PairSink band = tc ? PairSink{band_q, band_c, &ctl->band_cursor, cap, overflow} : no_band;
-        if (fused_counts) HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
         // all items of the join in this one batch: every unordered pair once (a query's pairs
         // must lie in one batch, and a shard owns its queries' pairs only)
-        const bool sym = tc && opts.shard_count <= 1 && b.b0 == 0 && b.b1 == nblocks;
+        const bool sym = (tc || warp) && opts.shard_count <= 1 && b.b0 == 0 && b.b1 == nblocks;
+        // otherwise the warp refine counts each query's pairs itself: the grouping then skips its
+        // counting pass
+        const bool fused_counts = warp && !sym;
+        if (fused_counts) HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
         HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, fused_counts ? qoff : nullptr,
                           sym));
         if (tc) HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, st));
@@ -1224,6 +1282,11 @@ struct StreamHandler : BatchHandler {
         return HJ_OK;
     }
     bool can_overlap() const override { return sink != nullptr; }
+    bool digest_only(DigestOut* o) const override {
+        if (sink || !cnt) return false;
+        *o = DigestOut{cnt, sum, xr};
+        return true;
+    }
     cudaEvent_t take_release() override {
         cudaEvent_t e = last_release;
         last_release = nullptr;

@@ -807,22 +807,6 @@ __global__ void __launch_bounds__(kPrepRows)
     }
 }
 
-// Marks the points of silent cells (a coordinate of 0) in bit 31 of a copy of perm.
-__global__ void k_flag_silent(const unsigned long long* __restrict__ cell_lid, const uint32_t* __restrict__ cell_start,
-                              uint32_t nC, HjGrid g, uint32_t* __restrict__ perm) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nC) return;
-    unsigned long long L = cell_lid[i];
-    bool silent = false;
-    for (uint32_t j = 0; j < g.k; ++j) {
-        const unsigned long long q = L / g.n_cells[j];
-        silent |= L == q * g.n_cells[j];
-        L = q;
-    }
-    if (!silent) return;
-    for (uint32_t p = cell_start[i]; p < cell_start[i + 1]; ++p) perm[p] |= 0x80000000u;
-}
-
 // Per-dimension minimum of the points: lanes walk a row's dimensions (coalesced
 // reads), warps stride over rows, one atomic per (block, dimension).
 __global__ void k_col_min(const float* __restrict__ pts, uint32_t n, uint32_t d, float* __restrict__ out) {
@@ -1161,23 +1145,6 @@ hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st) {
 void tc_set_dense(hj_index* ix, bool dense) {
     TcState* s = tc_state(ix);
     if (s) s->dense = dense;
-}
-
-// perm with the points of silent cells marked (bit 31), for the symmetric form;
-// the index's own perm where no cell is silent.
-static hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st) {
-    *out = ix->perm;
-    if (!ix->any_silent) return HJ_OK;
-    if (!ix->perm_flag) {
-        uint32_t* p = nullptr;
-        HJ_TRY(dalloc(&p, ix->n, st));
-        ix->perm_flag = p;
-        HJ_CUDA(cudaMemcpyAsync(p, ix->perm, (size_t)ix->n * 4, cudaMemcpyDeviceToDevice, st));
-        k_flag_silent<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->nC, ix->grid, p);
-        HJ_LAUNCHED();
-    }
-    *out = ix->perm_flag;
-    return HJ_OK;
 }
 
 // sym: blocks[0..nblocks) is the join's whole list, each unordered pair once.
