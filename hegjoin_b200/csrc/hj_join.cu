@@ -37,7 +37,7 @@ namespace hj {
 uint32_t plain_query_block(int dtype);
 hj_status launch_refine_plain(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                               const PairSink& sink, uint32_t count_only, unsigned long long* block_counts,
-                              cudaStream_t st);
+                              uint32_t* qcount, cudaStream_t st);
 bool warp_refine_supported(const hj_index* ix);
 uint32_t warp_query_block(uint32_t n);
 uint64_t warp_chunk_slack(uint32_t nblocks, double avg);
@@ -51,11 +51,12 @@ hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st);
 uint32_t tc_query_block(const hj_index* ix);
 hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                            const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
-                           unsigned long long* block_counts, unsigned long long* stats, uint32_t* err,
-                           cudaStream_t st);
+                           unsigned long long* block_counts, unsigned long long* stats, uint32_t* qcount,
+                           uint32_t* err, cudaStream_t st);
 hj_status launch_band_recheck(hj_index* ix, const uint32_t* bq, const uint32_t* bc,
                               const unsigned long long* band_used, unsigned long long band_cap,
-                              const PairSink& sink, uint32_t nblocks, bool sym, cudaStream_t st);
+                              const PairSink& sink, uint32_t nblocks, bool sym, uint32_t* qcount,
+                              cudaStream_t st);
 uint64_t plain_emit_warps(uint32_t nblocks);
 uint64_t tc_emit_warps(uint32_t nblocks);
 double tc_delta(const hj_index* ix);
@@ -186,70 +187,29 @@ __global__ void k_batch_reset(JoinCtl* c) {
     }
 }
 
-// Grouping a batch's pairs by query id: a counting sort.  Keys are query ids
-// below n (sentinel slots are skipped), so one pass counts the pairs per query,
-// an exclusive scan over the n + 1 counters gives every query's first slot, and
-// one more pass scatters each pair to its query's run.  Within a query the order
-// of its pairs is not defined, as in the reference (whose key sort is unstable).
+// Grouping a batch's pairs by query id: a counting sort.  The refine has counted
+// each query's pairs (one add per run of pairs where it writes runs), a scan gives
+// every query's first slot, and one pass scatters the pairs to their query's run.
+// Within a query the order of its pairs is not defined, as in the reference (whose
+// key sort is unstable).
 //
-// Both passes work on tiles of 4,096 consecutive pairs per block.  A tile comes
-// mostly from one or two work items, so it holds a few dozen distinct queries:
-// the block gathers them in a shared-memory table (key -> slot, open addressing;
-// lanes of a warp with the same key share one table operation) and issues one
-// global atomic per query per tile instead of one per query per warp.  Keys
-// that find the table full take their global atomics directly.
-constexpr uint32_t kGrpPer = 16;                       // pairs per thread per tile
+// A warp takes 32 consecutive pairs at a time; lanes with the same query share one
+// cursor atomic.  The refine writes a query's hits as runs of up to 64, so that is
+// about one atomic per run; the reversed orders of its symmetric form have keys of
+// their own each.  Eight steps are in flight per thread: the pass is bound by the
+// latency and rate of the atomics and by the scattered 4-byte stores (skewed 6-D,
+// 314M pairs; a shared-memory table of 1,024 keys per 4,096 pairs, which the
+// reversed orders overfill, took 8.9 ms and a counting pass 2.3 ms before it).
+// keys_out may be null (a result whose keys nobody asked for).
+constexpr uint32_t kGrpPer = 8;                        // pairs per thread
 constexpr uint32_t kGrpTile = 256 * kGrpPer;           // pairs per block-tile
-constexpr uint32_t kGrpSlots = 1024;                   // table slots (power of two)
-constexpr uint32_t kGrpFull = 0xFFFFFFFFu;
-
-// Slot of `key` in the block's table (inserting it), or kGrpFull.
-__device__ __forceinline__ uint32_t grp_slot(uint32_t* hk, uint32_t key) {
-    uint32_t h = (uint32_t)mix64(key) & (kGrpSlots - 1);
-    for (uint32_t probe = 0; probe < 64; ++probe) {
-        const uint32_t prev = atomicCAS(&hk[h], kSentinelKey, key);
-        if (prev == kSentinelKey || prev == key) return h;
-        h = (h + 1) & (kGrpSlots - 1);
-    }
-    return kGrpFull;
-}
-
-__global__ void __launch_bounds__(256) k_group_count(const uint32_t* __restrict__ keys, unsigned long long m,
-                                                      uint32_t* __restrict__ cnt) {
-    __shared__ uint32_t hk[kGrpSlots], hc[kGrpSlots];
-    for (unsigned long long base = (unsigned long long)blockIdx.x * kGrpTile; base < m;
-         base += (unsigned long long)gridDim.x * kGrpTile) {
-        for (uint32_t s = threadIdx.x; s < kGrpSlots; s += blockDim.x) { hk[s] = kSentinelKey; hc[s] = 0; }
-        __syncthreads();
-#pragma unroll 4
-        for (uint32_t j = 0; j < kGrpPer; ++j) {
-            const unsigned long long i = base + j * 256ull + threadIdx.x;
-            const uint32_t key = i < m ? keys[i] : kSentinelKey;
-            const uint32_t peers = __match_any_sync(0xffffffffu, key);
-            if (key != kSentinelKey && lane_id() == (uint32_t)(__ffs(peers) - 1)) {
-                const uint32_t sl = grp_slot(hk, key);
-                if (sl == kGrpFull) atomicAdd(&cnt[key], __popc(peers));
-                else atomicAdd(&hc[sl], __popc(peers));
-            }
-        }
-        __syncthreads();
-        for (uint32_t s = threadIdx.x; s < kGrpSlots; s += blockDim.x)
-            if (hk[s] != kSentinelKey) atomicAdd(&cnt[hk[s]], hc[s]);
-        __syncthreads();
-    }
-}
-
 __global__ void __launch_bounds__(256) k_group_scatter(const uint32_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ vals, unsigned long long m,
                                                         uint32_t* __restrict__ cursor, uint32_t* __restrict__ keys_out,
                                                         uint32_t* __restrict__ vals_out) {
-    __shared__ uint32_t hk[kGrpSlots], hc[kGrpSlots];
     for (unsigned long long base = (unsigned long long)blockIdx.x * kGrpTile; base < m;
          base += (unsigned long long)gridDim.x * kGrpTile) {
-        for (uint32_t s = threadIdx.x; s < kGrpSlots; s += blockDim.x) { hk[s] = kSentinelKey; hc[s] = 0; }
-        __syncthreads();
-        // pass 1: the tile's pairs per query (the thread keeps its keys and values)
-        uint32_t kk[kGrpPer], vv[kGrpPer];
+        uint32_t kk[kGrpPer], vv[kGrpPer], peers[kGrpPer], at[kGrpPer];
 #pragma unroll
         for (uint32_t j = 0; j < kGrpPer; ++j) {
             const unsigned long long i = base + j * 256ull + threadIdx.x;
@@ -258,45 +218,18 @@ __global__ void __launch_bounds__(256) k_group_scatter(const uint32_t* __restric
         }
 #pragma unroll
         for (uint32_t j = 0; j < kGrpPer; ++j) {
-            const uint32_t key = kk[j];
-            const uint32_t peers = __match_any_sync(0xffffffffu, key);
-            if (key != kSentinelKey && lane_id() == (uint32_t)(__ffs(peers) - 1)) {
-                const uint32_t sl = grp_slot(hk, key);
-                if (sl != kGrpFull) atomicAdd(&hc[sl], __popc(peers));
-            }
+            peers[j] = __match_any_sync(0xffffffffu, kk[j]);
+            at[j] = 0;
+            if (kk[j] != kSentinelKey && (peers[j] & lanemask_lt()) == 0u)
+                at[j] = atomicAdd(&cursor[kk[j]], __popc(peers[j]));
         }
-        __syncthreads();
-        // one global reservation per query of the tile; the slot's count becomes its cursor
-        for (uint32_t s = threadIdx.x; s < kGrpSlots; s += blockDim.x)
-            if (hk[s] != kSentinelKey) hc[s] = atomicAdd(&cursor[hk[s]], hc[s]);
-        __syncthreads();
-        // pass 2: place the pairs
 #pragma unroll
         for (uint32_t j = 0; j < kGrpPer; ++j) {
-            const uint32_t key = kk[j];
-            const uint32_t peers = __match_any_sync(0xffffffffu, key);
-            const uint32_t leader = __ffs(peers) - 1;
-            uint32_t first = 0;
-            if (key != kSentinelKey && lane_id() == leader) {
-                uint32_t sl = kGrpFull;
-                // the key is in the table unless the table was full when it came
-                uint32_t h = (uint32_t)mix64(key) & (kGrpSlots - 1);
-                for (uint32_t probe = 0; probe < 64; ++probe) {
-                    const uint32_t k2 = hk[h];
-                    if (k2 == key) { sl = h; break; }
-                    if (k2 == kSentinelKey) break;
-                    h = (h + 1) & (kGrpSlots - 1);
-                }
-                first = sl != kGrpFull ? atomicAdd(&hc[sl], __popc(peers)) : atomicAdd(&cursor[key], __popc(peers));
-            }
-            first = __shfl_sync(0xffffffffu, first, leader);
-            if (key != kSentinelKey) {
-                const uint32_t pos = first + __popc(peers & lanemask_lt());
-                keys_out[pos] = key;
-                vals_out[pos] = vv[j];
-            }
+            const uint32_t pos = __shfl_sync(0xffffffffu, at[j], __ffs(peers[j]) - 1) + __popc(peers[j] & lanemask_lt());
+            if (kk[j] == kSentinelKey) continue;
+            vals_out[pos] = vv[j];
+            if (keys_out) keys_out[pos] = kk[j];
         }
-        __syncthreads();
     }
 }
 
@@ -717,8 +650,17 @@ struct DigestOut {
 // What a join does with each grouped batch.
 struct BatchHandler {
     virtual ~BatchHandler() = default;
+    // Where a batch of `count` pairs is grouped to: arrays of the handler's own (keys may
+    // stay null if nobody reads them), or the join's (left as they are).
+    virtual hj_status grouped_to(uint64_t /*count*/, uint32_t** /*keys*/, uint32_t** /*vals*/, cudaStream_t) {
+        return HJ_OK;
+    }
+    // Whether grouped_to always gives arrays of the handler's own.
+    virtual bool own_arrays() const { return false; }
+    // After the last batch, before the join synchronises `st`.
+    virtual hj_status finish(cudaStream_t) { return HJ_OK; }
     // `count` pairs of batch `batch`: query ids (ascending) in keys, neighbour ids
-    // grouped by query in vals.  Both live in the join's reusable buffers and stay
+    // grouped by query in vals, in the arrays of grouped_to; the join's own stay
     // valid in the order of `st` until the next batch's refine is enqueued.  With
     // pairs, run_end (n entries, in the order of `st` until the next batch's grouping)
     // holds one past each query's last pair: query q's run is
@@ -878,9 +820,9 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             HJ_CUDA(cudaEventRecord(e0, st));
         }
         HJ_TRY(tc ? launch_refine_tc(ix, blk, nb, head, sink, band, count_only, sym, bc,
-                                     count_only ? nullptr : &ctl->tc_acc, &ctl->timeout, st)
+                                     count_only ? nullptr : &ctl->tc_acc, qcount, &ctl->timeout, st)
                : warp ? launch_refine_warp(ix, blk, nb, avg_work, head, sink, count_only, sym, bc, qcount, st)
-                      : launch_refine_plain(ix, blk, nb, head, sink, count_only, bc, st));
+                      : launch_refine_plain(ix, blk, nb, head, sink, count_only, bc, qcount, st));
         if (!count_only) HJ_CUDA(cudaEventRecord(e1, st));
         return HJ_OK;
     };
@@ -1008,10 +950,11 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     const uint64_t chunk_slack = tc     ? tc_emit_warps(nblocks) * kSinkChunk
                                  : warp ? warp_chunk_slack(nblocks, avg_work)
                                         : plain_emit_warps(nblocks) * kSinkChunk;
-    // keys, vals, their grouped copies (+ band pair ids; + a second set of grouped copies)
+    // keys, vals (+ band pair ids; + one or two sets of grouped copies unless the handler
+    // brings its own arrays)
     const bool overlap = opts.stream_overlap && handler.can_overlap();
-    const uint32_t base_words = tc ? 6u : 4u;
-    const uint32_t slot_words = base_words + (overlap ? 2u : 0u);
+    const uint32_t base_words = tc ? 4u : 2u;
+    const uint32_t slot_words = base_words + (handler.own_arrays() ? 0u : overlap ? 4u : 2u);
     const double bytes_per_slot = 4.0 * slot_words;
     const uint64_t want = (uint64_t)(total_est * 2.0) + chunk_slack + 4096;
     uint64_t cap = opts.result_capacity ? opts.result_capacity + chunk_slack : want;
@@ -1084,7 +1027,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     }
     std::reverse(batches.begin(), batches.end());   // used as a stack
 
-    // one allocation carved into keys, vals, their radix copies and the band pair ids;
+    // one allocation carved into keys, vals, the band pair ids and the grouped copies;
     // when the free-memory query was skipped and the allocation fails, query and retry smaller
     uint32_t* slab = nullptr;
     hj_status as = tmp.alloc(&slab, cap * slot_words);
@@ -1097,12 +1040,11 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         }
     }
     HJ_TRY(as);
-    uint32_t *keys = slab, *vals = slab + cap, *keys_tmp = slab + 2 * cap, *vals_tmp = slab + 3 * cap;
-    uint32_t* band_q = tc ? slab + 4 * cap : nullptr;
-    uint32_t* band_c = tc ? slab + 5 * cap : nullptr;
+    uint32_t *keys = slab, *vals = slab + cap;
+    uint32_t* band_q = tc ? slab + 2 * cap : nullptr;
+    uint32_t* band_c = tc ? slab + 3 * cap : nullptr;
     // the grouped copies, one set per batch parity with stream_overlap
-    uint32_t* grp_keys[2] = {keys_tmp, overlap ? slab + (size_t)base_words * cap : keys_tmp};
-    uint32_t* grp_vals[2] = {vals_tmp, overlap ? slab + (size_t)(base_words + 1) * cap : vals_tmp};
+    uint32_t* const copies = slab + (size_t)base_words * cap;
     cudaEvent_t release[2] = {nullptr, nullptr};   // a sink's events: the set is still being read
     uint32_t* qoff = nullptr;   // per-query counters, then first slots, of the grouping
     HJ_TRY(tmp.alloc(&qoff, (size_t)ix->n + 1));
@@ -1125,13 +1067,14 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         // all items of the join in this one batch: every unordered pair once (a query's pairs
         // must lie in one batch, and a shard owns its queries' pairs only)
         const bool sym = (tc || warp) && opts.shard_count <= 1 && b.b0 == 0 && b.b1 == nblocks;
-        // otherwise the warp refine counts each query's pairs itself: the grouping then skips its
-        // counting pass
-        const bool fused_counts = warp && !sym;
-        if (fused_counts) HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
-        HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, fused_counts ? qoff : nullptr,
-                          sym));
-        if (tc) HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, st));
+        HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
+        HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, qoff, sym));
+        if (tc)
+            HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, qoff, st));
+        // every query's first slot; qoff[n] = the batch's pairs
+        HJ_TRY(scan_u32_inplace(qoff, (uint64_t)ix->n + 1, st));
+        uint32_t valid = 0;
+        HJ_CUDA(cudaMemcpyAsync(&valid, qoff + ix->n, 4, cudaMemcpyDeviceToHost, st));
         JoinCtl hc;
         HJ_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
@@ -1156,27 +1099,6 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         S.band_pairs += hc.tc_band;
         auto t_g = std::chrono::steady_clock::now();
         const uint64_t slots = std::min<uint64_t>(used, cap);
-        uint32_t valid = 0;
-        if (slots) {
-            // group by query id: count (unless the refine counted), scan (qoff[n] = the batch's
-            // pairs), scatter into the copies
-            const unsigned g = (unsigned)std::min<uint64_t>((slots + kGrpTile - 1) / kGrpTile, (uint64_t)num_sms() * 8);
-            if (!fused_counts) {
-                HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
-                k_group_count<<<g, 256, 0, st>>>(keys, slots, qoff);
-                HJ_LAUNCHED();
-            }
-            HJ_TRY(scan_u32_inplace(qoff, (uint64_t)ix->n + 1, st));
-            HJ_CUDA(cudaMemcpyAsync(&valid, qoff + ix->n, 4, cudaMemcpyDeviceToHost, st));
-            const int set = overlap ? (int)(n_out & 1u) : 0;
-            if (release[set]) {   // the sink's reads of this set, two batches ago
-                HJ_CUDA(cudaStreamWaitEvent(st, release[set], 0));
-                release[set] = nullptr;
-            }
-            k_group_scatter<<<g, 256, 0, st>>>(keys, vals, slots, qoff, grp_keys[set], grp_vals[set]);
-            HJ_LAUNCHED();
-            HJ_CUDA(cudaStreamSynchronize(st));
-        }
         if (cap_bytes && kept + kept_bytes_per_pair * (double)valid > (double)cap_bytes) {
             // the estimate was low: refuse before the results pass the cap, asking for the
             // results so far extrapolated over the remaining work items (heaviest first, so
@@ -1194,11 +1116,20 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         kept += kept_bytes_per_pair * (double)valid;
         {
             const int set = overlap ? (int)(n_out & 1u) : 0;
-            if (release[set]) {   // an empty batch reuses the set without a scatter
+            if (release[set]) {   // the sink's reads of this set, two batches ago
                 HJ_CUDA(cudaStreamWaitEvent(st, release[set], 0));
                 release[set] = nullptr;
             }
-            HJ_TRY(handler.on_batch(n_out, grp_keys[set], grp_vals[set], valid, valid ? qoff : nullptr, st));
+            uint32_t *gk = copies + (size_t)(2 * set) * cap, *gv = gk + cap;
+            if (handler.own_arrays()) gk = gv = nullptr;
+            HJ_TRY(handler.grouped_to(valid, &gk, &gv, st));
+            if (slots) {
+                const unsigned g =
+                    (unsigned)std::min<uint64_t>((slots + kGrpTile - 1) / kGrpTile, (uint64_t)num_sms() * 8);
+                k_group_scatter<<<g, 256, 0, st>>>(keys, vals, slots, qoff, gk, gv);
+                HJ_LAUNCHED();
+            }
+            HJ_TRY(handler.on_batch(n_out, gk, gv, valid, valid ? qoff : nullptr, st));
             release[set] = handler.take_release();
         }
         ++n_out;
@@ -1207,6 +1138,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     }
     for (cudaEvent_t e : release)
         if (e) HJ_CUDA(cudaStreamWaitEvent(st, e, 0));   // the sink's last reads end before the join does
+    HJ_TRY(handler.finish(st));
     HJ_CUDA(cudaStreamSynchronize(st));
     S.ms_refine = ms_since(t_ref) - ms_group;
     S.ms_group = ms_group;
@@ -1224,31 +1156,37 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     return HJ_OK;
 }
 
-// hj_join: every batch's neighbour ids stay on the device (a copy per batch) and
-// the device neighbour table points into them.
+// hj_join: every batch is grouped into arrays that stay with the result, and the
+// device neighbour table points into them.
 struct RetainHandler : BatchHandler {
     hj_result* res;
     bool keep_keys;
     RetainHandler(hj_result* r, bool kk) : res(r), keep_keys(kk) {}
-    hj_status on_batch(uint32_t bi, const uint32_t* keys, const uint32_t* vals, uint64_t count,
-                       const uint32_t* run_end, cudaStream_t st) override {
-        uint32_t* bv = nullptr;
-        HJ_TRY(dalloc(&bv, count, st));
-        res->vals.push_back(bv);
+    bool own_arrays() const override { return true; }
+    hj_status grouped_to(uint64_t count, uint32_t** keys, uint32_t** vals, cudaStream_t st) override {
+        HJ_TRY(dalloc(vals, count, st));
+        res->vals.push_back(*vals);
         res->counts.push_back(count);
-        if (count) HJ_CUDA(cudaMemcpyAsync(bv, vals, count * 4, cudaMemcpyDeviceToDevice, st));
         if (keep_keys) {
-            uint32_t* bk = nullptr;
-            HJ_TRY(dalloc(&bk, count, st));
-            res->keys.push_back(bk);
-            if (count) HJ_CUDA(cudaMemcpyAsync(bk, keys, count * 4, cudaMemcpyDeviceToDevice, st));
+            HJ_TRY(dalloc(keys, count, st));
+            res->keys.push_back(*keys);
         }
+        return HJ_OK;
+    }
+    hj_status on_batch(uint32_t bi, const uint32_t*, const uint32_t*, uint64_t count, const uint32_t* run_end,
+                       cudaStream_t st) override {
         if (count) {
             k_table_runs<<<(res->n + 255) / 256, 256, 0, st>>>(run_end, res->n, bi, res->table);
             HJ_LAUNCHED();
         }
         res->total += count;
         return HJ_OK;
+    }
+    hj_status finish(cudaStream_t st) override {
+        if (res->vals.empty()) return HJ_OK;
+        HJ_TRY(dalloc(&res->d_batch_vals, res->vals.size(), st));
+        return cuda_status(cudaMemcpyAsync(res->d_batch_vals, res->vals.data(), res->vals.size() * sizeof(uint32_t*),
+                                           cudaMemcpyHostToDevice, st), "batch pointer table");
     }
 };
 
@@ -1380,13 +1318,6 @@ hj_status hj_join(hj_index* ix, const hj_join_opts* opts, void* stream, hj_resul
     RetainHandler h(res, keep_keys);
     hj_join_stats S{};
     if (s == HJ_OK) s = join_impl(ix, opts, st, h, keep_keys ? 8.0 : 4.0, (uint64_t)ix->n * sizeof(hj_nt_entry), &S);
-    if (s == HJ_OK && !res->vals.empty()) {
-        s = dalloc(&res->d_batch_vals, res->vals.size(), st);
-        if (s == HJ_OK)
-            s = cuda_status(cudaMemcpyAsync(res->d_batch_vals, res->vals.data(), res->vals.size() * sizeof(uint32_t*),
-                                            cudaMemcpyHostToDevice, st), "batch pointer table");
-    }
-    if (s == HJ_OK) s = cuda_status(cudaStreamSynchronize(st), "hj_join");
     if (stats) *stats = S;   // on an error: what was known (bytes_wanted when the cap refused)
     if (s != HJ_OK) {
         hj_result_destroy(res);

@@ -50,6 +50,7 @@ struct PlainArgs {
     PairSink sink;
     uint32_t count_only;
     unsigned long long* block_counts;   // count-only mode: pairs per work item
+    uint32_t* qcount;                   // else: pairs per query id, added up
 };
 
 // Packed FP32 pairs (sm_100): each lane's result is the IEEE-rounded scalar
@@ -177,7 +178,10 @@ __device__ __forceinline__ void warp_item(const PlainArgs<T>& a, const HjBlock& 
                     cid_w[lane] = valid ? a.perm[p] : 0u;
                     __syncwarp();
                     warp_emit_masks(a.sink, wc, mask,
-                                    [&](uint32_t owner, uint32_t b) { return make_uint2(qid_w[b], cid_w[owner]); });
+                                    [&](uint32_t owner, uint32_t b) {
+                                        atomicAdd(&a.qcount[qid_w[b]], 1u);
+                                        return make_uint2(qid_w[b], cid_w[owner]);
+                                    });
                     __syncwarp();
                 }
             }
@@ -413,6 +417,7 @@ __global__ void __launch_bounds__(256, 3) k_refine_plain(PlainArgs<T> a) {
                         warp_emit_masks(a.sink, wc, mask, [&](uint32_t owner, uint32_t b) {
                             const uint32_t ot = wbase + owner;
                             const uint32_t qi = (ot / TX) * RQ + b / RC, cj = (ot % TX) * RC + b % RC;
+                            atomicAdd(&a.qcount[qid_s[qi]], 1u);
                             return make_uint2(qid_s[qi], cid_s[cj]);
                         });
                     }
@@ -497,17 +502,17 @@ uint64_t plain_emit_warps(uint32_t nblocks) {
 // zero on entry.  count_only: per-item pair counts go to block_counts.
 hj_status launch_refine_plain(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                               const PairSink& sink, uint32_t count_only, unsigned long long* block_counts,
-                              cudaStream_t st) {
+                              uint32_t* qcount, cudaStream_t st) {
     if (nblocks == 0) return HJ_OK;
     if (ix->dtype == HJ_F32) {
         PlainArgs<float> a{(const float*)ix->pts, ix->perm, ix->cell_lid, ix->cell_start, ix->nC, cell_hash(ix), ix->d,
                            ix->grid,
-                           (float)ix->thr, blocks, nblocks, head, sink, count_only, block_counts};
+                           (float)ix->thr, blocks, nblocks, head, sink, count_only, block_counts, qcount};
         return dispatch_t<float>(a, ix->plain_shape, st);
     }
     PlainArgs<double> a{(const double*)ix->pts, ix->perm, ix->cell_lid, ix->cell_start, ix->nC, cell_hash(ix), ix->d,
                         ix->grid,
-                        ix->thr, blocks, nblocks, head, sink, count_only, block_counts};
+                        ix->thr, blocks, nblocks, head, sink, count_only, block_counts, qcount};
     return dispatch_t<double>(a, ix->plain_shape, st);
 }
 

@@ -112,6 +112,7 @@ struct TcArgs {
     uint32_t count_only;
     unsigned long long* block_counts;
     unsigned long long* stats;  // [0] accepted, [1] band
+    uint32_t* qcount;           // pairs per query id, added up (not in count-only mode)
     uint32_t* err;
     uint32_t fmt;               // operand format of the instruction descriptor (0 FP16, 1 BF16)
     long long wait_cycles;      // bound of every mbarrier wait (SM cycles)
@@ -531,6 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
                         if (self - c * 32u < 32u) self_hit |= (am[c] >> (self - c * 32u)) & 1u;
                     const uint32_t cnt = (fwd ? na : 0u) + (rev ? na - self_hit : 0u);
                     n_acc += cnt;
+                    if (rev && na > self_hit) atomicAdd(&a.qcount[cid], na - self_hit);
                     warp_emit_serial(a.sink, wc_acc, cnt, [&](auto&& put) {
 #pragma unroll
                         for (uint32_t c = 0; c < NCH; ++c) {
@@ -539,7 +541,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
                                 const uint32_t col = c * 32u + __ffs(m) - 1u;
                                 m &= m - 1u;
                                 const uint32_t qid = S.qid[col_base + col];
-                                if (fwd) put(qid, cid);
+                                if (fwd) {
+                                    put(qid, cid);
+                                    atomicAdd(&a.qcount[qid], 1u);
+                                }
                                 if (rev && col != self) put(cid, qid);
                             }
                         }
@@ -597,7 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
 __global__ void k_band_recheck(const float* __restrict__ pts, const uint32_t* __restrict__ perm, uint32_t d,
                                float thr, const uint32_t* __restrict__ bq, const uint32_t* __restrict__ bc,
                                const unsigned long long* __restrict__ band_used, unsigned long long band_cap,
-                               uint32_t sym, PairSink sink) {
+                               uint32_t sym, PairSink sink, uint32_t* __restrict__ qcount) {
     const unsigned long long n = min(*band_used, band_cap);
     WarpChunk wc;
     warp_chunk_init(wc);
@@ -623,6 +628,8 @@ __global__ void k_band_recheck(const float* __restrict__ pts, const uint32_t* __
                     cid = cw & 0x7FFFFFFFu;
                     fwd = !(qw >> 31);
                     rev = sym && !(cw >> 31) && qp != cp;
+                    if (fwd) atomicAdd(&qcount[qid], 1u);
+                    if (rev) atomicAdd(&qcount[cid], 1u);
                 }
             }
         }
@@ -1150,8 +1157,8 @@ void tc_set_dense(hj_index* ix, bool dense) {
 // sym: blocks[0..nblocks) is the join's whole list, each unordered pair once.
 hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                            const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
-                           unsigned long long* block_counts, unsigned long long* stats, uint32_t* err,
-                           cudaStream_t st) {
+                           unsigned long long* block_counts, unsigned long long* stats, uint32_t* qcount,
+                           uint32_t* err, cudaStream_t st) {
     if (nblocks == 0) return HJ_OK;
     TcState* s = tc_state(ix);
     if (!s) { set_error("tensor-core operands not prepared"); return HJ_ERR_INVALID; }
@@ -1173,7 +1180,8 @@ hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     a.lo = s->lo;
     a.sym = sym ? 1u : 0u;
     a.sink = sink; a.band = band;
-    a.count_only = count_only; a.block_counts = block_counts; a.stats = stats; a.err = err;
+    a.count_only = count_only; a.block_counts = block_counts; a.stats = stats;
+    a.qcount = qcount; a.err = err;
     a.fmt = ix->tc_kind == HJ_REFINE_TC_BF16 ? 1u : 0u;
     a.wait_cycles = kWaitCycles;
     unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)nblocks * a.parts);
@@ -1184,12 +1192,12 @@ hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
 
 hj_status launch_band_recheck(hj_index* ix, const uint32_t* bq, const uint32_t* bc,
                               const unsigned long long* band_used, unsigned long long band_cap, const PairSink& sink,
-                              uint32_t nblocks, bool sym, cudaStream_t st) {
+                              uint32_t nblocks, bool sym, uint32_t* qcount, cudaStream_t st) {
     const unsigned grid = recheck_grid(nblocks);
     const uint32_t* perm = ix->perm;
     if (sym) HJ_TRY(flagged_perm(ix, &perm, st));
     k_band_recheck<<<grid, 256, 0, st>>>((const float*)ix->pts, perm, ix->d, (float)ix->thr, bq, bc, band_used,
-                                         band_cap, sym ? 1u : 0u, sink);
+                                         band_cap, sym ? 1u : 0u, sink, qcount);
     HJ_LAUNCHED();
     return HJ_OK;
 }

@@ -34,14 +34,10 @@ static uint32_t warp_parts(uint32_t nblocks, double avg) {
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({64, (want + nb - 1) / nb, by_work}));
 }
 
-// Sink slots a warp reserves at a time: long lists take larger chunks (fewer
-// atomics on the one cursor).
-static uint32_t warp_chunk_slots(uint32_t nblocks) { return nblocks >= 16384 ? 1024u : kSinkChunk; }
-
 // Slots that partly filled chunks can leave unused in one launch.
 uint64_t warp_chunk_slack(uint32_t nblocks, double avg) {
     const uint64_t items = (uint64_t)std::max<uint32_t>(nblocks, 1) * warp_parts(nblocks, avg) + kWarpsPerBlock - 1;
-    return std::min<uint64_t>((uint64_t)kWarpMaxBlocks * kWarpsPerBlock * num_sms(), items) * warp_chunk_slots(nblocks);
+    return std::min<uint64_t>((uint64_t)kWarpMaxBlocks * kWarpsPerBlock * num_sms(), items) * kSinkChunk;
 }
 
 template <typename T>
@@ -60,15 +56,14 @@ static hj_status make_args(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     a->nblocks = nblocks;
     a->parts = warp_parts(nblocks, avg);
     a->sym = sym ? 1u : 0u;
-    a->chunk = warp_chunk_slots(nblocks);
     a->head = head;
     return HJ_OK;
 }
 
 // Runs the refine over work items blocks[0..nblocks).  `head` must be zero on
 // entry.  count_only: per-item pair counts go to block_counts.  sym: the items are
-// the join's whole list, each unordered pair once.  qcount (not with sym): each
-// query's pairs are added to it, by original id.
+// the join's whole list, each unordered pair once.  Each query's pairs are added to
+// qcount, by original id (not with count_only).
 hj_status launch_refine_warp(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
                              const PairSink& sink, uint32_t count_only, bool sym, unsigned long long* block_counts,
                              uint32_t* qcount, cudaStream_t st) {

@@ -61,12 +61,11 @@ struct WarpArgs {
     uint32_t nblocks;
     uint32_t parts;
     uint32_t sym;
-    uint32_t chunk;                   // sink slots a warp reserves at a time
     unsigned int* head;
     PairSink sink;
     uint32_t count_only;
     unsigned long long* block_counts; // count-only mode: pairs per work item
-    uint32_t* qcount;                 // optional (not with sym): pairs per query id, added up
+    uint32_t* qcount;                 // pairs per query id, added up (not in count-only mode)
     // digest kernel
     uint32_t* d_count;
     unsigned long long* d_sum;
@@ -190,7 +189,7 @@ struct WarpSlots {
     unsigned long long p0, p1;
     uint32_t room;
 };
-__device__ __forceinline__ bool warp_slots(const PairSink& s, WarpChunk& c, uint32_t chunk, uint32_t n, WarpSlots& o) {
+__device__ __forceinline__ bool warp_slots(const PairSink& s, WarpChunk& c, uint32_t n, WarpSlots& o) {
     o.p0 = c.base + c.used;
     o.room = c.cap - c.used;
     o.p1 = 0;
@@ -198,7 +197,7 @@ __device__ __forceinline__ bool warp_slots(const PairSink& s, WarpChunk& c, uint
         c.used += n;
         return true;
     }
-    const uint32_t need = (n - o.room + chunk - 1) / chunk * chunk;
+    const uint32_t need = (n - o.room + kSinkChunk - 1) / kSinkChunk * kSinkChunk;
     if (lane_id() == 0) o.p1 = atomicAdd(s.cursor, (unsigned long long)need);
     o.p1 = __shfl_sync(0xffffffffu, o.p1, 0);
     if (o.p1 + need > s.capacity) {
@@ -310,7 +309,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_
                     const uint32_t lt = lanemask_lt();
                     if (!a.sym) {
                         WarpSlots s;
-                        if (!warp_slots(a.sink, wc, a.chunk, n, s)) continue;
+                        if (!warp_slots(a.sink, wc, n, s)) continue;
 #pragma unroll
                         for (int c = 0; c < kWarpC; ++c) {
                             if (!hit[c]) continue;
@@ -328,7 +327,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_
                         const uint32_t r0 = __ballot_sync(0xffffffffu, rev[0]), r1 = __ballot_sync(0xffffffffu, rev[1]);
                         const uint32_t nf = fwd ? n : 0u, m0 = __popc(r0);
                         WarpSlots s;
-                        if (!warp_slots(a.sink, wc, a.chunk, nf + m0 + __popc(r1), s)) continue;
+                        if (!warp_slots(a.sink, wc, nf + m0 + __popc(r1), s)) continue;
 #pragma unroll
                         for (int c = 0; c < kWarpC; ++c) {
                             const uint32_t cid = cw[c] & 0x7FFFFFFFu;
@@ -343,6 +342,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_
                                 const unsigned long long pos = r < s.room ? s.p0 + r : s.p1 + (r - s.room);
                                 a.sink.keys[pos] = cid;
                                 a.sink.vals[pos] = qid;
+                                atomicAdd(&a.qcount[cid], 1u);
                             }
                         }
                     }
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_
         if (a.count_only) {
             const uint32_t t = __reduce_add_sync(0xffffffffu, my_count);
             if (lane == 0 && t) atomicAdd(&a.block_counts[bi], (unsigned long long)t);
-        } else if (a.qcount) {
+        } else if (fwd) {
             if (lane < nq && my_count) atomicAdd(&a.qcount[S.qid[lane]], my_count);
         }
     }
