@@ -213,8 +213,6 @@ hj_status radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp,
                              uint64_t n, uint32_t nbits, cudaStream_t st);
 hj_status radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                              uint64_t n, uint32_t nbits, cudaStream_t st);
-// Sum of n u64 values (device result).
-hj_status reduce_sum_u64(const uint64_t* in, uint64_t n, uint64_t* d_out, cudaStream_t st);
 
 // ---- device helpers -------------------------------------------------------------
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }

@@ -243,57 +243,105 @@ __global__ void k_gather_rows(const T* __restrict__ db, const uint32_t* __restri
 }  // namespace
 
 // Per non-empty cell: number of candidates in its stencil (kernel.cu:74-144).
-// One warp per cell; rows of the stencil (tuples over dimensions 1..k-1) are
-// split over the lanes, each row being one contiguous range of linear ids.
-__global__ void k_cell_workload(const unsigned long long* __restrict__ cell_lid, const uint32_t* __restrict__ cell_start,
-                                uint32_t nC, HjGrid grid, HjCellHash hash, uint32_t* __restrict__ cell_nb,
-                                unsigned long long* __restrict__ cell_work) {
-    uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= nC) return;
-    unsigned long long L = cell_lid[warp];
+// One warp per cell; the rows of the stencil (tuples over dimensions 1..k-1) are
+// split over the lanes, each row being one contiguous range of linear ids.  The
+// stencil is symmetric, so a cell looks only at the cells after it -- half of the
+// rows -- and adds each neighbour's points to its own count and its own points to
+// the neighbour's.  Silent cells (a coordinate of 0: they visit no cell) are
+// cleared by k_cell_keys.
+// Bound by the bitmap probes (L2 latency and ALU): 6.8M cells of the skewed 6-D
+// data, 122 rows each.
+__global__ void __launch_bounds__(256) k_cell_workload(const unsigned long long* __restrict__ cell_lid,
+                                                        const uint32_t* __restrict__ cell_start, uint32_t nC,
+                                                        HjGrid grid, HjCellHash hash, uint32_t* __restrict__ cell_nb) {
+    const uint32_t cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (cell >= nC) return;
+    const unsigned long long L = cell_lid[cell];
     uint32_t lo[kMaxK], w[kMaxK];
     uint32_t rows = 1;
-    bool empty = false;
     const uint32_t cl = lane_cell_coord(grid, L);
     for (uint32_t j = 0; j < grid.k; ++j) {
         const uint32_t c = __shfl_sync(0xffffffffu, cl, j);
-        uint32_t l = c - 1u;                                   // wraps at 0 (kernel.cu:113)
-        uint32_t h = min(grid.n_cells[j] - 1u, c + 1u);        // kernel.cu:114
-        if (l > h) empty = true;
-        lo[j] = l;
-        w[j] = h - l + 1;
+        lo[j] = c == 0u ? 0u : c - 1u;
+        w[j] = min(grid.n_cells[j] - 1u, c + 1u) - lo[j] + 1u;        // kernel.cu:113-114
         if (j > 0) rows *= w[j];
     }
-    unsigned long long cnt = 0;
-    if (!empty) {
-        const StencilRows sr = stencil_rows(grid, lo, rows);
-        for (uint32_t r = lane_id(); r < rows; r += 32) {
-            const uint2 sp = cell_span(hash, cell_start, stencil_row_id(grid, sr, lo, w, r), w[0]);
-            cnt += sp.y - sp.x;
+    const StencilRows sr = stencil_rows(grid, lo, rows);
+    const uint32_t r_own = own_row(grid, lo, w, cl);
+    const uint32_t pop = cell_start[cell + 1] - cell_start[cell];
+    uint32_t cnt = 0;
+    // four rows per lane at a time: their bitmap words are loaded together
+    for (uint32_t r0 = r_own; r0 < rows; r0 += 128) {
+        unsigned long long id[4];
+        uint32_t m[4];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const uint32_t r = r0 + i * 32 + lane_id();
+            m[i] = 0;
+            if (r >= rows) continue;
+            id[i] = stencil_row_id(grid, sr, lo, w, r);
+            m[i] = occ_row(hash, id[i], w[0]);
+            // of its own row, the cell itself and what follows
+            if (r == r_own) m[i] &= ~((1u << (uint32_t)(L - id[i])) - 1u);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            if (m[i] == 0u) continue;
+            const uint2 c = cell_range(hash, id[i], m[i]);
+            if (c.x == kNoCell) continue;
+            uint32_t s = cell_start[c.x];
+            for (uint32_t j = c.x; j <= c.y; ++j) {
+                const uint32_t e = cell_start[j + 1];
+                cnt += e - s;
+                if (j != cell) atomicAdd(&cell_nb[j], pop);
+                s = e;
+            }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if (lane_id() == 0) {
-        cell_nb[warp] = (uint32_t)cnt;
-        cell_work[warp] = cnt * (unsigned long long)(cell_start[warp + 1] - cell_start[warp]);
-    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane_id() == 0) atomicAdd(&cell_nb[cell], cnt);
 }
 
 namespace {
 
-__global__ void k_desc_keys(const uint32_t* __restrict__ nb, uint32_t nC, uint32_t* __restrict__ keys,
-                            uint32_t* __restrict__ vals) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nC) return;
-    keys[i] = ~nb[i];     // ascending order of the complement = descending candidates
-    vals[i] = i;
-}
-
-__global__ void k_max_u32(const uint32_t* __restrict__ a, uint32_t n, uint32_t* out) {
-    uint32_t m = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, a[i]);
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-    if (lane_id() == 0) atomicMax(out, m);
+// After k_cell_workload: clears the silent cells' counts, writes the sort keys of
+// the workload order (top - candidates: ascending keys, descending candidates) and
+// folds totalCandidates and the largest count into out[0], out[1].
+__global__ void __launch_bounds__(256) k_cell_keys(const unsigned long long* __restrict__ cell_lid,
+                                                    const uint32_t* __restrict__ cell_start, uint32_t nC, HjGrid g,
+                                                    uint32_t any_silent, uint32_t top, uint32_t* __restrict__ cell_nb,
+                                                    uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                    unsigned long long* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long work = 0;
+    uint32_t nb = 0;
+    if (i < nC) {
+        nb = cell_nb[i];
+        if (any_silent) {
+            unsigned long long L = cell_lid[i];
+            bool silent = false;
+            for (uint32_t j = 0; j < g.k; ++j) {
+                const unsigned long long q = L / g.n_cells[j];
+                silent |= L == q * g.n_cells[j];
+                L = q;
+            }
+            if (silent) cell_nb[i] = nb = 0;
+        }
+        keys[i] = top - nb;
+        vals[i] = i;
+        work = (unsigned long long)nb * (cell_start[i + 1] - cell_start[i]);
+    }
+    for (int o = 16; o > 0; o >>= 1) work += __shfl_down_sync(0xffffffffu, work, o);
+    nb = __reduce_max_sync(0xffffffffu, nb);
+    __shared__ unsigned long long ws[8];
+    __shared__ uint32_t wm[8];
+    if (lane_id() == 0) { ws[threadIdx.x >> 5] = work; wm[threadIdx.x >> 5] = nb; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < 8; ++j) { work += ws[j]; nb = max(nb, wm[j]); }
+        if (work) atomicAdd(&out[0], work);
+        if (nb) atomicMax(&out[1], (unsigned long long)nb);
+    }
 }
 
 __global__ void k_block_counts(const uint32_t* __restrict__ order, const uint32_t* __restrict__ cell_start, uint32_t nC,
@@ -422,21 +470,22 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
 // The first cell of each group inserts the group's entry: key, first cell, mask
 // of the group's ids (its cells are the next ones in the table, at most four).
 // The key word pair is claimed with a 64-bit compare-and-swap on the entry's
-// first 8 bytes; first cell and mask are written after it.
+// first 8 bytes; first cell and mask are written after it.  The first cell of
+// each segment of 32 ids sets the segment's bits in the bitmap.
 __global__ void k_hash_insert(const unsigned long long* __restrict__ lid, uint32_t nC, uint4* entries,
-                              unsigned long long mask, uint32_t* occ, unsigned long long occ_mask) {
+                              unsigned long long mask, uint32_t* occ, uint32_t occ_shift) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nC) return;
-    const unsigned long long g = lid[i] >> 2;
-    if (i > 0 && (lid[i - 1] >> 2) == g) return;
+    const unsigned long long me = lid[i], before = i > 0 ? lid[i - 1] : ~me;
+    if (i == 0 || (before >> 5) != (me >> 5)) {
+        uint32_t bits = 0;
+        for (uint32_t j = i; j < nC && (lid[j] >> 5) == (me >> 5); ++j) bits |= 1u << (uint32_t)(lid[j] & 31u);
+        atomicOr(occ + occ_word(me, occ_shift), bits);
+    }
+    const unsigned long long g = me >> 2;
+    if (i > 0 && (before >> 2) == g) return;
     uint32_t m = 0;
     for (uint32_t j = i; j < nC && j < i + 4 && (lid[j] >> 2) == g; ++j) m |= 1u << (uint32_t)(lid[j] & 3u);
-    if (occ) {
-        unsigned long long w;
-        uint32_t b;
-        occ_bits(g, occ_mask, &w, &b);
-        atomicOr(occ + w, b);
-    }
     unsigned long long s = mix64(g) & mask;
     for (unsigned long long probe = 0; probe <= mask; ++probe) {   // the table is at most half full
         unsigned long long* kw = reinterpret_cast<unsigned long long*>(&entries[s]);
@@ -475,28 +524,21 @@ hj_status build_row_offsets(hj_index* ix, cudaStream_t st) {
     return HJ_OK;
 }
 
-// Smallest table (entries) that gets an occupancy filter: 32 MB of entries.
-constexpr unsigned long long kOccMinCap = 1ull << 21;
-
 // The cell hash of an index whose cell table is built (capacity: the power of
 // two at least twice the number of cells, an upper bound on the groups that
-// needs no count from the device, at least 64).  From kOccMinCap entries on, an
-// occupancy filter of capacity / 4 words (16 bits per cell, a sixteenth of the
-// table's bytes) goes with it.
+// needs no count from the device, at least 64) and its bitmap (a word per entry).
 hj_status build_cell_hash(hj_index* ix, cudaStream_t st) {
     unsigned long long cap = 64;
     while (cap < 2ull * ix->nC) cap <<= 1;
     HJ_TRY(dalloc(&ix->hash_entries, (size_t)cap, st));
     HJ_CUDA(cudaMemsetAsync(ix->hash_entries, 0xFF, (size_t)cap * sizeof(uint4), st));
     ix->hash_mask = cap - 1;
-    if (cap >= kOccMinCap) {
-        HJ_TRY(dalloc(&ix->hash_occ, (size_t)(cap / 4), st));
-        HJ_CUDA(cudaMemsetAsync(ix->hash_occ, 0, (size_t)cap, st));
-        ix->occ_mask = cap / 4 - 1;
-    }
+    HJ_TRY(dalloc(&ix->hash_occ, (size_t)cap, st));
+    HJ_CUDA(cudaMemsetAsync(ix->hash_occ, 0, (size_t)cap * 4, st));
+    ix->occ_shift = 65 - bits_for(cap);   // cap = 2^(bits - 1)
     if (ix->nC) {
         k_hash_insert<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->nC, ix->hash_entries, ix->hash_mask,
-                                                           ix->hash_occ, ix->occ_mask);
+                                                           ix->hash_occ, ix->occ_shift);
         HJ_LAUNCHED();
     }
     return HJ_OK;
@@ -736,32 +778,31 @@ hj_status hj_sort_by_workload(hj_index* ix, void* stream, uint64_t* total_candid
         dfree(ix->cell_nb, st);
         dfree(ix->cell_order, st);
         Scratch tmp(st);
-        unsigned long long* work = nullptr;
-        uint32_t *keys = nullptr, *keys_tmp = nullptr, *vals_tmp = nullptr, *dmax = nullptr;
-        uint64_t* dsum = nullptr;
+        unsigned long long* folded = nullptr;   // totalCandidates, largest count
+        uint32_t *keys = nullptr, *keys_tmp = nullptr, *vals_tmp = nullptr;
         HJ_TRY(dalloc(&ix->cell_nb, nC, st));
-        HJ_TRY(tmp.alloc(&work, nC));
-        unsigned g = (unsigned)(((uint64_t)nC * 32 + 255) / 256);
-        k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, cell_hash(ix), ix->cell_nb,
-                                           work);
-        HJ_LAUNCHED();
-        HJ_TRY(tmp.alloc(&dsum, 1));
-        HJ_TRY(reduce_sum_u64(reinterpret_cast<uint64_t*>(work), nC, dsum, st));
-        HJ_TRY(tmp.alloc(&dmax, 1));
-        HJ_CUDA(cudaMemsetAsync(dmax, 0, 4, st));
-        k_max_u32<<<std::min<unsigned>((nC + 255) / 256, num_sms() * 4), 256, 0, st>>>(ix->cell_nb, nC, dmax);
-        HJ_LAUNCHED();
+        HJ_TRY(dalloc(&ix->cell_order, nC, st));
+        HJ_TRY(tmp.alloc(&folded, 2));
         HJ_TRY(tmp.alloc(&keys, nC));
         HJ_TRY(tmp.alloc(&keys_tmp, nC));
         HJ_TRY(tmp.alloc(&vals_tmp, nC));
-        HJ_TRY(dalloc(&ix->cell_order, nC, st));
-        k_desc_keys<<<(nC + 255) / 256, 256, 0, st>>>(ix->cell_nb, nC, keys, ix->cell_order);
+        HJ_CUDA(cudaMemsetAsync(ix->cell_nb, 0, (size_t)nC * 4, st));
+        HJ_CUDA(cudaMemsetAsync(folded, 0, 2 * sizeof(unsigned long long), st));
+        unsigned g = (unsigned)(((uint64_t)nC * 32 + 255) / 256);
+        k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, cell_hash(ix), ix->cell_nb);
         HJ_LAUNCHED();
-        HJ_TRY(radix_sort_u32_u32(keys, ix->cell_order, keys_tmp, vals_tmp, nC, 32, st));
-        uint64_t tot = 0;
-        HJ_CUDA(cudaMemcpyAsync(&tot, dsum, 8, cudaMemcpyDeviceToHost, st));
-        HJ_CUDA(cudaMemcpyAsync(&ix->max_nb, dmax, 4, cudaMemcpyDeviceToHost, st));
+        // no count exceeds n: the sort needs only that many bits
+        const uint32_t nbits = bits_for(ix->n);
+        k_cell_keys<<<(nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, ix->any_silent,
+                                                      (uint32_t)((1ull << nbits) - 1), ix->cell_nb, keys,
+                                                      ix->cell_order, folded);
+        HJ_LAUNCHED();
+        HJ_TRY(radix_sort_u32_u32(keys, ix->cell_order, keys_tmp, vals_tmp, nC, nbits, st));
+        unsigned long long hf[2] = {0, 0};
+        HJ_CUDA(cudaMemcpyAsync(hf, folded, sizeof(hf), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
+        const uint64_t tot = hf[0];
+        ix->max_nb = (uint32_t)hf[1];
         ix->total_candidates = tot;
         ix->have_workload = true;
     }

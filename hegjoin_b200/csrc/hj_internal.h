@@ -28,16 +28,17 @@ constexpr uint32_t kRowOffMaxK = 7;   // at most 729 offsets
 // power of two at least twice the number of cells (so at most half full of
 // groups); free entries hold the key
 // kEmptyLid (no group can have it: linear ids stay below 2^63).
-// A table too large for L2 gets an occupancy filter beside it: two bits of one
-// 32-bit word per group (16 bits per cell), set at insertion.  A probe of an
-// absent group, the common case on sparse data, then costs one load of a
-// filter small enough to stay in L2 instead of a random DRAM read of the table;
-// about 2% of absent groups pass the filter and read the table as before.
+// Beside it lies an occupancy bitmap: ids in segments of 32, each segment a word
+// picked by a multiplicative hash (segments may share one), each cell its bit.  A
+// stencil row is one load of one word -- from L2, where the table itself does not
+// fit -- and three bits: the common case on sparse data, a row without cells, ends
+// there.  4 bytes per table entry, 64 to 128 bits per cell: 3 to 5% of the empty
+// rows find a stranger's bit and go on to the table.
 struct HjCellHash {
     const uint4* entries;
     unsigned long long mask;       // capacity - 1
-    const uint32_t* occ;           // occupancy filter, or null (small tables)
-    unsigned long long occ_mask;   // filter words - 1
+    const uint32_t* occ;           // occupancy bitmap
+    uint32_t occ_shift;            // 64 - log2(its words)
 };
 
 // Work item of the refine kernels: queries q0..q1 (sorted positions) of cell
@@ -70,8 +71,8 @@ struct hj_index {
     uint32_t nC = 0;
     uint4* hash_entries = nullptr;   // cell hash (HjCellHash)
     unsigned long long hash_mask = 0;
-    uint32_t* hash_occ = nullptr;    // its occupancy filter (large tables only)
-    unsigned long long occ_mask = 0;
+    uint32_t* hash_occ = nullptr;    // its occupancy bitmap
+    uint32_t occ_shift = 0;
     unsigned long long* row_off = nullptr;   // grid.row_off
 
     // workload (hj_sort_by_workload)
@@ -121,16 +122,12 @@ constexpr unsigned long long kEmptyLid = ~0ull;
 constexpr uint32_t kNoCell = 0xFFFFFFFFu;
 
 inline HjCellHash cell_hash(const hj_index* ix) {
-    return HjCellHash{ix->hash_entries, ix->hash_mask, ix->hash_occ, ix->occ_mask};
+    return HjCellHash{ix->hash_entries, ix->hash_mask, ix->hash_occ, ix->occ_shift};
 }
 
-// The filter word of group g and the two bits the group sets in it (a second
-// hash of g, independent of the slot index).
-__host__ __device__ __forceinline__ void occ_bits(unsigned long long g, unsigned long long occ_mask,
-                                                  unsigned long long* word, uint32_t* bits) {
-    const uint64_t z = mix64(g ^ 0xD6E8FEB86659FD93ull);
-    *word = z & occ_mask;
-    *bits = (1u << (uint32_t)((z >> 52) & 31u)) | (1u << (uint32_t)((z >> 58) & 31u));
+// Bitmap word of the segment of 32 ids that holds `lid`.
+__host__ __device__ __forceinline__ unsigned long long occ_word(unsigned long long lid, uint32_t occ_shift) {
+    return ((lid >> 5) * 0x9E3779B97F4A7C15ull) >> occ_shift;
 }
 
 // Coordinate of the cell with linear id L along dimension lane_id() for the
@@ -181,16 +178,22 @@ __device__ __forceinline__ unsigned long long stencil_row_id(const HjGrid& g, co
     return id;
 }
 
+// The row of a full stencil box (or an edge box) that holds the cell itself: rows
+// are in ascending order of their linear ids, so the cells after the cell lie in its
+// own row, past it, and in the rows after that one.
+__device__ __forceinline__ uint32_t own_row(const HjGrid& g, const uint32_t* lo, const uint32_t* w, uint32_t cl) {
+    uint32_t r = 0, radix = 1;
+    for (uint32_t j = 1; j < g.k; ++j) {
+        r += (__shfl_sync(0xffffffffu, cl, j) - lo[j]) * radix;   // cl: lane_cell_coord
+        radix *= w[j];
+    }
+    return r;
+}
+
 // The entry of group g: (first cell, id mask), or a zero mask when the group has
 // no cell.  Probes stop at a free entry; the table is at most half full, so the
 // loop ends after a few probes (and after capacity probes at the very most).
 __device__ __forceinline__ uint2 group_find(const HjCellHash& h, unsigned long long g) {
-    if (h.occ) {
-        unsigned long long w;
-        uint32_t b;
-        occ_bits(g, h.occ_mask, &w, &b);
-        if ((__ldg(h.occ + w) & b) != b) return make_uint2(kNoCell, 0u);
-    }
     unsigned long long i = mix64(g) & h.mask;
     for (unsigned long long probe = 0; probe <= h.mask; ++probe) {
         const uint4 e = h.entries[i];
@@ -202,26 +205,49 @@ __device__ __forceinline__ uint2 group_find(const HjCellHash& h, unsigned long l
     return make_uint2(kNoCell, 0u);
 }
 
-// Points of the existing cells with linear ids lo .. lo + w - 1 (consecutive
-// along dimension 0, w <= 4): one contiguous span [x, y) of the cell-ordered
-// points, because the non-empty cells are sorted by linear id.
-__device__ __forceinline__ uint2 cell_span(const HjCellHash& h, const uint32_t* cell_start, unsigned long long lo,
-                                           uint32_t w) {
-    const unsigned long long hi = lo + w - 1;
+// Bit i set: the bitmap knows a cell lo + i, i < w <= 4 (or one that shares its bit).
+__device__ __forceinline__ uint32_t occ_row(const HjCellHash& h, unsigned long long lo, uint32_t w) {
+    const uint32_t b = (uint32_t)lo & 31u;
+    uint32_t m = __ldg(h.occ + occ_word(lo, h.occ_shift)) >> b;
+    if (b + w > 32u) m |= __ldg(h.occ + occ_word(lo + w - 1, h.occ_shift)) << (32u - b);
+    return m & ((1u << w) - 1u);
+}
+
+// The existing cells among those named by `m` (occ_row's answer) from id lo on:
+// consecutive in the cell table, [x, y] (x == kNoCell: none).
+__device__ __forceinline__ uint2 cell_range(const HjCellHash& h, unsigned long long lo, uint32_t m) {
     uint32_t first = kNoCell, last = kNoCell;
-    for (unsigned long long g = lo >> 2; g <= (hi >> 2); ++g) {
+    while (m) {
+        const unsigned long long id = lo + (__ffs(m) - 1);
+        const unsigned long long g = id >> 2;
         const uint2 e = group_find(h, g);
-        const uint32_t b0 = g == (lo >> 2) ? (uint32_t)(lo & 3u) : 0u;
-        const uint32_t b1 = g == (hi >> 2) ? (uint32_t)(hi & 3u) : 3u;
-        const uint32_t m = e.y & ((2u << b1) - 1u) & ~((1u << b0) - 1u);   // the group's ids in [lo, hi]
-        if (m == 0u) continue;
-        const uint32_t f = e.x + __popc(e.y & ((1u << (__ffs(m) - 1)) - 1u));
-        const uint32_t l = e.x + __popc(e.y & ((2u << (31 - __clz(m))) - 1u)) - 1u;
+        // this group's ids among m: bit b of the group is id g * 4 + b
+        const long long sh = (long long)(g * 4ull - lo);
+        const uint32_t want = (sh >= 0 ? m >> sh : m << -sh) & 15u;
+        m &= ~(sh >= 0 ? 15u << sh : 15u >> -sh);
+        const uint32_t have = e.y & want;
+        if (have == 0u) continue;
+        const uint32_t f = e.x + __popc(e.y & ((1u << (__ffs(have) - 1)) - 1u));
+        const uint32_t l = e.x + __popc(e.y & ((2u << (31 - __clz(have))) - 1u)) - 1u;
         if (first == kNoCell) first = f;
         last = l;
     }
-    if (first == kNoCell) return make_uint2(0u, 0u);
-    return make_uint2(cell_start[first], cell_start[last + 1]);
+    return make_uint2(first, last);
+}
+
+// Points of the existing cells with linear ids lo .. lo + w - 1 (consecutive
+// along dimension 0, w <= 4): one contiguous span [x, y) of the cell-ordered
+// points, because the non-empty cells are sorted by linear id.
+__device__ __forceinline__ uint2 cell_points(const HjCellHash& h, const uint32_t* cell_start, unsigned long long lo,
+                                             uint32_t m) {
+    const uint2 c = cell_range(h, lo, m);
+    if (c.x == kNoCell) return make_uint2(0u, 0u);
+    return make_uint2(cell_start[c.x], cell_start[c.y + 1]);
+}
+__device__ __forceinline__ uint2 cell_span(const HjCellHash& h, const uint32_t* cell_start, unsigned long long lo,
+                                           uint32_t w) {
+    const uint32_t m = occ_row(h, lo, w);
+    return m ? cell_points(h, cell_start, lo, m) : make_uint2(0u, 0u);
 }
 
 }  // namespace hj

@@ -106,6 +106,7 @@ struct WarpBox {
     uint32_t rows;
     bool silent;
     unsigned long long L;
+    uint32_t r_own;           // the row that holds the cell itself
     StencilRows sr;
 };
 __device__ __forceinline__ void warp_box(const HjGrid& g, unsigned long long L, WarpBox& b) {
@@ -122,6 +123,7 @@ __device__ __forceinline__ void warp_box(const HjGrid& g, unsigned long long L, 
         if (j > 0) b.rows *= b.w[j];
     }
     b.sr = stencil_rows(g, b.lo, b.rows);
+    b.r_own = own_row(g, b.lo, b.w, cl);
 }
 
 // One round of stencil rows: their non-empty point ranges, compacted into S, and
@@ -131,26 +133,25 @@ __device__ __forceinline__ uint32_t warp_round(const HjGrid& g, const HjCellHash
                                                const WarpBox& b, uint32_t row0, bool sym, uint32_t q0, S_& S,
                                                uint32_t* n_ranges) {
     uint32_t run = 0, nr = 0;
+    // the lanes' bitmap words are loaded together; most rows of sparse data end there
+    unsigned long long id[kWarpRows / 32];
+    uint32_t m[kWarpRows / 32];
 #pragma unroll
     for (uint32_t sl = 0; sl < kWarpRows / 32; ++sl) {
         const uint32_t r = row0 + sl * 32 + lane_id();
+        m[sl] = 0;
+        if (r >= b.rows) continue;
+        id[sl] = stencil_row_id(g, b.sr, b.lo, b.w, r);
+        m[sl] = occ_row(hash, id[sl], b.w[0]);
+        // symmetric form: of its own row, the cell itself and what follows
+        if (sym && r == b.r_own) m[sl] &= ~((1u << (uint32_t)(b.L - id[sl])) - 1u);
+    }
+#pragma unroll
+    for (uint32_t sl = 0; sl < kWarpRows / 32; ++sl) {
         uint2 sp = make_uint2(0u, 0u);
-        if (r < b.rows) {
-            unsigned long long id = stencil_row_id(g, b.sr, b.lo, b.w, r);
-            uint32_t wid = b.w[0];
-            bool own = false;
-            if (sym) {
-                // rows before the cell's own are skipped; its own row starts at the cell itself
-                own = id <= b.L && b.L < id + wid;
-                if (own) {
-                    wid -= (uint32_t)(b.L - id);
-                    id = b.L;
-                } else if (id < b.L) {
-                    wid = 0;
-                }
-            }
-            if (wid) sp = cell_span(hash, cell_start, id, wid);
-            if (own) sp.x = q0;
+        if (m[sl]) {
+            sp = cell_points(hash, cell_start, id[sl], m[sl]);
+            if (sym && row0 + sl * 32 + lane_id() == b.r_own) sp.x = q0;
         }
         const uint32_t len = sp.y - sp.x;
         const uint32_t some = __ballot_sync(0xffffffffu, len != 0u);
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_
         if (lane < nq) S.qid[lane] = a.perm[q0 + lane] & 0x7FFFFFFFu;
         const bool fwd = !box.silent;
         uint32_t my_count = 0;               // lane b: pairs of query b (or, counting only, any pairs)
-        for (uint32_t row0 = 0; row0 < box.rows; row0 += kWarpRows) {
+        for (uint32_t row0 = a.sym ? box.r_own : 0u; row0 < box.rows; row0 += kWarpRows) {
             uint32_t nr;
             const uint32_t run = warp_round(a.grid, a.hash, a.cell_start, box, row0, a.sym != 0u, q0, S, &nr);
             const uint32_t c_lo = (uint32_t)((unsigned long long)run * part / a.parts);

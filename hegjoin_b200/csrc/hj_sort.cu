@@ -233,14 +233,6 @@ hj_status radix_sort(K* keys, uint32_t* vals, K* keys_tmp, uint32_t* vals_tmp, u
     return HJ_OK;
 }
 
-__global__ void k_reduce_u64(const uint64_t* __restrict__ in, uint64_t n, unsigned long long* out) {
-    unsigned long long acc = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        acc += in[i];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane_id() == 0 && acc) atomicAdd(out, acc);
-}
-
 }  // namespace
 
 hj_status scan_u32_to_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t st) {
@@ -260,13 +252,4 @@ hj_status radix_sort_u32_u32(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp,
                              uint32_t nbits, cudaStream_t st) {
     return radix_sort<uint32_t>(keys, vals, keys_tmp, vals_tmp, n, nbits, st);
 }
-hj_status reduce_sum_u64(const uint64_t* in, uint64_t n, uint64_t* d_out, cudaStream_t st) {
-    HJ_CUDA(cudaMemsetAsync(d_out, 0, sizeof(uint64_t), st));
-    if (n == 0) return HJ_OK;
-    unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)num_sms() * 8);
-    k_reduce_u64<<<grid, 256, 0, st>>>(in, n, reinterpret_cast<unsigned long long*>(d_out));
-    HJ_LAUNCHED();
-    return HJ_OK;
-}
-
 }  // namespace hj
