@@ -252,37 +252,28 @@ __global__ void k_gather_rows(const T* __restrict__ db, const uint32_t* __restri
 // Bound by the bitmap probes (L2 latency and ALU): 6.8M cells of the skewed 6-D
 // data, 122 rows each.
 __global__ void __launch_bounds__(256) k_cell_workload(const unsigned long long* __restrict__ cell_lid,
-                                                        const uint32_t* __restrict__ cell_start, uint32_t nC,
-                                                        HjGrid grid, HjCellHash hash, uint32_t* __restrict__ cell_nb) {
+                                                        const uint32_t* __restrict__ cell_start,
+                                                        const uint8_t* __restrict__ cell_edge, uint32_t nC, HjGrid grid,
+                                                        HjCellHash hash, uint32_t* __restrict__ cell_nb) {
     const uint32_t cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (cell >= nC) return;
-    const unsigned long long L = cell_lid[cell];
-    uint32_t lo[kMaxK], w[kMaxK];
-    uint32_t rows = 1;
-    const uint32_t cl = lane_cell_coord(grid, L);
-    for (uint32_t j = 0; j < grid.k; ++j) {
-        const uint32_t c = __shfl_sync(0xffffffffu, cl, j);
-        lo[j] = c == 0u ? 0u : c - 1u;
-        w[j] = min(grid.n_cells[j] - 1u, c + 1u) - lo[j] + 1u;        // kernel.cu:113-114
-        if (j > 0) rows *= w[j];
-    }
-    const StencilRows sr = stencil_rows(grid, lo, rows);
-    const uint32_t r_own = own_row(grid, lo, w, cl);
+    CellBox box;
+    cell_box(grid, cell_lid[cell], cell_edge[cell] != 0, box);
     const uint32_t pop = cell_start[cell + 1] - cell_start[cell];
     uint32_t cnt = 0;
     // four rows per lane at a time: their bitmap words are loaded together
-    for (uint32_t r0 = r_own; r0 < rows; r0 += 128) {
+    for (uint32_t r0 = box.r_own; r0 < box.rows; r0 += 128) {
         unsigned long long id[4];
         uint32_t m[4];
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
             const uint32_t r = r0 + i * 32 + lane_id();
             m[i] = 0;
-            if (r >= rows) continue;
-            id[i] = stencil_row_id(grid, sr, lo, w, r);
-            m[i] = occ_row(hash, id[i], w[0]);
+            if (r >= box.rows) continue;
+            id[i] = cell_box_row(grid, box, r);
+            m[i] = occ_row(hash, id[i], box.w0);
             // of its own row, the cell itself and what follows
-            if (r == r_own) m[i] &= ~((1u << (uint32_t)(L - id[i])) - 1u);
+            if (r == box.r_own) m[i] &= ~((1u << (uint32_t)(box.L - id[i])) - 1u);
         }
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
@@ -471,12 +462,24 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
 // of the group's ids (its cells are the next ones in the table, at most four).
 // The key word pair is claimed with a 64-bit compare-and-swap on the entry's
 // first 8 bytes; first cell and mask are written after it.  The first cell of
-// each segment of 32 ids sets the segment's bits in the bitmap.
-__global__ void k_hash_insert(const unsigned long long* __restrict__ lid, uint32_t nC, uint4* entries,
-                              unsigned long long mask, uint32_t* occ, uint32_t occ_shift) {
+// each segment of 32 ids sets the segment's bits in the bitmap.  Every cell notes
+// whether a coordinate lies at the grid's edge.
+__global__ void k_hash_insert(const unsigned long long* __restrict__ lid, uint32_t nC, HjGrid grid, uint4* entries,
+                              unsigned long long mask, uint32_t* occ, uint32_t occ_shift, uint8_t* __restrict__ edge) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nC) return;
     const unsigned long long me = lid[i], before = i > 0 ? lid[i - 1] : ~me;
+    {
+        unsigned long long rest = me;
+        bool e = false;
+        for (uint32_t j = 0; j < grid.k; ++j) {
+            const unsigned long long q = rest / grid.n_cells[j];
+            const uint32_t c = (uint32_t)(rest - q * grid.n_cells[j]);
+            e |= c == 0u || c + 1u >= grid.n_cells[j];
+            rest = q;
+        }
+        edge[i] = e ? 1 : 0;
+    }
     if (i == 0 || (before >> 5) != (me >> 5)) {
         uint32_t bits = 0;
         for (uint32_t j = i; j < nC && (lid[j] >> 5) == (me >> 5); ++j) bits |= 1u << (uint32_t)(lid[j] & 31u);
@@ -518,6 +521,8 @@ hj_status build_row_offsets(hj_index* ix, cudaStream_t st) {
     for (uint32_t j = 1; j < ix->grid.k; ++j) rows *= 3;
     HJ_TRY(dalloc(&ix->row_off, rows, st));
     ix->grid.full_rows = rows;
+    ix->grid.full_base = 1;
+    for (uint32_t j = 1; j < ix->grid.k; ++j) ix->grid.full_base += ix->grid.mult[j];
     k_row_offsets<<<(rows + 255) / 256, 256, 0, st>>>(ix->grid, ix->row_off);
     HJ_LAUNCHED();
     ix->grid.row_off = ix->row_off;
@@ -535,10 +540,11 @@ hj_status build_cell_hash(hj_index* ix, cudaStream_t st) {
     ix->hash_mask = cap - 1;
     HJ_TRY(dalloc(&ix->hash_occ, (size_t)cap, st));
     HJ_CUDA(cudaMemsetAsync(ix->hash_occ, 0, (size_t)cap * 4, st));
+    HJ_TRY(dalloc(&ix->cell_edge, ix->nC, st));
     ix->occ_shift = 65 - bits_for(cap);   // cap = 2^(bits - 1)
     if (ix->nC) {
-        k_hash_insert<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->nC, ix->hash_entries, ix->hash_mask,
-                                                           ix->hash_occ, ix->occ_shift);
+        k_hash_insert<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->nC, ix->grid, ix->hash_entries,
+                                                           ix->hash_mask, ix->hash_occ, ix->occ_shift, ix->cell_edge);
         HJ_LAUNCHED();
     }
     return HJ_OK;
@@ -548,6 +554,7 @@ void free_index(hj_index* ix, cudaStream_t st) {
     tc_release(ix);
     dfree(ix->hash_entries, st);
     dfree(ix->hash_occ, st);
+    dfree(ix->cell_edge, st);
     dfree(ix->row_off, st);
     ix->grid.row_off = nullptr;
     ix->grid.full_rows = 0;
@@ -789,7 +796,8 @@ hj_status hj_sort_by_workload(hj_index* ix, void* stream, uint64_t* total_candid
         HJ_CUDA(cudaMemsetAsync(ix->cell_nb, 0, (size_t)nC * 4, st));
         HJ_CUDA(cudaMemsetAsync(folded, 0, 2 * sizeof(unsigned long long), st));
         unsigned g = (unsigned)(((uint64_t)nC * 32 + 255) / 256);
-        k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, cell_hash(ix), ix->cell_nb);
+        k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->cell_edge, nC, ix->grid, cell_hash(ix),
+                                           ix->cell_nb);
         HJ_LAUNCHED();
         // no count exceeds n: the sort needs only that many bits
         const uint32_t nbits = bits_for(ix->n);

@@ -14,6 +14,7 @@ struct HjGrid {
     // full_rows 0) for k > kRowOffMaxK.
     const unsigned long long* row_off;
     uint32_t full_rows;
+    unsigned long long full_base;   // linear id of a cell minus that of its full box's first cell
 };
 constexpr uint32_t kRowOffMaxK = 7;   // at most 729 offsets
 
@@ -72,6 +73,7 @@ struct hj_index {
     uint4* hash_entries = nullptr;   // cell hash (HjCellHash)
     unsigned long long hash_mask = 0;
     uint32_t* hash_occ = nullptr;    // its occupancy bitmap
+    uint8_t* cell_edge = nullptr;    // per cell: 1 if its stencil box is not full (a coordinate at the grid's edge)
     uint32_t occ_shift = 0;
     unsigned long long* row_off = nullptr;   // grid.row_off
 
@@ -178,16 +180,46 @@ __device__ __forceinline__ unsigned long long stencil_row_id(const HjGrid& g, co
     return id;
 }
 
-// The row of a full stencil box (or an edge box) that holds the cell itself: rows
-// are in ascending order of their linear ids, so the cells after the cell lie in its
-// own row, past it, and in the rows after that one.
-__device__ __forceinline__ uint32_t own_row(const HjGrid& g, const uint32_t* lo, const uint32_t* w, uint32_t cl) {
-    uint32_t r = 0, radix = 1;
-    for (uint32_t j = 1; j < g.k; ++j) {
-        r += (__shfl_sync(0xffffffffu, cl, j) - lo[j]) * radix;   // cl: lane_cell_coord
-        radix *= w[j];
+// The stencil box of a cell (kernel.cu:778-783), whole warp.  Rows are in ascending
+// order of their linear ids, so the cells after the cell itself lie in its own row,
+// past it, and in the rows after that one.  A full box (the cell is off the grid's
+// edges; cell_edge says so) needs no coordinate: its rows are at fixed offsets from
+// the cell's id.  The others take one 64-bit division per lane for the coordinates.
+struct CellBox {
+    unsigned long long L;
+    uint32_t rows, r_own, w0;   // rows, the row that holds the cell, cells per row
+    bool full, silent;          // silent: a coordinate is 0
+    uint32_t lo[hj::kMaxK], w[hj::kMaxK];
+};
+__device__ __forceinline__ void cell_box(const HjGrid& g, unsigned long long L, bool edge, CellBox& b) {
+    b.L = L;
+    b.full = !edge && g.row_off != nullptr;
+    b.silent = false;
+    if (b.full) {
+        b.rows = g.full_rows;
+        b.r_own = g.full_rows >> 1;
+        b.w0 = 3;
+        return;
     }
-    return r;
+    b.rows = 1;
+    b.r_own = 0;
+    const uint32_t cl = lane_cell_coord(g, L);
+    for (uint32_t j = 0; j < g.k; ++j) {
+        const uint32_t c = __shfl_sync(0xffffffffu, cl, j);
+        b.silent |= c == 0u;
+        b.lo[j] = c == 0u ? 0u : c - 1u;
+        b.w[j] = min(g.n_cells[j] - 1u, c + 1u) - b.lo[j] + 1u;
+        if (j > 0) {
+            b.r_own += (c - b.lo[j]) * b.rows;
+            b.rows *= b.w[j];
+        }
+    }
+    b.w0 = b.w[0];
+}
+// Linear id of the first cell of row r.
+__device__ __forceinline__ unsigned long long cell_box_row(const HjGrid& g, const CellBox& b, uint32_t r) {
+    if (b.full) return b.L - g.full_base + __ldg(g.row_off + r);
+    return stencil_row_id(g, StencilRows{false, 0ull}, b.lo, b.w, r);
 }
 
 // The entry of group g: (first cell, id mask), or a zero mask when the group has

@@ -276,35 +276,55 @@ __global__ void k_csr_copy(const hj_nt_entry* __restrict__ t, uint32_t* const* _
 constexpr uint32_t kWarpSortMax = 1024;
 constexpr uint32_t kSortWarps = 4;
 
+// In-lane steps of one merge: strides K/2 .. 1, ascending.
+template <int K>
+__device__ __forceinline__ void lane_merge(uint32_t (&v)[K]) {
+#pragma unroll
+    for (int stride = K / 2; stride > 0; stride >>= 1)
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+            if (r & stride) continue;
+            const uint32_t lo = min(v[r], v[r + stride]), hi = max(v[r], v[r + stride]);
+            v[r] = lo;
+            v[r + stride] = hi;
+        }
+}
+// Descending merges run ascending on complemented values.  The loops over lane
+// distances stay loops: unrolled, the six sizes were more code than the instruction
+// cache holds, and warps waited for instructions half of the time.
 template <int K>
 __device__ __forceinline__ void warp_sort(uint32_t (&v)[K]) {
     const uint32_t lane = lane_id();
+    // a lane's own K values, by sizes 2, 4, .. K / 2: directions alternate by register
 #pragma unroll
-    for (uint32_t size = 2; size <= 32u * K; size <<= 1) {
+    for (int size = 2; size < K; size <<= 1)
 #pragma unroll
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= K) {
-                const uint32_t lm = stride / K;
-                // ascending where the block of `size` values has an even index
-                const bool up = (lane & (size / K)) == 0 || size == 32u * K;
-                const bool keep_min = ((lane & lm) == 0) == up;
+        for (int stride = size / 2; stride > 0; stride >>= 1)
 #pragma unroll
-                for (int r = 0; r < K; ++r) {
-                    const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], lm);
-                    v[r] = keep_min ? min(v[r], o) : max(v[r], o);
-                }
-            } else {
+            for (int r = 0; r < K; ++r) {
+                if (r & stride) continue;
+                const uint32_t lo = min(v[r], v[r + stride]), hi = max(v[r], v[r + stride]);
+                v[r] = (r & size) ? hi : lo;
+                v[r + stride] = (r & size) ? lo : hi;
+            }
+    // then merges over 1, 2, 4, .. 32 lanes: descending where the merged group's index is odd
+    uint32_t flipped = 0;
+#pragma unroll 1
+    for (uint32_t lanes = 1; lanes <= 32; lanes <<= 1) {
+        const uint32_t flip = (lane & lanes) ? 0xFFFFFFFFu : 0u;
 #pragma unroll
-                for (int r = 0; r < K; ++r) {
-                    const int o = r ^ (int)stride;
-                    if (o < r) continue;
-                    const bool up = size >= K ? ((lane & (size / K)) == 0 || size == 32u * K) : (r & size) == 0;
-                    const uint32_t lo = min(v[r], v[o]), hi = max(v[r], v[o]);
-                    v[r] = up ? lo : hi;
-                    v[o] = up ? hi : lo;
-                }
+        for (int r = 0; r < K; ++r) v[r] ^= flip ^ flipped;
+        flipped = flip;
+#pragma unroll 1
+        for (uint32_t lm = lanes >> 1; lm > 0; lm >>= 1) {
+            const bool keep_min = (lane & lm) == 0;
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], lm);
+                v[r] = keep_min ? min(v[r], o) : max(v[r], o);
             }
         }
+        lane_merge<K>(v);
     }
 }
 

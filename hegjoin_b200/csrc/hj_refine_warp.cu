@@ -49,6 +49,7 @@ static hj_status make_args(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     if (sym) HJ_TRY(flagged_perm(ix, &a->perm, st));
     a->cell_lid = ix->cell_lid;
     a->cell_start = ix->cell_start;
+    a->cell_edge = ix->cell_edge;
     a->hash = cell_hash(ix);
     a->grid = ix->grid;
     a->thr = (T)ix->thr;

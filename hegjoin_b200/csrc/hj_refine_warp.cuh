@@ -54,6 +54,7 @@ struct WarpArgs {
     const uint32_t* perm;             // sorted position -> original id (sym: bit 31 set in silent cells)
     const unsigned long long* cell_lid;
     const uint32_t* cell_start;
+    const uint8_t* cell_edge;
     HjCellHash hash;
     HjGrid grid;
     T thr;
@@ -100,37 +101,11 @@ __device__ __forceinline__ unsigned long long wfma2(unsigned long long a, unsign
     return d;
 }
 
-// The stencil box of an item's cell (kernel.cu:778-783); silent: a coordinate is 0.
-struct WarpBox {
-    uint32_t lo[kMaxK], w[kMaxK];
-    uint32_t rows;
-    bool silent;
-    unsigned long long L;
-    uint32_t r_own;           // the row that holds the cell itself
-    StencilRows sr;
-};
-__device__ __forceinline__ void warp_box(const HjGrid& g, unsigned long long L, WarpBox& b) {
-    b.L = L;
-    b.rows = 1;
-    b.silent = false;
-    const uint32_t cl = lane_cell_coord(g, L);
-    for (uint32_t j = 0; j < g.k; ++j) {
-        const uint32_t c = __shfl_sync(0xffffffffu, cl, j);
-        const uint32_t h = min(g.n_cells[j] - 1u, c + 1u);
-        b.silent |= c == 0u;
-        b.lo[j] = c == 0u ? 0u : c - 1u;
-        b.w[j] = h - b.lo[j] + 1u;
-        if (j > 0) b.rows *= b.w[j];
-    }
-    b.sr = stencil_rows(g, b.lo, b.rows);
-    b.r_own = own_row(g, b.lo, b.w, cl);
-}
-
 // One round of stencil rows: their non-empty point ranges, compacted into S, and
 // the round's candidates (0: nothing).  Whole warp.
 template <typename S_>
 __device__ __forceinline__ uint32_t warp_round(const HjGrid& g, const HjCellHash& hash, const uint32_t* cell_start,
-                                               const WarpBox& b, uint32_t row0, bool sym, uint32_t q0, S_& S,
+                                               const CellBox& b, uint32_t row0, bool sym, uint32_t q0, S_& S,
                                                uint32_t* n_ranges) {
     uint32_t run = 0, nr = 0;
     // the lanes' bitmap words are loaded together; most rows of sparse data end there
@@ -141,8 +116,8 @@ __device__ __forceinline__ uint32_t warp_round(const HjGrid& g, const HjCellHash
         const uint32_t r = row0 + sl * 32 + lane_id();
         m[sl] = 0;
         if (r >= b.rows) continue;
-        id[sl] = stencil_row_id(g, b.sr, b.lo, b.w, r);
-        m[sl] = occ_row(hash, id[sl], b.w[0]);
+        id[sl] = cell_box_row(g, b, r);
+        m[sl] = occ_row(hash, id[sl], b.w0);
         // symmetric form: of its own row, the cell itself and what follows
         if (sym && r == b.r_own) m[sl] &= ~((1u << (uint32_t)(b.L - id[sl])) - 1u);
     }
@@ -226,8 +201,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_
         const uint32_t bi = it / a.parts, part = it - bi * a.parts;
         const HjBlock blk = a.blocks[bi];
         const uint32_t q0 = blk.q0, nq = blk.q1 - blk.q0;
-        WarpBox box;
-        warp_box(a.grid, a.cell_lid[blk.cell], box);
+        CellBox box;
+        cell_box(a.grid, a.cell_lid[blk.cell], a.cell_edge[blk.cell] != 0, box);
         if (box.silent && !a.sym) continue;
         __syncwarp();
         for (uint32_t f = lane; f < nq * D; f += 32) {
@@ -388,8 +363,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_refine_digest(const __g
         const uint32_t bi = it / a.parts, part = it - bi * a.parts;
         const HjBlock blk = a.blocks[bi];
         const uint32_t q0 = blk.q0, nq = blk.q1 - blk.q0;
-        WarpBox box;
-        warp_box(a.grid, a.cell_lid[blk.cell], box);
+        CellBox box;
+        cell_box(a.grid, a.cell_lid[blk.cell], a.cell_edge[blk.cell] != 0, box);
         if (box.silent) continue;
         T qv[D];
 #pragma unroll
