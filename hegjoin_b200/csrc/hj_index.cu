@@ -255,30 +255,19 @@ __global__ void __launch_bounds__(256) k_cell_workload(const unsigned long long*
                                                         const uint32_t* __restrict__ cell_start,
                                                         const uint8_t* __restrict__ cell_edge, uint32_t nC, HjGrid grid,
                                                         HjCellHash hash, uint32_t* __restrict__ cell_nb) {
+    __shared__ uint32_t lists[8][kBoxRows];
     const uint32_t cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (cell >= nC) return;
     CellBox box;
     cell_box(grid, cell_lid[cell], cell_edge[cell] != 0, box);
     const uint32_t pop = cell_start[cell + 1] - cell_start[cell];
     uint32_t cnt = 0;
-    // four rows per lane at a time: their bitmap words are loaded together
-    for (uint32_t r0 = box.r_own; r0 < box.rows; r0 += 128) {
-        unsigned long long id[4];
-        uint32_t m[4];
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            const uint32_t r = r0 + i * 32 + lane_id();
-            m[i] = 0;
-            if (r >= box.rows) continue;
-            id[i] = cell_box_row(grid, box, r);
-            m[i] = occ_row(hash, id[i], box.w0);
-            // of its own row, the cell itself and what follows
-            if (r == box.r_own) m[i] &= ~((1u << (uint32_t)(box.L - id[i])) - 1u);
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            if (m[i] == 0u) continue;
-            const uint2 c = cell_range(hash, id[i], m[i]);
+    uint32_t* list = lists[threadIdx.x >> 5];
+    for (uint32_t r0 = box.r_own; r0 < box.rows; r0 += kBoxRows) {
+        const uint32_t n = box_rows_present(grid, hash, box, r0, true, list);
+        for (uint32_t i = lane_id(); i < n; i += 32) {
+            const uint32_t x = list[i];
+            const uint2 c = cell_range(hash, cell_box_row(grid, box, x & 0x0FFFFFFFu), x >> 28);
             if (c.x == kNoCell) continue;
             uint32_t s = cell_start[c.x];
             for (uint32_t j = c.x; j <= c.y; ++j) {
@@ -288,6 +277,7 @@ __global__ void __launch_bounds__(256) k_cell_workload(const unsigned long long*
                 s = e;
             }
         }
+        __syncwarp();
     }
     cnt = __reduce_add_sync(0xffffffffu, cnt);
     if (lane_id() == 0) atomicAdd(&cell_nb[cell], cnt);

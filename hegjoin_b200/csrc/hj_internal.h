@@ -267,6 +267,35 @@ __device__ __forceinline__ uint2 cell_range(const HjCellHash& h, unsigned long l
     return make_uint2(first, last);
 }
 
+// Rows row0 .. row0 + 127 of a box that the bitmap does not rule out, compacted into
+// `list` (row | cells << 28), and their number.  The lanes' bitmap words are loaded
+// together; what is left of sparse data -- a few rows -- then goes through the
+// table side by side instead of one slot of 32 rows after the other.  after: only
+// the cell itself and the cells after it.  Whole warp.
+constexpr uint32_t kBoxRows = 128;
+__device__ __forceinline__ uint32_t box_rows_present(const HjGrid& g, const HjCellHash& h, const CellBox& b,
+                                                     uint32_t row0, bool after, uint32_t* list) {
+    uint32_t m[kBoxRows / 32];
+#pragma unroll
+    for (uint32_t i = 0; i < kBoxRows / 32; ++i) {
+        const uint32_t r = row0 + i * 32 + lane_id();
+        m[i] = 0;
+        if (r >= b.rows) continue;
+        const unsigned long long id = cell_box_row(g, b, r);
+        m[i] = occ_row(h, id, b.w0);
+        if (after && r == b.r_own) m[i] &= ~((1u << (uint32_t)(b.L - id)) - 1u);
+    }
+    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kBoxRows / 32; ++i) {
+        const uint32_t some = __ballot_sync(0xffffffffu, m[i] != 0u);
+        if (m[i]) list[n + __popc(some & lanemask_lt())] = (row0 + i * 32 + lane_id()) | m[i] << 28;
+        n += __popc(some);
+    }
+    __syncwarp();
+    return n;
+}
+
 // Points of the existing cells with linear ids lo .. lo + w - 1 (consecutive
 // along dimension 0, w <= 4): one contiguous span [x, y) of the cell-ordered
 // points, because the non-empty cells are sorted by linear id.

@@ -45,7 +45,7 @@ namespace hj {
 constexpr int kWarpC = 2;             // candidates per lane and step
 constexpr uint32_t kWarpsPerBlock = 4;
 constexpr uint32_t kWarpQ = 32;       // queries per work item
-constexpr uint32_t kWarpRows = 128;   // stencil rows per round
+constexpr uint32_t kWarpRows = kBoxRows;   // stencil rows per round
 constexpr uint32_t kWarpMaxBlocks = 8;   // resident blocks per SM at most
 
 template <typename T>
@@ -108,29 +108,19 @@ __device__ __forceinline__ uint32_t warp_round(const HjGrid& g, const HjCellHash
                                                const CellBox& b, uint32_t row0, bool sym, uint32_t q0, S_& S,
                                                uint32_t* n_ranges) {
     uint32_t run = 0, nr = 0;
-    // the lanes' bitmap words are loaded together; most rows of sparse data end there
-    unsigned long long id[kWarpRows / 32];
-    uint32_t m[kWarpRows / 32];
-#pragma unroll
-    for (uint32_t sl = 0; sl < kWarpRows / 32; ++sl) {
-        const uint32_t r = row0 + sl * 32 + lane_id();
-        m[sl] = 0;
-        if (r >= b.rows) continue;
-        id[sl] = cell_box_row(g, b, r);
-        m[sl] = occ_row(hash, id[sl], b.w0);
-        // symmetric form: of its own row, the cell itself and what follows
-        if (sym && r == b.r_own) m[sl] &= ~((1u << (uint32_t)(b.L - id[sl])) - 1u);
-    }
-#pragma unroll
-    for (uint32_t sl = 0; sl < kWarpRows / 32; ++sl) {
+    const uint32_t n = box_rows_present(g, hash, b, row0, sym, S.pre);
+    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
         uint2 sp = make_uint2(0u, 0u);
-        if (m[sl]) {
-            sp = cell_points(hash, cell_start, id[sl], m[sl]);
-            if (sym && row0 + sl * 32 + lane_id() == b.r_own) sp.x = q0;
+        const uint32_t x = i0 + lane_id() < n ? S.pre[i0 + lane_id()] : 0u;
+        if (x) {
+            const uint32_t r = x & 0x0FFFFFFFu;
+            sp = cell_points(hash, cell_start, cell_box_row(g, b, r), x >> 28);
+            if (sym && r == b.r_own) sp.x = q0;
         }
+        // ranges replace the row list from its start: at most as many as rows read so far
+        __syncwarp();
         const uint32_t len = sp.y - sp.x;
         const uint32_t some = __ballot_sync(0xffffffffu, len != 0u);
-        if (some == 0u) continue;
         uint32_t incl = len;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -144,6 +134,7 @@ __device__ __forceinline__ uint32_t warp_round(const HjGrid& g, const HjCellHash
         }
         run += __shfl_sync(0xffffffffu, incl, 31);
         nr += __popc(some);
+        __syncwarp();
     }
     if (lane_id() == 0) S.pre[nr] = run;
     *n_ranges = nr;
