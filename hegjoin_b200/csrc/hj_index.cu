@@ -207,23 +207,26 @@ __global__ void k_cell_ids(const T* __restrict__ db, uint32_t n, uint32_t d, Geo
     if (zero) atomicExch(silent, 1u);
 }
 
+// 1 where a run of equal keys begins.
 __global__ void k_run_flags(const unsigned long long* __restrict__ keys, uint32_t n, uint32_t* __restrict__ flags) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
 }
 
-__global__ void k_cells(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ flags,
-                        const uint32_t* __restrict__ pos, uint32_t n, unsigned long long* __restrict__ cell_lid,
-                        uint32_t* __restrict__ cell_start, uint32_t* n_cells_out) {
+// pos: exclusive scan of the run flags.
+__global__ void k_cells(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ pos, uint32_t n,
+                        unsigned long long* __restrict__ cell_lid, uint32_t* __restrict__ cell_start,
+                        uint32_t* n_cells_out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (flags[i]) {
+    const bool first = i == 0 || keys[i] != keys[i - 1];
+    if (first) {
         cell_lid[pos[i]] = keys[i];
         cell_start[pos[i]] = i;
     }
     if (i == n - 1) {
-        uint32_t nc = pos[i] + flags[i];
+        uint32_t nc = pos[i] + (first ? 1u : 0u);
         cell_start[nc] = n;
         *n_cells_out = nc;
     }
@@ -402,7 +405,7 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
     // temporaries: freed on every return path; the index's own arrays are freed by free_index on failure
     Scratch tmp(st);
     unsigned long long *keys = nullptr, *keys_tmp = nullptr;
-    uint32_t *vals_tmp = nullptr, *flags = nullptr, *pos = nullptr, *scalars = nullptr;
+    uint32_t *vals_tmp = nullptr, *pos = nullptr, *scalars = nullptr;
     HJ_TRY(tmp.alloc(&keys, n));
     HJ_TRY(tmp.alloc(&keys_tmp, n));
     HJ_TRY(dalloc(&ix->perm, n, st));
@@ -418,15 +421,13 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
                               vals_tmp, n, nbits, st));
     tmp.release(keys_tmp);
     tmp.release(vals_tmp);
-    HJ_TRY(tmp.alloc(&flags, n));
     HJ_TRY(tmp.alloc(&pos, n));
-    k_run_flags<<<grid1, 256, 0, st>>>(keys, n, flags);
+    k_run_flags<<<grid1, 256, 0, st>>>(keys, n, pos);
     HJ_LAUNCHED();
-    HJ_CUDA(cudaMemcpyAsync(pos, flags, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
     HJ_TRY(scan_u32_inplace(pos, n, st));
     HJ_TRY(dalloc(&ix->cell_lid, (size_t)n, st));
     HJ_TRY(dalloc(&ix->cell_start, (size_t)n + 1, st));
-    k_cells<<<grid1, 256, 0, st>>>(keys, flags, pos, n, ix->cell_lid, ix->cell_start, scalars + 1);
+    k_cells<<<grid1, 256, 0, st>>>(keys, pos, n, ix->cell_lid, ix->cell_start, scalars + 1);
     HJ_LAUNCHED();
     T* pts = nullptr;
     HJ_TRY(dalloc(&pts, (size_t)n * d, st));
@@ -452,11 +453,24 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
 // of the group's ids (its cells are the next ones in the table, at most four).
 // The key word pair is claimed with a 64-bit compare-and-swap on the entry's
 // first 8 bytes; first cell and mask are written after it.  The first cell of
-// each segment of 32 ids sets the segment's bits in the bitmap.  Every cell notes
-// whether a coordinate lies at the grid's edge.
+// each segment of 32 ids clears the segment's bits in the bitmap (a clear bit is a
+// cell: the bitmap and the table start as one array of set bits).  Every cell notes
+// whether a coordinate lies at the grid's edge.  The first threads also write the
+// grid's row offsets (HjGrid::row_off): entry r is the sum over j >= 1 of r's base-3
+// digits times the multipliers.
 __global__ void k_hash_insert(const unsigned long long* __restrict__ lid, uint32_t nC, HjGrid grid, uint4* entries,
-                              unsigned long long mask, uint32_t* occ, uint32_t occ_shift, uint8_t* __restrict__ edge) {
+                              unsigned long long mask, uint32_t* occ, uint32_t occ_shift, uint8_t* __restrict__ edge,
+                              unsigned long long* __restrict__ row_off) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < grid.full_rows) {
+        uint32_t rem = i;
+        unsigned long long o = 0;
+        for (uint32_t j = 1; j < grid.k; ++j) {
+            o += (unsigned long long)(rem % 3u) * grid.mult[j];
+            rem /= 3u;
+        }
+        row_off[i] = o;
+    }
     if (i >= nC) return;
     const unsigned long long me = lid[i], before = i > 0 ? lid[i - 1] : ~me;
     {
@@ -473,7 +487,7 @@ __global__ void k_hash_insert(const unsigned long long* __restrict__ lid, uint32
     if (i == 0 || (before >> 5) != (me >> 5)) {
         uint32_t bits = 0;
         for (uint32_t j = i; j < nC && (lid[j] >> 5) == (me >> 5); ++j) bits |= 1u << (uint32_t)(lid[j] & 31u);
-        atomicOr(occ + occ_word(me, occ_shift), bits);
+        atomicAnd(occ + occ_word(me, occ_shift), ~bits);
     }
     const unsigned long long g = me >> 2;
     if (i > 0 && (before >> 2) == g) return;
@@ -492,58 +506,41 @@ __global__ void k_hash_insert(const unsigned long long* __restrict__ lid, uint32
     }
 }
 
-// The grid's row-offset table (HjGrid::row_off), for k <= kRowOffMaxK.
-__global__ void k_row_offsets(HjGrid g, unsigned long long* off) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= g.full_rows) return;
-    uint32_t rem = r;
-    unsigned long long o = 0;
-    for (uint32_t j = 1; j < g.k; ++j) {
-        o += (unsigned long long)(rem % 3u) * g.mult[j];
-        rem /= 3u;
-    }
-    off[r] = o;
-}
-
-hj_status build_row_offsets(hj_index* ix, cudaStream_t st) {
-    if (ix->grid.k == 0 || ix->grid.k > kRowOffMaxK) return HJ_OK;
-    uint32_t rows = 1;
-    for (uint32_t j = 1; j < ix->grid.k; ++j) rows *= 3;
-    HJ_TRY(dalloc(&ix->row_off, rows, st));
-    ix->grid.full_rows = rows;
-    ix->grid.full_base = 1;
-    for (uint32_t j = 1; j < ix->grid.k; ++j) ix->grid.full_base += ix->grid.mult[j];
-    k_row_offsets<<<(rows + 255) / 256, 256, 0, st>>>(ix->grid, ix->row_off);
-    HJ_LAUNCHED();
-    ix->grid.row_off = ix->row_off;
-    return HJ_OK;
-}
-
-// The cell hash of an index whose cell table is built (capacity: the power of
-// two at least twice the number of cells, an upper bound on the groups that
-// needs no count from the device, at least 64) and its bitmap (a word per entry).
+// The cell hash of an index whose cell table is built: the table (capacity: the
+// power of two at least twice the number of cells, an upper bound on the groups
+// that needs no count from the device, at least 64), its bitmap (a word per entry)
+// and, for k <= kRowOffMaxK, the grid's row offsets.
 hj_status build_cell_hash(hj_index* ix, cudaStream_t st) {
     unsigned long long cap = 64;
     while (cap < 2ull * ix->nC) cap <<= 1;
-    HJ_TRY(dalloc(&ix->hash_entries, (size_t)cap, st));
-    HJ_CUDA(cudaMemsetAsync(ix->hash_entries, 0xFF, (size_t)cap * sizeof(uint4), st));
+    HJ_TRY(dalloc(&ix->hash_entries, (size_t)(cap + cap / 4), st));
+    HJ_CUDA(cudaMemsetAsync(ix->hash_entries, 0xFF, (size_t)(cap + cap / 4) * sizeof(uint4), st));
     ix->hash_mask = cap - 1;
-    HJ_TRY(dalloc(&ix->hash_occ, (size_t)cap, st));
-    HJ_CUDA(cudaMemsetAsync(ix->hash_occ, 0, (size_t)cap * 4, st));
-    HJ_TRY(dalloc(&ix->cell_edge, ix->nC, st));
+    ix->hash_occ = reinterpret_cast<uint32_t*>(ix->hash_entries + cap);
     ix->occ_shift = 65 - bits_for(cap);   // cap = 2^(bits - 1)
-    if (ix->nC) {
-        k_hash_insert<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->nC, ix->grid, ix->hash_entries,
-                                                           ix->hash_mask, ix->hash_occ, ix->occ_shift, ix->cell_edge);
-        HJ_LAUNCHED();
+    HJ_TRY(dalloc(&ix->cell_edge, ix->nC, st));
+    if (ix->grid.k <= kRowOffMaxK) {
+        uint32_t rows = 1;
+        ix->grid.full_base = 1;
+        for (uint32_t j = 1; j < ix->grid.k; ++j) {
+            rows *= 3;
+            ix->grid.full_base += ix->grid.mult[j];
+        }
+        HJ_TRY(dalloc(&ix->row_off, rows, st));
+        ix->grid.full_rows = rows;
+        ix->grid.row_off = ix->row_off;
     }
+    k_hash_insert<<<(std::max(ix->nC, ix->grid.full_rows) + 255) / 256, 256, 0, st>>>(
+        ix->cell_lid, ix->nC, ix->grid, ix->hash_entries, ix->hash_mask, ix->hash_occ, ix->occ_shift, ix->cell_edge,
+        ix->row_off);
+    HJ_LAUNCHED();
     return HJ_OK;
 }
 
 void free_index(hj_index* ix, cudaStream_t st) {
     tc_release(ix);
     dfree(ix->hash_entries, st);
-    dfree(ix->hash_occ, st);
+    ix->hash_occ = nullptr;   // part of the table's allocation
     dfree(ix->cell_edge, st);
     dfree(ix->row_off, st);
     ix->grid.row_off = nullptr;
@@ -706,7 +703,6 @@ hj_status hj_index_create(const void* d_db, uint32_t n, uint32_t d, uint32_t k, 
                       : index_create_t<double>((const double*)d_db, n, d, k, eps, h_min_arr, h_n_cells, st, ix);
     // linear ids are below totalCells <= 2^64 - 1, so none equals the hash's free-slot mark
     if (s == HJ_OK) s = build_cell_hash(ix, st);
-    if (s == HJ_OK) s = build_row_offsets(ix, st);
     if (s != HJ_OK) {
         free_index(ix, st);
         cudaStreamSynchronize(st);

@@ -238,11 +238,12 @@ __device__ __forceinline__ uint2 group_find(const HjCellHash& h, unsigned long l
 }
 
 // Bit i set: the bitmap knows a cell lo + i, i < w <= 4 (or one that shares its bit).
+// In the bitmap itself a cell's bit is clear.
 __device__ __forceinline__ uint32_t occ_row(const HjCellHash& h, unsigned long long lo, uint32_t w) {
     const uint32_t b = (uint32_t)lo & 31u;
     uint32_t m = __ldg(h.occ + occ_word(lo, h.occ_shift)) >> b;
     if (b + w > 32u) m |= __ldg(h.occ + occ_word(lo + w - 1, h.occ_shift)) << (32u - b);
-    return m & ((1u << w) - 1u);
+    return ~m & ((1u << w) - 1u);
 }
 
 // The existing cells among those named by `m` (occ_row's answer) from id lo on:

@@ -4,8 +4,9 @@
 // (GPU.cu:249-251, GPU.cu:285, GPU.cu:1543).  The radix sort is a
 // reduce-then-scan LSD sort with 8-bit digits: per pass a tile histogram
 // kernel, an exclusive scan of the (digit-major) histogram table and a stable
-// scatter that ranks each tile's keys in shared memory.  Only the low `nbits`
-// key bits are sorted, so a 21-bit point-id key costs three passes.
+// scatter that ranks each tile's keys warp by warp.  Only the low `nbits` key bits
+// are sorted, so a 21-bit point-id key costs three passes.  A small input is sorted
+// by one block in one launch.
 
 #include "hj_common.cuh"
 
@@ -152,52 +153,136 @@ __global__ void k_rs_hist(const K* __restrict__ keys, uint64_t n, uint32_t shift
     }
 }
 
-// Stable scatter: tile elements are visited in order (round r covers tile
-// positions [r*256, r*256+256)), ranked by (earlier rounds, earlier warps,
-// earlier lanes) among keys with the same digit.
+// Ranks of a warp's keys among the warp's earlier keys with the same digit, key by
+// key in order: cnt (256 counters of this warp, zeroed) holds the digits' counts
+// afterwards.  dgt 256 marks a lane without a key.
+__device__ __forceinline__ uint32_t warp_rank(uint32_t dgt, uint32_t* cnt) {
+    const uint32_t peers = __match_any_sync(0xffffffffu, dgt);
+    const uint32_t before = peers & lanemask_lt();
+    const uint32_t first = dgt < kRadix ? cnt[dgt] : 0u;
+    __syncwarp();
+    if (before == 0u && dgt < kRadix) cnt[dgt] = first + __popc(peers);
+    __syncwarp();
+    return first + __popc(before);
+}
+
+// Stable scatter of one tile.  Each warp takes 512 consecutive keys and ranks them
+// among its own (no block barrier); one prefix over the warps per digit then gives
+// every key its place.  Two barriers per tile; ranking 256 keys at a time over the
+// whole block took four per 256 keys.  10M (u64, u32) pairs per pass: 134 us before.
 template <typename K>
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__ keys, const uint32_t* __restrict__ vals,
                                                            K* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                            uint64_t n, uint32_t shift, const uint32_t* __restrict__ offs,
                                                            uint32_t ntiles) {
-    __shared__ uint32_t run[kRadix];           // running count per digit (tile-global offset)
-    __shared__ uint32_t wcnt[kRsWarps][kRadix + 1];
-    for (int dgt = threadIdx.x; dgt < kRadix; dgt += kRsThreads) run[dgt] = offs[(uint64_t)dgt * ntiles + blockIdx.x];
-    for (int i = threadIdx.x; i < kRsWarps * (kRadix + 1); i += kRsThreads) (&wcnt[0][0])[i] = 0;
-    __syncthreads();
-    uint64_t base = (uint64_t)blockIdx.x * kRsTile;
+    __shared__ uint32_t wcnt[kRsWarps][kRadix];
+    static_assert(kRsThreads == kRadix, "a thread per digit");
     const uint32_t w = threadIdx.x >> 5, lane = lane_id();
+    for (int i = lane; i < kRadix; i += 32) wcnt[w][i] = 0;
+    __syncwarp();
+    const uint64_t base = (uint64_t)blockIdx.x * kRsTile + w * (kRsTile / kRsWarps);
+    K key[kRsItems];
+    uint32_t val[kRsItems], rank[kRsItems];
+#pragma unroll
     for (int r = 0; r < kRsItems; ++r) {
-        uint64_t idx = base + (uint64_t)r * kRsThreads + threadIdx.x;
-        bool valid = idx < n;
-        K key = valid ? keys[idx] : K(0);
-        uint32_t val = valid ? vals[idx] : 0u;
-        uint32_t dgt = valid ? ((uint32_t)(key >> shift) & 0xFFu) : (uint32_t)kRadix;
-        uint32_t peers = __match_any_sync(0xffffffffu, dgt);
-        uint32_t rank = __popc(peers & lanemask_lt());
-        uint32_t leader = __ffs(peers) - 1;
-        if (lane == leader) wcnt[w][dgt] = __popc(peers);
+        const uint64_t idx = base + (uint64_t)r * 32 + lane;
+        key[r] = idx < n ? keys[idx] : K(0);
+        val[r] = idx < n ? vals[idx] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < kRsItems; ++r) {
+        const bool valid = base + (uint64_t)r * 32 + lane < n;
+        rank[r] = warp_rank(valid ? (uint32_t)(key[r] >> shift) & 0xFFu : (uint32_t)kRadix, wcnt[w]);
+    }
+    __syncthreads();
+    uint32_t acc = offs[(uint64_t)threadIdx.x * ntiles + blockIdx.x];
+#pragma unroll
+    for (int j = 0; j < kRsWarps; ++j) {
+        const uint32_t c = wcnt[j][threadIdx.x];
+        wcnt[j][threadIdx.x] = acc;
+        acc += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRsItems; ++r) {
+        if (base + (uint64_t)r * 32 + lane >= n) continue;
+        const uint32_t dst = wcnt[w][(uint32_t)(key[r] >> shift) & 0xFFu] + rank[r];
+        keys_out[dst] = key[r];
+        vals_out[dst] = val[r];
+    }
+}
+
+// A whole sort of up to kRsSmall pairs by one block, in shared memory: every pass of
+// a small input in one launch instead of three each.
+constexpr uint32_t kRsSmall = 7168;
+constexpr int kRsSmallThreads = 1024;
+template <typename K>
+constexpr size_t rs_small_bytes(uint64_t n) {
+    return 2 * n * (sizeof(K) + sizeof(uint32_t)) + (kRsSmallThreads / 32) * kRadix * sizeof(uint32_t);
+}
+template <typename K>
+__global__ void __launch_bounds__(kRsSmallThreads) k_rs_small(K* keys, uint32_t* vals, uint32_t n, uint32_t passes) {
+    extern __shared__ __align__(16) unsigned char rs_smem[];
+    K* kb[2] = {reinterpret_cast<K*>(rs_smem), reinterpret_cast<K*>(rs_smem) + n};
+    uint32_t* vb[2] = {reinterpret_cast<uint32_t*>(kb[1] + n), reinterpret_cast<uint32_t*>(kb[1] + n) + n};
+    uint32_t* cnt = vb[1] + n;                       // [32 warps][256]
+    __shared__ uint32_t wtot[8];
+    constexpr uint32_t kWarps = kRsSmallThreads / 32;
+    const uint32_t w = threadIdx.x >> 5, lane = lane_id();
+    for (uint32_t i = threadIdx.x; i < n; i += kRsSmallThreads) {
+        kb[0][i] = keys[i];
+        vb[0][i] = vals[i];
+    }
+    const uint32_t per = ((n + kWarps - 1) / kWarps + 31) / 32 * 32;   // consecutive keys per warp
+    uint32_t src = 0;
+    for (uint32_t p = 0; p < passes; ++p) {
+        for (uint32_t i = threadIdx.x; i < kWarps * kRadix; i += kRsSmallThreads) cnt[i] = 0;
         __syncthreads();
-        // per digit: exclusive prefix across warps, then advance the running count
-        for (int dd = threadIdx.x; dd < kRadix; dd += kRsThreads) {
-            uint32_t acc = run[dd];
-            for (int j = 0; j < kRsWarps; ++j) {
-                uint32_t c = wcnt[j][dd];
-                wcnt[j][dd] = acc;
-                acc += c;
+        for (uint32_t i0 = 0; i0 < per; i0 += 32) {
+            const uint32_t i = w * per + i0 + lane;
+            warp_rank(i < n ? (uint32_t)(kb[src][i] >> (8 * p)) & 0xFFu : (uint32_t)kRadix, cnt + w * kRadix);
+        }
+        __syncthreads();
+        // first place of every (digit, warp): prefix over the warps, then over the digits
+        uint32_t total = 0, incl = 0;
+        if (threadIdx.x < kRadix) {
+            for (uint32_t j = 0; j < kWarps; ++j) {
+                const uint32_t c = cnt[j * kRadix + threadIdx.x];
+                cnt[j * kRadix + threadIdx.x] = total;
+                total += c;
             }
-            run[dd] = acc;
+            incl = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += x;
+            }
+            if (lane == 31) wtot[w] = incl;
         }
         __syncthreads();
-        if (valid) {
-            uint32_t dst = wcnt[w][dgt] + rank;
-            keys_out[dst] = key;
-            vals_out[dst] = val;
+        if (threadIdx.x < kRadix) {
+            uint32_t first = incl - total;
+            for (uint32_t j = 0; j < w; ++j) first += wtot[j];
+            for (uint32_t j = 0; j < kWarps; ++j) cnt[j * kRadix + threadIdx.x] += first;
         }
         __syncthreads();
-        // every digit slot now holds a prefix value; reset the table for the next round
-        for (int j = threadIdx.x; j < kRsWarps * (kRadix + 1); j += kRsThreads) (&wcnt[0][0])[j] = 0;
+        for (uint32_t i0 = 0; i0 < per; i0 += 32) {
+            const uint32_t i = w * per + i0 + lane;
+            const bool valid = i < n;
+            const K key = valid ? kb[src][i] : K(0);
+            const uint32_t dst =
+                warp_rank(valid ? (uint32_t)(key >> (8 * p)) & 0xFFu : (uint32_t)kRadix, cnt + w * kRadix);
+            if (valid) {
+                kb[src ^ 1][dst] = key;
+                vb[src ^ 1][dst] = vb[src][i];
+            }
+        }
+        src ^= 1;
         __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += kRsSmallThreads) {
+        keys[i] = kb[src][i];
+        vals[i] = vb[src][i];
     }
 }
 
@@ -209,13 +294,20 @@ hj_status radix_sort(K* keys, uint32_t* vals, K* keys_tmp, uint32_t* vals_tmp, u
         set_error("radix sort: %llu elements exceed 2^32", (unsigned long long)n);
         return HJ_ERR_INVALID;
     }
+    const uint32_t passes = (nbits + 7) / 8;
+    if (n <= kRsSmall) {
+        const size_t smem = rs_small_bytes<K>(n);
+        HJ_TRY(ensure_smem(k_rs_small<K>, smem));
+        k_rs_small<K><<<1, kRsSmallThreads, smem, st>>>(keys, vals, (uint32_t)n, passes);
+        HJ_LAUNCHED();
+        return HJ_OK;
+    }
     uint32_t ntiles = (uint32_t)((n + kRsTile - 1) / kRsTile);
     Scratch tmp(st);
     uint32_t* hist = nullptr;
     HJ_TRY(tmp.alloc(&hist, (size_t)kRadix * ntiles));
     K* src_k = keys; uint32_t* src_v = vals;
     K* dst_k = keys_tmp; uint32_t* dst_v = vals_tmp;
-    uint32_t passes = (nbits + 7) / 8;
     for (uint32_t p = 0; p < passes; ++p) {
         uint32_t shift = p * 8;
         k_rs_hist<K><<<ntiles, kRsThreads, 0, st>>>(src_k, n, shift, hist, ntiles);
