@@ -54,6 +54,21 @@ bool injected_alloc_failure() {
     return g_fail_alloc_in.fetch_sub(1, std::memory_order_relaxed) == 1;
 }
 
+namespace {
+struct Readback {
+    void* p = nullptr;
+    ~Readback() {
+        if (p) cudaFreeHost(p);
+    }
+};
+thread_local Readback t_readback;
+}  // namespace
+hj_status readback_buffer(void** p) {
+    if (!t_readback.p) HJ_CUDA(cudaMallocHost(&t_readback.p, kReadbackBytes));
+    *p = t_readback.p;
+    return HJ_OK;
+}
+
 hj_status ensure_smem_ptr(const void* kern, size_t bytes) {
     static std::mutex mu;
     static std::map<const void*, size_t> done;
@@ -157,14 +172,16 @@ __global__ void k_minmax(const T* __restrict__ db, uint32_t n, uint32_t d, uint3
 template <typename T>
 hj_status geometry_t(const T* db, uint32_t n, uint32_t d, uint32_t k, T eps, double* h_min, double* h_max,
                      uint32_t* h_ncells, uint64_t* h_total, cudaStream_t st) {
-    const int blocks = std::min<int>(num_sms() * 4, std::max<uint32_t>(1, (n + 255) / 256));
+    const int blocks = std::min<int>(std::min(num_sms() * 4, 592), std::max<uint32_t>(1, (n + 255) / 256));
     Scratch tmp(st);
     T* part = nullptr;
     HJ_TRY(tmp.alloc(&part, (size_t)2 * blocks * k));
     k_minmax<T><<<blocks, 256, 0, st>>>(db, n, d, k, part, part + (size_t)k * blocks);
     HJ_LAUNCHED();
-    std::vector<T> hp((size_t)2 * blocks * k);
-    HJ_CUDA(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(T), cudaMemcpyDeviceToHost, st));
+    static_assert(2 * 592 * kMaxK * sizeof(double) <= kReadbackBytes, "partials of 592 blocks");
+    T* hp = nullptr;
+    HJ_TRY(readback_buffer(reinterpret_cast<void**>(&hp)));
+    HJ_CUDA(cudaMemcpyAsync(hp, part, (size_t)2 * blocks * k * sizeof(T), cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaStreamSynchronize(st));
     uint64_t total = 1;
     for (uint32_t j = 0; j < k; ++j) {
@@ -331,6 +348,7 @@ __global__ void __launch_bounds__(256) k_cell_keys(const unsigned long long* __r
 __global__ void k_block_counts(const uint32_t* __restrict__ order, const uint32_t* __restrict__ cell_start, uint32_t nC,
                                uint32_t qb, uint32_t align, uint32_t* __restrict__ cnt) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == nC) cnt[nC] = 0;   // the scan's total goes there
     if (i >= nC) return;
     uint32_t c = order[i];
     uint32_t s = cell_start[c] & ~(align - 1u);
@@ -435,8 +453,9 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
     unsigned grid2 = (unsigned)std::min<uint64_t>(((uint64_t)n * d + 255) / 256, (uint64_t)num_sms() * 16);
     k_gather_rows<T><<<grid2, 256, 0, st>>>(d_db, ix->perm, n, d, pts);
     HJ_LAUNCHED();
-    uint32_t hs[3];
-    HJ_CUDA(cudaMemcpyAsync(hs, scalars, sizeof(hs), cudaMemcpyDeviceToHost, st));
+    uint32_t* hs = nullptr;
+    HJ_TRY(readback_buffer(reinterpret_cast<void**>(&hs)));
+    HJ_CUDA(cudaMemcpyAsync(hs, scalars, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaStreamSynchronize(st));
     ix->aliasing = hs[0];
     ix->nC = hs[1];
@@ -589,24 +608,66 @@ hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st) {
     return HJ_OK;
 }
 
-hj_status build_blocks(const hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
+// Launches of the workload order; *folded (in tmp) then holds totalCandidates and the
+// largest count, for workload_done.
+static hj_status workload_launch(hj_index* ix, Scratch& tmp, unsigned long long** folded_out, cudaStream_t st) {
+    const uint32_t nC = ix->nC;
+    // a previous attempt that failed part-way may have left these allocated
+    dfree(ix->cell_nb, st);
+    dfree(ix->cell_order, st);
+    unsigned long long* folded = nullptr;
+    uint32_t *keys = nullptr, *keys_tmp = nullptr, *vals_tmp = nullptr;
+    HJ_TRY(dalloc(&ix->cell_nb, nC, st));
+    HJ_TRY(dalloc(&ix->cell_order, nC, st));
+    HJ_TRY(tmp.alloc(&folded, 2));
+    HJ_TRY(tmp.alloc(&keys, nC));
+    HJ_TRY(tmp.alloc(&keys_tmp, nC));
+    HJ_TRY(tmp.alloc(&vals_tmp, nC));
+    HJ_CUDA(cudaMemsetAsync(ix->cell_nb, 0, (size_t)nC * 4, st));
+    HJ_CUDA(cudaMemsetAsync(folded, 0, 2 * sizeof(unsigned long long), st));
+    unsigned g = (unsigned)(((uint64_t)nC * 32 + 255) / 256);
+    k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->cell_edge, nC, ix->grid, cell_hash(ix),
+                                       ix->cell_nb);
+    HJ_LAUNCHED();
+    // no count exceeds n: the sort needs only that many bits
+    const uint32_t nbits = bits_for(ix->n);
+    k_cell_keys<<<(nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, ix->any_silent,
+                                                  (uint32_t)((1ull << nbits) - 1), ix->cell_nb, keys, ix->cell_order,
+                                                  folded);
+    HJ_LAUNCHED();
+    HJ_TRY(radix_sort_u32_u32(keys, ix->cell_order, keys_tmp, vals_tmp, nC, nbits, st));
+    *folded_out = folded;
+    return HJ_OK;
+}
+static void workload_done(hj_index* ix, const unsigned long long* folded) {
+    ix->total_candidates = folded[0];
+    ix->max_nb = (uint32_t)folded[1];
+    ix->have_workload = true;
+}
+
+hj_status build_blocks(hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
                        cudaStream_t st) {
-    uint32_t nC = ix->nC;
+    const uint32_t nC = ix->nC;
     Scratch tmp(st);
+    unsigned long long *folded = nullptr, *back = nullptr;
+    HJ_TRY(readback_buffer(reinterpret_cast<void**>(&back)));
+    if (!ix->have_workload) {
+        HJ_TRY(workload_launch(ix, tmp, &folded, st));
+        HJ_CUDA(cudaMemcpyAsync(back + 1, folded, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    }
     uint32_t* cnt = nullptr;
     HJ_TRY(tmp.alloc(&cnt, (size_t)nC + 1));
-    unsigned g = (nC + 255) / 256;
-    k_block_counts<<<g, 256, 0, st>>>(ix->cell_order, ix->cell_start, nC, qb, align, cnt);
+    k_block_counts<<<nC / 256 + 1, 256, 0, st>>>(ix->cell_order, ix->cell_start, nC, qb, align, cnt);
     HJ_LAUNCHED();
-    HJ_CUDA(cudaMemsetAsync(cnt + nC, 0, 4, st));
     HJ_TRY(scan_u32_inplace(cnt, (uint64_t)nC + 1, st));
-    uint32_t nb = 0;
-    HJ_CUDA(cudaMemcpyAsync(&nb, cnt + nC, 4, cudaMemcpyDeviceToHost, st));
+    HJ_CUDA(cudaMemcpyAsync(back, cnt + nC, 4, cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaStreamSynchronize(st));
+    if (folded) workload_done(ix, back + 1);
+    const uint32_t nb = *reinterpret_cast<const uint32_t*>(back);
     HjBlock* blocks = nullptr;
     HJ_TRY(tmp.alloc_pool(&blocks, (size_t)std::max<uint32_t>(nb, 1)));   // handed to the caller
-    k_make_blocks<<<g, 256, 0, st>>>(ix->cell_order, ix->cell_start, ix->cell_nb, cnt, nC, qb, align,
-                                      blocks);
+    k_make_blocks<<<(nC + 255) / 256, 256, 0, st>>>(ix->cell_order, ix->cell_start, ix->cell_nb, cnt, nC, qb, align,
+                                                    blocks);
     HJ_LAUNCHED();
     *d_blocks = tmp.keep(blocks);
     *n_blocks = nb;
@@ -766,39 +827,13 @@ hj_status hj_sort_by_workload(hj_index* ix, void* stream, uint64_t* total_candid
     if (!ix) { set_error("hj_sort_by_workload: null index"); return HJ_ERR_INVALID; }
     cudaStream_t st = as_stream(stream);
     if (!ix->have_workload) {
-        uint32_t nC = ix->nC;
-        // a previous attempt that failed part-way may have left these allocated
-        dfree(ix->cell_nb, st);
-        dfree(ix->cell_order, st);
         Scratch tmp(st);
-        unsigned long long* folded = nullptr;   // totalCandidates, largest count
-        uint32_t *keys = nullptr, *keys_tmp = nullptr, *vals_tmp = nullptr;
-        HJ_TRY(dalloc(&ix->cell_nb, nC, st));
-        HJ_TRY(dalloc(&ix->cell_order, nC, st));
-        HJ_TRY(tmp.alloc(&folded, 2));
-        HJ_TRY(tmp.alloc(&keys, nC));
-        HJ_TRY(tmp.alloc(&keys_tmp, nC));
-        HJ_TRY(tmp.alloc(&vals_tmp, nC));
-        HJ_CUDA(cudaMemsetAsync(ix->cell_nb, 0, (size_t)nC * 4, st));
-        HJ_CUDA(cudaMemsetAsync(folded, 0, 2 * sizeof(unsigned long long), st));
-        unsigned g = (unsigned)(((uint64_t)nC * 32 + 255) / 256);
-        k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->cell_edge, nC, ix->grid, cell_hash(ix),
-                                           ix->cell_nb);
-        HJ_LAUNCHED();
-        // no count exceeds n: the sort needs only that many bits
-        const uint32_t nbits = bits_for(ix->n);
-        k_cell_keys<<<(nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, ix->any_silent,
-                                                      (uint32_t)((1ull << nbits) - 1), ix->cell_nb, keys,
-                                                      ix->cell_order, folded);
-        HJ_LAUNCHED();
-        HJ_TRY(radix_sort_u32_u32(keys, ix->cell_order, keys_tmp, vals_tmp, nC, nbits, st));
-        unsigned long long hf[2] = {0, 0};
-        HJ_CUDA(cudaMemcpyAsync(hf, folded, sizeof(hf), cudaMemcpyDeviceToHost, st));
+        unsigned long long *folded = nullptr, *back = nullptr;
+        HJ_TRY(readback_buffer(reinterpret_cast<void**>(&back)));
+        HJ_TRY(hj::workload_launch(ix, tmp, &folded, st));
+        HJ_CUDA(cudaMemcpyAsync(back, folded, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
-        const uint64_t tot = hf[0];
-        ix->max_nb = (uint32_t)hf[1];
-        ix->total_candidates = tot;
-        ix->have_workload = true;
+        hj::workload_done(ix, back);
     }
     if (total_candidates) *total_candidates = ix->total_candidates;
     return HJ_OK;

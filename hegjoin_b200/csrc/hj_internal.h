@@ -116,8 +116,9 @@ hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st);
 // hj_index.cu
 // Work items of up to qb queries per cell, in the workload order; `align` (a
 // power of two): a cell's items after its first start at multiples of it and
-// fill whole groups, the first begins at the cell's first point.
-hj_status build_blocks(const hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
+// fill whole groups, the first begins at the cell's first point.  Makes the workload
+// order first if the index has none yet (one synchronisation for both).
+hj_status build_blocks(hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_blocks, uint32_t* n_blocks,
                        cudaStream_t st);
 
 constexpr unsigned long long kEmptyLid = ~0ull;

@@ -82,13 +82,18 @@ namespace {
 // The estimator's sample: every stride-th work item, of each at most max_q queries
 // (the estimate is a rate per query).
 __global__ void k_pick_samples(const HjBlock* __restrict__ blocks, uint32_t nblocks, uint32_t stride,
-                               uint32_t nsamp, uint32_t max_q, HjBlock* __restrict__ out) {
+                               uint32_t nsamp, uint32_t max_q, HjBlock* __restrict__ out,
+                               unsigned long long* __restrict__ cnt) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nsamp) return;
+    cnt[i] = 0;
     HjBlock b = blocks[min(nblocks - 1, i * stride)];
     b.q1 = min(b.q1, b.q0 + max_q);
     out[i] = b;
 }
+
+// Largest result buffer that is sized by the number of candidates instead of an estimate.
+constexpr double kBoundedBytes = 64.0 * 1024 * 1024;
 
 // Queries per sampled item of the warp refine, whose cost is queries x candidates
 // (the tensor-core filter's is candidate tiles: it takes whole items).
@@ -173,10 +178,13 @@ struct JoinCtl {
     uint32_t pad_;
 };
 
-// Start of a batch: both sink cursors, the overflow flag, the queue head and the
-// filter's counters (the host adds up those of the batches that did not overflow).
-__global__ void k_batch_reset(JoinCtl* c) {
-    if (threadIdx.x == 0) {
+// Start of a batch: both sink cursors, the overflow flag, the queue head, the filter's
+// counters (the host adds up those of the batches that did not overflow) and the
+// per-query counts.
+__global__ void __launch_bounds__(256) k_batch_reset(JoinCtl* c, uint32_t* __restrict__ qcount, uint64_t m) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
+        qcount[i] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         c->cursor = 0;
         c->band_cursor = 0;
         c->valid = 0;
@@ -716,8 +724,6 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     Scratch tmp(st);
     uint64_t launches0 = thread_launch_count();
     hj_join_stats S{};
-    HJ_TRY(hj_sort_by_workload(ix, st, nullptr));
-
     // ---- refine kind
     int refine = opts.refine;
     const bool auto_kind = refine == HJ_REFINE_AUTO;
@@ -846,17 +852,6 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         if (!count_only) HJ_CUDA(cudaEventRecord(e1, st));
         return HJ_OK;
     };
-    auto check_timeout = [&]() -> hj_status {
-        uint32_t to = 0;
-        HJ_CUDA(cudaMemcpyAsync(&to, &ctl->timeout, 4, cudaMemcpyDeviceToHost, st));
-        HJ_CUDA(cudaStreamSynchronize(st));
-        if (to) {
-            set_error("hj_join: a bounded device-side wait expired in the tensor-core pipeline");
-            return HJ_ERR_TIMEOUT;
-        }
-        return HJ_OK;
-    };
-
     // ---- digests that nobody wants the pairs of: one launch, no estimate, no batches.  Only
     // without limits on buffers and batches, which such a join would never meet.
     DigestOut dig;
@@ -869,11 +864,12 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         HJ_CUDA(cudaEventRecord(kev.ev[0].first, st));
         HJ_TRY(launch_refine_digest(ix, blocks, nblocks, avg_work, head, dig.count, dig.sum, dig.xr, &ctl->valid, st));
         HJ_CUDA(cudaEventRecord(kev.ev[0].second, st));
-        JoinCtl hc;
-        HJ_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
+        JoinCtl* hc = nullptr;
+        HJ_TRY(readback_buffer(reinterpret_cast<void**>(&hc)));
+        HJ_CUDA(cudaMemcpyAsync(hc, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
         HJ_CUDA(cudaEventElapsedTime(&S.ms_refine_kernel, kev.ev[0].first, kev.ev[0].second));
-        S.total_pairs = S.estimated_pairs = hc.valid;
+        S.total_pairs = S.estimated_pairs = hc->valid;
         S.n_batches = nblocks ? 1 : 0;
         S.refine_launches = nblocks ? 1 : 0;
         S.ms_total = ms_since(t_start);
@@ -882,6 +878,19 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         if (stats) *stats = S;
         return HJ_OK;
     }
+
+    // ---- slots of the result buffer
+    // slack for partly filled warp chunks: every warp that can emit during a batch holds
+    // at most one (sized from the launch grids, so small joins get small buffers)
+    const uint64_t chunk_slack = tc     ? tc_emit_warps(nblocks) * kSinkChunk
+                                 : warp ? warp_chunk_slack(nblocks, avg_work)
+                                        : plain_emit_warps(nblocks) * kSinkChunk;
+    // keys, vals (+ band pair ids; + one or two sets of grouped copies unless the handler
+    // brings its own arrays)
+    const bool overlap = opts.stream_overlap && handler.can_overlap();
+    const uint32_t base_words = tc ? 4u : 2u;
+    const uint32_t slot_words = base_words + (handler.own_arrays() ? 0u : overlap ? 4u : 2u);
+    const double bytes_per_slot = 4.0 * slot_words;
 
     // ---- estimator (GPUBatchEst_v2, GPU.cu:403-779)
     auto t_est = std::chrono::steady_clock::now();
@@ -900,16 +909,27 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         }
     }
     double total_est = 0, cand_total = 0;
-    double* pest = nullptr;   // exclusive prefix of the per-item estimates (nblocks + 1)
-    double* dsum = nullptr;
-    if (nsamp) {
+    double* pest = nullptr;   // exclusive prefix of the per-item estimates (nblocks + 1), then the candidates
+    // A join's pairs are among its candidates: where a buffer for all of those is small,
+    // it takes the place of the estimate (a tenth of a small join's time).
+    const uint64_t bound_slots = ix->total_candidates + chunk_slack + 4096;
+    const double bound_bytes = (double)bound_slots * bytes_per_slot;
+    const bool bounded = !opts.result_capacity && bound_bytes <= kBoundedBytes &&
+                         (!opts.device_bytes_cap ||
+                          bound_bytes + 1.1 * kept_bytes_per_pair * (double)ix->total_candidates +
+                                  (double)fixed_kept_bytes <= (double)opts.device_bytes_cap);
+    if (bounded) {
+        total_est = cand_total = (double)ix->total_candidates;
+        int tuned = 0;
+        if (!tc && !warp && tune_lookup(tune_key(refine, ix->d, ix->dtype), &tuned)) ix->plain_shape = tuned;
+    }
+    if (nsamp && !bounded) {
         HjBlock* sblocks = nullptr;
         unsigned long long* scnt = nullptr;
         HJ_TRY(tmp.alloc(&sblocks, nsamp));
         HJ_TRY(tmp.alloc(&scnt, nsamp));
-        HJ_CUDA(cudaMemsetAsync(scnt, 0, nsamp * sizeof(unsigned long long), st));
         k_pick_samples<<<(nsamp + 255) / 256, 256, 0, st>>>(blocks, nblocks, stride, nsamp,
-                                                           warp ? kSampleQueries : 0x7FFFFFFFu, sblocks);
+                                                           warp ? kSampleQueries : 0x7FFFFFFFu, sblocks, scnt);
         HJ_LAUNCHED();
         PairSink none{nullptr, nullptr, nullptr, 0, overflow};
         int tuned = 0;
@@ -942,21 +962,24 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         } else {
             if (!tc) ix->plain_shape = tuned;
             HJ_TRY(run_refine(sblocks, nsamp, none, no_band, 1, scnt));
-            HJ_TRY(check_timeout());
         }
         // per-item estimates and their exclusive prefix on the device; the host reads the
         // totals only (the item list of a sparse dataset runs to millions of entries)
-        HJ_TRY(tmp.alloc(&pest, (size_t)nblocks + 1));
-        HJ_TRY(tmp.alloc(&dsum, 1));
-        HJ_CUDA(cudaMemsetAsync(dsum, 0, sizeof(double), st));
+        HJ_TRY(tmp.alloc(&pest, (size_t)nblocks + 2));
+        HJ_CUDA(cudaMemsetAsync(pest + nblocks + 1, 0, sizeof(double), st));
         k_item_estimates<<<(nblocks + 256) / 256, 256, 0, st>>>(blocks, nblocks, stride, nsamp, sblocks, scnt, pest,
-                                                                 dsum);
+                                                                 pest + nblocks + 1);
         HJ_LAUNCHED();
         HJ_TRY(scan_f64_inplace(pest, (uint64_t)nblocks + 1, st));
-        double hsum[2] = {0, 0};
-        HJ_CUDA(cudaMemcpyAsync(&hsum[0], pest + nblocks, sizeof(double), cudaMemcpyDeviceToHost, st));
-        HJ_CUDA(cudaMemcpyAsync(&hsum[1], dsum, sizeof(double), cudaMemcpyDeviceToHost, st));
+        double* hsum = nullptr;
+        HJ_TRY(readback_buffer(reinterpret_cast<void**>(&hsum)));
+        HJ_CUDA(cudaMemcpyAsync(hsum, pest + nblocks, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+        HJ_CUDA(cudaMemcpyAsync(hsum + 2, &ctl->timeout, 4, cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
+        if (*reinterpret_cast<const uint32_t*>(hsum + 2)) {
+            set_error("hj_join: a bounded device-side wait expired in the tensor-core pipeline");
+            return HJ_ERR_TIMEOUT;
+        }
         total_est = hsum[0];
         cand_total = hsum[1];
     }
@@ -965,18 +988,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     if (tc) tc_set_dense(ix, dense_for(total_est, cand_total));
 
     // ---- result buffer capacity
-    // slack for partly filled warp chunks: every warp that can emit during a batch holds
-    // at most one (sized from the launch grids, so small joins get small buffers)
-    const uint64_t chunk_slack = tc     ? tc_emit_warps(nblocks) * kSinkChunk
-                                 : warp ? warp_chunk_slack(nblocks, avg_work)
-                                        : plain_emit_warps(nblocks) * kSinkChunk;
-    // keys, vals (+ band pair ids; + one or two sets of grouped copies unless the handler
-    // brings its own arrays)
-    const bool overlap = opts.stream_overlap && handler.can_overlap();
-    const uint32_t base_words = tc ? 4u : 2u;
-    const uint32_t slot_words = base_words + (handler.own_arrays() ? 0u : overlap ? 4u : 2u);
-    const double bytes_per_slot = 4.0 * slot_words;
-    const uint64_t want = (uint64_t)(total_est * 2.0) + chunk_slack + 4096;
+    const uint64_t want = bounded ? bound_slots : (uint64_t)(total_est * 2.0) + chunk_slack + 4096;
     uint64_t cap = opts.result_capacity ? opts.result_capacity + chunk_slack : want;
     if (cap < chunk_slack * 2) cap = chunk_slack * 2;
     const double result_bytes = kept_bytes_per_pair * total_est * 1.1;   // what the handler keeps
@@ -1020,7 +1032,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     if (nblocks) {
         const double budget = 0.5 * (double)(cap - chunk_slack);
         std::vector<uint32_t> cuts;
-        if (nblocks > 1 && total_est >= budget) {
+        if (nblocks > 1 && !bounded && total_est >= budget) {
             uint32_t* dcuts = nullptr;
             unsigned int* dn = nullptr;
             HJ_TRY(tmp.alloc(&dcuts, nblocks));
@@ -1080,24 +1092,26 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             set_error("hj_join: batch limit %u reached", opts.max_batches);
             return HJ_ERR_OVERFLOW;
         }
-        k_batch_reset<<<1, 32, 0, st>>>(ctl);
+        k_batch_reset<<<(unsigned)std::min<uint64_t>(((uint64_t)ix->n + 256) / 256, (uint64_t)num_sms() * 8), 256, 0,
+                        st>>>(ctl, qoff, (uint64_t)ix->n + 1);
         HJ_LAUNCHED();
         PairSink sink{keys, vals, &ctl->cursor, cap, overflow};
         PairSink band = tc ? PairSink{band_q, band_c, &ctl->band_cursor, cap, overflow} : no_band;
         // all items of the join in this one batch: every unordered pair once (a query's pairs
         // must lie in one batch, and a shard owns its queries' pairs only)
         const bool sym = (tc || warp) && opts.shard_count <= 1 && b.b0 == 0 && b.b1 == nblocks;
-        HJ_CUDA(cudaMemsetAsync(qoff, 0, ((size_t)ix->n + 1) * 4, st));
         HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, qoff, sym));
         if (tc)
             HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, qoff, st));
         // every query's first slot; qoff[n] = the batch's pairs
         HJ_TRY(scan_u32_inplace(qoff, (uint64_t)ix->n + 1, st));
-        uint32_t valid = 0;
-        HJ_CUDA(cudaMemcpyAsync(&valid, qoff + ix->n, 4, cudaMemcpyDeviceToHost, st));
-        JoinCtl hc;
-        HJ_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
+        struct { JoinCtl ctl; uint32_t valid; }* back = nullptr;
+        HJ_TRY(readback_buffer(reinterpret_cast<void**>(&back)));
+        HJ_CUDA(cudaMemcpyAsync(&back->valid, qoff + ix->n, 4, cudaMemcpyDeviceToHost, st));
+        HJ_CUDA(cudaMemcpyAsync(&back->ctl, ctl, sizeof(JoinCtl), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
+        const uint32_t valid = back->valid;
+        const JoinCtl hc = back->ctl;
         if (hc.timeout) {
             set_error("hj_join: a bounded device-side wait expired in the tensor-core pipeline");
             return HJ_ERR_TIMEOUT;
