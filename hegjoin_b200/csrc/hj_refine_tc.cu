@@ -25,7 +25,7 @@
 //   rechecked otherwise, in FP32 in the reference's order (fma chain).
 // The result set is therefore identical to the exact path.
 //
-// Kernel shape (one CTA per SM, persistent, 19 warps):
+// Kernel shape (one CTA per SM, persistent, 20 or 22 warps):
 //   warp 0      loads: the work item's up to 512 query columns once, candidate
 //               tiles through a ring of shared-memory stages, by bulk copies;
 //   warps 1, 2  MMA issuers, one per TMEM accumulator (2 x 256 columns, all of
@@ -33,20 +33,24 @@
 //               of this pattern issued 128 x 128 x 16 MMAs at 42% of the tensor
 //               pipe's rate and 128 x 256 x 16 ones at 98%;
 //   warps 3..18 epilogue, a set of 8 per accumulator: tcgen05.ld, signs ORed or
-//               gathered into masks, accumulator released, hits emitted.
+//               gathered into masks, accumulator released;
+//   the rest    emit the hits, which reach them as records in shared memory.
 //
 // What bounds it, at d = 18 (two K steps per tile; 400,000 points, 12,500
-// accumulator uses per SM): the hand-over chain of an accumulator, ~1,700 cycles
-// for a use (issue ~200, MMAs 273, wake ~100, four TMEM reads with their ORs ~600,
-// release ~100, and the hits' emission, which holds back its own set), two
-// accumulators overlapping.  The floor of each part is 273 cycles per use on the
-// tensor pipe and 256 on the ALU (one OR per value at 128 per cycle).  Measured
-// there: 15.9 ms before the sign test, symmetric form and whole-warp waits, 6.4 ms
-// now; at 90-D and 150,000 points 6.7 -> 2.5 ms; at 18-D and 100,000 points, where
-// half of the 32 x 32 chunks hold a hit, 4.7 -> 1.2 ms.  Tried and not kept: one
-// set of 16 warps on every use (a warp that emits holds back both accumulators:
-// 8.6 ms), 64-column reads (spills: 9.8 ms), named barriers instead of mbarriers
-// for the release (6.5 ms), three accumulators of 160 columns.
+// accumulator uses per SM): the hand-over chain of an accumulator, ~1,690 cycles
+// for a use (waking and issue ~330, MMAs 273 and the other accumulator's share of
+// the pipe, waking the epilogue ~100, four TMEM reads with their ORs ~700, vote and
+// release ~110), two accumulators overlapping.  The floor of each part is 273
+// cycles per use on the tensor pipe and 256 on the ALU (one OR per value at 128 per
+// cycle); the chain without data dependence reached ~500.  Measured there: 15.9 ms
+// before the sign test, symmetric form and whole-warp waits, 6.5 ms with the
+// epilogue emitting, 5.8 ms now; at 90-D and 150,000 points 6.7 -> 2.5 -> 2.05 ms; at
+// 18-D and 100,003 points, where half of the 32 x 32 chunks hold a hit, 4.7 -> 1.25
+// -> 1.06 ms.  Tried and not kept: one set of 16 warps on every use (8.6 ms with
+// emission, 6.3 ms without), 64-column reads (spills: 9.8 ms), named barriers instead
+// of mbarriers for the release (6.5 ms), releasing before the last chunk is ORed
+// (6.6 ms against 5.8), two chunks in flight (6.2 ms), three accumulators of 160
+// columns.
 // Every wait is bounded; a timeout raises an error flag that ends every later wait
 // at once, and the roles walk their loops to the end (on garbage that the host
 // discards, within the item's ranges), leave time for copies in flight and return.
@@ -76,7 +80,12 @@ constexpr uint32_t kKBlockBytes = kTileRows * kRowBytes;   // one K block of a c
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kMaxRanges = 256;
 constexpr int kEpiWarps = 16;                // 8 per accumulator: 4 TMEM lane quarters x 2 column halves
-constexpr int kThreads = 32 * (1 + kAcc + kEpiWarps);
+// warps that emit the hits which the epilogue finds: one keeps up with rare hits and
+// leaves the most issue slots, dense hits take three (18-D, 100,003 points: 1.48 and
+// 1.06 ms; 18-D, 400,000: 5.83 and 5.97 ms)
+constexpr int hit_warps(bool dense) { return dense ? 3 : 1; }
+constexpr int tc_threads(bool dense) { return 32 * (1 + kAcc + kEpiWarps + hit_warps(dense)); }
+constexpr uint32_t kRing = 512;              // records between them
 constexpr long long kWaitCycles = 4000000000ll;     // ~2 s at 1.9 GHz
 
 // Operand forms in memory: K-block planes [kb][row][64 bytes], a row's four
@@ -118,7 +127,7 @@ struct TcArgs {
     long long wait_cycles;      // bound of every mbarrier wait (SM cycles)
 };
 
-struct TcShared {
+struct __align__(16) TcShared {
     uint64_t full_a[kMaxStages];
     uint64_t empty_a[kMaxStages];
     uint64_t full_acc[kAcc];
@@ -128,6 +137,11 @@ struct TcShared {
     uint32_t item;
     uint32_t abort;
     uint32_t ntiles, nr;
+    // ring of hit records, epilogue -> emitting warps: record k lies in slot k % kRing, which is
+    // free for it when seq is k, filled when k + 1
+    uint32_t produced, taken, done;        // records reserved, records taken, epilogue warps through
+    uint32_t seq[kRing];
+    uint4 ring[kRing];                     // tile, row | chunk of 32 query columns << 7, hits, accepts
     uint32_t qid[kQBMax];                  // original ids of the query columns
     uint32_t rs[kMaxRanges];               // range start (sorted position)
     uint32_t rl[kMaxRanges];               // range length
@@ -216,6 +230,22 @@ __device__ __forceinline__ uint32_t below_mask(const uint32_t (&v)[32], float lo
 }
 __device__ __forceinline__ uint32_t low_bits(uint32_t n) { return n >= 32u ? 0xFFFFFFFFu : (1u << n) - 1u; }
 
+// Wait until a ring slot's sequence number is `want` (bounded like mbar_wait).
+__device__ __forceinline__ void ring_wait(const uint32_t& seq, uint32_t want, volatile uint32_t* abort, uint32_t* err,
+                                          long long limit_cycles) {
+    const volatile uint32_t* p = &seq;
+    if (*p != want) {
+        const long long t0 = clock64();
+        while (*p != want && !*abort) {
+            if (clock64() - t0 > limit_cycles) {
+                *abort = 1u;
+                atomicExch(err, 1u);
+            }
+        }
+    }
+    __threadfence_block();
+}
+
 // DENSE: every chunk's signs go into a mask at once (one instruction per value);
 // otherwise they are only ORed (half an instruction per value) and the chunks
 // with a hit are read again before the accumulator is released.
@@ -230,11 +260,15 @@ __device__ __forceinline__ uint32_t low_bits(uint32_t n) { return n >= 32u ? 0xF
 // only (candidate, query) orders, and a silent candidate (bit 31 of perm) only
 // (query, candidate).
 //
+// The epilogue does not emit: a warp that did (ids, a scan, stores: some 2,000 cycles)
+// held back its whole set.  Lanes with a hit pass a record on through a ring in shared
+// memory, and the hit warps take 32 records at a time, one per lane.
+//
 // Work of one item.  With more than 256 query columns every tile is multiplied
 // with both halves of the columns, half h by issuer h into accumulator h; an item
 // of up to 256 columns alternates its tiles between the accumulators.
 template <bool DENSE>
-__global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
+__global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid_constant__ TcArgs a) {
     extern __shared__ uint8_t smem_raw[];
     // operand tiles need 1024-byte alignment for the swizzle pattern
     uint32_t base = tc::smem_u32(smem_raw);
@@ -326,6 +360,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
                 S.rs[r] = sp.x;
                 S.rl[r] = sp.y - sp.x;
             }
+            for (uint32_t i = tid; i < kRing; i += blockDim.x) S.seq[i] = i;
+            if (tid == 0) S.produced = S.taken = S.done = 0u;
             for (uint32_t i = tid; i < ncols; i += blockDim.x) S.qid[i] = a.perm[qbase + i] & 0x7FFFFFFFu;
             __syncthreads();
             if (warp == 0) {
@@ -429,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
                 if (++stage == a.stages) { stage = 0; ++use_a; }
             }
             ++items_loaded;
-        } else {
+        } else if (warp <= kAcc + kEpiWarps) {
             // ---------------- epilogue: warps 3 .. 18, a set of 8 per accumulator, so that a slow
             // warp holds back only its own accumulator.  TMEM lane quarter = warp % 4; each warp
             // reads half of the accumulator's columns.
@@ -437,8 +473,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
             const uint32_t j = ew / (kEpiWarps / kAcc);   // the accumulator this warp drains
             const uint32_t quarter = warp & 3u;
             const uint32_t row = quarter * 32u + lane;
-            // per-thread pair counts of one launch stay far below 2^32 (bounded by the sink)
-            uint32_t n_acc = 0, n_band = 0;
             // this warp's columns of the accumulator, read in chunks of 32
             constexpr uint32_t COLS = kAccCols / 2, NCH = COLS / 32;
             const uint32_t acc_col = ((ew >> 2) & 1u) * COLS;
@@ -446,7 +480,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
             const uint32_t col_base = acc_col + (both ? j * kAccCols : 0u);   // in query columns
             // chunks that hold queries of this item (the rest of the accumulator is stale)
             const uint32_t nch = ncols > col_base ? min(NCH, (ncols - col_base + 31u) / 32u) : 0u;
-            TileWalk tw;
             for (uint32_t t = t_lo + (both ? 0u : j); t < t_hi; t += both ? 1u : 2u) {
                 tc::mbar_wait(&S.full_acc[j], uses & 1u, abort, a.err, a.wait_cycles);
                 tc::fence_after();
@@ -454,16 +487,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
                 uint32_t hm[NCH], am[NCH];
 #pragma unroll
                 for (uint32_t c = 0; c < NCH; ++c) hm[c] = am[c] = 0u;
+                auto release = [&] {
+                    tc::fence_before();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&S.empty_acc[j]);
+                };
                 if constexpr (DENSE) {
+                    // the accumulator goes back as soon as the last chunk is in registers
+                    uint32_t any = 0;
+                    if (nch == 0u) release();
 #pragma unroll
                     for (uint32_t c = 0; c < NCH; ++c) {
                         if (c >= nch) break;
                         uint32_t v[32];
                         tc::tmem_ld_32(acc + c * 32u, v);
                         tc::tmem_wait_32(v);
+                        if (c + 1 == nch) release();
                         hm[c] = sign_mask(v);
-                        if (!a.count_only && __any_sync(0xffffffffu, hm[c])) am[c] = hm[c] & below_mask(v, a.lo);
+                        if (__any_sync(0xffffffffu, hm[c])) {
+                            any = 1u;
+                            if (!a.count_only) am[c] = hm[c] & below_mask(v, a.lo);
+                        }
                     }
+                    ++uses;
+                    if (!any) continue;
                 } else {
                     uint32_t seen = 0, v[32];
 #pragma unroll
@@ -485,85 +532,122 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
                             am[c] = hm[c] & below_mask(v, a.lo);
                         }
                     }
+                    release();
+                    ++uses;
+                    if (!seen) continue;
                 }
-                // every column of this warp has been read: release the accumulator
-                tc::fence_before();
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&S.empty_acc[j]);
-                ++uses;
-                uint32_t any = 0;
-#pragma unroll
-                for (uint32_t c = 0; c < NCH; ++c) any |= hm[c];
-                if (!__any_sync(0xffffffffu, any)) continue;
-
-                // rows past the range's end and columns past the queries are other points'; in the
-                // symmetric form a candidate pairs with the queries up to its own position
-                tw.locate(S, t);
-                const uint32_t cpos = tw.start + row;
-                const bool in = row >= tw.first && row < tw.end;
-                const uint32_t lim = in ? (a.sym ? min(ncols, cpos - qbase + 1u) : ncols) : 0u;
-                const uint32_t skip = q0 - qbase;   // columns below 8 that precede the item's queries
-                uint32_t na = 0, nb = 0;
-                uint32_t self = 0xFFFFFFFFu;   // column of the candidate itself
-                if (a.sym && in && cpos < blk.q1) self = cpos - qbase - col_base;
+                // lanes with a hit pass it on
 #pragma unroll
                 for (uint32_t c = 0; c < NCH; ++c) {
-                    const uint32_t c0 = col_base + c * 32u;
-                    hm[c] &= lim > c0 ? low_bits(lim - c0) : 0u;
-                    if (c0 == 0u) hm[c] &= ~low_bits(skip);
-                    am[c] &= hm[c];
-                    hm[c] &= ~am[c];          // band
-                    na += __popc(am[c]);
-                    nb += __popc(hm[c]);
+                    const uint32_t who = __ballot_sync(0xffffffffu, hm[c] != 0u);
+                    if (who == 0u) continue;
+                    uint32_t k = 0;
+                    if (lane == 0) k = atomicAdd(&S.produced, __popc(who));
+                    k = __shfl_sync(0xffffffffu, k, 0) + __popc(who & lanemask_lt());
+                    if (hm[c]) {
+                        ring_wait(S.seq[k % kRing], k, abort, a.err, a.wait_cycles);
+                        S.ring[k % kRing] = make_uint4(t, row | ((col_base >> 5) + c) << 7, hm[c], am[c]);
+                        __threadfence_block();
+                        *(volatile uint32_t*)&S.seq[k % kRing] = k + 1;
+                    }
+                    __syncwarp();
                 }
+            }
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) atomicAdd(&S.done, 1u);
+        } else {
+            // ---------------- hits: batches of up to 32 records, one per lane
+            uint32_t n_acc = 0, n_band = 0;
+            for (;;) {
+                uint32_t k = 0, avail = 0;
+                if (lane == 0) {
+                    k = atomicAdd(&S.taken, 32u);
+                    // a whole batch, or what is left once every epilogue warp is through
+                    const long long t0 = clock64();
+                    for (;;) {
+                        const uint32_t d = *(volatile uint32_t*)&S.done;
+                        __threadfence_block();
+                        avail = *(volatile uint32_t*)&S.produced;
+                        if ((int)(avail - k) >= 32 || d == (uint32_t)kEpiWarps || *abort) break;
+                        if (clock64() - t0 > a.wait_cycles) {
+                            *abort = 1u;
+                            atomicExch(a.err, 1u);
+                            break;
+                        }
+                        __nanosleep(500);
+                    }
+                }
+                k = __shfl_sync(0xffffffffu, k, 0);
+                avail = __shfl_sync(0xffffffffu, avail, 0);
+                const uint32_t n = (int)(avail - k) > 0 ? min(32u, avail - k) : 0u;
+                if (n == 0u) break;
+                uint4 rec = make_uint4(0u, 0u, 0u, 0u);
+                if (lane < n) {
+                    const uint32_t slot = (k + lane) % kRing;
+                    ring_wait(S.seq[slot], k + lane + 1u, abort, a.err, a.wait_cycles);
+                    rec = S.ring[slot];
+                    __threadfence_block();
+                    *(volatile uint32_t*)&S.seq[slot] = k + lane + kRing;
+                }
+                __syncwarp();
+                // the tile's range: the last r with tp[r] <= tile
+                uint32_t r = 0;
+#pragma unroll
+                for (uint32_t step = kMaxRanges / 2; step > 0; step >>= 1)
+                    if (r + step < S.nr && S.tp[r + step] <= rec.x) r += step;
+                const uint32_t rs = S.rs[r], off = (rec.x - S.tp[r]) * kTileRows, skip = rs & 7u;
+                const uint32_t row = rec.y & 127u, in_range = off + row;   // from the range's aligned start
+                const uint32_t cpos = (rs & ~7u) + in_range;
+                const uint32_t pos0 = qbase + (rec.y >> 7) * 32u;          // query position of bit 0
+                // rows past the range's end and columns past the queries are other points'; in the
+                // symmetric form a candidate pairs with the queries up to its own position
+                const bool in = rec.z != 0u && in_range >= skip && in_range < skip + S.rl[r];
+                const uint32_t lim = in ? (a.sym ? min(blk.q1, cpos + 1u) : blk.q1) : 0u;
+                uint32_t hits = lim > pos0 ? rec.z & low_bits(lim - pos0) : 0u;
+                if (pos0 < q0) hits &= ~low_bits(q0 - pos0);
+                uint32_t acc = hits & rec.w;
+                uint32_t bnd = hits & ~rec.w;
+                const uint32_t na = __popc(acc), nb = __popc(bnd);
                 if (a.count_only) {
                     n_band += na + nb;
-                    continue;
-                }
-                // accepted pairs go out in both orders (symmetric form), the pair of a point with itself once
-                if (__any_sync(0xffffffffu, na)) {
-                    const uint32_t cw = na ? a.perm[cpos] : 0u;
-                    const uint32_t cid = cw & 0x7FFFFFFFu;
-                    const bool fwd = !q_silent;
-                    const bool rev = a.sym && !(cw >> 31);
-                    uint32_t self_hit = 0;
-#pragma unroll
-                    for (uint32_t c = 0; c < NCH; ++c)
-                        if (self - c * 32u < 32u) self_hit |= (am[c] >> (self - c * 32u)) & 1u;
-                    const uint32_t cnt = (fwd ? na : 0u) + (rev ? na - self_hit : 0u);
-                    n_acc += cnt;
-                    if (rev && na > self_hit) atomicAdd(&a.qcount[cid], na - self_hit);
-                    warp_emit_serial(a.sink, wc_acc, cnt, [&](auto&& put) {
-#pragma unroll
-                        for (uint32_t c = 0; c < NCH; ++c) {
-                            uint32_t m = am[c];
-                            while (m) {
-                                const uint32_t col = c * 32u + __ffs(m) - 1u;
-                                m &= m - 1u;
-                                const uint32_t qid = S.qid[col_base + col];
+                } else {
+                    const uint32_t self = a.sym && in ? cpos - pos0 : 0xFFFFFFFFu;   // bit of the candidate itself
+                    // accepted pairs go out in both orders (symmetric form), that of a point with itself once
+                    if (__any_sync(0xffffffffu, na)) {
+                        const uint32_t cw = na ? a.perm[cpos] : 0u;
+                        const uint32_t cid = cw & 0x7FFFFFFFu;
+                        const bool fwd = !q_silent;
+                        const bool rev = a.sym && !(cw >> 31);
+                        const uint32_t self_hit = self < 32u ? (acc >> self) & 1u : 0u;
+                        const uint32_t cnt = (fwd ? na : 0u) + (rev ? na - self_hit : 0u);
+                        n_acc += cnt;
+                        if (rev && na > self_hit) atomicAdd(&a.qcount[cid], na - self_hit);
+                        warp_emit_serial(a.sink, wc_acc, cnt, [&](auto&& put) {
+                            while (acc) {
+                                const uint32_t b = __ffs(acc) - 1u;
+                                acc &= acc - 1u;
+                                const uint32_t qid = S.qid[pos0 - qbase + b];
                                 if (fwd) {
                                     put(qid, cid);
                                     atomicAdd(&a.qcount[qid], 1u);
                                 }
-                                if (rev && col != self) put(cid, qid);
+                                if (rev && b != self) put(cid, qid);
                             }
-                        }
-                    });
-                }
-                if (__any_sync(0xffffffffu, nb)) {
-                    n_band += a.sym ? 2u * nb : nb;
-                    warp_emit_serial(a.band, wc_band, nb, [&](auto&& put) {
-#pragma unroll
-                        for (uint32_t c = 0; c < NCH; ++c) {
-                            uint32_t m = hm[c];
-                            while (m) {
-                                const uint32_t col = c * 32u + __ffs(m) - 1u;
-                                m &= m - 1u;
-                                put(qbase + col_base + col, cpos);
+                        });
+                    }
+                    if (__any_sync(0xffffffffu, nb)) {
+                        n_band += a.sym ? 2u * nb : nb;
+                        warp_emit_serial(a.band, wc_band, nb, [&](auto&& put) {
+                            while (bnd) {
+                                const uint32_t b = __ffs(bnd) - 1u;
+                                bnd &= bnd - 1u;
+                                put(pos0 + b, cpos);
                             }
-                        }
-                    });
+                        });
+                    }
                 }
+                if (n < 32u) break;
             }
             unsigned long long w_acc = n_acc, w_band = n_band;
             for (int o = 16; o > 0; o >>= 1) {
@@ -580,7 +664,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_refine_tc(TcArgs a) {
             }
         }
     }
-    if (warp > kAcc && !a.count_only) {
+    if (warp > kAcc + kEpiWarps && !a.count_only) {
         warp_chunk_close(a.sink, wc_acc);
         warp_chunk_close(a.band, wc_band);
     }
@@ -984,10 +1068,10 @@ static unsigned recheck_grid(uint32_t nblocks) {
 }
 
 // Upper bound on the warps that reserve chunks of one sink during one batch: the
-// refine's epilogue warps (at most 16 per CTA, one CTA per SM) and the band
-// recheck's warps (8 per block), each holding at most one partly filled chunk.
+// refine's hit warps (one CTA per SM) and the band recheck's warps (8 per block),
+// each holding at most one partly filled chunk.
 uint64_t tc_emit_warps(uint32_t nblocks) {
-    return std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)std::max<uint32_t>(nblocks, 1) * tc_parts(nblocks)) * 16ull +
+    return std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)std::max<uint32_t>(nblocks, 1) * tc_parts(nblocks)) * (uint64_t)hit_warps(true) +
            (uint64_t)recheck_grid(nblocks) * 8ull;
 }
 
@@ -1185,7 +1269,7 @@ hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     a.fmt = ix->tc_kind == HJ_REFINE_TC_BF16 ? 1u : 0u;
     a.wait_cycles = kWaitCycles;
     unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)nblocks * a.parts);
-    kern<<<grid, kThreads, smem, st>>>(a);
+    kern<<<grid, tc_threads(s->dense), smem, st>>>(a);
     HJ_LAUNCHED();
     return HJ_OK;
 }
