@@ -175,11 +175,11 @@ class Scratch {
     std::vector<void*> held_;
 };
 
-// Readbacks land in pinned memory of the calling thread (kReadbackBytes, allocated on
-// its first use and given back when it ends), so that several copies and the wait
+// Readbacks land in pinned memory of the calling thread (kReadbackBytes, taken on
+// its first use and handed on when it ends), so that several copies and the wait
 // for them cost one synchronisation: a copy to pageable memory waits by itself.
 // Valid until the thread's next readback.
-constexpr size_t kReadbackBytes = 160 * 1024;
+constexpr size_t kReadbackBytes = 40 * 1024;
 hj_status readback_buffer(void** p);   // hj_index.cu
 
 // Raise a kernel's dynamic shared-memory limit once per (kernel, size), safe

@@ -55,16 +55,37 @@ bool injected_alloc_failure() {
 }
 
 namespace {
+// Buffers of ended threads wait for the next thread (a server's workers come and go
+// with it, and allocating pinned memory stops the device for a moment); at most
+// kReadbackKept of them.
+constexpr size_t kReadbackKept = 32;
+std::mutex g_readback_mu;
+std::vector<void*> g_readback_free;
 struct Readback {
     void* p = nullptr;
     ~Readback() {
-        if (p) cudaFreeHost(p);
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lk(g_readback_mu);
+            if (g_readback_free.size() < kReadbackKept) {
+                g_readback_free.push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);
     }
 };
 thread_local Readback t_readback;
 }  // namespace
 hj_status readback_buffer(void** p) {
-    if (!t_readback.p) HJ_CUDA(cudaMallocHost(&t_readback.p, kReadbackBytes));
+    if (!t_readback.p) {
+        std::lock_guard<std::mutex> lk(g_readback_mu);
+        if (!g_readback_free.empty()) {
+            t_readback.p = g_readback_free.back();
+            g_readback_free.pop_back();
+        }
+    }
+    if (!t_readback.p) HJ_CUDA(cudaHostAlloc(&t_readback.p, kReadbackBytes, cudaHostAllocPortable));
     *p = t_readback.p;
     return HJ_OK;
 }
@@ -172,13 +193,14 @@ __global__ void k_minmax(const T* __restrict__ db, uint32_t n, uint32_t d, uint3
 template <typename T>
 hj_status geometry_t(const T* db, uint32_t n, uint32_t d, uint32_t k, T eps, double* h_min, double* h_max,
                      uint32_t* h_ncells, uint64_t* h_total, cudaStream_t st) {
-    const int blocks = std::min<int>(std::min(num_sms() * 4, 592), std::max<uint32_t>(1, (n + 255) / 256));
+    constexpr int kGeoBlocks = 148;
+    const int blocks = std::min<int>(kGeoBlocks, std::max<uint32_t>(1, (n + 1023) / 1024));
     Scratch tmp(st);
     T* part = nullptr;
     HJ_TRY(tmp.alloc(&part, (size_t)2 * blocks * k));
-    k_minmax<T><<<blocks, 256, 0, st>>>(db, n, d, k, part, part + (size_t)k * blocks);
+    k_minmax<T><<<blocks, 1024, 0, st>>>(db, n, d, k, part, part + (size_t)k * blocks);
     HJ_LAUNCHED();
-    static_assert(2 * 592 * kMaxK * sizeof(double) <= kReadbackBytes, "partials of 592 blocks");
+    static_assert(2 * kGeoBlocks * kMaxK * sizeof(double) <= kReadbackBytes, "the blocks' partials are read back");
     T* hp = nullptr;
     HJ_TRY(readback_buffer(reinterpret_cast<void**>(&hp)));
     HJ_CUDA(cudaMemcpyAsync(hp, part, (size_t)2 * blocks * k * sizeof(T), cudaMemcpyDeviceToHost, st));

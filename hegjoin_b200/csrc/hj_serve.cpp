@@ -28,6 +28,7 @@
 
 namespace hj {
 void result_set_stream(hj_result* r, cudaStream_t s);   // hj_join.cu
+hj_status readback_buffer(void** p);                    // hj_index.cu
 }
 
 namespace {
@@ -99,6 +100,8 @@ void worker_main(hj_server* S) {
     cudaSetDevice(S->device);
     cudaStream_t st;
     cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    void* pinned = nullptr;
+    hj::readback_buffer(&pinned);   // taken before the first request rather than in it
     // the worker's device workspace: the temporaries of its requests' index builds and
     // joins come from it, so a small request makes no allocator calls for them
     hj::Workspace ws;
