@@ -26,23 +26,26 @@ uint32_t warp_query_block(uint32_t n) {
 
 // Items per block of queries: a list that would leave warps idle (fewer than two
 // items per resident warp) is cut so that an item still has about 8,192 pairs to
-// evaluate; `avg` = mean pairs (queries x candidates) per block of the join.
-static uint32_t warp_parts(uint32_t nblocks, double avg) {
+// evaluate; `avg` = mean pairs (queries x candidates) per block of the join.  The
+// estimator's sample is cut whatever the mean: its first items are the heaviest of
+// the join, and one of them alone took as long as the join (6-D, 20,011 points: 142
+// us of 270).
+static uint32_t warp_parts(uint32_t nblocks, double avg, bool sample) {
     const uint64_t want = 2ull * kWarpMaxBlocks * kWarpsPerBlock * (uint64_t)num_sms();
     const uint64_t nb = std::max<uint32_t>(nblocks, 1);
-    const uint64_t by_work = (uint64_t)(avg / 8192.0);
+    const uint64_t by_work = sample ? 64u : (uint64_t)(avg / 8192.0);
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({64, (want + nb - 1) / nb, by_work}));
 }
 
 // Slots that partly filled chunks can leave unused in one launch.
 uint64_t warp_chunk_slack(uint32_t nblocks, double avg) {
-    const uint64_t items = (uint64_t)std::max<uint32_t>(nblocks, 1) * warp_parts(nblocks, avg) + kWarpsPerBlock - 1;
+    const uint64_t items = (uint64_t)std::max<uint32_t>(nblocks, 1) * warp_parts(nblocks, avg, false) + kWarpsPerBlock - 1;
     return std::min<uint64_t>((uint64_t)kWarpMaxBlocks * kWarpsPerBlock * num_sms(), items) * kSinkChunk;
 }
 
 template <typename T>
-static hj_status make_args(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, bool sym,
-                           unsigned int* head, WarpArgs<T>* a, cudaStream_t st) {
+static hj_status make_args(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, bool sample,
+                           bool sym, unsigned int* head, WarpArgs<T>* a, cudaStream_t st) {
     *a = WarpArgs<T>{};
     a->pts = (const T*)ix->pts;
     a->perm = ix->perm;
@@ -55,7 +58,7 @@ static hj_status make_args(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     a->thr = (T)ix->thr;
     a->blocks = blocks;
     a->nblocks = nblocks;
-    a->parts = warp_parts(nblocks, avg);
+    a->parts = warp_parts(nblocks, avg, sample);
     a->sym = sym ? 1u : 0u;
     a->head = head;
     return HJ_OK;
@@ -72,7 +75,7 @@ hj_status launch_refine_warp(hj_index* ix, const HjBlock* blocks, uint32_t nbloc
     auto run = [&](auto zero, auto refine) -> hj_status {
         using T = decltype(zero);
         WarpArgs<T> a;
-        HJ_TRY(make_args<T>(ix, blocks, nblocks, avg, sym, head, &a, st));
+        HJ_TRY(make_args<T>(ix, blocks, nblocks, avg, count_only != 0u, sym, head, &a, st));
         a.sink = sink;
         a.count_only = count_only;
         a.block_counts = block_counts;
@@ -91,7 +94,7 @@ hj_status launch_refine_digest(hj_index* ix, const HjBlock* blocks, uint32_t nbl
     auto run = [&](auto zero, auto refine) -> hj_status {
         using T = decltype(zero);
         WarpArgs<T> a;
-        HJ_TRY(make_args<T>(ix, blocks, nblocks, avg, false, head, &a, st));
+        HJ_TRY(make_args<T>(ix, blocks, nblocks, avg, false, false, head, &a, st));
         a.d_count = d_count;
         a.d_sum = d_sum;
         a.d_xor = d_xor;

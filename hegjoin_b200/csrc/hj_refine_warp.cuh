@@ -179,7 +179,7 @@ __device__ __forceinline__ bool warp_slots(const PairSink& s, WarpChunk& c, uint
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 6 ? 6 : 4) k_refine_warp(const __grid_constant__ WarpArgs<T> a) {
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, D <= 8 ? 6 : 5) k_refine_warp(const __grid_constant__ WarpArgs<T> a) {
     using Smem = WarpSmem<T, D>;
     constexpr bool F32 = std::is_same<T, float>::value;
     __shared__ Smem smem[kWarpsPerBlock];
