@@ -521,7 +521,7 @@ bool tuning_enabled() {
 }
 
 // Tensor-core epilogue: with fewer than ~3% of its 32 x 32 chunks holding a hit, ORing the
-// signs and reading the hit chunks again beats building every chunk's mask.
+// signs and reading the hit chunks again beats a vote per chunk and masks at once.
 // HJ_TC_DEFER=0/1 forces masks or ORs (tests).
 bool dense_for(double pairs, double cand) {
     if (const char* e = std::getenv("HJ_TC_DEFER")) return e[0] != '1';

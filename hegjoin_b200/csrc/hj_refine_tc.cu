@@ -6,7 +6,7 @@
 // is a GEMM on the 5th-generation tensor cores:
 //
 //   A (M = 128 candidates, streamed by TMA) = [-2 c~, 1, 1, N_c hi, N_c lo, 0...]
-//   B (N = 256 queries, resident)           = [  q~, N_q hi, N_q lo, 1, 1, 0...]
+//   B (N = 128 queries, resident)           = [  q~, N_q hi, N_q lo, 1, 1, 0...]
 //   D' = A B^T = N_q + N_c - 2 q~.c~        (FP32 accumulate in TMEM)
 //
 // where x~ is the FP16 (or BF16) rounding of (x - origin) * 2^s and the norm
@@ -25,32 +25,35 @@
 //   rechecked otherwise, in FP32 in the reference's order (fma chain).
 // The result set is therefore identical to the exact path.
 //
-// Kernel shape (one CTA per SM, persistent, 20 or 22 warps):
+// Kernel shape (one CTA per SM, persistent, 22 or 24 warps):
 //   warp 0      loads: the work item's up to 512 query columns once, candidate
 //               tiles through a ring of shared-memory stages, by bulk copies;
-//   warps 1, 2  MMA issuers, one per TMEM accumulator (2 x 256 columns, all of
-//               TMEM): M = 128 x N = 256 MMAs.  N = 256 matters: a microbenchmark
-//               of this pattern issued 128 x 128 x 16 MMAs at 42% of the tensor
-//               pipe's rate and 128 x 256 x 16 ones at 98%;
-//   warps 3..18 epilogue, a set of 8 per accumulator: tcgen05.ld, signs ORed or
+//   warps 1..4  MMA issuers, one per TMEM accumulator (4 x 128 columns, all of
+//               TMEM): M = 128 x N = 128 MMAs;
+//   warps 5..20 epilogue, a set of 4 per accumulator: tcgen05.ld, signs ORed or
 //               gathered into masks, accumulator released;
 //   the rest    emit the hits, which reach them as records in shared memory.
 //
-// What bounds it, at d = 18 (two K steps per tile; 400,000 points, 12,500
-// accumulator uses per SM): the hand-over chain of an accumulator, ~1,690 cycles
-// for a use (waking and issue ~330, MMAs 273 and the other accumulator's share of
-// the pipe, waking the epilogue ~100, four TMEM reads with their ORs ~700, vote and
-// release ~110), two accumulators overlapping.  The floor of each part is 273
-// cycles per use on the tensor pipe and 256 on the ALU (one OR per value at 128 per
-// cycle); the chain without data dependence reached ~500.  Measured there: 15.9 ms
-// before the sign test, symmetric form and whole-warp waits, 6.5 ms with the
-// epilogue emitting, 5.8 ms now; at 90-D and 150,000 points 6.7 -> 2.5 -> 2.05 ms; at
-// 18-D and 100,003 points, where half of the 32 x 32 chunks hold a hit, 4.7 -> 1.25
-// -> 1.06 ms.  Tried and not kept: one set of 16 warps on every use (8.6 ms with
-// emission, 6.3 ms without), 64-column reads (spills: 9.8 ms), named barriers instead
-// of mbarriers for the release (6.5 ms), releasing before the last chunk is ORed
-// (6.6 ms against 5.8), two chunks in flight (6.2 ms), three accumulators of 160
-// columns.
+// What bounds it: the hand-over chain of an accumulator (waking the issuer and
+// issuing ~330 cycles, MMAs, waking the epilogue ~100, TMEM reads with their ORs,
+// vote and release ~110), the accumulators overlapping.  Per 256 columns and tile the
+// floor is 273 cycles on the tensor pipe at d = 18 (two K steps) and 256 on the ALU
+// (one OR per value at 128 per cycle); with the ORs left out a tile took ~350, with
+// them and no hits ~750, with the hits of the data below ~820.
+// Refine of 18-D points, 400,000 / 100,003 (half of the 32 x 32 chunks hold a hit),
+// 90-D, 150,000 and 32-D BF16, 150,001, in ms:
+//   before the sign test, symmetric form and whole-warp waits   15.9  4.7   6.7
+//   the epilogue emitting                                         6.5  1.25  2.5
+//   one ring of hits for all, two accumulators of 256 columns     5.83 1.06  2.06  2.21
+//   sign masks in four chains of shifts, a ring per epilogue
+//   warp, the accumulator released once its last read is done     5.56 0.93  1.86  1.82
+//   four accumulators of 128 columns, waits without a sleep hint  5.11 0.89  1.73  1.72
+// (a microbenchmark had issued N = 128 MMAs at 42% of the tensor pipe's rate, N = 256
+// ones at 98%; the shorter chain is worth more).  Tried and not kept: one set of 16
+// warps on every use (8.6 ms with emission, 6.3 ms without), 24 epilogue warps (5.84 ms
+// against 5.83), 64-column reads (spills: 9.8 ms), named barriers instead of mbarriers
+// for the release (6.5 ms), two chunks in flight (6.2 ms), three accumulators of 160
+// columns, masks of the groups of four columns that hold a hit only (6.2 ms against 5.6).
 // Every wait is bounded; a timeout raises an error flag that ends every later wait
 // at once, and the roles walk their loops to the end (on garbage that the host
 // discards, within the item's ranges), leave time for copies in flight and return.
@@ -69,9 +72,9 @@ namespace hj {
 namespace {
 
 constexpr int kTileRows = 128;               // candidate rows per tile (M of every MMA)
-constexpr int kAcc = 2;                      // TMEM accumulators
-constexpr int kAccCols = 256;                // N of one MMA: columns of one accumulator
-constexpr int kQBMax = 2 * kAccCols;         // query columns per work item at most
+constexpr int kAcc = 4;                      // TMEM accumulators (a power of two)
+constexpr int kAccCols = 128;                // N of one MMA: columns of one accumulator
+constexpr int kQBMax = kAcc * kAccCols;      // query columns per work item at most
 constexpr int kProbeThreads = 192;   // tile probe: load warp, MMA warp, 4 epilogue warps
 constexpr int kProbeQB = 512;                // the tile probe evaluates 512 query rows
 constexpr int kMaxStages = 8;
@@ -79,13 +82,15 @@ constexpr uint32_t kRowBytes = 64;           // one row of one K block: 32 halve
 constexpr uint32_t kKBlockBytes = kTileRows * kRowBytes;   // one K block of a candidate tile
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kMaxRanges = 256;
-constexpr int kEpiWarps = 16;                // 8 per accumulator: 4 TMEM lane quarters x 2 column halves
+constexpr int kEpiWarps = 16;                // 4 per accumulator: one per TMEM lane quarter
 // warps that emit the hits which the epilogue finds: one keeps up with rare hits and
-// leaves the most issue slots, dense hits take three (18-D, 100,003 points: 1.48 and
-// 1.06 ms; 18-D, 400,000: 5.83 and 5.97 ms)
+// leaves the most issue slots, dense hits take three (one, two and three at 18-D, 100,003
+// points: 1.41, 1.03 and 0.93 ms; at 18-D, 400,000: 5.56, 5.63 and 5.77 ms)
 constexpr int hit_warps(bool dense) { return dense ? 3 : 1; }
 constexpr int tc_threads(bool dense) { return 32 * (1 + kAcc + kEpiWarps + hit_warps(dense)); }
-constexpr uint32_t kRing = 512;              // records between them
+// hit records between an epilogue warp and the hit warps (at least the 32 of one chunk; 32 and
+// 64: 5.21 and 5.12 ms at 18-D, 400,000 points)
+constexpr uint32_t kRing = 64;
 constexpr long long kWaitCycles = 4000000000ll;     // ~2 s at 1.9 GHz
 
 // Operand forms in memory: K-block planes [kb][row][64 bytes], a row's four
@@ -137,11 +142,12 @@ struct __align__(16) TcShared {
     uint32_t item;
     uint32_t abort;
     uint32_t ntiles, nr;
-    // ring of hit records, epilogue -> emitting warps: record k lies in slot k % kRing, which is
-    // free for it when seq is k, filled when k + 1
-    uint32_t produced, taken, done;        // records reserved, records taken, epilogue warps through
-    uint32_t seq[kRing];
-    uint4 ring[kRing];                     // tile, row | chunk of 32 query columns << 7, hits, accepts
+    // a ring of hit records per epilogue warp, written by it and read by one hit warp:
+    // record k lies in slot k % kRing
+    uint32_t done;                         // epilogue warps through with the item
+    uint32_t produced[kEpiWarps];          // records written so far
+    uint32_t consumed[kEpiWarps];          // and taken
+    uint4 ring[kEpiWarps][kRing];          // tile, row | chunk of 32 query columns << 7, hits, accepts
     uint32_t qid[kQBMax];                  // original ids of the query columns
     uint32_t rs[kMaxRanges];               // range start (sorted position)
     uint32_t rl[kMaxRanges];               // range length
@@ -214,29 +220,34 @@ __device__ __forceinline__ uint32_t or_all(const uint32_t (&v)[32]) {
     for (int i = 0; i < 8; ++i) m[i] = (v[i] | v[i + 8]) | (v[i + 16] | v[i + 24]);
     return ((m[0] | m[1]) | (m[2] | m[3])) | ((m[4] | m[5]) | (m[6] | m[7]));
 }
-// Bit i = sign of v[i].
-__device__ __forceinline__ uint32_t sign_mask(const uint32_t (&v)[32]) {
-    uint32_t m = 0;
+// Bit i = sign of at(i), in four independent chains of funnel shifts: a single chain
+// of 32 took as long as the rest of an accumulator's epilogue.
+template <typename At>
+__device__ __forceinline__ uint32_t sign_bits(At&& at) {
+    uint32_t m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int i = 31; i >= 0; --i) m = __funnelshift_l(v[i], m, 1);
-    return m;
+    for (int i = 7; i >= 0; --i)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) m[g] = __funnelshift_l(at(8 * g + i), m[g], 1);
+    return (m[0] | m[1] << 8) | (m[2] << 16 | m[3] << 24);
+}
+__device__ __forceinline__ uint32_t sign_mask(const uint32_t (&v)[32]) {
+    return sign_bits([&](int i) { return v[i]; });
 }
 // Bit i = (v[i] < lo), lo negative.
 __device__ __forceinline__ uint32_t below_mask(const uint32_t (&v)[32], float lo) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int i = 31; i >= 0; --i) m = __funnelshift_l(__float_as_uint(__uint_as_float(v[i]) - lo), m, 1);
-    return m;
+    return sign_bits([&](int i) { return __float_as_uint(__uint_as_float(v[i]) - lo); });
 }
 __device__ __forceinline__ uint32_t low_bits(uint32_t n) { return n >= 32u ? 0xFFFFFFFFu : (1u << n) - 1u; }
 
-// Wait until a ring slot's sequence number is `want` (bounded like mbar_wait).
-__device__ __forceinline__ void ring_wait(const uint32_t& seq, uint32_t want, volatile uint32_t* abort, uint32_t* err,
-                                          long long limit_cycles) {
-    const volatile uint32_t* p = &seq;
-    if (*p != want) {
+// Wait until a ring's counter has reached `want` (bounded like mbar_wait).
+__device__ __forceinline__ uint32_t ring_wait(const uint32_t& counter, uint32_t want, volatile uint32_t* abort,
+                                              uint32_t* err, long long limit_cycles) {
+    const volatile uint32_t* p = &counter;
+    uint32_t v = *p;
+    if ((int)(v - want) < 0) {
         const long long t0 = clock64();
-        while (*p != want && !*abort) {
+        while ((int)((v = *p) - want) < 0 && !*abort) {
             if (clock64() - t0 > limit_cycles) {
                 *abort = 1u;
                 atomicExch(err, 1u);
@@ -244,11 +255,14 @@ __device__ __forceinline__ void ring_wait(const uint32_t& seq, uint32_t want, vo
         }
     }
     __threadfence_block();
+    return v;
 }
 
-// DENSE: every chunk's signs go into a mask at once (one instruction per value);
-// otherwise they are only ORed (half an instruction per value) and the chunks
-// with a hit are read again before the accumulator is released.
+// DENSE: a chunk with a hit has its signs gathered into masks while it is in
+// registers (a vote per chunk); otherwise chunks are only ORed (one vote per
+// accumulator) and those with a hit are read again before the accumulator is
+// released.  18-D, 400,000 points: 5.34 and 5.11 ms; 18-D, 100,003 (half of the chunks
+// hold a hit, three hit warps): 0.89 and 0.93 ms; 32-D: 1.72 and 1.78 ms.
 //
 // Symmetric form (a.sym): d2 is the same number for (q, c) and (c, q), so a join
 // that runs all its work items in one batch evaluates each unordered pair once
@@ -261,12 +275,12 @@ __device__ __forceinline__ void ring_wait(const uint32_t& seq, uint32_t want, vo
 // (query, candidate).
 //
 // The epilogue does not emit: a warp that did (ids, a scan, stores: some 2,000 cycles)
-// held back its whole set.  Lanes with a hit pass a record on through a ring in shared
-// memory, and the hit warps take 32 records at a time, one per lane.
+// held back its whole set.  Lanes with a hit pass a record on through their warp's ring in
+// shared memory, and the hit warps take up to 32 records at a time, one per lane.
 //
-// Work of one item.  With more than 256 query columns every tile is multiplied
-// with both halves of the columns, half h by issuer h into accumulator h; an item
-// of up to 256 columns alternates its tiles between the accumulators.
+// Work of one item.  Its query columns make one, two or four groups of up to 128; each
+// tile is multiplied with all of them, group g into an accumulator h with h % groups == g,
+// and an item of fewer than four groups deals its tiles to the accumulators in turn.
 template <bool DENSE>
 __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid_constant__ TcArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -283,7 +297,7 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
     if (tid == 0) {
         for (uint32_t s = 0; s < a.stages; ++s) {
             tc::mbar_init(&S.full_a[s], 1);
-            tc::mbar_init(&S.empty_a[s], 2);   // two commits: one by each issuer, or both by the tile's
+            tc::mbar_init(&S.empty_a[s], kAcc);   // commits by the tile's issuers
         }
         for (int j = 0; j < kAcc; ++j) {
             tc::mbar_init(&S.full_acc[j], 1);
@@ -321,7 +335,10 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
         const HjBlock blk = a.blocks[bi];
         // query columns: positions qbase + [0, ncols), of which the first q0 - qbase are not the item's
         const uint32_t q0 = blk.q0, qbase = q0 & ~7u, ncols = blk.q1 - qbase;
-        const bool both = ncols > (uint32_t)kAccCols;
+        // column groups: accumulator h takes group h % groups of every (kAcc / groups)-th tile
+        uint32_t groups = 1;
+        while (groups * kAccCols < ncols) groups *= 2;
+        const uint32_t round = kAcc / groups;
         bool q_silent = false;
         {
             // stencil rows of the block's cell -> candidate ranges, a row per thread
@@ -360,8 +377,8 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                 S.rs[r] = sp.x;
                 S.rl[r] = sp.y - sp.x;
             }
-            for (uint32_t i = tid; i < kRing; i += blockDim.x) S.seq[i] = i;
-            if (tid == 0) S.produced = S.taken = S.done = 0u;
+            if (tid < (uint32_t)kEpiWarps) S.produced[tid] = S.consumed[tid] = 0u;
+            if (tid == 0) S.done = 0u;
             for (uint32_t i = tid; i < ncols; i += blockDim.x) S.qid[i] = a.perm[qbase + i] & 0x7FFFFFFFu;
             __syncthreads();
             if (warp == 0) {
@@ -415,7 +432,7 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
             __syncwarp();
             TileWalk tw;
             for (uint32_t t = t_lo; t < t_hi; ++t) {
-                if (use_a > 0) tc::mbar_wait(&S.empty_a[stage], (use_a - 1) & 1u, abort, a.err, a.wait_cycles);
+                if (use_a > 0) tc::mbar_wait<false>(&S.empty_a[stage], (use_a - 1) & 1u, abort, a.err, a.wait_cycles);
                 tw.locate(S, t);
                 if (tc::elect_one()) {
                     tc::mbar_arrive_expect_tx(&S.full_a[stage], tile_bytes);
@@ -428,25 +445,23 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                 if (++stage == a.stages) { stage = 0; ++use_a; }
             }
         } else if (warp <= kAcc) {
-            // ---------------- MMA issuer h (warp 1: h = 0, warp 2: h = 1), into accumulator h.
+            // ---------------- MMA issuer h (warp 1 + h), into accumulator h
             const uint32_t h = warp - 1;
             tc::mbar_wait(&S.bfull, items_loaded & 1u, abort, a.err, a.wait_cycles);
+            const uint32_t first_col = h % groups * kAccCols, turn = h / groups;
             const uint64_t a_desc = tc::desc_kmajor_sw64(tc::smem_u32(a_tiles));
             const uint64_t b_desc =
-                tc::desc_kmajor_sw64(tc::smem_u32(b_tiles) + (both ? h * (uint32_t)kAccCols * kRowBytes : 0u));
-            // N = this half's query columns in whole groups of 32
-            const uint32_t cols = both ? (h ? ncols - kAccCols : (uint32_t)kAccCols) : ncols;
+                tc::desc_kmajor_sw64(tc::smem_u32(b_tiles) + first_col * kRowBytes);
+            // N = this group's query columns in whole groups of 32
+            const uint32_t cols = ncols > first_col ? min((uint32_t)kAccCols, ncols - first_col) : 32u;
             const uint32_t idesc = tc::idesc_f16(a.fmt, kTileRows, (cols + 31u) & ~31u);
-            // both: this issuer takes every tile; otherwise every second one
             for (uint32_t t = t_lo; t < t_hi; ++t) {
-                if (both || ((t - t_lo) & 1u) == h) {
-                    tc::mbar_wait(&S.full_a[stage], use_a & 1u, abort, a.err, a.wait_cycles);
-                    if (uses > 0) tc::mbar_wait(&S.empty_acc[h], (uses - 1) & 1u, abort, a.err, a.wait_cycles);
+                if (((t - t_lo) & (round - 1u)) == turn) {
+                    tc::mbar_wait<false>(&S.full_a[stage], use_a & 1u, abort, a.err, a.wait_cycles);
+                    if (uses > 0) tc::mbar_wait<false>(&S.empty_acc[h], (uses - 1) & 1u, abort, a.err, a.wait_cycles);
                     ++uses;
                     if (tc::elect_one()) {
                         tc::fence_after();
-                        // M = 128 candidates x N = 256 queries per MMA: the shape that keeps the
-                        // tensor pipe busy (N = 128 MMAs issue at well under half its rate)
                         uint64_t ad = a_desc + ((stage * tile_bytes) >> 4), bd = b_desc;
                         tc::mma_f16(tmem + h * kAccCols, ad, bd, idesc, 0u);
                         tc::mma_f16(tmem + h * kAccCols, ad + 2u, bd + 2u, idesc, 1u);
@@ -457,8 +472,7 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                             tc::mma_f16(tmem + h * kAccCols, ad + 2u, bd + 2u, idesc, 1u);
                         }
                         tc::mma_commit(&S.full_acc[h]);
-                        tc::mma_commit(&S.empty_a[stage]);
-                        if (!both) tc::mma_commit(&S.empty_a[stage]);
+                        for (uint32_t i = 0; i < round; ++i) tc::mma_commit(&S.empty_a[stage]);
                     }
                     __syncwarp();
                 }
@@ -466,22 +480,30 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
             }
             ++items_loaded;
         } else if (warp <= kAcc + kEpiWarps) {
-            // ---------------- epilogue: warps 3 .. 18, a set of 8 per accumulator, so that a slow
-            // warp holds back only its own accumulator.  TMEM lane quarter = warp % 4; each warp
-            // reads half of the accumulator's columns.
+            // ---------------- epilogue: warps 5 .. 20, a set of 4 per accumulator, so that a slow
+            // warp holds back only its own accumulator.  TMEM lane quarter = warp % 4.
             const uint32_t ew = warp - 1 - kAcc;
-            const uint32_t j = ew / (kEpiWarps / kAcc);   // the accumulator this warp drains
+            constexpr uint32_t SET = kEpiWarps / kAcc;
+            const uint32_t j = ew / SET;   // the accumulator this warp drains
             const uint32_t quarter = warp & 3u;
             const uint32_t row = quarter * 32u + lane;
             // this warp's columns of the accumulator, read in chunks of 32
-            constexpr uint32_t COLS = kAccCols / 2, NCH = COLS / 32;
-            const uint32_t acc_col = ((ew >> 2) & 1u) * COLS;
+            constexpr uint32_t COLS = kAccCols / (SET / 4), NCH = COLS / 32;
+            const uint32_t acc_col = ew % SET / 4u * COLS;
             const uint32_t acc = tmem + ((quarter * 32u) << 16) + j * kAccCols + acc_col;
-            const uint32_t col_base = acc_col + (both ? j * kAccCols : 0u);   // in query columns
+            const uint32_t col_base = acc_col + j % groups * kAccCols;   // in query columns
             // chunks that hold queries of this item (the rest of the accumulator is stale)
             const uint32_t nch = ncols > col_base ? min(NCH, (ncols - col_base + 31u) / 32u) : 0u;
-            for (uint32_t t = t_lo + (both ? 0u : j); t < t_hi; t += both ? 1u : 2u) {
-                tc::mbar_wait(&S.full_acc[j], uses & 1u, abort, a.err, a.wait_cycles);
+            uint32_t prod = 0, room = kRing;   // records written, and how many may be before a look at the reader
+            auto publish = [&] {
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) *(volatile uint32_t*)&S.produced[ew] = prod;
+                __syncwarp();
+            };
+            for (uint32_t t = t_lo + j / groups; t < t_hi; t += round) {
+                tc::mbar_wait<false>(&S.full_acc[j], uses & 1u, abort, a.err, a.wait_cycles);
+                ++uses;
                 tc::fence_after();
                 // per chunk: signs (candidate hits) and outright accepts of this lane's row
                 uint32_t hm[NCH], am[NCH];
@@ -492,9 +514,9 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&S.empty_acc[j]);
                 };
+                uint32_t seen = 0;
                 if constexpr (DENSE) {
                     // the accumulator goes back as soon as the last chunk is in registers
-                    uint32_t any = 0;
                     if (nch == 0u) release();
 #pragma unroll
                     for (uint32_t c = 0; c < NCH; ++c) {
@@ -503,16 +525,13 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                         tc::tmem_ld_32(acc + c * 32u, v);
                         tc::tmem_wait_32(v);
                         if (c + 1 == nch) release();
+                        if (!__any_sync(0xffffffffu, (int)or_all(v) < 0)) continue;
+                        seen = 1u;
                         hm[c] = sign_mask(v);
-                        if (__any_sync(0xffffffffu, hm[c])) {
-                            any = 1u;
-                            if (!a.count_only) am[c] = hm[c] & below_mask(v, a.lo);
-                        }
+                        am[c] = hm[c] & below_mask(v, a.lo);
                     }
-                    ++uses;
-                    if (!any) continue;
                 } else {
-                    uint32_t seen = 0, v[32];
+                    uint32_t v[32];
 #pragma unroll
                     for (uint32_t c = 0; c < NCH; ++c) {
                         if (c >= nch) break;
@@ -521,76 +540,93 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                         seen |= (or_all(v) >> 31) << c;
                     }
                     seen = __reduce_or_sync(0xffffffffu, seen);
-                    if (seen) {
-                        // rare: the accumulator is still held
-#pragma unroll
-                        for (uint32_t c = 0; c < NCH; ++c) {
-                            if (!((seen >> c) & 1u)) continue;
-                            tc::tmem_ld_32(acc + c * 32u, v);
-                            tc::tmem_wait_32(v);
-                            hm[c] = sign_mask(v);
-                            am[c] = hm[c] & below_mask(v, a.lo);
-                        }
+                    if (!seen) {
+                        release();
+                        continue;
                     }
-                    release();
-                    ++uses;
-                    if (!seen) continue;
+#pragma unroll
+                    for (uint32_t c = 0; c < NCH; ++c) {
+                        if (!((seen >> c) & 1u)) continue;
+                        tc::tmem_ld_32(acc + c * 32u, v);
+                        tc::tmem_wait_32(v);
+                        if (seen >> c == 1u) release();   // the last one to be read again
+                        hm[c] = sign_mask(v);
+                        am[c] = hm[c] & below_mask(v, a.lo);
+                    }
                 }
+                if (!seen) continue;
                 // lanes with a hit pass it on
 #pragma unroll
                 for (uint32_t c = 0; c < NCH; ++c) {
                     const uint32_t who = __ballot_sync(0xffffffffu, hm[c] != 0u);
                     if (who == 0u) continue;
-                    uint32_t k = 0;
-                    if (lane == 0) k = atomicAdd(&S.produced, __popc(who));
-                    k = __shfl_sync(0xffffffffu, k, 0) + __popc(who & lanemask_lt());
-                    if (hm[c]) {
-                        ring_wait(S.seq[k % kRing], k, abort, a.err, a.wait_cycles);
-                        S.ring[k % kRing] = make_uint4(t, row | ((col_base >> 5) + c) << 7, hm[c], am[c]);
-                        __threadfence_block();
-                        *(volatile uint32_t*)&S.seq[k % kRing] = k + 1;
+                    const uint32_t n = __popc(who);
+                    if (prod + n > room) {
+                        publish();
+                        room = ring_wait(S.consumed[ew], prod + n - kRing, abort, a.err, a.wait_cycles) + kRing;
+                        __syncwarp();
+                        room = __shfl_sync(0xffffffffu, room, 0);
                     }
-                    __syncwarp();
+                    if (hm[c])
+                        S.ring[ew][(prod + __popc(who & lanemask_lt())) % kRing] =
+                            make_uint4(t, row | ((col_base >> 5) + c) << 7, hm[c], am[c]);
+                    prod += n;
                 }
+                publish();
             }
             __threadfence_block();
             __syncwarp();
             if (lane == 0) atomicAdd(&S.done, 1u);
         } else {
-            // ---------------- hits: batches of up to 32 records, one per lane
+            // ---------------- hits: batches of up to 32 records, one per lane, from this warp's rings:
+            // lane l keeps the account of ring hw + l * HW
+            constexpr uint32_t HW = hit_warps(DENSE), RINGS = ((uint32_t)kEpiWarps + HW - 1) / HW;
+            const uint32_t hw = warp - 1 - kAcc - kEpiWarps, ring = hw + lane * HW;
+            const bool mine = ring < (uint32_t)kEpiWarps;
+            uint32_t taken = 0;
             uint32_t n_acc = 0, n_band = 0;
             for (;;) {
-                uint32_t k = 0, avail = 0;
-                if (lane == 0) {
-                    k = atomicAdd(&S.taken, 32u);
-                    // a whole batch, or what is left once every epilogue warp is through
-                    const long long t0 = clock64();
-                    for (;;) {
-                        const uint32_t d = *(volatile uint32_t*)&S.done;
-                        __threadfence_block();
-                        avail = *(volatile uint32_t*)&S.produced;
-                        if ((int)(avail - k) >= 32 || d == (uint32_t)kEpiWarps || *abort) break;
-                        if (clock64() - t0 > a.wait_cycles) {
-                            *abort = 1u;
-                            atomicExch(a.err, 1u);
-                            break;
-                        }
-                        __nanosleep(500);
-                    }
-                }
-                k = __shfl_sync(0xffffffffu, k, 0);
-                avail = __shfl_sync(0xffffffffu, avail, 0);
-                const uint32_t n = (int)(avail - k) > 0 ? min(32u, avail - k) : 0u;
-                if (n == 0u) break;
-                uint4 rec = make_uint4(0u, 0u, 0u, 0u);
-                if (lane < n) {
-                    const uint32_t slot = (k + lane) % kRing;
-                    ring_wait(S.seq[slot], k + lane + 1u, abort, a.err, a.wait_cycles);
-                    rec = S.ring[slot];
+                uint32_t avail, incl, total;
+                const long long t0 = clock64();
+                for (uint32_t polls = 0;; ++polls) {
+                    // a whole batch, a ring that is half full, what is left once every epilogue warp
+                    // is through, or what has waited (its writer may need the room)
+                    const uint32_t d = __shfl_sync(0xffffffffu, *(volatile uint32_t*)&S.done, 0);
                     __threadfence_block();
-                    *(volatile uint32_t*)&S.seq[slot] = k + lane + kRing;
+                    avail = mine ? *(volatile uint32_t*)&S.produced[ring] - taken : 0u;
+                    const uint32_t stop = *abort;
+                    incl = avail;
+#pragma unroll
+                    for (uint32_t o = 1; o < RINGS; o <<= 1) {
+                        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += x;
+                    }
+                    total = __shfl_sync(0xffffffffu, incl, RINGS - 1);
+                    if (__any_sync(0xffffffffu, total >= 32u || avail >= kRing / 2 || d == (uint32_t)kEpiWarps || stop ||
+                                                  (total && polls >= 8u)))
+                        break;
+                    if (clock64() - t0 > a.wait_cycles) {
+                        *abort = 1u;
+                        atomicExch(a.err, 1u);
+                    }
+                    __nanosleep(500);
                 }
+                __threadfence_block();
+                const uint32_t n = min(32u, total);
+                if (n == 0u) break;
+                const uint32_t excl = incl - avail;
+                uint32_t src = 0;   // the lane whose ring holds record `lane` of the batch
+#pragma unroll
+                for (uint32_t l = 0; l + 1 < RINGS; ++l) src += __shfl_sync(0xffffffffu, incl, l) <= lane;
+                const uint32_t at = lane - __shfl_sync(0xffffffffu, excl, src) + __shfl_sync(0xffffffffu, taken, src);
+                uint4 rec = make_uint4(0u, 0u, 0u, 0u);
+                if (lane < n) rec = S.ring[min(hw + src * HW, (uint32_t)kEpiWarps - 1u)][at % kRing];
+                __threadfence_block();
                 __syncwarp();
+                if (mine && excl < n && avail) {
+                    taken += min(avail, n - excl);
+                    *(volatile uint32_t*)&S.consumed[ring] = taken;
+                }
                 // the tile's range: the last r with tp[r] <= tile
                 uint32_t r = 0;
 #pragma unroll
@@ -647,7 +683,6 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                         });
                     }
                 }
-                if (n < 32u) break;
             }
             unsigned long long w_acc = n_acc, w_band = n_band;
             for (int o = 16; o > 0; o >>= 1) {
@@ -1021,7 +1056,7 @@ constexpr size_t kSmemBudget = 225 * 1024;
 
 // Query columns per work item: 512 (each candidate tile fetched once for both
 // accumulators: half the L2 traffic per pair) where three stages fit beside them.
-uint32_t tc_qcols(uint32_t nkb) { return tc_smem_bytes(nkb, kQBMax, 3) <= kSmemBudget ? kQBMax : kAccCols; }
+uint32_t tc_qcols(uint32_t nkb) { return tc_smem_bytes(nkb, kQBMax, 3) <= kSmemBudget ? kQBMax : kQBMax / 2; }
 
 uint32_t tc_stages(uint32_t nkb) {
     uint32_t s = kMaxStages;
@@ -1046,7 +1081,7 @@ bool tc_supported(const hj_index* ix, int kind) {
     if (ix->dtype != HJ_F32 || ix->d < 8) return false;
     if (kind != HJ_REFINE_TC_F16 && kind != HJ_REFINE_TC_BF16) return false;
     uint32_t nkb = kpad_for(ix->d) / 32;
-    if (tc_smem_bytes(nkb, kAccCols, 2) > kSmemBudget) return false;
+    if (tc_smem_bytes(nkb, kQBMax / 2, 2) > kSmemBudget) return false;
     uint32_t rows = 1;
     for (uint32_t j = 1; j < ix->k; ++j) rows *= 3;
     return rows <= kMaxRanges && ix->n < 0x7FFFFF00u;
