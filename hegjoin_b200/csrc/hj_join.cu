@@ -16,10 +16,10 @@
 //     batch; batches are cut at half the buffer (the reference allocates twice
 //     its nominal buffer, GPU.cu:1042-1062) and a batch whose pairs overflow
 //     the buffer is split in two and re-run, instead of writing out of bounds;
-//   * pairs are grouped by query id on the device with the library's radix
-//     sort, and the neighbour table (the device form of neighborTableLookup,
-//     structs.h:35-41) is built on the device; nothing crosses PCIe unless the
-//     caller exports it.
+//   * pairs are grouped by query id on the device by a counting sort (the refine
+//     counts while it emits), and the neighbour table (the device form of
+//     neighborTableLookup, structs.h:35-41) is built on the device; nothing crosses
+//     PCIe unless the caller exports it.
 
 #include <algorithm>
 #include <chrono>
@@ -164,6 +164,9 @@ __global__ void k_gather_items(const HjBlock* __restrict__ in, const uint32_t* _
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m) out[i] = in[idx[i]];
 }
+
+// Candidate pairs per launch of a digest-only join.
+constexpr double kDigestBatchPairs = 17179869184.0;
 
 // Counters and flags of one join, in one device allocation.
 struct JoinCtl {
@@ -852,8 +855,10 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         if (!count_only) HJ_CUDA(cudaEventRecord(e1, st));
         return HJ_OK;
     };
-    // ---- digests that nobody wants the pairs of: one launch, no estimate, no batches.  Only
-    // without limits on buffers and batches, which such a join would never meet.
+    // ---- digests that nobody wants the pairs of: no estimate and no pair buffer.  Only
+    // without limits on buffers and batches, which such a join would never meet.  A batch is
+    // a launch of about 2^34 candidate pairs (some 10 ms), so that a join of any length lets
+    // other streams' kernels in between.
     DigestOut dig;
     if (warp && crowded && !opts.result_capacity && !opts.device_bytes_cap && !opts.max_batches &&
         handler.digest_only(&dig)) {
@@ -862,7 +867,13 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         HJ_TRY(event_acquire(&kev.ev[0].first));
         HJ_TRY(event_acquire(&kev.ev[0].second));
         HJ_CUDA(cudaEventRecord(kev.ev[0].first, st));
-        HJ_TRY(launch_refine_digest(ix, blocks, nblocks, avg_work, head, dig.count, dig.sum, dig.xr, &ctl->valid, st));
+        const uint32_t per_batch = (uint32_t)std::min(
+            (double)std::max<uint32_t>(nblocks, 1), std::max(1.0, kDigestBatchPairs / std::max(avg_work, 1.0)));
+        for (uint32_t b = 0; b < nblocks; b += std::min(per_batch, nblocks - b), ++S.n_batches) {
+            if (b) HJ_CUDA(cudaMemsetAsync(head, 0, sizeof(unsigned int), st));
+            HJ_TRY(launch_refine_digest(ix, blocks + b, std::min(per_batch, nblocks - b), avg_work, head, dig.count,
+                                        dig.sum, dig.xr, &ctl->valid, st));
+        }
         HJ_CUDA(cudaEventRecord(kev.ev[0].second, st));
         JoinCtl* hc = nullptr;
         HJ_TRY(readback_buffer(reinterpret_cast<void**>(&hc)));
@@ -870,8 +881,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         HJ_CUDA(cudaStreamSynchronize(st));
         HJ_CUDA(cudaEventElapsedTime(&S.ms_refine_kernel, kev.ev[0].first, kev.ev[0].second));
         S.total_pairs = S.estimated_pairs = hc->valid;
-        S.n_batches = nblocks ? 1 : 0;
-        S.refine_launches = nblocks ? 1 : 0;
+        S.refine_launches = S.n_batches;
         S.ms_total = ms_since(t_start);
         S.ms_refine = S.ms_total - S.ms_setup;
         S.kernel_launches = (uint32_t)(thread_launch_count() - launches0);
@@ -1021,7 +1031,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         HJ_TRY(max_cap_from_free(&max_cap));
         cap = std::min(cap, max_cap);
     }
-    cap = std::min<uint64_t>(cap, 0xF0000000ull);   // radix sort and 32-bit counts per batch
+    cap = std::min<uint64_t>(cap, 0xF0000000ull);   // 32-bit slots and counts per batch
     if (cap <= chunk_slack) {
         set_error("hj_join: not enough device memory for a result buffer");
         return HJ_ERR_OOM;

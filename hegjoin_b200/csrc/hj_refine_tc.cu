@@ -5,7 +5,7 @@
 // loop is a dense distance evaluation; here each (candidate tile x query block)
 // is a GEMM on the 5th-generation tensor cores:
 //
-//   A (M = 128 candidates, streamed by TMA) = [-2 c~, 1, 1, N_c hi, N_c lo, 0...]
+//   A (M = 128 candidates, in bulk copies)  = [-2 c~, 1, 1, N_c hi, N_c lo, 0...]
 //   B (N = 128 queries, resident)           = [  q~, N_q hi, N_q lo, 1, 1, 0...]
 //   D' = A B^T = N_q + N_c - 2 q~.c~        (FP32 accumulate in TMEM)
 //
@@ -1198,7 +1198,7 @@ static hj_status launch_prep(const hj_index* ix, int kind, const float* origin, 
 hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st) {
     if (ix->tc_kind == kind && ix->tc_state) return HJ_OK;
     // Drop the previous operand forms before anything else: if a step below
-    // fails, no tensor map may be left pointing at freed buffers.
+    // fails, nothing may be left pointing at freed buffers.
     tc_release(ix);
     ix->tc_kind = -1;
     dfree(ix->tc_a, st);
