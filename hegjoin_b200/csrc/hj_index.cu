@@ -124,6 +124,20 @@ void init_memory_pool() {
     cudaGetLastError();
 }
 
+// Bytes that the memory pool holds and nobody uses (0 when it cannot say).
+uint64_t pool_idle_bytes() {
+    int dev = 0;
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return reserved > used ? reserved - used : 0;
+}
+
 template <typename T>
 static T sq_threshold_t(T eps) {
     // sqrt is correctly rounded and monotone, so {x : RN(sqrt(x)) <= eps} is

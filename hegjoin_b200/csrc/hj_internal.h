@@ -101,6 +101,7 @@ double sq_threshold(double eps, int dtype);
 
 // Keep freed stream-ordered allocations mapped for reuse (called once per process).
 void init_memory_pool();
+uint64_t pool_idle_bytes();
 
 // hj_refine_tc.cu
 void tc_release(hj_index* ix);

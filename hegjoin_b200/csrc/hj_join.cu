@@ -165,6 +165,9 @@ __global__ void k_gather_items(const HjBlock* __restrict__ in, const uint32_t* _
     if (i < m) out[i] = in[idx[i]];
 }
 
+// Share of the free device memory that a join's buffers may take.
+constexpr double kDefaultMemFraction = 0.6;
+
 // Candidate pairs per launch of a digest-only join.
 constexpr double kDigestBatchPairs = 17179869184.0;
 
@@ -719,7 +722,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     hj_join_opts opts;
     if (opts_in) opts = *opts_in; else hj_join_opts_default(&opts);
     if (opts.sample_rate <= 0 || opts.sample_rate > 1) opts.sample_rate = 0.02;
-    if (opts.mem_fraction <= 0 || opts.mem_fraction > 0.95) opts.mem_fraction = 0.6;
+    if (opts.mem_fraction <= 0 || opts.mem_fraction > 0.95) opts.mem_fraction = kDefaultMemFraction;
     if (opts.shard_count > 1 && opts.shard_index >= opts.shard_count) {
         set_error("hj_join: shard_index %u out of range for %u shards", opts.shard_index, opts.shard_count);
         return HJ_ERR_INVALID;
@@ -1025,8 +1028,12 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         *out = std::min<uint64_t>((uint64_t)(opts.mem_fraction * usable / bytes_per_slot), 0xF0000000ull);
         return HJ_OK;
     };
+    // and the memory pool does not hold them idle already (at the default share): the call takes
+    // 0.1 ms alone and up to 82 ms while other processes use the driver, beside a join of 20 ms
     const bool large = (double)cap * bytes_per_slot + result_bytes > 1024.0 * 1024 * 1024;
-    if (large) {
+    bool queried = false;
+    if (large && !(opts.mem_fraction == kDefaultMemFraction && (double)cap * bytes_per_slot <= (double)pool_idle_bytes())) {
+        queried = true;
         uint64_t max_cap = 0;
         HJ_TRY(max_cap_from_free(&max_cap));
         cap = std::min(cap, max_cap);
@@ -1073,7 +1080,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     // when the free-memory query was skipped and the allocation fails, query and retry smaller
     uint32_t* slab = nullptr;
     hj_status as = tmp.alloc(&slab, cap * slot_words);
-    if (as == HJ_ERR_OOM && !large && !opts.result_capacity) {
+    if (as == HJ_ERR_OOM && !queried && !opts.result_capacity) {
         uint64_t max_cap = 0;
         HJ_TRY(max_cap_from_free(&max_cap));
         if (max_cap < cap && max_cap > chunk_slack) {
@@ -1333,7 +1340,7 @@ void hj_join_opts_default(hj_join_opts* o) {
     *o = hj_join_opts{};
     o->refine = HJ_REFINE_AUTO;
     o->sample_rate = 0.02;
-    o->mem_fraction = 0.6;
+    o->mem_fraction = kDefaultMemFraction;
     o->use_graphs = 0;
     o->keep_keys = 0;
 }
