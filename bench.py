@@ -60,6 +60,11 @@ class ClockSampler:
             self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.index), f"--query-gpu={q}",
                                           "--format=csv,noheader,nounits", "-lms", "200"],
                                          stdout=self.f, stderr=subprocess.DEVNULL)
+            # its start-up holds driver locks for a second or so: the timed region begins after
+            # the first sample
+            t0 = time.time()
+            while os.path.getsize(self.path) == 0 and time.time() - t0 < 10.0 and self.proc.poll() is None:
+                time.sleep(0.05)
         except Exception:
             self.proc = None
         return self
@@ -696,21 +701,24 @@ def main():
     pk, pk_kind = peaks()
     tc = refine_used in (hj.HJ_REFINE_TC_F16, hj.HJ_REFINE_TC_BF16)
     cand_rank = cand / ws
+    # a join in one batch on one GPU evaluates each unordered pair once
+    once = 0.5 if ws == 1 and int(recs[-1][8]) == 1 else 1.0
     if tc:
-        flops = 2.0 * wl.d * cand_rank
+        flops = 2.0 * wl.d * cand_rank * once
         peak = pk.get("bf16_tflops_sustained", pk.get("bf16_tflops"))
         achieved = flops / (kern_ms / 1e3) / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "kernel": "k_refine_tc",
                 "peak_kind": f"{pk_kind} bf16 dense, sustained (kernel runs inside a seconds-long step)",
-                "algorithmic": "2*d flops per candidate pair (C = sum over queries of stencil candidates)"}
+                "algorithmic": f"2*d flops per evaluated pair: {once} C (C = sum over queries of stencil candidates)"}
     else:
         # queries read once, each 64-query block reads its candidates once, pairs written as two u32
         s = 4 if wl.dtype == "f32" else 8
         byts = (wl.n / ws) * wl.d * s + (cand_rank / 64.0) * wl.d * s + 8.0 * pairs
         achieved = byts / (kern_ms / 1e3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / pk["hbm_gbs"], "traffic": None, "kernel": "k_refine_plain",
+                "frac": achieved / pk["hbm_gbs"], "traffic": None,
+                "kernel": "k_refine_warp" if wl.d <= (12 if s == 4 else 8) else "k_refine_plain",
                 "peak_kind": f"{pk_kind} copy bandwidth",
                 "algorithmic": "n*d*s + (C/64)*d*s + 8*P bytes per launch"}
     traffic_path = os.path.join(ROOT, "profiles", f"traffic_{wl.name}.txt")
@@ -820,9 +828,11 @@ def main():
         c3 = wlmod.WORKLOADS["c3_90d"]
         cand3 = t3["plain_fp32"]["candidates"]
         # plain FP32: 3 d flops per candidate (sub, multiply, add) on the FP32 pipe; the filter:
-        # 2 d per candidate on the tensor pipe (the MMA itself does 2 Kpad)
+        # 2 d per evaluated pair on the tensor pipe, half of the candidates in one batch (the MMA
+        # itself does 2 Kpad)
         for arm, flops_per, peak_key in (("plain_fp32", 3.0 * c3.d, "fp32x2_fma_tflops"),
-                                          ("tc_filter", 2.0 * c3.d, "f16_mma_tflops")):
+                                          ("tc_filter", (1.0 if t3["tc_filter"]["batches"] == 1 else 2.0) * c3.d,
+                                           "f16_mma_tflops")):
             ach = flops_per * cand3 / (t3[arm]["refine_kernel_ms"] / 1e3) / 1e12
             t3[arm]["roofline"] = {"achieved_tflops": ach, "own_peak_tflops": own[peak_key],
                                    "frac_of_own_peak": ach / own[peak_key], "peak": peak_key}
