@@ -722,6 +722,9 @@ __global__ void k_band_recheck(const float* __restrict__ pts, const uint32_t* __
                                float thr, const uint32_t* __restrict__ bq, const uint32_t* __restrict__ bc,
                                const unsigned long long* __restrict__ band_used, unsigned long long band_cap,
                                uint32_t sym, PairSink sink, uint32_t* __restrict__ qcount) {
+    // after an overflow the band holds slots that were reserved and never written (the batch is
+    // run again in any case)
+    if (*(volatile const uint32_t*)sink.overflow) return;
     const unsigned long long n = min(*band_used, band_cap);
     WarpChunk wc;
     warp_chunk_init(wc);
