@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
     if (tid == 0) {
         for (uint32_t s = 0; s < a.stages; ++s) {
             tc::mbar_init(&S.full_a[s], 1);
-            tc::mbar_init(&S.empty_a[s], kAcc);   // commits by the tile's issuers
+            tc::mbar_init(&S.empty_a[s], kAcc);   // one arrival for each issuer
         }
         for (int j = 0; j < kAcc; ++j) {
             tc::mbar_init(&S.full_acc[j], 1);
@@ -455,9 +455,17 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
             // N = this group's query columns in whole groups of 32
             const uint32_t cols = ncols > first_col ? min((uint32_t)kAccCols, ncols - first_col) : 32u;
             const uint32_t idesc = tc::idesc_f16(a.fmt, kTileRows, (cols + 31u) & ~31u);
+            // A wait names a barrier's phase by one bit, so an issuer may be at most one fill of a
+            // stage ahead of the last one that it saw.  Where the stages are a multiple of the round
+            // (4 or 8 of them: d <= 124), a stage's tiles within an item are all the same issuer's.
+            // Otherwise (2 or 3 stages) every issuer waits for every tile, and those that a tile is
+            // not for arrive at the stage's release themselves: no fill is missed, none is overrun.
+            const bool in_step = a.stages % round != 0u;
+            const uint32_t commits = in_step ? 1u : round;
             for (uint32_t t = t_lo; t < t_hi; ++t) {
-                if (((t - t_lo) & (round - 1u)) == turn) {
-                    tc::mbar_wait<false>(&S.full_a[stage], use_a & 1u, abort, a.err, a.wait_cycles);
+                const bool mine = ((t - t_lo) & (round - 1u)) == turn;
+                if (mine || in_step) tc::mbar_wait<false>(&S.full_a[stage], use_a & 1u, abort, a.err, a.wait_cycles);
+                if (mine) {
                     if (uses > 0) tc::mbar_wait<false>(&S.empty_acc[h], (uses - 1) & 1u, abort, a.err, a.wait_cycles);
                     ++uses;
                     if (tc::elect_one()) {
@@ -472,8 +480,11 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                             tc::mma_f16(tmem + h * kAccCols, ad + 2u, bd + 2u, idesc, 1u);
                         }
                         tc::mma_commit(&S.full_acc[h]);
-                        for (uint32_t i = 0; i < round; ++i) tc::mma_commit(&S.empty_a[stage]);
+                        for (uint32_t i = 0; i < commits; ++i) tc::mma_commit(&S.empty_a[stage]);
                     }
+                    __syncwarp();
+                } else if (in_step) {
+                    if (lane == 0) tc::mbar_arrive(&S.empty_a[stage]);
                     __syncwarp();
                 }
                 if (++stage == a.stages) { stage = 0; ++use_a; }
