@@ -90,10 +90,13 @@ hj_status readback_buffer(void** p) {
     return HJ_OK;
 }
 
+constexpr size_t kDefaultSmem = 48 * 1024;
+constexpr size_t kStaticSmemMax = 16 * 1024;   // no kernel here that takes dynamic shared memory has more
 hj_status ensure_smem_ptr(const void* kern, size_t bytes) {
     static std::mutex mu;
     static std::map<const void*, size_t> done;
-    if (bytes <= 48 * 1024) return HJ_OK;
+    // the 48 KB that need no raised limit hold the kernel's static shared memory too
+    if (bytes <= kDefaultSmem - kStaticSmemMax) return HJ_OK;
     std::lock_guard<std::mutex> lk(mu);
     size_t& have = done[kern];
     if (bytes <= have) return HJ_OK;
