@@ -271,7 +271,7 @@ __global__ void k_cell_ids(const T* __restrict__ db, uint32_t n, uint32_t d, Geo
         lid += (unsigned long long)c * grid.mult[j];
     }
     keys[i] = lid;
-    vals[i] = i;
+    vals[i] = zero ? i | 0x80000000u : i;   // the sort carries the mark to the point's place
     if (al) atomicExch(alias, 1u);
     if (zero) atomicExch(silent, 1u);
 }
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) k_gather_rows(const T* __restrict__ db, c
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; r0 < n; r0 += warps * 32u) {
         const uint32_t rows = min(32u, n - r0);
-        const uint32_t id = lane_id() < rows ? perm[r0 + lane_id()] : 0u;
+        const uint32_t id = lane_id() < rows ? perm[r0 + lane_id()] & 0x7FFFFFFFu : 0u;
         T* dst = out + (size_t)r0 * d;
         for (uint32_t f0 = 0; f0 < rows * d; f0 += 32) {
             const uint32_t f = f0 + lane_id();
@@ -318,6 +318,16 @@ __global__ void __launch_bounds__(256) k_gather_rows(const T* __restrict__ db, c
             if (f < rows * d) dst[f] = db[(size_t)src * d + l];
         }
     }
+}
+
+// The sorted lookup array with the marks of silent cells' points (bit 31) into `marked`,
+// and without them in place.
+__global__ void k_split_marks(uint32_t* __restrict__ perm, uint32_t* __restrict__ marked, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t x = perm[i];
+    marked[i] = x;
+    perm[i] = x & 0x7FFFFFFFu;
 }
 
 // ---- workload ------------------------------------------------------------------------
@@ -544,6 +554,11 @@ hj_status index_create_t(const T* d_db, uint32_t n, uint32_t d, uint32_t k, T ep
                   "(epsilon below the coordinates' rounding granularity); unsupported");
         return HJ_ERR_UNSUPPORTED;
     }
+    if (ix->any_silent) {
+        HJ_TRY(dalloc(&ix->perm_flag, n, st));
+        k_split_marks<<<grid1, 256, 0, st>>>(ix->perm, ix->perm_flag, n);
+        HJ_LAUNCHED();
+    }
     return HJ_OK;
 }
 
@@ -654,38 +669,7 @@ void free_index(hj_index* ix, cudaStream_t st) {
     dfree(ix->perm_flag, st);
 }
 
-// Marks the points of silent cells (a coordinate of 0) in bit 31 of a copy of perm.
-__global__ void k_flag_silent(const unsigned long long* __restrict__ cell_lid, const uint32_t* __restrict__ cell_start,
-                              uint32_t nC, HjGrid g, uint32_t* __restrict__ perm) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nC) return;
-    unsigned long long L = cell_lid[i];
-    bool silent = false;
-    for (uint32_t j = 0; j < g.k; ++j) {
-        const unsigned long long q = L / g.n_cells[j];
-        silent |= L == q * g.n_cells[j];
-        L = q;
-    }
-    if (!silent) return;
-    for (uint32_t p = cell_start[i]; p < cell_start[i + 1]; ++p) perm[p] |= 0x80000000u;
-}
-
 }  // namespace
-
-hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st) {
-    *out = ix->perm;
-    if (!ix->any_silent) return HJ_OK;
-    if (!ix->perm_flag) {
-        uint32_t* p = nullptr;
-        HJ_TRY(dalloc(&p, ix->n, st));
-        ix->perm_flag = p;
-        HJ_CUDA(cudaMemcpyAsync(p, ix->perm, (size_t)ix->n * 4, cudaMemcpyDeviceToDevice, st));
-        k_flag_silent<<<(ix->nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->nC, ix->grid, p);
-        HJ_LAUNCHED();
-    }
-    *out = ix->perm_flag;
-    return HJ_OK;
-}
 
 // Launches of the workload order; *folded (in tmp) then holds totalCandidates and the
 // largest count, for workload_done.

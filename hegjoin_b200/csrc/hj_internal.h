@@ -87,7 +87,7 @@ struct hj_index {
     // tensor-core operands (built on first use)
     void* tc_a = nullptr;            // query form: K-block planes (hj_refine_tc.cu)
     void* tc_b = nullptr;            // candidate form
-    uint32_t* perm_flag = nullptr;   // perm with bit 31 set for points of silent cells (built on first use)
+    uint32_t* perm_flag = nullptr;   // perm with bit 31 set for points of silent cells (null without such cells)
     uint32_t tc_kpad = 0;
     int plain_shape = 0;             // exact refine tile shape (0 or 1; autotuned per d and dtype)
     int tc_kind = -1;                // HJ_REFINE_TC_F16 / _BF16 the operands hold
@@ -111,8 +111,9 @@ constexpr int kWarpMaxD32 = 12;
 constexpr int kWarpMaxD64 = 8;
 
 // perm with the points of silent cells marked (bit 31), for the refines' symmetric
-// form; the index's own perm where no cell is silent.
-hj_status flagged_perm(hj_index* ix, const uint32_t** out, cudaStream_t st);
+// form; the index's own perm where no cell is silent.  Part of the index from its
+// creation: joins of one index may run side by side on several threads and streams.
+inline const uint32_t* flagged_perm(const hj_index* ix) { return ix->perm_flag ? ix->perm_flag : ix->perm; }
 
 // hj_index.cu
 // Work items of up to qb queries per cell, in the workload order; `align` (a

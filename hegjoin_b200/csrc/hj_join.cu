@@ -41,19 +41,19 @@ hj_status launch_refine_plain(const hj_index* ix, const HjBlock* blocks, uint32_
 bool warp_refine_supported(const hj_index* ix);
 uint32_t warp_query_block(uint32_t n);
 uint64_t warp_chunk_slack(uint32_t nblocks, double avg);
-hj_status launch_refine_warp(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
+hj_status launch_refine_warp(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
                              const PairSink& sink, uint32_t count_only, bool sym, unsigned long long* block_counts,
                              uint32_t* qcount, cudaStream_t st);
-hj_status launch_refine_digest(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
+hj_status launch_refine_digest(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
                                uint32_t* d_count, unsigned long long* d_sum, unsigned long long* d_xor,
                                unsigned long long* total, cudaStream_t st);
 hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st);
 uint32_t tc_query_block(const hj_index* ix);
-hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
+hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                            const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
                            unsigned long long* block_counts, unsigned long long* stats, uint32_t* qcount,
                            uint32_t* err, cudaStream_t st);
-hj_status launch_band_recheck(hj_index* ix, const uint32_t* bq, const uint32_t* bc,
+hj_status launch_band_recheck(const hj_index* ix, const uint32_t* bq, const uint32_t* bc,
                               const unsigned long long* band_used, unsigned long long band_cap,
                               const PairSink& sink, uint32_t nblocks, bool sym, uint32_t* qcount,
                               cudaStream_t st);

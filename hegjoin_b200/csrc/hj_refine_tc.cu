@@ -1288,7 +1288,7 @@ void tc_set_dense(hj_index* ix, bool dense) {
 }
 
 // sym: blocks[0..nblocks) is the join's whole list, each unordered pair once.
-hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
+hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
                            const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
                            unsigned long long* block_counts, unsigned long long* stats, uint32_t* qcount,
                            uint32_t* err, cudaStream_t st) {
@@ -1303,8 +1303,7 @@ hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     HJ_TRY(ensure_smem(kern, smem));
     TcArgs a{};
     a.blocks = blocks; a.nblocks = nblocks; a.parts = tc_parts(nblocks); a.head = head;
-    a.perm = ix->perm;
-    if (sym) HJ_TRY(flagged_perm(ix, &a.perm, st));
+    a.perm = sym ? flagged_perm(ix) : ix->perm;
     a.cell_lid = ix->cell_lid; a.cell_start = ix->cell_start; a.grid = ix->grid;
     a.hash = cell_hash(ix);
     a.qform = (const uint8_t*)ix->tc_a; a.cform = (const uint8_t*)ix->tc_b;
@@ -1323,12 +1322,11 @@ hj_status launch_refine_tc(hj_index* ix, const HjBlock* blocks, uint32_t nblocks
     return HJ_OK;
 }
 
-hj_status launch_band_recheck(hj_index* ix, const uint32_t* bq, const uint32_t* bc,
+hj_status launch_band_recheck(const hj_index* ix, const uint32_t* bq, const uint32_t* bc,
                               const unsigned long long* band_used, unsigned long long band_cap, const PairSink& sink,
                               uint32_t nblocks, bool sym, uint32_t* qcount, cudaStream_t st) {
     const unsigned grid = recheck_grid(nblocks);
-    const uint32_t* perm = ix->perm;
-    if (sym) HJ_TRY(flagged_perm(ix, &perm, st));
+    const uint32_t* perm = sym ? flagged_perm(ix) : ix->perm;
     k_band_recheck<<<grid, 256, 0, st>>>((const float*)ix->pts, perm, ix->d, (float)ix->thr, bq, bc, band_used,
                                          band_cap, sym ? 1u : 0u, sink, qcount);
     HJ_LAUNCHED();

@@ -44,38 +44,36 @@ uint64_t warp_chunk_slack(uint32_t nblocks, double avg) {
 }
 
 template <typename T>
-static hj_status make_args(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, bool sample,
-                           bool sym, unsigned int* head, WarpArgs<T>* a, cudaStream_t st) {
-    *a = WarpArgs<T>{};
-    a->pts = (const T*)ix->pts;
-    a->perm = ix->perm;
-    if (sym) HJ_TRY(flagged_perm(ix, &a->perm, st));
-    a->cell_lid = ix->cell_lid;
-    a->cell_start = ix->cell_start;
-    a->cell_edge = ix->cell_edge;
-    a->hash = cell_hash(ix);
-    a->grid = ix->grid;
-    a->thr = (T)ix->thr;
-    a->blocks = blocks;
-    a->nblocks = nblocks;
-    a->parts = warp_parts(nblocks, avg, sample);
-    a->sym = sym ? 1u : 0u;
-    a->head = head;
-    return HJ_OK;
+static WarpArgs<T> make_args(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, bool sample,
+                             bool sym, unsigned int* head) {
+    WarpArgs<T> a{};
+    a.pts = (const T*)ix->pts;
+    a.perm = sym ? flagged_perm(ix) : ix->perm;
+    a.cell_lid = ix->cell_lid;
+    a.cell_start = ix->cell_start;
+    a.cell_edge = ix->cell_edge;
+    a.hash = cell_hash(ix);
+    a.grid = ix->grid;
+    a.thr = (T)ix->thr;
+    a.blocks = blocks;
+    a.nblocks = nblocks;
+    a.parts = warp_parts(nblocks, avg, sample);
+    a.sym = sym ? 1u : 0u;
+    a.head = head;
+    return a;
 }
 
 // Runs the refine over work items blocks[0..nblocks).  `head` must be zero on
 // entry.  count_only: per-item pair counts go to block_counts.  sym: the items are
 // the join's whole list, each unordered pair once.  Each query's pairs are added to
 // qcount, by original id (not with count_only).
-hj_status launch_refine_warp(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
+hj_status launch_refine_warp(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
                              const PairSink& sink, uint32_t count_only, bool sym, unsigned long long* block_counts,
                              uint32_t* qcount, cudaStream_t st) {
     if (nblocks == 0) return HJ_OK;
     auto run = [&](auto zero, auto refine) -> hj_status {
         using T = decltype(zero);
-        WarpArgs<T> a;
-        HJ_TRY(make_args<T>(ix, blocks, nblocks, avg, count_only != 0u, sym, head, &a, st));
+        WarpArgs<T> a = make_args<T>(ix, blocks, nblocks, avg, count_only != 0u, sym, head);
         a.sink = sink;
         a.count_only = count_only;
         a.block_counts = block_counts;
@@ -87,14 +85,13 @@ hj_status launch_refine_warp(hj_index* ix, const HjBlock* blocks, uint32_t nbloc
 
 // The digests of hj_result_digest for every query of the items, and the number of
 // pairs, without writing a pair.  The arrays and *total are added to.
-hj_status launch_refine_digest(hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
+hj_status launch_refine_digest(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, double avg, unsigned int* head,
                                uint32_t* d_count, unsigned long long* d_sum, unsigned long long* d_xor,
                                unsigned long long* total, cudaStream_t st) {
     if (nblocks == 0) return HJ_OK;
     auto run = [&](auto zero, auto refine) -> hj_status {
         using T = decltype(zero);
-        WarpArgs<T> a;
-        HJ_TRY(make_args<T>(ix, blocks, nblocks, avg, false, false, head, &a, st));
+        WarpArgs<T> a = make_args<T>(ix, blocks, nblocks, avg, false, false, head);
         a.d_count = d_count;
         a.d_sum = d_sum;
         a.d_xor = d_xor;
