@@ -50,7 +50,7 @@ hj_status launch_refine_digest(const hj_index* ix, const HjBlock* blocks, uint32
 hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st);
 uint32_t tc_query_block(const hj_index* ix);
 hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
-                           const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
+                           const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym, bool dense,
                            unsigned long long* block_counts, unsigned long long* stats, uint32_t* qcount,
                            uint32_t* err, cudaStream_t st);
 hj_status launch_band_recheck(const hj_index* ix, const uint32_t* bq, const uint32_t* bc,
@@ -62,7 +62,6 @@ uint64_t tc_emit_warps(uint32_t nblocks);
 double tc_delta(const hj_index* ix);
 double tc_band_ratio(const hj_index* ix);
 bool tc_supported(const hj_index* ix, int kind);
-void tc_set_dense(hj_index* ix, bool dense);
 }  // namespace hj
 
 struct hj_result {
@@ -837,6 +836,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     PairSink no_band{nullptr, nullptr, nullptr, 0, overflow};
 
     EventPairs kev;   // refine kernel launches of the join proper
+    bool dense = false;   // the filter's epilogue: known after the estimate
     // head_reset: zero the work-item queue head first (batches reset it with the rest)
     auto run_refine = [&](const HjBlock* blk, uint32_t nb, const PairSink& sink, const PairSink& band,
                           uint32_t count_only, unsigned long long* bc, bool head_reset = true,
@@ -851,7 +851,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             e1 = kev.ev.back().second;
             HJ_CUDA(cudaEventRecord(e0, st));
         }
-        HJ_TRY(tc ? launch_refine_tc(ix, blk, nb, head, sink, band, count_only, sym, bc,
+        HJ_TRY(tc ? launch_refine_tc(ix, blk, nb, head, sink, band, count_only, sym, dense, bc,
                                      count_only ? nullptr : &ctl->tc_acc, qcount, &ctl->timeout, st)
                : warp ? launch_refine_warp(ix, blk, nb, avg_work, head, sink, count_only, sym, bc, qcount, st)
                       : launch_refine_plain(ix, blk, nb, head, sink, count_only, bc, qcount, st));
@@ -998,7 +998,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     }
     S.estimated_pairs = (uint64_t)total_est;
     S.ms_estimate = ms_since(t_est);
-    if (tc) tc_set_dense(ix, dense_for(total_est, cand_total));
+    dense = tc && dense_for(total_est, cand_total);
 
     // ---- result buffer capacity
     const uint64_t want = bounded ? bound_slots : (uint64_t)(total_est * 2.0) + chunk_slack + 4096;

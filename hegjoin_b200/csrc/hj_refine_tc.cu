@@ -1081,7 +1081,6 @@ uint32_t tc_stages(uint32_t nkb) {
 }  // namespace
 
 struct TcState {
-    bool dense = false;       // masks at once (set from the estimated pair density)
     float gamma_acc = 0;
     int scale_exp = 0;        // operand forms hold (x - origin) * 2^scale_exp
     double thr_s = 0;         // the squared threshold in those units: thr * 4^scale_exp, exact
@@ -1282,24 +1281,20 @@ hj_status tc_prepare(hj_index* ix, int kind, cudaStream_t st) {
     return HJ_OK;
 }
 
-void tc_set_dense(hj_index* ix, bool dense) {
-    TcState* s = tc_state(ix);
-    if (s) s->dense = dense;
-}
-
-// sym: blocks[0..nblocks) is the join's whole list, each unordered pair once.
+// sym: blocks[0..nblocks) is the join's whole list, each unordered pair once.  dense:
+// the epilogue's form (k_refine_tc), a choice of this launch's caller alone.
 hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t nblocks, unsigned int* head,
-                           const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym,
+                           const PairSink& sink, const PairSink& band, uint32_t count_only, bool sym, bool dense,
                            unsigned long long* block_counts, unsigned long long* stats, uint32_t* qcount,
                            uint32_t* err, cudaStream_t st) {
     if (nblocks == 0) return HJ_OK;
-    TcState* s = tc_state(ix);
+    const TcState* s = tc_state(ix);
     if (!s) { set_error("tensor-core operands not prepared"); return HJ_ERR_INVALID; }
     const uint32_t nkb = ix->tc_kpad / 32, qcols = tc_qcols(nkb), stages = tc_stages(nkb);
     size_t smem = tc_smem_bytes(nkb, qcols, stages);
     // one CTA per SM: ask for more than half of the SM's shared memory
     smem = std::max<size_t>(smem, 116 * 1024);
-    auto kern = s->dense ? k_refine_tc<true> : k_refine_tc<false>;
+    auto kern = dense ? k_refine_tc<true> : k_refine_tc<false>;
     HJ_TRY(ensure_smem(kern, smem));
     TcArgs a{};
     a.blocks = blocks; a.nblocks = nblocks; a.parts = tc_parts(nblocks); a.head = head;
@@ -1317,7 +1312,7 @@ hj_status launch_refine_tc(const hj_index* ix, const HjBlock* blocks, uint32_t n
     a.fmt = ix->tc_kind == HJ_REFINE_TC_BF16 ? 1u : 0u;
     a.wait_cycles = kWaitCycles;
     unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)num_sms(), (uint64_t)nblocks * a.parts);
-    kern<<<grid, tc_threads(s->dense), smem, st>>>(a);
+    kern<<<grid, tc_threads(dense), smem, st>>>(a);
     HJ_LAUNCHED();
     return HJ_OK;
 }

@@ -17,7 +17,7 @@ from hegjoin_b200 import workloads
 pytestmark = pytest.mark.gpu
 
 
-def _join_together(ix, streams, refines, off, vals):
+def _join_together(ix, streams, options, off, vals):
     import torch
     import hegjoin_b200 as hj
     start = threading.Barrier(len(streams))
@@ -28,7 +28,7 @@ def _join_together(ix, streams, refines, off, vals):
             start.wait()
             for _ in range(3):
                 with torch.cuda.stream(streams[i]):
-                    o, v = hj.join(ix, refine=refines[i]).to_csr(sort_lists=True)
+                    o, v = hj.join(ix, **options[i]).to_csr(sort_lists=True)
                     got[i] = (o.cpu().numpy().astype(np.uint64), v.cpu().numpy().astype(np.uint32))
                 assert np.array_equal(got[i][0], off) and np.array_equal(got[i][1], vals)
         except BaseException as e:
@@ -56,4 +56,21 @@ def test_exact_joins_of_one_index(cuda, d, k, eps, offset):
         ix = hj.GridIndex(torch.from_numpy(db).to(cuda), k, eps)
         ix.sort_by_workload()
         torch.cuda.synchronize()
-        _join_together(ix, streams, ["exact"] * 4, off, vals)
+        _join_together(ix, streams, [{"refine": "exact"}] * 4, off, vals)
+
+
+def test_filter_joins_of_one_index(cuda):
+    # operand forms made by the tile probe: the joins count their samples in the filter's sparse
+    # form and then run the dense one, each on its own account
+    import torch
+    import hegjoin_b200 as hj
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    db = workloads.exp40(310, 6000, 18, np.float32)
+    eps = np.float32(0.07)
+    off, vals = oracle.join(db, 6, eps)
+    for _ in range(8):
+        ix = hj.GridIndex(torch.from_numpy(db).to(cuda), 6, float(eps))
+        ix.sort_by_workload()
+        hj.probe_tc_tile(ix, "tc_f16", 0, 0)
+        torch.cuda.synchronize()
+        _join_together(ix, streams, [{"refine": "tc_f16"}] * 4, off, vals)
