@@ -653,6 +653,8 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                 const uint32_t lim = in ? (a.sym ? min(blk.q1, cpos + 1u) : blk.q1) : 0u;
                 uint32_t hits = lim > pos0 ? rec.z & low_bits(lim - pos0) : 0u;
                 if (pos0 < q0) hits &= ~low_bits(q0 - pos0);
+                // a silent candidate of a silent query: the pair is neither's
+                if (a.sym && q_silent && hits && (a.perm[cpos] >> 31)) hits = 0u;
                 uint32_t acc = hits & rec.w;
                 uint32_t bnd = hits & ~rec.w;
                 const uint32_t na = __popc(acc), nb = __popc(bnd);
