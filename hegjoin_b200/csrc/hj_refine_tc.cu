@@ -654,7 +654,9 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                 uint32_t hits = lim > pos0 ? rec.z & low_bits(lim - pos0) : 0u;
                 if (pos0 < q0) hits &= ~low_bits(q0 - pos0);
                 // a silent candidate of a silent query: the pair is neither's
-                if (a.sym && q_silent && hits && (a.perm[cpos] >> 31)) hits = 0u;
+                const uint32_t cw = hits && !a.count_only ? a.perm[cpos] : 0u, cid = cw & 0x7FFFFFFFu;
+                const bool fwd = !q_silent, rev = a.sym && !(cw >> 31);
+                if (a.sym && !fwd && !rev) hits = 0u;
                 uint32_t acc = hits & rec.w;
                 uint32_t bnd = hits & ~rec.w;
                 const uint32_t na = __popc(acc), nb = __popc(bnd);
@@ -663,15 +665,14 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                 } else {
                     const uint32_t self = a.sym && in ? cpos - pos0 : 0xFFFFFFFFu;   // bit of the candidate itself
                     // accepted pairs go out in both orders (symmetric form), that of a point with itself once
+                    const uint32_t self_bit = self < 32u ? 1u << self : 0u;
+                    // orders that the named pairs stand for, and those of them with the candidate first
+                    auto reversed = [&](uint32_t m) { return rev ? (uint32_t)__popc(m & ~self_bit) : 0u; };
+                    auto orders = [&](uint32_t m) { return (fwd ? (uint32_t)__popc(m) : 0u) + reversed(m); };
                     if (__any_sync(0xffffffffu, na)) {
-                        const uint32_t cw = na ? a.perm[cpos] : 0u;
-                        const uint32_t cid = cw & 0x7FFFFFFFu;
-                        const bool fwd = !q_silent;
-                        const bool rev = a.sym && !(cw >> 31);
-                        const uint32_t self_hit = self < 32u ? (acc >> self) & 1u : 0u;
-                        const uint32_t cnt = (fwd ? na : 0u) + (rev ? na - self_hit : 0u);
+                        const uint32_t cnt = orders(acc), cnt_rev = reversed(acc);
                         n_acc += cnt;
-                        if (rev && na > self_hit) atomicAdd(&a.qcount[cid], na - self_hit);
+                        if (cnt_rev) atomicAdd(&a.qcount[cid], cnt_rev);
                         warp_emit_serial(a.sink, wc_acc, cnt, [&](auto&& put) {
                             while (acc) {
                                 const uint32_t b = __ffs(acc) - 1u;
@@ -686,7 +687,7 @@ __global__ void __launch_bounds__(tc_threads(DENSE), 1) k_refine_tc(const __grid
                         });
                     }
                     if (__any_sync(0xffffffffu, nb)) {
-                        n_band += a.sym ? 2u * nb : nb;
+                        n_band += orders(bnd);
                         warp_emit_serial(a.band, wc_band, nb, [&](auto&& put) {
                             while (bnd) {
                                 const uint32_t b = __ffs(bnd) - 1u;

@@ -115,8 +115,9 @@ typedef struct {
     uint64_t total_pairs;
     uint32_t n_batches;
     uint32_t n_retries;            /* batches re-run after an overflow */
-    uint64_t band_pairs;           /* tensor-core filter: pairs that needed the exact recheck */
-    uint64_t tc_accepts;           /* tensor-core filter: pairs accepted outside the band */
+    uint64_t band_pairs;           /* tensor-core filter: ordered pairs decided by the exact recheck (both
+                                      orders of a pair are decided by one) */
+    uint64_t tc_accepts;           /* tensor-core filter: ordered pairs accepted outside the band */
     uint64_t estimated_pairs;      /* selectivity estimate before the join */
     double filter_delta;           /* guard band half-width on d2 (tensor-core filter) */
     float ms_estimate, ms_refine, ms_group, ms_total;
