@@ -474,8 +474,12 @@ __global__ void k_digest(const hj_nt_entry* __restrict__ t, uint32_t* const* __r
     }
 }
 
+// Work items list[b0 .. b1): of the join's list, or the halves of an item whose pairs
+// outgrew the buffer by themselves.
 struct Batch {
     uint32_t b0, b1;
+    const HjBlock* list;
+    uint32_t upto;   // items of the join's list up to this batch's end
 };
 
 // ---- autotuner ------------------------------------------------------------------------
@@ -1069,10 +1073,10 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         }
         uint32_t b0 = 0;
         for (uint32_t c : cuts) {
-            batches.push_back({b0, c});
+            batches.push_back({b0, c, blocks, c});
             b0 = c;
         }
-        batches.push_back({b0, nblocks});
+        batches.push_back({b0, nblocks, blocks, nblocks});
     }
     std::reverse(batches.begin(), batches.end());   // used as a stack
 
@@ -1116,8 +1120,8 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         PairSink band = tc ? PairSink{band_q, band_c, &ctl->band_cursor, cap, overflow} : no_band;
         // all items of the join in this one batch: every unordered pair once (a query's pairs
         // must lie in one batch, and a shard owns its queries' pairs only)
-        const bool sym = (tc || warp) && opts.shard_count <= 1 && b.b0 == 0 && b.b1 == nblocks;
-        HJ_TRY(run_refine(blocks + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, qoff, sym));
+        const bool sym = (tc || warp) && opts.shard_count <= 1 && b.list == blocks && b.b0 == 0 && b.b1 == nblocks;
+        HJ_TRY(run_refine(b.list + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, qoff, sym));
         if (tc)
             HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, qoff, st));
         // every query's first slot; qoff[n] = the batch's pairs
@@ -1135,15 +1139,30 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         }
         const unsigned long long used = hc.cursor;
         if (hc.overflow) {
-            if (b.b1 - b.b0 <= 1) {
-                set_error("hj_join: one work item produces more pairs than the result buffer holds (%llu)",
+            S.n_retries++;
+            if (b.b1 - b.b0 > 1) {   // of the join's list: halves come one at a time
+                const uint32_t mid = b.b0 + (b.b1 - b.b0) / 2;
+                batches.push_back({mid, b.b1, blocks, b.b1});
+                batches.push_back({b.b0, mid, blocks, mid});
+                continue;
+            }
+            // one item: its queries in two halves, down to a single query
+            HjBlock half[2];
+            HJ_CUDA(cudaMemcpyAsync(half, b.list + b.b0, sizeof(HjBlock), cudaMemcpyDeviceToHost, st));
+            HJ_CUDA(cudaStreamSynchronize(st));
+            if (half[0].q1 - half[0].q0 <= 1) {
+                set_error("hj_join: one query produces more pairs than the result buffer holds (%llu)",
                           (unsigned long long)cap);
                 return HJ_ERR_OVERFLOW;
             }
-            uint32_t mid = b.b0 + (b.b1 - b.b0) / 2;
-            batches.push_back({mid, b.b1});
-            batches.push_back({b.b0, mid});
-            S.n_retries++;
+            half[1] = half[0];
+            half[0].q1 = half[1].q0 = half[0].q0 + (half[0].q1 - half[0].q0) / 2;
+            HjBlock* halves = nullptr;
+            HJ_TRY(tmp.alloc(&halves, 2));
+            HJ_CUDA(cudaMemcpyAsync(halves, half, sizeof(half), cudaMemcpyHostToDevice, st));
+            HJ_CUDA(cudaStreamSynchronize(st));   // `half` is read by the copy above
+            batches.push_back({1, 2, halves, b.upto});
+            batches.push_back({0, 1, halves, b.upto});
             continue;
         }
         S.tc_accepts += hc.tc_acc;
@@ -1156,7 +1175,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
             // this errs high)
             const double slab_b = (double)cap * bytes_per_slot;
             const double so_far = kept - (double)fixed_kept_bytes - slab_b + kept_bytes_per_pair * (double)valid;
-            const double frac = (double)std::max<uint32_t>(1, b.b1) / nblocks;
+            const double frac = (double)std::max<uint32_t>(1, b.upto) / nblocks;
             S.bytes_wanted = std::max<uint64_t>(
                 S.bytes_wanted, (uint64_t)((double)fixed_kept_bytes + slab_b + 1.1 * so_far / frac));
             set_error("hj_join: the results outgrow the cap of %llu device bytes",
