@@ -529,6 +529,22 @@ bool tuning_enabled() {
     return !(e && e[0] == '0');
 }
 
+// The warp refine's symmetric form saves half of the distances, and pays with reversed
+// pairs that the grouping scatters one by one (with their keys, where somebody reads
+// those) instead of in runs.  It is the faster one from about 40 coordinates evaluated
+// per result pair on, 80 with keys.  Symmetric and plain form, whole join / with a sink,
+// in ms:
+//   2-D, 100,000 points, 800 neighbours   5 per pair  1.40  0.90 / 1.91  1.08
+//   3-D, 300,000 points, 100 neighbours  18           0.92  0.83 / 1.14  0.93
+//   4-D, 300,000 points, 100 neighbours  51           1.11  1.17 / 1.31  1.25
+//   5-D, 100,000 points, 800 neighbours  74           2.31  2.48 / 2.89  2.67
+//   6-D, 300,000 points, 100 neighbours 309           2.23  3.09 / 2.42  3.20
+// (2-D, 1,000,000 points and 1.2e9 pairs with a sink: 39.7 and 15.7 ms.)
+constexpr double kSymWork = 40.0;
+bool symmetric_pays(uint32_t d, double pairs, double cand, bool keys) {
+    return (double)d * cand >= (keys ? 2.0 * kSymWork : kSymWork) * pairs;
+}
+
 // Tensor-core epilogue: with fewer than ~3% of its 32 x 32 chunks holding a hit, ORing the
 // signs and reading the hit chunks again beats a vote per chunk and masks at once.
 // HJ_TC_DEFER=0/1 forces masks or ORs (tests).
@@ -694,6 +710,8 @@ struct BatchHandler {
     }
     // Whether grouped_to always gives arrays of the handler's own.
     virtual bool own_arrays() const { return false; }
+    // Whether the grouped keys are wanted.
+    virtual bool reads_keys() const { return true; }
     // After the last batch, before the join synchronises `st`.
     virtual hj_status finish(cudaStream_t) { return HJ_OK; }
     // `count` pairs of batch `batch`: query ids (ascending) in keys, neighbour ids
@@ -1119,8 +1137,10 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         PairSink sink{keys, vals, &ctl->cursor, cap, overflow};
         PairSink band = tc ? PairSink{band_q, band_c, &ctl->band_cursor, cap, overflow} : no_band;
         // all items of the join in this one batch: every unordered pair once (a query's pairs
-        // must lie in one batch, and a shard owns its queries' pairs only)
-        const bool sym = (tc || warp) && opts.shard_count <= 1 && b.list == blocks && b.b0 == 0 && b.b1 == nblocks;
+        // must lie in one batch, and a shard owns its queries' pairs only).  A join that is
+        // sized by its candidates knows nothing of its pairs, and either form suits it.
+        const bool sym = (tc || (warp && (bounded || symmetric_pays(ix->d, total_est, cand_total, handler.reads_keys())))) &&
+                         opts.shard_count <= 1 && b.list == blocks && b.b0 == 0 && b.b1 == nblocks;
         HJ_TRY(run_refine(b.list + b.b0, b.b1 - b.b0, sink, band, 0, nullptr, false, qoff, sym));
         if (tc)
             HJ_TRY(launch_band_recheck(ix, band_q, band_c, &ctl->band_cursor, cap, sink, b.b1 - b.b0, sym, qoff, st));
@@ -1233,6 +1253,7 @@ struct RetainHandler : BatchHandler {
     bool keep_keys;
     RetainHandler(hj_result* r, bool kk) : res(r), keep_keys(kk) {}
     bool own_arrays() const override { return true; }
+    bool reads_keys() const override { return keep_keys; }
     hj_status grouped_to(uint64_t count, uint32_t** keys, uint32_t** vals, cudaStream_t st) override {
         HJ_TRY(dalloc(vals, count, st));
         res->vals.push_back(*vals);
