@@ -178,7 +178,8 @@ class Scratch {
 // Readbacks land in pinned memory of the calling thread (kReadbackBytes, taken on
 // its first use and handed on when it ends), so that several copies and the wait
 // for them cost one synchronisation: a copy to pageable memory waits by itself.
-// Valid until the thread's next readback.
+// Valid until the thread's next readback, so a caller returns with no copy into it
+// under way: the wait follows its copies at once.
 constexpr size_t kReadbackBytes = 40 * 1024;
 hj_status readback_buffer(void** p);   // hj_index.cu
 

@@ -714,15 +714,15 @@ hj_status build_blocks(hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_bl
     Scratch tmp(st);
     unsigned long long *folded = nullptr, *back = nullptr;
     HJ_TRY(readback_buffer(reinterpret_cast<void**>(&back)));
-    if (!ix->have_workload) {
-        HJ_TRY(workload_launch(ix, tmp, &folded, st));
-        HJ_CUDA(cudaMemcpyAsync(back + 1, folded, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    }
+    if (!ix->have_workload) HJ_TRY(workload_launch(ix, tmp, &folded, st));
     uint32_t* cnt = nullptr;
     HJ_TRY(tmp.alloc(&cnt, (size_t)nC + 1));
     k_block_counts<<<nC / 256 + 1, 256, 0, st>>>(ix->cell_order, ix->cell_start, nC, qb, align, cnt);
     HJ_LAUNCHED();
     HJ_TRY(scan_u32_inplace(cnt, (uint64_t)nC + 1, st));
+    // nothing that can fail for want of memory stands between a copy and the wait for it
+    if (folded)
+        HJ_CUDA(cudaMemcpyAsync(back + 1, folded, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaMemcpyAsync(back, cnt + nC, 4, cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaStreamSynchronize(st));
     if (folded) workload_done(ix, back + 1);

@@ -47,3 +47,4 @@ def test_one_query_too_many_is_refused(cuda):
     with pytest.raises(hj.HJError) as e:
         hj.join(ix, refine="exact", result_capacity=1, shard_count=n // 64, shard_index=0)
     assert e.value.status == hj.HJ_ERR_OVERFLOW
+    ix.close()
