@@ -175,8 +175,12 @@ class Scratch {
     std::vector<void*> held_;
 };
 
+// Id of the current context (0: none yet).  A context that replaces another after
+// cudaDeviceReset has the same handle but an id of its own.
+uint64_t context_id();   // hj_index.cu
+
 // Readbacks land in pinned memory of the calling thread (kReadbackBytes, taken on
-// its first use and handed on when it ends), so that several copies and the wait
+// its first use in a context and handed on when it ends), so that several copies and the wait
 // for them cost one synchronisation: a copy to pageable memory waits by itself.
 // Valid until the thread's next readback, so a caller returns with no copy into it
 // under way: the wait follows its copies at once.

@@ -22,6 +22,8 @@
 #include <map>
 #include <mutex>
 
+#include <cuda.h>
+
 #include "hj_internal.h"
 
 namespace hj {
@@ -54,39 +56,84 @@ bool injected_alloc_failure() {
     return g_fail_alloc_in.fetch_sub(1, std::memory_order_relaxed) == 1;
 }
 
+// Through the runtime's driver entry-point query (the library does not link libcuda).
+uint64_t context_id() {
+    using Current = CUresult (*)(CUcontext*);
+    using Id = CUresult (*)(CUcontext, unsigned long long*);
+    auto entry = [](const char* name) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+                   ? p
+                   : nullptr;
+    };
+    static const Current current = reinterpret_cast<Current>(entry("cuCtxGetCurrent"));
+    static const Id id_of = reinterpret_cast<Id>(entry("cuCtxGetId"));
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (current && id_of && current(&c) == CUDA_SUCCESS && c) id_of(c, &id);
+    return id;
+}
+
 namespace {
+// A readback buffer lives as long as the context that it was allocated in.
+struct Pinned {
+    void* p;
+    int dev;
+    uint64_t ctx;
+};
 // Buffers of ended threads wait for the next thread (a server's workers come and go
 // with it, and allocating pinned memory stops the device for a moment); at most
-// kReadbackKept of them.
+// kReadbackKept of them.  Those of a context that is gone are forgotten.
 constexpr size_t kReadbackKept = 32;
 std::mutex g_readback_mu;
-std::vector<void*> g_readback_free;
+std::vector<Pinned> g_readback_free;
 struct Readback {
-    void* p = nullptr;
+    std::vector<Pinned> bufs;   // one per context that the thread has used
     ~Readback() {
-        if (!p) return;
-        {
-            std::lock_guard<std::mutex> lk(g_readback_mu);
-            if (g_readback_free.size() < kReadbackKept) {
-                g_readback_free.push_back(p);
-                return;
+        for (const Pinned& b : bufs) {
+            if (cudaSetDevice(b.dev) != cudaSuccess || context_id() != b.ctx) continue;
+            {
+                std::lock_guard<std::mutex> lk(g_readback_mu);
+                if (g_readback_free.size() < kReadbackKept) {
+                    g_readback_free.push_back(b);
+                    continue;
+                }
             }
+            cudaFreeHost(b.p);
         }
-        cudaFreeHost(p);
     }
 };
 thread_local Readback t_readback;
 }  // namespace
 hj_status readback_buffer(void** p) {
-    if (!t_readback.p) {
+    Pinned b{nullptr, 0, context_id()};
+    if (b.ctx == 0) {
+        HJ_CUDA(cudaFree(nullptr));   // makes the device's context current
+        b.ctx = context_id();
+    }
+    for (const Pinned& have : t_readback.bufs)
+        if (have.ctx == b.ctx) {
+            *p = have.p;
+            return HJ_OK;
+        }
+    HJ_CUDA(cudaGetDevice(&b.dev));
+    auto gone = [&](const Pinned& x) { return x.dev == b.dev && x.ctx != b.ctx; };
+    auto& bufs = t_readback.bufs;
+    bufs.erase(std::remove_if(bufs.begin(), bufs.end(), gone), bufs.end());
+    {
         std::lock_guard<std::mutex> lk(g_readback_mu);
-        if (!g_readback_free.empty()) {
-            t_readback.p = g_readback_free.back();
-            g_readback_free.pop_back();
+        auto& free = g_readback_free;
+        free.erase(std::remove_if(free.begin(), free.end(), gone), free.end());
+        auto it = std::find_if(free.begin(), free.end(), [&](const Pinned& x) { return x.ctx == b.ctx; });
+        if (it != free.end()) {
+            b.p = it->p;
+            free.erase(it);
         }
     }
-    if (!t_readback.p) HJ_CUDA(cudaHostAlloc(&t_readback.p, kReadbackBytes, cudaHostAllocPortable));
-    *p = t_readback.p;
+    if (!b.p) HJ_CUDA(cudaHostAlloc(&b.p, kReadbackBytes, cudaHostAllocDefault));
+    bufs.push_back(b);
+    *p = b.p;
     return HJ_OK;
 }
 
