@@ -187,7 +187,7 @@ uint64_t context_id();   // hj_index.cu
 constexpr size_t kReadbackBytes = 40 * 1024;
 hj_status readback_buffer(void** p);   // hj_index.cu
 
-// Raise a kernel's dynamic shared-memory limit once per (kernel, size), safe
+// Raise a kernel's dynamic shared-memory limit once per (context, kernel, size), safe
 // when several host threads launch joins concurrently.
 hj_status ensure_smem_ptr(const void* kern, size_t bytes);   // hj_index.cu
 template <typename K>

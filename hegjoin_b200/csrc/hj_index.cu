@@ -141,11 +141,11 @@ constexpr size_t kDefaultSmem = 48 * 1024;
 constexpr size_t kStaticSmemMax = 16 * 1024;   // no kernel here that takes dynamic shared memory has more
 hj_status ensure_smem_ptr(const void* kern, size_t bytes) {
     static std::mutex mu;
-    static std::map<const void*, size_t> done;
+    static std::map<std::pair<uint64_t, const void*>, size_t> done;   // by context: each has its own limits
     // the 48 KB that need no raised limit hold the kernel's static shared memory too
     if (bytes <= kDefaultSmem - kStaticSmemMax) return HJ_OK;
     std::lock_guard<std::mutex> lk(mu);
-    size_t& have = done[kern];
+    size_t& have = done[{context_id(), kern}];
     if (bytes <= have) return HJ_OK;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) {

@@ -1,8 +1,9 @@
 """Index builds after the process has reset its device.
 
 cudaDeviceReset ends the process's context, and with it the pinned buffer that
-readbacks of an earlier call went through.  The next call works in a new context.  In
-a process of its own, through the C interface.
+readbacks of an earlier call went through and the shared-memory limits that were
+raised for its kernels.  The next call works in a new context.  In a process of its
+own, through the C interface; up to 7,168 points the sort needs a raised limit.
 """
 import os
 import subprocess
@@ -23,7 +24,7 @@ CHILD = textwrap.dedent("""
     import hegjoin_b200 as hj
     from hegjoin_b200 import workloads
     from cuda.bindings import runtime as rt
-    for n in (20000, 30000):
+    for n in (20000, 30000, 3000, 7000):
         db = workloads.exp40(800, n, 2, np.float32)
         mn, _, nc, _ = oracle.geometry(db, 2, np.float32(0.01))
         cells = len(oracle.index(db, 2, np.float32(0.01), mn, nc)[0])
