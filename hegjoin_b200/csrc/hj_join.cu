@@ -1050,11 +1050,13 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         *out = std::min<uint64_t>((uint64_t)(opts.mem_fraction * usable / bytes_per_slot), 0xF0000000ull);
         return HJ_OK;
     };
-    // and the memory pool does not hold them idle already (at the default share): the call takes
-    // 0.1 ms alone and up to 82 ms while other processes use the driver, beside a join of 20 ms
-    const bool large = (double)cap * bytes_per_slot + result_bytes > 1024.0 * 1024 * 1024;
+    // and the memory pool does not hold them and the results idle already (at the default share):
+    // the call takes 0.1 ms alone and up to 82 ms while other processes use the driver, beside a
+    // join of 20 ms
+    const double join_bytes = (double)cap * bytes_per_slot + result_bytes;
+    const bool large = join_bytes > 1024.0 * 1024 * 1024;
     bool queried = false;
-    if (large && !(opts.mem_fraction == kDefaultMemFraction && (double)cap * bytes_per_slot <= (double)pool_idle_bytes())) {
+    if (large && !(opts.mem_fraction == kDefaultMemFraction && join_bytes <= (double)pool_idle_bytes())) {
         queried = true;
         uint64_t max_cap = 0;
         HJ_TRY(max_cap_from_free(&max_cap));
@@ -1100,9 +1102,10 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
 
     // one allocation carved into keys, vals, the band pair ids and the grouped copies;
     // when the free-memory query was skipped and the allocation fails, query and retry smaller
+    // (a small buffer of a named capacity is taken as named)
     uint32_t* slab = nullptr;
     hj_status as = tmp.alloc(&slab, cap * slot_words);
-    if (as == HJ_ERR_OOM && !queried && !opts.result_capacity) {
+    if (as == HJ_ERR_OOM && !queried && (large || !opts.result_capacity)) {
         uint64_t max_cap = 0;
         HJ_TRY(max_cap_from_free(&max_cap));
         if (max_cap < cap && max_cap > chunk_slack) {
