@@ -546,7 +546,9 @@ bool symmetric_pays(uint32_t d, double pairs, double cand, bool keys) {
 }
 
 // Tensor-core epilogue: with fewer than ~3% of its 32 x 32 chunks holding a hit, ORing the
-// signs and reading the hit chunks again beats a vote per chunk and masks at once.
+// signs and reading the hit chunks again beats a vote per chunk and masks at once.  A join
+// that is sized by its candidates (pairs == cand here) is dense by the same rule: each
+// of its queries pairs with itself, and it has fewer than 34,133 candidates per query.
 // HJ_TC_DEFER=0/1 forces masks or ORs (tests).
 bool dense_for(double pairs, double cand) {
     if (const char* e = std::getenv("HJ_TC_DEFER")) return e[0] != '1';
@@ -818,6 +820,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     const double avg_work = (double)ix->total_candidates / std::max<uint32_t>(1, nblocks);   // pairs evaluated per item
     // items hold 8 queries on average: enough for the digest kernel, whose lanes are queries
     const bool crowded = (uint64_t)ix->n >= 8ull * nblocks;
+    uint64_t candidates = ix->total_candidates;   // of this call's items
     if (opts.shard_count > 1) {
         // the item list on the host, for the costs of the share
         std::vector<HjBlock> hblocks(nblocks);
@@ -832,6 +835,8 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         std::vector<uint32_t> mine(std::max<uint32_t>(nblocks, 1));
         uint32_t n_mine = 0;
         HJ_TRY(hj_shard_plan_lpt(cost.data(), nblocks, opts.shard_count, opts.shard_index, mine.data(), &n_mine));
+        candidates = 0;
+        for (uint32_t i = 0; i < n_mine; ++i) candidates += cost[mine[i]];
         uint32_t* d_items = nullptr;
         HjBlock* sel = nullptr;
         HJ_TRY(tmp.alloc(&d_items, std::max<uint32_t>(n_mine, 1)));
@@ -947,14 +952,14 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     double* pest = nullptr;   // exclusive prefix of the per-item estimates (nblocks + 1), then the candidates
     // A join's pairs are among its candidates: where a buffer for all of those is small,
     // it takes the place of the estimate (a tenth of a small join's time).
-    const uint64_t bound_slots = ix->total_candidates + chunk_slack + 4096;
+    const uint64_t bound_slots = candidates + chunk_slack + 4096;
     const double bound_bytes = (double)bound_slots * bytes_per_slot;
     const bool bounded = !opts.result_capacity && bound_bytes <= kBoundedBytes &&
                          (!opts.device_bytes_cap ||
-                          bound_bytes + 1.1 * kept_bytes_per_pair * (double)ix->total_candidates +
-                                  (double)fixed_kept_bytes <= (double)opts.device_bytes_cap);
+                          bound_bytes + 1.1 * kept_bytes_per_pair * (double)candidates + (double)fixed_kept_bytes <=
+                              (double)opts.device_bytes_cap);
     if (bounded) {
-        total_est = cand_total = (double)ix->total_candidates;
+        total_est = cand_total = (double)candidates;
         int tuned = 0;
         if (!tc && !warp && tune_lookup(tune_key(refine, ix->d, ix->dtype), &tuned)) ix->plain_shape = tuned;
     }
@@ -1018,7 +1023,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         total_est = hsum[0];
         cand_total = hsum[1];
     }
-    S.estimated_pairs = (uint64_t)total_est;
+    S.estimated_pairs = bounded ? 0 : (uint64_t)total_est;   // without an estimate: the pairs, at the end
     S.ms_estimate = ms_since(t_est);
     dense = tc && dense_for(total_est, cand_total);
 
@@ -1242,6 +1247,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     }
     cudaGetLastError();
     S.total_pairs = total;
+    if (bounded) S.estimated_pairs = total;
     S.n_batches = n_out;
     S.ms_total = ms_since(t_start);
     S.kernel_launches = (uint32_t)(thread_launch_count() - launches0);

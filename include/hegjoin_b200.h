@@ -118,7 +118,8 @@ typedef struct {
     uint64_t band_pairs;           /* tensor-core filter: ordered pairs decided by the exact recheck (both
                                       orders of a pair are decided by one) */
     uint64_t tc_accepts;           /* tensor-core filter: ordered pairs accepted outside the band */
-    uint64_t estimated_pairs;      /* selectivity estimate before the join */
+    uint64_t estimated_pairs;      /* selectivity estimate before the join; where it makes none (a small
+                                      join, or one that only digests are wanted of) its total_pairs */
     double filter_delta;           /* guard band half-width on d2 (tensor-core filter) */
     float ms_estimate, ms_refine, ms_group, ms_total;
     float ms_refine_kernel;        /* device time of the refine kernels (CUDA events on the join's stream) */
@@ -127,7 +128,8 @@ typedef struct {
     uint32_t kernel_launches;      /* kernels launched by this join */
     float ms_setup;                /* workload order, refine choice, operand forms, work items (wall clock) */
     uint64_t bytes_wanted;         /* device bytes of result buffers + kept results the join asks for by
-                                      its estimate (one batch); also filled when the cap refuses it */
+                                      its estimate, or by its candidates where it makes none (one batch;
+                                      0 for digests alone); also filled when the cap refuses it */
 } hj_join_stats;
 
 /* ---- errors / library ---------------------------------------------------- */
