@@ -124,6 +124,13 @@ __global__ void k_item_estimates(const HjBlock* __restrict__ blocks, uint32_t nb
     if (lane_id() == 0 && c > 0) atomicAdd(cand, c);
 }
 
+// Queries x candidates per item, for a prefix that cuts digest launches; work[nblocks] = 0.
+__global__ void k_item_work(const HjBlock* __restrict__ blocks, uint32_t nblocks, double* __restrict__ work) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > nblocks) return;
+    work[i] = i < nblocks ? (double)blocks[i].nb * (double)(blocks[i].q1 - blocks[i].q0) : 0.0;
+}
+
 // Batch cuts: item i > 0 starts a batch where the exclusive prefix of the
 // estimates crosses a multiple of the budget, so a batch's estimate stays below
 // the budget plus its last item's.
@@ -885,24 +892,56 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         if (!count_only) HJ_CUDA(cudaEventRecord(e1, st));
         return HJ_OK;
     };
+    // First items (but 0) of the batches that an exclusive prefix over the items gives.
+    auto batch_cuts = [&](const double* pre, double budget, std::vector<uint32_t>* cuts) -> hj_status {
+        uint32_t* dcuts = nullptr;
+        unsigned int* dn = nullptr;
+        HJ_TRY(tmp.alloc(&dcuts, nblocks));
+        HJ_TRY(tmp.alloc(&dn, 1));
+        HJ_CUDA(cudaMemsetAsync(dn, 0, sizeof(unsigned int), st));
+        k_batch_cuts<<<(nblocks + 254) / 256, 256, 0, st>>>(pre, nblocks, budget, dcuts, dn);
+        HJ_LAUNCHED();
+        unsigned int ncut = 0;
+        HJ_CUDA(cudaMemcpyAsync(&ncut, dn, sizeof(ncut), cudaMemcpyDeviceToHost, st));
+        HJ_CUDA(cudaStreamSynchronize(st));
+        cuts->resize(ncut);
+        if (ncut) {
+            HJ_CUDA(cudaMemcpyAsync(cuts->data(), dcuts, (size_t)ncut * 4, cudaMemcpyDeviceToHost, st));
+            HJ_CUDA(cudaStreamSynchronize(st));
+        }
+        std::sort(cuts->begin(), cuts->end());
+        return HJ_OK;
+    };
+
     // ---- digests that nobody wants the pairs of: no estimate and no pair buffer.  Only
     // without limits on buffers and batches, which such a join would never meet.  A batch is
-    // a launch of about 2^34 candidate pairs (some 10 ms), so that a join of any length lets
-    // other streams' kernels in between.
+    // a launch of about 2^34 candidate pairs (some 10 ms; at most one item more), so that a
+    // join of any length lets other streams' kernels in between.
     DigestOut dig;
     if (warp && crowded && !opts.result_capacity && !opts.device_bytes_cap && !opts.max_batches &&
         handler.digest_only(&dig)) {
+        std::vector<uint32_t> ends;   // one past each launch's last item
+        if ((double)candidates > kDigestBatchPairs) {
+            double* work = nullptr;
+            HJ_TRY(tmp.alloc(&work, (size_t)nblocks + 1));
+            k_item_work<<<nblocks / 256 + 1, 256, 0, st>>>(blocks, nblocks, work);
+            HJ_LAUNCHED();
+            HJ_TRY(scan_f64_inplace(work, (uint64_t)nblocks + 1, st));
+            HJ_TRY(batch_cuts(work, kDigestBatchPairs, &ends));
+        }
+        if (nblocks) ends.push_back(nblocks);
         S.ms_setup = ms_since(t_start);
         kev.ev.emplace_back(nullptr, nullptr);
         HJ_TRY(event_acquire(&kev.ev[0].first));
         HJ_TRY(event_acquire(&kev.ev[0].second));
         HJ_CUDA(cudaEventRecord(kev.ev[0].first, st));
-        const uint32_t per_batch = (uint32_t)std::min(
-            (double)std::max<uint32_t>(nblocks, 1), std::max(1.0, kDigestBatchPairs / std::max(avg_work, 1.0)));
-        for (uint32_t b = 0; b < nblocks; b += std::min(per_batch, nblocks - b), ++S.n_batches) {
+        uint32_t b = 0;
+        for (uint32_t e : ends) {
             if (b) HJ_CUDA(cudaMemsetAsync(head, 0, sizeof(unsigned int), st));
-            HJ_TRY(launch_refine_digest(ix, blocks + b, std::min(per_batch, nblocks - b), avg_work, head, dig.count,
-                                        dig.sum, dig.xr, &ctl->valid, st));
+            HJ_TRY(launch_refine_digest(ix, blocks + b, e - b, avg_work, head, dig.count, dig.sum, dig.xr, &ctl->valid,
+                                        st));
+            b = e;
+            ++S.n_batches;
         }
         HJ_CUDA(cudaEventRecord(kev.ev[0].second, st));
         JoinCtl* hc = nullptr;
@@ -1078,24 +1117,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     if (nblocks) {
         const double budget = 0.5 * (double)(cap - chunk_slack);
         std::vector<uint32_t> cuts;
-        if (nblocks > 1 && !bounded && total_est >= budget) {
-            uint32_t* dcuts = nullptr;
-            unsigned int* dn = nullptr;
-            HJ_TRY(tmp.alloc(&dcuts, nblocks));
-            HJ_TRY(tmp.alloc(&dn, 1));
-            HJ_CUDA(cudaMemsetAsync(dn, 0, sizeof(unsigned int), st));
-            k_batch_cuts<<<(nblocks + 254) / 256, 256, 0, st>>>(pest, nblocks, budget, dcuts, dn);
-            HJ_LAUNCHED();
-            unsigned int ncut = 0;
-            HJ_CUDA(cudaMemcpyAsync(&ncut, dn, sizeof(ncut), cudaMemcpyDeviceToHost, st));
-            HJ_CUDA(cudaStreamSynchronize(st));
-            cuts.resize(ncut);
-            if (ncut) {
-                HJ_CUDA(cudaMemcpyAsync(cuts.data(), dcuts, (size_t)ncut * 4, cudaMemcpyDeviceToHost, st));
-                HJ_CUDA(cudaStreamSynchronize(st));
-            }
-            std::sort(cuts.begin(), cuts.end());
-        }
+        if (nblocks > 1 && !bounded && total_est >= budget) HJ_TRY(batch_cuts(pest, budget, &cuts));
         uint32_t b0 = 0;
         for (uint32_t c : cuts) {
             batches.push_back({b0, c, blocks, c});
