@@ -745,9 +745,12 @@ struct BatchHandler {
 // temporary lives in `tmp` and is freed on every return path.
 // kept_bytes_per_pair: device bytes the handler keeps per result pair (left free);
 // fixed_kept_bytes: what the caller already holds for the result (counted against
-// opts.device_bytes_cap).
+// opts.device_bytes_cap).  *unsized (in): size large buffers by the free memory in any
+// case; (out): the join left that out, so that an HJ_ERR_OOM may come of it.
 hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, BatchHandler& handler,
-                    double kept_bytes_per_pair, uint64_t fixed_kept_bytes, hj_join_stats* stats) {
+                    double kept_bytes_per_pair, uint64_t fixed_kept_bytes, hj_join_stats* stats, bool* unsized) {
+    const bool always_query = *unsized;
+    *unsized = false;
     auto t_start = std::chrono::steady_clock::now();
     hj_join_opts opts;
     if (opts_in) opts = *opts_in; else hj_join_opts_default(&opts);
@@ -1094,13 +1097,12 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
         *out = std::min<uint64_t>((uint64_t)(opts.mem_fraction * usable / bytes_per_slot), 0xF0000000ull);
         return HJ_OK;
     };
-    // and the memory pool does not hold them and the results idle already (at the default share):
-    // the call takes 0.1 ms alone and up to 82 ms while other processes use the driver, beside a
-    // join of 20 ms
-    const double join_bytes = (double)cap * bytes_per_slot + result_bytes;
-    const bool large = join_bytes > 1024.0 * 1024 * 1024;
+    // and the memory pool does not hold them idle already (at the default share): the call takes
+    // 0.1 ms alone and up to 82 ms while other processes use the driver, beside a join of 20 ms
+    const bool large = (double)cap * bytes_per_slot + result_bytes > 1024.0 * 1024 * 1024;
     bool queried = false;
-    if (large && !(opts.mem_fraction == kDefaultMemFraction && join_bytes <= (double)pool_idle_bytes())) {
+    if (large && (always_query || opts.mem_fraction != kDefaultMemFraction ||
+                  (double)cap * bytes_per_slot > (double)pool_idle_bytes())) {
         queried = true;
         uint64_t max_cap = 0;
         HJ_TRY(max_cap_from_free(&max_cap));
@@ -1130,6 +1132,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
     // one allocation carved into keys, vals, the band pair ids and the grouped copies;
     // when the free-memory query was skipped and the allocation fails, query and retry smaller
     // (a small buffer of a named capacity is taken as named)
+    *unsized = large && !queried;
     uint32_t* slab = nullptr;
     hj_status as = tmp.alloc(&slab, cap * slot_words);
     if (as == HJ_ERR_OOM && !queried && (large || !opts.result_capacity)) {
@@ -1230,6 +1233,7 @@ hj_status join_impl(hj_index* ix, const hj_join_opts* opts_in, cudaStream_t st, 
                 S.bytes_wanted, (uint64_t)((double)fixed_kept_bytes + slab_b + 1.1 * so_far / frac));
             set_error("hj_join: the results outgrow the cap of %llu device bytes",
                       (unsigned long long)cap_bytes);
+            *unsized = false;
             if (stats) *stats = S;
             return HJ_ERR_OOM;
         }
@@ -1416,11 +1420,21 @@ void hj_join_opts_default(hj_join_opts* o) {
     o->keep_keys = 0;
 }
 
-hj_status hj_result_destroy(hj_result* r) {
-    if (!r) return HJ_OK;
+// Frees what a result holds of its batches (the table stays).
+static void drop_batches(hj_result* r) {
     for (auto* p : r->vals) cudaFreeAsync(p, r->stream);
     for (auto* p : r->keys) cudaFreeAsync(p, r->stream);
     if (r->d_batch_vals) cudaFreeAsync(r->d_batch_vals, r->stream);
+    r->vals.clear();
+    r->keys.clear();
+    r->counts.clear();
+    r->d_batch_vals = nullptr;
+    r->total = 0;
+}
+
+hj_status hj_result_destroy(hj_result* r) {
+    if (!r) return HJ_OK;
+    drop_batches(r);
     if (r->table) cudaFreeAsync(r->table, r->stream);
     delete r;
     return HJ_OK;
@@ -1439,7 +1453,19 @@ hj_status hj_join(hj_index* ix, const hj_join_opts* opts, void* stream, hj_resul
     const bool keep_keys = opts && opts->keep_keys;
     RetainHandler h(res, keep_keys);
     hj_join_stats S{};
-    if (s == HJ_OK) s = join_impl(ix, opts, st, h, keep_keys ? 8.0 : 4.0, (uint64_t)ix->n * sizeof(hj_nt_entry), &S);
+    bool unsized = false;
+    auto run = [&] {
+        return join_impl(ix, opts, st, h, keep_keys ? 8.0 : 4.0, (uint64_t)ix->n * sizeof(hj_nt_entry), &S, &unsized);
+    };
+    if (s == HJ_OK) s = run();
+    if (s == HJ_ERR_OOM && unsized) {
+        // the buffer came from the pool without a look at the free memory, and the results found
+        // none: once more with a buffer that leaves them room
+        drop_batches(res);
+        s = cuda_status(cudaMemsetAsync(res->table, 0, (size_t)ix->n * sizeof(hj_nt_entry), st),
+                        "clear the neighbour table");
+        if (s == HJ_OK) s = run();
+    }
     if (stats) *stats = S;   // on an error: what was known (bytes_wanted when the cap refused)
     if (s != HJ_OK) {
         hj_result_destroy(res);
@@ -1463,7 +1489,8 @@ hj_status hj_join_stream(hj_index* ix, const hj_join_opts* opts, hj_batch_sink s
         HJ_CUDA(cudaMemsetAsync(d_xor, 0, (size_t)ix->n * 8, st));
     }
     StreamHandler h(sink, user, d_count, d_sum, d_xor);
-    HJ_TRY(join_impl(ix, opts, st, h, 0.0, 0, stats));
+    bool unsized = false;
+    HJ_TRY(join_impl(ix, opts, st, h, 0.0, 0, stats, &unsized));
     HJ_CUDA(cudaStreamSynchronize(st));
     return HJ_OK;
 }
