@@ -425,7 +425,7 @@ namespace {
 
 // After k_cell_workload: clears the silent cells' counts, writes the sort keys of
 // the workload order (top - candidates: ascending keys, descending candidates) and
-// folds totalCandidates and the largest count into out[0], out[1].
+// adds totalCandidates up in *out.
 __global__ void __launch_bounds__(256) k_cell_keys(const unsigned long long* __restrict__ cell_lid,
                                                     const uint32_t* __restrict__ cell_start, uint32_t nC, HjGrid g,
                                                     uint32_t any_silent, uint32_t top, uint32_t* __restrict__ cell_nb,
@@ -433,9 +433,8 @@ __global__ void __launch_bounds__(256) k_cell_keys(const unsigned long long* __r
                                                     unsigned long long* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long work = 0;
-    uint32_t nb = 0;
     if (i < nC) {
-        nb = cell_nb[i];
+        uint32_t nb = cell_nb[i];
         if (any_silent) {
             unsigned long long L = cell_lid[i];
             bool silent = false;
@@ -451,15 +450,12 @@ __global__ void __launch_bounds__(256) k_cell_keys(const unsigned long long* __r
         work = (unsigned long long)nb * (cell_start[i + 1] - cell_start[i]);
     }
     for (int o = 16; o > 0; o >>= 1) work += __shfl_down_sync(0xffffffffu, work, o);
-    nb = __reduce_max_sync(0xffffffffu, nb);
     __shared__ unsigned long long ws[8];
-    __shared__ uint32_t wm[8];
-    if (lane_id() == 0) { ws[threadIdx.x >> 5] = work; wm[threadIdx.x >> 5] = nb; }
+    if (lane_id() == 0) ws[threadIdx.x >> 5] = work;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int j = 1; j < 8; ++j) { work += ws[j]; nb = max(nb, wm[j]); }
-        if (work) atomicAdd(&out[0], work);
-        if (nb) atomicMax(&out[1], (unsigned long long)nb);
+        for (int j = 1; j < 8; ++j) work += ws[j];
+        if (work) atomicAdd(out, work);
     }
 }
 
@@ -718,23 +714,22 @@ void free_index(hj_index* ix, cudaStream_t st) {
 
 }  // namespace
 
-// Launches of the workload order; *folded (in tmp) then holds totalCandidates and the
-// largest count, for workload_done.
-static hj_status workload_launch(hj_index* ix, Scratch& tmp, unsigned long long** folded_out, cudaStream_t st) {
+// Launches of the workload order; **total (in tmp) then holds totalCandidates, for workload_done.
+static hj_status workload_launch(hj_index* ix, Scratch& tmp, unsigned long long** total_out, cudaStream_t st) {
     const uint32_t nC = ix->nC;
     // a previous attempt that failed part-way may have left these allocated
     dfree(ix->cell_nb, st);
     dfree(ix->cell_order, st);
-    unsigned long long* folded = nullptr;
+    unsigned long long* total = nullptr;
     uint32_t *keys = nullptr, *keys_tmp = nullptr, *vals_tmp = nullptr;
     HJ_TRY(dalloc(&ix->cell_nb, nC, st));
     HJ_TRY(dalloc(&ix->cell_order, nC, st));
-    HJ_TRY(tmp.alloc(&folded, 2));
+    HJ_TRY(tmp.alloc(&total, 1));
     HJ_TRY(tmp.alloc(&keys, nC));
     HJ_TRY(tmp.alloc(&keys_tmp, nC));
     HJ_TRY(tmp.alloc(&vals_tmp, nC));
     HJ_CUDA(cudaMemsetAsync(ix->cell_nb, 0, (size_t)nC * 4, st));
-    HJ_CUDA(cudaMemsetAsync(folded, 0, 2 * sizeof(unsigned long long), st));
+    HJ_CUDA(cudaMemsetAsync(total, 0, sizeof(unsigned long long), st));
     unsigned g = (unsigned)(((uint64_t)nC * 32 + 255) / 256);
     k_cell_workload<<<g, 256, 0, st>>>(ix->cell_lid, ix->cell_start, ix->cell_edge, nC, ix->grid, cell_hash(ix),
                                        ix->cell_nb);
@@ -743,15 +738,14 @@ static hj_status workload_launch(hj_index* ix, Scratch& tmp, unsigned long long*
     const uint32_t nbits = bits_for(ix->n);
     k_cell_keys<<<(nC + 255) / 256, 256, 0, st>>>(ix->cell_lid, ix->cell_start, nC, ix->grid, ix->any_silent,
                                                   (uint32_t)((1ull << nbits) - 1), ix->cell_nb, keys, ix->cell_order,
-                                                  folded);
+                                                  total);
     HJ_LAUNCHED();
     HJ_TRY(radix_sort_u32_u32(keys, ix->cell_order, keys_tmp, vals_tmp, nC, nbits, st));
-    *folded_out = folded;
+    *total_out = total;
     return HJ_OK;
 }
-static void workload_done(hj_index* ix, const unsigned long long* folded) {
-    ix->total_candidates = folded[0];
-    ix->max_nb = (uint32_t)folded[1];
+static void workload_done(hj_index* ix, unsigned long long total) {
+    ix->total_candidates = total;
     ix->have_workload = true;
 }
 
@@ -759,20 +753,19 @@ hj_status build_blocks(hj_index* ix, uint32_t qb, uint32_t align, HjBlock** d_bl
                        cudaStream_t st) {
     const uint32_t nC = ix->nC;
     Scratch tmp(st);
-    unsigned long long *folded = nullptr, *back = nullptr;
+    unsigned long long *total = nullptr, *back = nullptr;
     HJ_TRY(readback_buffer(reinterpret_cast<void**>(&back)));
-    if (!ix->have_workload) HJ_TRY(workload_launch(ix, tmp, &folded, st));
+    if (!ix->have_workload) HJ_TRY(workload_launch(ix, tmp, &total, st));
     uint32_t* cnt = nullptr;
     HJ_TRY(tmp.alloc(&cnt, (size_t)nC + 1));
     k_block_counts<<<nC / 256 + 1, 256, 0, st>>>(ix->cell_order, ix->cell_start, nC, qb, align, cnt);
     HJ_LAUNCHED();
     HJ_TRY(scan_u32_inplace(cnt, (uint64_t)nC + 1, st));
     // nothing that can fail for want of memory stands between a copy and the wait for it
-    if (folded)
-        HJ_CUDA(cudaMemcpyAsync(back + 1, folded, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    if (total) HJ_CUDA(cudaMemcpyAsync(back + 1, total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaMemcpyAsync(back, cnt + nC, 4, cudaMemcpyDeviceToHost, st));
     HJ_CUDA(cudaStreamSynchronize(st));
-    if (folded) workload_done(ix, back + 1);
+    if (total) workload_done(ix, back[1]);
     const uint32_t nb = *reinterpret_cast<const uint32_t*>(back);
     HjBlock* blocks = nullptr;
     HJ_TRY(tmp.alloc_pool(&blocks, (size_t)std::max<uint32_t>(nb, 1)));   // handed to the caller
@@ -938,12 +931,12 @@ hj_status hj_sort_by_workload(hj_index* ix, void* stream, uint64_t* total_candid
     cudaStream_t st = as_stream(stream);
     if (!ix->have_workload) {
         Scratch tmp(st);
-        unsigned long long *folded = nullptr, *back = nullptr;
+        unsigned long long *total = nullptr, *back = nullptr;
         HJ_TRY(readback_buffer(reinterpret_cast<void**>(&back)));
-        HJ_TRY(hj::workload_launch(ix, tmp, &folded, st));
-        HJ_CUDA(cudaMemcpyAsync(back, folded, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        HJ_TRY(hj::workload_launch(ix, tmp, &total, st));
+        HJ_CUDA(cudaMemcpyAsync(back, total, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         HJ_CUDA(cudaStreamSynchronize(st));
-        hj::workload_done(ix, back);
+        hj::workload_done(ix, *back);
     }
     if (total_candidates) *total_candidates = ix->total_candidates;
     return HJ_OK;

@@ -82,7 +82,6 @@ struct hj_index {
     uint64_t total_candidates = 0;
     uint32_t* cell_nb = nullptr;     // candidates per cell (cell order)
     uint32_t* cell_order = nullptr;  // cells, heaviest first
-    uint32_t max_nb = 0;
 
     // tensor-core operands (built on first use)
     void* tc_a = nullptr;            // query form: K-block planes (hj_refine_tc.cu)

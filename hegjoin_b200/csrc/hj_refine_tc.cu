@@ -1071,8 +1071,8 @@ size_t tc_smem_bytes(uint32_t nkb, uint32_t qcols, uint32_t stages) {
 }
 constexpr size_t kSmemBudget = 225 * 1024;
 
-// Query columns per work item: 512 (each candidate tile fetched once for both
-// accumulators: half the L2 traffic per pair) where three stages fit beside them.
+// Query columns per work item: 512 (each candidate tile fetched once for all four
+// accumulators) where three stages fit beside them, else 256.
 uint32_t tc_qcols(uint32_t nkb) { return tc_smem_bytes(nkb, kQBMax, 3) <= kSmemBudget ? kQBMax : kQBMax / 2; }
 
 uint32_t tc_stages(uint32_t nkb) {
