@@ -652,7 +652,7 @@ def main():
             pairs = res.total_pairs
             res.close()
         out = (pairs, cand, st.ms_refine_kernel, st.refine_launches, st.refine_used, st.band_pairs,
-               st.tc_accepts, st.filter_delta, int(st.n_batches))
+               st.tc_accepts, st.filter_delta, int(st.n_batches), int(st.bytes_wanted))
         ix.close()
         return out
 
@@ -712,15 +712,21 @@ def main():
                 "peak_kind": f"{pk_kind} bf16 dense, sustained (kernel runs inside a seconds-long step)",
                 "algorithmic": f"2*d flops per evaluated pair: {once} C (C = sum over queries of stencil candidates)"}
     else:
-        # queries read once, each 64-query block reads its candidates once, pairs written as two u32
+        # points read once; pairs written as two u32, or per-query digests (count, sum, xor) alone
         s = 4 if wl.dtype == "f32" else 8
-        byts = (wl.n / ws) * wl.d * s + (cand_rank / 64.0) * wl.d * s + 8.0 * pairs
+        warp = wl.d <= (12 if s == 4 else 8)
+        digest = stream_mode and recs[-1][9] == 0       # no pair buffer
+        byts = (wl.n / ws) * wl.d * s + (20.0 * wl.n if digest else 8.0 * pairs)
         achieved = byts / (kern_ms / 1e3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / pk["hbm_gbs"], "traffic": None,
-                "kernel": "k_refine_warp" if wl.d <= (12 if s == 4 else 8) else "k_refine_plain",
+                "kernel": "k_refine_digest" if digest else "k_refine_warp" if warp else "k_refine_plain",
                 "peak_kind": f"{pk_kind} copy bandwidth",
-                "algorithmic": "n*d*s + (C/64)*d*s + 8*P bytes per launch"}
+                "algorithmic": "n*d*s + 20*n bytes per step" if digest else "n*d*s + 8*P bytes per step"}
+        # its operations: 3*d flops per evaluated pair, each unordered pair once in the symmetric
+        # form (one batch, 40 evaluated coordinates per result pair)
+        sym = warp and not digest and once < 1.0 and wl.d * cand >= 40.0 * pairs
+        roof["tflops"] = 3.0 * wl.d * cand_rank * (0.5 if sym else 1.0) / (kern_ms / 1e3) / 1e12
     traffic_path = os.path.join(ROOT, "profiles", f"traffic_{wl.name}.txt")
     if os.path.exists(traffic_path):
         try:
@@ -815,6 +821,9 @@ def main():
         if tc:
             roof["own_mma_peak_tflops"] = own["f16_mma_tflops"]
             roof["frac_of_own_mma_peak"] = roof["achieved"] / own["f16_mma_tflops"]
+        else:
+            key = "fp32_fma_tflops" if wl.dtype == "f32" else "fp64_fma_tflops"
+            roof["frac_of_own_pipe_peak"] = roof["tflops"] / own[key]
 
     # the north-star comparisons, each with its own clock record (single GPU only)
     extras = {}
