@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(256) k_batch_reset(JoinCtl* c, uint32_t* __res
 // cursor atomic.  The refine writes a query's hits as runs of up to 64, so that is
 // about one atomic per run; the reversed orders of its symmetric form have keys of
 // their own each.  Eight steps are in flight per thread: the pass is bound by the
-// latency and rate of the atomics and by the scattered 4-byte stores (skewed 6-D,
-// 314M pairs; a shared-memory table of 1,024 keys per 4,096 pairs, which the
+// latency and rate of the atomics and by the scattered 4-byte stores: skewed 6-D, 314M
+// pairs, 4.0 ms (a shared-memory table of 1,024 keys per 4,096 pairs, which the
 // reversed orders overfill, took 8.9 ms and a counting pass 2.3 ms before it).
 // keys_out may be null (a result whose keys nobody asked for).
 constexpr uint32_t kGrpPer = 8;                        // pairs per thread
@@ -290,9 +290,10 @@ __global__ void k_csr_copy(const hj_nt_entry* __restrict__ t, uint32_t* const* _
 // go through shared memory (one padding word per 32, conflict-free for every K) so
 // that the stores are coalesced.  Lists longer than kWarpSortMax are noted for
 // k_csr_sort_long.
-// Bound by shuffles and the lists' two trips through memory: 314M neighbours in
-// lists of 80 on average (4M points) take ~1 ms; the radix sort of (query, id) keys
-// that this replaces took seven passes over 12 bytes a pair, 62 ms.
+// Bound by instruction issue (59% of the slots; shuffles) and the latency of the lists'
+// loads: 314M neighbours in lists of 80 on average (4M points) take 5.6 ms with the long
+// lists' sort; the radix sort of (query, id) keys that this replaces took seven passes
+// over 12 bytes a pair, 62 ms.
 constexpr uint32_t kWarpSortMax = 1024;
 constexpr uint32_t kSortWarps = 4;
 

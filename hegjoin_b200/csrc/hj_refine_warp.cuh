@@ -26,8 +26,8 @@
 // 120,000 points 1.5 -> 1.1 ms.
 //
 // Symmetric form (a.sym): d2 is the same number for (q, c) and (c, q), so a join
-// that runs in one batch evaluates each unordered pair once and emits both orders:
-// an item takes the cells after its own in linear-id order and, of its own cell,
+// that runs in one batch may evaluate each unordered pair once and emit both orders
+// (symmetric_pays in hj_join.cu says when that is the faster form): an item takes the cells after its own in linear-id order and, of its own cell,
 // the points from its first query on.  Cells with a coordinate of 0 visit no cell
 // in the reference's stencil (kernel.cu:780 wraps) although their neighbours visit
 // them: an item of such a cell emits only (candidate, query), a candidate of one
